@@ -131,7 +131,7 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
                           const int* __restrict__ type_in, const double4* __restrict__ pos_in,
                           const double4* __restrict__ vel_in, int* __restrict__ pidx_out,
                           int* __restrict__ type_out, double4* __restrict__ pos_out,
-                          double4* __restrict__ vel_out, double4* __restrict__ snap) {
+                          double4* __restrict__ vel_out, double2* __restrict__ xv, double4* __restrict__ snap) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int s = vals[i];
@@ -140,7 +140,14 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
     const double4 p = pos_in[s];
     pos_out[i] = p;
     snap[i] = p;
-    vel_out[i] = vel_in[s];
+    const double4 v = vel_in[s];
+    vel_out[i] = v;
+    if (xv) {
+        double2* q = xv + 3 * (size_t)i;
+        q[0] = make_double2(p.x, p.y);
+        q[1] = make_double2(p.z, v.x);
+        q[2] = make_double2(v.y, v.z);
+    }
 }
 
 // Neighbour list (main.cpp:1329-1585), one warp per home key: the particles
@@ -422,9 +429,9 @@ void launch_cell_ranges(const SimConst& c, const int* keys, int* cellstart, cuda
 
 void launch_reorder(const SimConst& c, const int* vals, const int* pidx_in, const int* type_in,
                     const double4* pos_in, const double4* vel_in, int* pidx_out, int* type_out,
-                    double4* pos_out, double4* vel_out, double4* snap, cudaStream_t s) {
+                    double4* pos_out, double4* vel_out, double2* xv, double4* snap, cudaStream_t s) {
     k_reorder<<<blocks(c.n, 256), 256, 0, s>>>(c.n, vals, pidx_in, type_in, pos_in, vel_in, pidx_out,
-                                               type_out, pos_out, vel_out, snap);
+                                               type_out, pos_out, vel_out, xv, snap);
 }
 
 // Bound of the prefilter (see k_neighbor_list).  An FP32 coordinate in

@@ -61,7 +61,48 @@ __device__ __forceinline__ double omod_q(double x, double w, unsigned long long 
     return ((unsigned long long)__double_as_longlong(x) < q75) ? x : omod(x, w);
 }
 
+// The record the pair sweeps gather per neighbour: position and velocity, 48
+// bytes as three 16-byte words {x, y}, {z, vx}, {vy, vz}, written by the move
+// (k_move) and by the reorder.  The sweeps are bound by the L1 data pipe: a
+// warp's gather of one neighbour per lane costs it 50-57 cycles as two 32-byte
+// double4 (four 16-byte loads), 37 as two 32-byte loads and 27-32 as this record
+// (measured with 40 to 1000 records in reach of a warp).  Force sweep 299 -> 255
+// us on the 258,392-particle dam break and 3.08 -> 2.90 ms on the 2,779,256 one,
+// sweep A 49 -> 43 us and 0.39 -> 0.36 ms, the move, which writes the records,
+// 13 -> 16 us and 0.058 -> 0.082 ms.
+struct XV {
+    double2 a, b, c;
+};
+__device__ __forceinline__ XV ld_xv(const double2* __restrict__ xv, int j) {
+    const double2* p = xv + 3 * (size_t)j;
+    XV r;
+    r.a = __ldg(p);
+    r.b = __ldg(p + 1);
+    r.c = __ldg(p + 2);
+    return r;
+}
+// One 32-byte record of a 32-byte aligned array in one load (18-19 cycles of
+// the L1 data pipe per warp-wide gather; two 16-byte loads take about 27).
+__device__ __forceinline__ double4 ld_d4(const double4* __restrict__ a, int j) {
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w)
+        : "l"(a + j));
+    return r;
+}
+__device__ __forceinline__ void st_xv(double2* __restrict__ xv, int i, const double4& p, const double4& v) {
+    double2* q = xv + 3 * (size_t)i;
+    q[0] = make_double2(p.x, p.y);
+    q[1] = make_double2(p.z, v.x);
+    q[2] = make_double2(v.y, v.z);
+}
+
 // Minimum-image displacement x_j - x_i (main.cpp:1680 and every sweep).
+__device__ __forceinline__ void disp(const SimConst& c, const XV& pi, const XV& pj, double* x) {
+    x[0] = omod_q(pj.a.x - pi.a.x + c.half_width[0], c.width[0], c.q75_bits[0]) - c.half_width[0];
+    x[1] = omod_q(pj.a.y - pi.a.y + c.half_width[1], c.width[1], c.q75_bits[1]) - c.half_width[1];
+    x[2] = omod_q(pj.b.x - pi.b.x + c.half_width[2], c.width[2], c.q75_bits[2]) - c.half_width[2];
+}
 __device__ __forceinline__ void disp(const SimConst& c, const double4& pi, const double4& pj, double* x) {
     x[0] = omod_q(pj.x - pi.x + c.half_width[0], c.width[0], c.q75_bits[0]) - c.half_width[0];
     x[1] = omod_q(pj.y - pi.y + c.half_width[1], c.width[1], c.q75_bits[1]) - c.half_width[1];
@@ -101,7 +142,7 @@ __device__ __forceinline__ int type_of(const double4& p) { return (int)p.w; }
 template <bool GRAPH>
 __global__ void __launch_bounds__(256)
 k_move(SimConst c, const int* __restrict__ cellstart, double4* __restrict__ pos, double4* __restrict__ vel,
-       const double4* __restrict__ snap, const double* __restrict__ wall_center, StepScalars* __restrict__ scal,
+       double2* __restrict__ xv, const double4* __restrict__ snap, const double* __restrict__ wall_center, StepScalars* __restrict__ scal,
        cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_sweep) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool stopped = GRAPH && *reinterpret_cast<volatile int*>(&scal->stop) != 0;
@@ -109,8 +150,8 @@ k_move(SimConst c, const int* __restrict__ cellstart, double4* __restrict__ pos,
     if (i < c.n && !stopped) {
         const int nf = cellstart[c.tot], we = cellstart[2 * c.tot];
         double4 p = pos[i];
+        double4 v = vel[i];
         if (i < nf) {
-            const double4 v = vel[i];
             p.x += v.x * c.dt;
             p.y += v.y * c.dt;
             p.z += v.z * c.dt;
@@ -124,7 +165,6 @@ k_move(SimConst c, const int* __restrict__ cellstart, double4* __restrict__ pos,
             r0 = R[0][0] * r0 + R[0][1] * r1 + R[0][2] * r2;   // in place, as main.cpp:2033-2035
             r1 = R[1][0] * r0 + R[1][1] * r1 + R[1][2] * r2;
             r2 = R[2][0] * r0 + R[2][1] * r1 + R[2][2] * r2;
-            double4 v = vel[i];
             v.x = W[1] * r2 - W[2] * r1 + U[0];
             v.y = W[2] * r0 - W[0] * r2 + U[1];
             v.z = W[0] * r1 - W[1] * r0 + U[2];
@@ -137,6 +177,7 @@ k_move(SimConst c, const int* __restrict__ cellstart, double4* __restrict__ pos,
         p.y = omod_fast(p.y - c.dmin[1], c.width[1]) + c.dmin[1];
         p.z = omod_fast(p.z - c.dmin[2], c.width[2]) + c.dmin[2];
         pos[i] = p;
+        st_xv(xv, i, p, v);
         const double4 q = snap[i];
         double d[3];
         d[0] = omod_fast(p.x - q.x + c.half_width[0], c.width[0]) - c.half_width[0];
@@ -191,18 +232,15 @@ __device__ __forceinline__ double s_dwv(const SimConst& c, double q) { return c.
 // calculatePhysicalCoefficients (1631-1662) and the PressureP / PressureA
 // values (1904-1906, 1735-1740).  Every division of the reference is an
 // exactly rounded div_rn (mph_exact.cuh) against one reciprocal per pair.
-// DA: DensityA and PressureA are computed here, over the whole list.  Without
-// surface tension the step does not use them (PressureA is zero and its force
-// terms are not evaluated), so the step leaves them to k_density_a, run only
-// when they are read, and visits only the short sublist (the pairs that can
-// lie within RadiusP, in list order).
-// SPLIT (with surface tension): DensityP and DivergenceP over the short
-// sublist (ncount_p, nlist_p: the list's entries within RadiusP+MARGIN, in list
-// order, so the same sums), DensityA and GravityCenter over the list; the
-// pressure block then no longer runs with most lanes masked off.
-template <bool ST, bool RATIO, bool DA, bool SPLIT>
+// DensityP and DivergenceP visit the short sublist (ncount_p, nlist_p: the
+// list's entries within RadiusP+MARGIN, in list order, so every pair within
+// RadiusP in the reference's order).  With surface tension DensityA and
+// GravityCenter visit the list in a loop of their own; without, the step does
+// not use DensityA (PressureA is zero and its force terms are not evaluated),
+// and k_density_a computes it when it is read.
+template <bool ST, bool RATIO>
 __global__ void __launch_bounds__(128, ST ? MPH_SWEEP_MINB_ST : MPH_SWEEP_MINB)
-k_sweep_a(SimConst c, const double4* __restrict__ pos, const double4* __restrict__ vel,
+k_sweep_a(SimConst c, const double2* __restrict__ xv, const int* __restrict__ type,
           const int* __restrict__ ncount, const int* __restrict__ nlist, const int* __restrict__ ncount_p,
           const int* __restrict__ nlist_p, double* __restrict__ dens_a,
           double* __restrict__ strain_p, double* __restrict__ div_p, double4* __restrict__ velp,
@@ -215,35 +253,31 @@ k_sweep_a(SimConst c, const double4* __restrict__ pos, const double4* __restrict
         if (t >= 2) wall_center[3 * t + d] += c.wall_velocity[t][d] * c.dt;
     }
     if (i >= c.n) return;
-    const double4 pi = pos[i];
-    const double4 vi = vel[i];
-    const int ti = type_of(pi);
-    const int cnt = ncount[i];
+    const XV pi = ld_xv(xv, i);
+    const int ti = type[i];
     const size_t n = (size_t)c.n;
     double sum_a = 0.0, sum_p = 0.0, sum_d = 0.0;
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    if (SPLIT) {  // DensityP, DivergenceP over the short sublist (main.cpp:1831-1896)
+    {  // DensityP, DivergenceP: indices two entries ahead, the neighbour's record one ahead
         const int cs = ncount_p[i];
         const int* lq = nlist_p + i;
         int q1 = cs > 0 ? __ldg(lq) : i;
         int q2 = cs > 1 ? __ldg(lq + n) : i;
         lq += 2 * n;
-        double4 qn = pos[q1], qv = vel[q1];
+        XV qn = ld_xv(xv, q1);
         for (int k = 0; k < cs; ++k) {
             const int j = q1;
-            const double4 pj = qn;
-            const double4 vjn = qv;
+            const XV pj = qn;
             q1 = q2;
             if (k + 2 < cs) q2 = __ldg(lq);
             lq += n;
-            if (k + 1 < cs) {
-                qn = pos[q1];
-                qv = vel[q1];
-            }
+            if (k + 1 < cs) qn = ld_xv(xv, q1);
             if (j == i) continue;
             double x[3];
             disp(c, pi, pj, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            // R*R - r2 >= 0 (main.cpp:1683 and the other density sums) is r2 <= R*R:
+            // with gradual underflow a - b is zero only when a == b, and its sign exact
             if (!(r2 <= c.rp2)) continue;
             const double r = sqrt(r2);
             const double qp = div_rs(r, c.rp, c.inv_rp);
@@ -251,67 +285,56 @@ k_sweep_a(SimConst c, const double4* __restrict__ pos, const double4* __restrict
             const double dw = s_dwp(c, qp);
             const double ri = __drcp_rn(r);
             const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-            const double u0 = vjn.x - vi.x, u1 = vjn.y - vi.y, u2 = vjn.z - vi.z;
+            const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
             sum_d -= u0 * e0 * dw;
             sum_d -= u1 * e1 * dw;
             sum_d -= u2 * e2 * dw;
         }
     }
-    // indices two entries ahead, the neighbour's position and velocity one ahead
-    const int* lp = nlist + i;
-    int j1 = cnt > 0 ? __ldg(lp) : i;
-    int j2 = cnt > 1 ? __ldg(lp + n) : i;
-    lp += 2 * n;
-    double4 pn = pos[j1], vq = vel[j1];
-    for (int k = 0; k < cnt; ++k) {
-        const int j = j1;
-        const double4 pj = pn;
-        const double4 vjn = vq;
-        j1 = j2;
-        if (k + 2 < cnt) j2 = __ldg(lp);
-        lp += n;
-        if (k + 1 < cnt) {
-            pn = pos[j1];
-            vq = vel[j1];
+    if (ST) {  // DensityA, GravityCenter
+        const int cnt = ncount[i];
+        const int* lp = nlist + i;
+        int j1 = cnt > 0 ? __ldg(lp) : i;
+        int j2 = cnt > 1 ? __ldg(lp + n) : i;
+        lp += 2 * n;
+        XV pn = ld_xv(xv, j1);  // the words that are not used are not loaded
+        int tn = RATIO ? __ldg(type + j1) : 0;
+        for (int k = 0; k < cnt; ++k) {
+            const int j = j1;
+            const XV pj = pn;
+            const int tj = tn;
+            j1 = j2;
+            if (k + 2 < cnt) j2 = __ldg(lp);
+            lp += n;
+            if (k + 1 < cnt) {
+                pn = ld_xv(xv, j1);
+                if (RATIO) tn = __ldg(type + j1);
+            }
+            if (j == i) continue;
+            double x[3];
+            disp(c, pi, pj, x);
+            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            const bool in_a = r2 <= c.ra2;
+            const bool in_g = r2 <= c.rg2;
+            if (!(in_a || in_g)) continue;
+            const double r = sqrt(r2);
+            double ratio = 1.0;
+            if (RATIO) ratio = c.ratio[ti][tj];
+            const double qa = div_rs(r, c.ra, c.inv_ra);
+            if (in_a) {
+                const double w = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
+                sum_a += w;
+            }
+            if (in_g) {
+                const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                const double w = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
+                g0 += div_rs(x[0] * w, c.r2g, c.inv_r2g) * c.rg;
+                g1 += div_rs(x[1] * w, c.r2g, c.inv_r2g) * c.rg;
+                g2 += div_rs(x[2] * w, c.r2g, c.inv_r2g) * c.rg;
+            }
         }
-        if (j == i) continue;
-        double x[3];
-        disp(c, pi, pj, x);
-        const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        // R*R - r2 >= 0 (main.cpp:1683 and the other density sums) is r2 <= R*R:
-        // with gradual underflow a - b is zero only when a == b, and its sign exact
-        const bool in_a = DA && (r2 <= c.ra2);
-        const bool in_p = !SPLIT && r2 <= c.rp2;
-        const bool in_g = ST && (r2 <= c.rg2);
-        if (!(in_a || in_p || in_g)) continue;
-        const double r = sqrt(r2);
-        double ratio = 1.0;
-        if (RATIO) ratio = c.ratio[ti][type_of(pj)];
-        const double qa = div_rs(r, c.ra, c.inv_ra);
-        if (in_a) {
-            const double w = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
-            sum_a += w;
-        }
-        if (ST && in_g) {
-            const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
-            const double w = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
-            g0 += div_rs(x[0] * w, c.r2g, c.inv_r2g) * c.rg;
-            g1 += div_rs(x[1] * w, c.r2g, c.inv_r2g) * c.rg;
-            g2 += div_rs(x[2] * w, c.r2g, c.inv_r2g) * c.rg;
-        }
-        if (in_p) {
-            const double qp = div_rs(r, c.rp, c.inv_rp);
-            sum_p += s_wp(c, qp);
-            const double dw = s_dwp(c, qp);
-            const double ri = __drcp_rn(r);
-            const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-            const double u0 = vjn.x - vi.x, u1 = vjn.y - vi.y, u2 = vjn.z - vi.z;
-            sum_d -= u0 * e0 * dw;
-            sum_d -= u1 * e1 * dw;
-            sum_d -= u2 * e2 * dw;
-        }
+        dens_a[i] = sum_a;
     }
-    if (DA) dens_a[i] = sum_a;
     const double strain = sum_p - c.n0p;
     strain_p[i] = strain;
     div_p[i] = sum_d;
@@ -319,14 +342,14 @@ k_sweep_a(SimConst c, const double4* __restrict__ pos, const double4* __restrict
     if (strain < 0.0) kappa = 0.0;
     const double lambda = c.bulk_viscosity[ti];
     const double pp = -lambda * sum_d + kappa * strain;
-    double pa = 0.0;
-    if (DA) {
-        pa = c.cof_a[ti] * (sum_a - c.n0a) / c.l0;
+    // sweep B gathers PressureP and {GravityCenter, PressureA} per neighbour;
+    // without surface tension the latter stay zero (PressureA: k_density_a)
+    velp[i] = make_double4(pi.b.y, pi.c.x, pi.c.y, pp);
+    if (ST) {
+        double pa = c.cof_a[ti] * (sum_a - c.n0a) / c.l0;
         if (c.n0a <= sum_a) pa = 0.0;
+        gcpa[i] = make_double4(g0, g1, g2, pa);
     }
-    // sweep B gathers {v, PressureP} and {GravityCenter, PressureA} per neighbour
-    velp[i] = make_double4(vi.x, vi.y, vi.z, pp);
-    gcpa[i] = make_double4(g0, g1, g2, pa);
 }
 
 // DensityA (main.cpp:1665-1692) and PressureA (1735-1740) alone, for the
@@ -367,76 +390,74 @@ __global__ void __launch_bounds__(128) k_density_a(SimConst c, const double4* __
 // (1742-1775), DiffuseInterface (1782-1828, aj uses the type of i as in the
 // reference), ViscosityV (1943-1984); Force = 0 + fP + fA + fDI + fV, then
 // Gravity (1988-1998) and Acceleration (2000-2010) for fluid particles.
+// The PressureP force visits only pairs within RadiusP, all of which are in
+// the short sublist, in list order (the argument of k_neighbor_list), so that
+// sum runs as its own loop over the short sublist and the main loop carries
+// the other terms.  The terms and their order in each sum are the reference's;
+// the main loop does not run the pressure block under a branch that some lane
+// takes on nearly every entry while most lanes wait.
 // LRN: the learned form.  The PressureA, DiffuseInterface and ViscosityV pair
 // terms are not evaluated; fluid particle i adds instead the sum of its
 // edge-MLP pair forces eforce[eoff[i] .. eoff[i+1]) (FP32, in edge order),
 // which is also stored in lsum[i].
-// SPLIT (not learned): the PressureP force visits only
-// pairs within RadiusP, all of which are in the short sublist, in list order
-// (the argument of k_neighbor_list), so that sum runs as its own loop over the
-// short sublist and the main loop carries ViscosityV alone.  The terms and
-// their order in each sum are the reference's; the main loop no longer runs
-// the pressure block under a branch that some lane takes on nearly every
-// entry while most lanes wait.
-template <bool ST, bool RATIO, bool LRN, bool SPLIT>
+// MU1: visc_c * muij is one number for every pair of types, so the type of j
+// is not gathered.
+template <bool ST, bool RATIO, bool LRN, bool MU1>
 __global__ void __launch_bounds__(128, ST ? MPH_SWEEPB_MINB_ST : MPH_SWEEPB_MINB)
-k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double4* __restrict__ pos,
-          const double4* __restrict__ velp, double4* __restrict__ vel_out, const double4* __restrict__ gcpa,
-          const int* __restrict__ ncount, const int* __restrict__ nlist, const int* __restrict__ ncount_s,
-          const int* __restrict__ nlist_s, double4* __restrict__ force,
+k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restrict__ xv,
+          const int* __restrict__ type, const double4* __restrict__ velp, double4* __restrict__ vel_out,
+          const double4* __restrict__ gcpa, const int* __restrict__ ncount, const int* __restrict__ nlist,
+          const int* __restrict__ ncount_s, const int* __restrict__ nlist_s, double4* __restrict__ force,
           StepScalars* __restrict__ scal, const int* __restrict__ eoff, const float4* __restrict__ eforce,
           float4* __restrict__ lsum, int part, int i0, int i1, double* __restrict__ vel_host) {
     const int i = i0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);  // particles [i0, i1)
     if (i >= i1) return;
     const int nf = cellstart[c.tot];
-    const double4 vi = velp[i];   // .w = PressureP
+    const XV pi = ld_xv(xv, i);
     // part 1: fluid only; a wall keeps its velocity (what the full sweep
     // writes for it) and its force is left for part 2 (output only)
     if (part == 1 && i >= nf) {
-        vel_out[i] = make_double4(vi.x, vi.y, vi.z, 0.0);
+        vel_out[i] = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
         if (vel_host) {
-            vel_host[3 * (size_t)i] = vi.x;
-            vel_host[3 * (size_t)i + 1] = vi.y;
-            vel_host[3 * (size_t)i + 2] = vi.z;
+            vel_host[3 * (size_t)i] = pi.b.y;
+            vel_host[3 * (size_t)i + 1] = pi.c.x;
+            vel_host[3 * (size_t)i + 2] = pi.c.y;
         }
         return;
     }
     if (part == 2 && i < nf) return;
-    const double4 pi = pos[i];
-    const int ti = type_of(pi);
-    const double ai = c.a_k[ti];
-    double4 gci = make_double4(0, 0, 0, 0);
-    if (ST) gci = gcpa[i];        // .w = PressureA
-    const int cnt = ncount[i];
+    const int ti = type[i];
     const size_t n = (size_t)c.n;
     double fp0 = 0.0, fp1 = 0.0, fp2 = 0.0;
     double fa0 = 0.0, fa1 = 0.0, fa2 = 0.0;
     double fd0 = 0.0, fd1 = 0.0, fd2 = 0.0;
     double fv0 = 0.0, fv1 = 0.0, fv2 = 0.0;
-    if (SPLIT) {  // PressureP force (main.cpp:1908-1938) over the short sublist
-        // indices two entries ahead, the neighbour's records one entry ahead
+    {  // PressureP force (main.cpp:1908-1938) over the short sublist
+        // indices two entries ahead, the neighbour's position and PressureP one ahead
+        const double ppi = velp[i].w;
         const int cs = ncount_s[i];
         const int* lq = nlist_s + i;
         int q1 = cs > 0 ? __ldg(lq) : i;
         int q2 = cs > 1 ? __ldg(lq + n) : i;
         lq += 2 * n;
-        double4 qn = pos[q1];
+        XV qn = ld_xv(xv, q1);
         double qp1 = velp[q1].w;
         for (int k = 0; k < cs; ++k) {
             const int j = q1;
-            const double4 pj = qn;
+            const XV pj = qn;
             const double pjp = qp1;  // PressureP of j
             q1 = q2;
             if (k + 2 < cs) q2 = __ldg(lq);
             lq += n;
             if (k + 1 < cs) {
-                qn = pos[q1];
+                qn = ld_xv(xv, q1);
                 qp1 = velp[q1].w;
             }
             if (j == i) continue;
             double x[3];
             disp(c, pi, pj, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            // R*R - r2 > 0 (main.cpp:1926 and the other force sums) is r2 < R*R
             if (!(r2 < c.rp2)) continue;
             const double r = sqrt(r2);
             const double ri = __drcp_rn(r);
@@ -444,100 +465,97 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double4* __restri
             const double dw = s_dwp(c, qp);
             const double gw0 = div_rs(dw * x[0], r, ri), gw1 = div_rs(dw * x[1], r, ri),
                          gw2 = div_rs(dw * x[2], r, ri);
-            const double ps = vi.w + pjp;
+            const double ps = ppi + pjp;
             fp0 += ps * gw0 * c.vol;
             fp1 += ps * gw1 * c.vol;
             fp2 += ps * gw2 * c.vol;
         }
     }
-    // software pipeline: list indices two entries ahead, the neighbour's two
-    // records (position, velocity + PressureP) one entry ahead, so their
-    // gathers overlap the previous pair's FP64 arithmetic
-    const int* lp = nlist + i;
-    int j1 = cnt > 0 ? __ldg(lp) : i;
-    int j2 = cnt > 1 ? __ldg(lp + n) : i;
-    lp += 2 * n;
-    double4 pn = pos[j1], vn1 = velp[j1];
-    for (int k = 0; k < cnt; ++k) {
-        const int j = j1;
-        const double4 pj = pn;
-        const double4 vj = vn1;   // .w = PressureP of j
-        j1 = j2;
-        if (k + 2 < cnt) j2 = __ldg(lp);
-        lp += n;
-        if (k + 1 < cnt) {
-            pn = pos[j1];
-            vn1 = velp[j1];
-        }
-        if (j == i) continue;
-        double x[3];
-        disp(c, pi, pj, x);
-        const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        // Without surface tension every CofA is 0, PressureA is +-0 and each
-        // PressureA term adds a signed zero to a sum that starts at +0: the sum
-        // stays +0 exactly, so the term is skipped (ST == false).
-        // R*R - r2 > 0 (main.cpp:1926 and the other force sums) is r2 < R*R
-        const bool in_p = !SPLIT && r2 < c.rp2;
-        const bool in_a = !LRN && ST && (r2 < c.ra2);
-        const bool in_g = !LRN && ST && (r2 < c.rg2);
-        const bool in_v = !LRN && r2 < c.rv2;
-        if (!(in_p || in_a || in_g || in_v)) continue;
-        const int tj = type_of(pj);
-        const double r = sqrt(r2);
-        const double ri = __drcp_rn(r);
-        const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-        const double qa = div_rs(r, c.ra, c.inv_ra);
-        double rij = 1.0, rji = 1.0;
-        if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
-        if (in_p) {
-            const double qp = div_rs(r, c.rp, c.inv_rp);
-            const double dw = s_dwp(c, qp);
-            const double gw0 = div_rs(dw * x[0], r, ri), gw1 = div_rs(dw * x[1], r, ri),
-                         gw2 = div_rs(dw * x[2], r, ri);
-            const double ps = vi.w + vj.w;
-            fp0 += ps * gw0 * c.vol;
-            fp1 += ps * gw1 * c.vol;
-            fp2 += ps * gw2 * c.vol;
-        }
-        if (in_a) {
-            const double dwa = s_dwa(c, qa);
-            const double dwij = RATIO ? rij * dwa : dwa;
-            const double dwji = RATIO ? rji * dwa : dwa;
-            const double s = gci.w * dwij + gcpa[j].w * dwji;
-            fa0 += s * e0 * c.vol;
-            fa1 += s * e1 * c.vol;
-            fa2 += s * e2 * c.vol;
-        }
-        if (ST && in_g) {
-            const double4 gcj = gcpa[j];
-            const double aj = ai;
-            const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
-            const double wg = s_wg(c, qg);
-            const double wij = RATIO ? rij * wg : wg;
-            const double wji = RATIO ? rji * wg : wg;
-            fd0 -= div_rs(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-            fd1 -= div_rs(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-            fd2 -= div_rs(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-            const double dg = s_dwg(c, qg);
-            const double dwij = RATIO ? rij * dg : dg;
-            const double dwji = RATIO ? rji * dg : dg;
-            double gr = 0.0;
-            gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
-            gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
-            gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
-            fd0 -= div_rs((gr) * e0, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-            fd1 -= div_rs((gr) * e1, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-            fd2 -= div_rs((gr) * e2, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-        }
-        if (in_v) {
-            const double qv = c.rv_eq_ra ? qa : div_rs(r, c.rv, c.inv_rv);
-            const double dw = -s_dwv(c, qv);
-            const double u0 = vj.x - vi.x, u1 = vj.y - vi.y, u2 = vj.z - vi.z;
-            const double cm = c.visc_mu[ti][tj];
-            const double dot = u0 * e0 + u1 * e1 + u2 * e2;
-            fv0 += div_rs(cm * dot * e0 * dw, r, ri) * c.vol;
-            fv1 += div_rs(cm * dot * e1 * dw, r, ri) * c.vol;
-            fv2 += div_rs(cm * dot * e2 * dw, r, ri) * c.vol;
+    if (!LRN) {
+        // software pipeline: list indices two entries ahead, the neighbour's
+        // record one ahead, so the gathers overlap the previous pair's FP64
+        // arithmetic
+        const double ai = ST ? c.a_k[ti] : 0.0;
+        double4 gci = make_double4(0, 0, 0, 0);
+        if (ST) gci = gcpa[i];        // .w = PressureA
+        const int cnt = ncount[i];
+        const int* lp = nlist + i;
+        int j1 = cnt > 0 ? __ldg(lp) : i;
+        int j2 = cnt > 1 ? __ldg(lp + n) : i;
+        lp += 2 * n;
+        constexpr bool TYPES = RATIO || !MU1;
+        XV pn = ld_xv(xv, j1);
+        int tn = TYPES ? __ldg(type + j1) : 0;
+        for (int k = 0; k < cnt; ++k) {
+            const int j = j1;
+            const XV pj = pn;
+            const int tj = tn;
+            j1 = j2;
+            if (k + 2 < cnt) j2 = __ldg(lp);
+            lp += n;
+            if (k + 1 < cnt) {
+                pn = ld_xv(xv, j1);
+                if (TYPES) tn = __ldg(type + j1);
+            }
+            if (j == i) continue;
+            double x[3];
+            disp(c, pi, pj, x);
+            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            // Without surface tension every CofA is 0, PressureA is +-0 and each
+            // PressureA term adds a signed zero to a sum that starts at +0: the sum
+            // stays +0 exactly, so the term is skipped (ST == false).
+            const bool in_a = ST && (r2 < c.ra2);
+            const bool in_g = ST && (r2 < c.rg2);
+            const bool in_v = r2 < c.rv2;
+            if (!(in_a || in_g || in_v)) continue;
+            const double r = sqrt(r2);
+            const double ri = __drcp_rn(r);
+            const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
+            const double qa = div_rs(r, c.ra, c.inv_ra);
+            double rij = 1.0, rji = 1.0;
+            if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
+            if (ST) {
+                const double4 gcj = ld_d4(gcpa, j);  // .w = PressureA
+                if (in_a) {
+                    const double dwa = s_dwa(c, qa);
+                    const double dwij = RATIO ? rij * dwa : dwa;
+                    const double dwji = RATIO ? rji * dwa : dwa;
+                    const double s = gci.w * dwij + gcj.w * dwji;
+                    fa0 += s * e0 * c.vol;
+                    fa1 += s * e1 * c.vol;
+                    fa2 += s * e2 * c.vol;
+                }
+                if (in_g) {
+                    const double aj = ai;
+                    const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                    const double wg = s_wg(c, qg);
+                    const double wij = RATIO ? rij * wg : wg;
+                    const double wji = RATIO ? rji * wg : wg;
+                    fd0 -= div_rs(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd1 -= div_rs(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd2 -= div_rs(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    const double dg = s_dwg(c, qg);
+                    const double dwij = RATIO ? rij * dg : dg;
+                    const double dwji = RATIO ? rji * dg : dg;
+                    double gr = 0.0;
+                    gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
+                    gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
+                    gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
+                    fd0 -= div_rs((gr) * e0, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd1 -= div_rs((gr) * e1, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd2 -= div_rs((gr) * e2, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                }
+            }
+            if (in_v) {
+                const double qv = c.rv_eq_ra ? qa : div_rs(r, c.rv, c.inv_rv);
+                const double dw = -s_dwv(c, qv);
+                const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
+                const double cm = MU1 ? c.visc_mu[0][0] : c.visc_mu[ti][tj];
+                const double dot = u0 * e0 + u1 * e1 + u2 * e2;
+                fv0 += div_rs(cm * dot * e0 * dw, r, ri) * c.vol;
+                fv1 += div_rs(cm * dot * e1 * dw, r, ri) * c.vol;
+                fv2 += div_rs(cm * dot * e2 * dw, r, ri) * c.vol;
+            }
         }
     }
     if (LRN) {
@@ -560,7 +578,7 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double4* __restri
     F0 += fa0; F1 += fa1; F2 += fa2;
     F0 += fd0; F1 += fd1; F2 += fd2;
     F0 += fv0; F1 += fv1; F2 += fv2;
-    double4 vn = make_double4(vi.x, vi.y, vi.z, 0.0);
+    double4 vn = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
     if (i < nf) {
         const double m = c.density[ti] * c.vol;
         F0 += m * c.gravity[0];
@@ -609,8 +627,9 @@ __device__ __forceinline__ SumOp sweep_b_sum(int s) {
 
 template <bool ST, bool RATIO>
 __global__ void __launch_bounds__(32 * kWarpSweepWarps)
-k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __restrict__ pos,
-            const double4* __restrict__ velp, double4* __restrict__ vel_out, const double4* __restrict__ gcpa,
+k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __restrict__ xv,
+            const int* __restrict__ type, const double4* __restrict__ velp, double4* __restrict__ vel_out,
+            const double4* __restrict__ gcpa,
             const int* __restrict__ ncount, const int* __restrict__ nlist, double4* __restrict__ force,
             StepScalars* __restrict__ scal, int part, double* __restrict__ vel_host) {
     constexpr int NV = ST ? 15 : 6;  // terms per entry: fp 3, fv 3 [, fa 3, fd 3 + 3]
@@ -621,21 +640,21 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
     const int i = blockIdx.x * kWarpSweepWarps + w;
     if (i >= c.n) return;  // whole warp
     const int nf = cellstart[c.tot];
-    const double4 vi = velp[i];   // .w = PressureP
+    const XV pi = ld_xv(xv, i);
     if (part == 1 && i >= nf) {   // a wall keeps its velocity (see k_sweep_b)
         if (lane == 0) {
-            vel_out[i] = make_double4(vi.x, vi.y, vi.z, 0.0);
+            vel_out[i] = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
             if (vel_host) {
-                vel_host[3 * (size_t)i] = vi.x;
-                vel_host[3 * (size_t)i + 1] = vi.y;
-                vel_host[3 * (size_t)i + 2] = vi.z;
+                vel_host[3 * (size_t)i] = pi.b.y;
+                vel_host[3 * (size_t)i + 1] = pi.c.x;
+                vel_host[3 * (size_t)i + 2] = pi.c.y;
             }
         }
         return;
     }
     if (part == 2 && i < nf) return;
-    const double4 pi = pos[i];
-    const int ti = type_of(pi);
+    const double ppi = velp[i].w;
+    const int ti = type[i];
     const double ai = c.a_k[ti];
     double4 gci = make_double4(0, 0, 0, 0);
     if (ST) gci = gcpa[i];        // .w = PressureA
@@ -651,7 +670,7 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
         for (int q = 0; q < NV; ++q) v[q] = 0.0;
         const int j = k < cnt ? __ldg(nlist + (size_t)k * n + i) : i;
         if (j != i) {
-            const double4 pj = pos[j];
+            const XV pj = ld_xv(xv, j);
             double x[3];
             disp(c, pi, pj, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
@@ -660,8 +679,7 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
             const bool in_g = ST && (r2 < c.rg2);
             const bool in_v = r2 < c.rv2;
             if (in_p || in_a || in_g || in_v) {
-                const double4 vj = velp[j];   // .w = PressureP of j
-                const int tj = type_of(pj);
+                const int tj = __ldg(type + j);
                 const double r = sqrt(r2);
                 const double ri = __drcp_rn(r);
                 const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
@@ -673,7 +691,7 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
                     const double dw = s_dwp(c, qp);
                     const double gw0 = div_rs(dw * x[0], r, ri), gw1 = div_rs(dw * x[1], r, ri),
                                  gw2 = div_rs(dw * x[2], r, ri);
-                    const double ps = vi.w + vj.w;
+                    const double ps = ppi + velp[j].w;
                     v[0] = ps * gw0 * c.vol;
                     v[1] = ps * gw1 * c.vol;
                     v[2] = ps * gw2 * c.vol;
@@ -682,7 +700,7 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
                 if (in_v) {
                     const double qv = c.rv_eq_ra ? qa : div_rs(r, c.rv, c.inv_rv);
                     const double dw = -s_dwv(c, qv);
-                    const double u0 = vj.x - vi.x, u1 = vj.y - vi.y, u2 = vj.z - vi.z;
+                    const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
                     const double cm = c.visc_mu[ti][tj];
                     const double dot = u0 * e0 + u1 * e1 + u2 * e2;
                     v[3] = div_rs(cm * dot * e0 * dw, r, ri) * c.vol;
@@ -759,7 +777,7 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
     F0 += fa0; F1 += fa1; F2 += fa2;
     F0 += fd0; F1 += fd1; F2 += fd2;
     F0 += fv0; F1 += fv1; F2 += fv2;
-    double4 vn = make_double4(vi.x, vi.y, vi.z, 0.0);
+    double4 vn = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
     if (i < nf) {
         const double m = c.density[ti] * c.vol;
         F0 += m * c.gravity[0];
@@ -784,9 +802,9 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double4* __rest
 // Sweep A, warp per particle: sums DensityA (lane 0, bit 1), DensityP (lane 1,
 // bit 2), DivergenceP (lane 2, bit 2, three subtractions per entry) and
 // GravityCenter (lanes 3-5, bit 4), as k_sweep_a adds them.
-template <bool ST, bool RATIO, bool DA>
+template <bool ST, bool RATIO>
 __global__ void __launch_bounds__(32 * kWarpSweepWarps)
-k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restrict__ vel,
+k_sweep_a_w(SimConst c, const double2* __restrict__ xv, const int* __restrict__ type,
             const int* __restrict__ ncount, const int* __restrict__ nlist, double* __restrict__ dens_a,
             double* __restrict__ strain_p, double* __restrict__ div_p, double4* __restrict__ velp,
             double4* __restrict__ gcpa, double* __restrict__ wall_center) {
@@ -800,9 +818,8 @@ k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restri
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * kWarpSweepWarps + w;
     if (i >= c.n) return;  // whole warp
-    const double4 pi = pos[i];
-    const double4 vi = vel[i];
-    const int ti = type_of(pi);
+    const XV pi = ld_xv(xv, i);
+    const int ti = type[i];
     const int cnt = ncount[i];
     const size_t n = (size_t)c.n;
     // lane s's sum: 0 DensityA, 1 DensityP, 2 DivergenceP, 3-5 GravityCenter
@@ -816,17 +833,17 @@ k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restri
         for (int q = 0; q < 8; ++q) v[q] = 0.0;
         const int j = k < cnt ? __ldg(nlist + (size_t)k * n + i) : i;
         if (j != i) {
-            const double4 pj = pos[j];
+            const XV pj = ld_xv(xv, j);
             double x[3];
             disp(c, pi, pj, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-            const bool in_a = DA && (r2 <= c.ra2);
+            const bool in_a = ST && (r2 <= c.ra2);
             const bool in_p = r2 <= c.rp2;
             const bool in_g = ST && (r2 <= c.rg2);
             if (in_a || in_p || in_g) {
                 const double r = sqrt(r2);
                 double ratio = 1.0;
-                if (RATIO) ratio = c.ratio[ti][type_of(pj)];
+                if (RATIO) ratio = c.ratio[ti][__ldg(type + j)];
                 const double qa = div_rs(r, c.ra, c.inv_ra);
                 if (in_a) {
                     v[0] = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
@@ -841,13 +858,12 @@ k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restri
                     fl |= 4u;
                 }
                 if (in_p) {
-                    const double4 vjn = vel[j];
                     const double qp = div_rs(r, c.rp, c.inv_rp);
                     v[1] = s_wp(c, qp);
                     const double dw = s_dwp(c, qp);
                     const double ri = __drcp_rn(r);
                     const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-                    const double u0 = vjn.x - vi.x, u1 = vjn.y - vi.y, u2 = vjn.z - vi.z;
+                    const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
                     v[2] = u0 * e0 * dw;
                     v[3] = u1 * e1 * dw;
                     v[4] = u2 * e2 * dw;
@@ -884,7 +900,7 @@ k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restri
     const double g1 = __shfl_sync(0xffffffffu, acc, 4);
     const double g2 = __shfl_sync(0xffffffffu, acc, 5);
     if (lane != 0) return;
-    if (DA) dens_a[i] = sum_a;
+    if (ST) dens_a[i] = sum_a;
     const double strain = sum_p - c.n0p;
     strain_p[i] = strain;
     div_p[i] = sum_d;
@@ -892,13 +908,12 @@ k_sweep_a_w(SimConst c, const double4* __restrict__ pos, const double4* __restri
     if (strain < 0.0) kappa = 0.0;
     const double lambda = c.bulk_viscosity[ti];
     const double pp = -lambda * sum_d + kappa * strain;
-    double pa = 0.0;
-    if (DA) {
-        pa = c.cof_a[ti] * (sum_a - c.n0a) / c.l0;
+    velp[i] = make_double4(pi.b.y, pi.c.x, pi.c.y, pp);
+    if (ST) {
+        double pa = c.cof_a[ti] * (sum_a - c.n0a) / c.l0;
         if (c.n0a <= sum_a) pa = 0.0;
+        gcpa[i] = make_double4(g0, g1, g2, pa);
     }
-    velp[i] = make_double4(vi.x, vi.y, vi.z, pp);
-    gcpa[i] = make_double4(ST ? g0 : 0.0, ST ? g1 : 0.0, ST ? g2 : 0.0, pa);
 }
 
 // Self-check of div_rn against the hardware IEEE division: operands with
@@ -1254,45 +1269,38 @@ k_force_compare(int nf, const double4* __restrict__ fa, const double4* __restric
 
 }  // namespace
 
-void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4* vel, const double4* snap,
-                 const double* wall_center, StepScalars* scal, cudaStream_t s) {
-    k_move<false><<<blocks(c.n, 256), 256, 0, s>>>(c, cellstart, pos, vel, snap, wall_center, scal, 0, 0);
+void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
+                 const double4* snap, const double* wall_center, StepScalars* scal, cudaStream_t s) {
+    k_move<false><<<blocks(c.n, 256), 256, 0, s>>>(c, cellstart, pos, vel, xv, snap, wall_center, scal, 0, 0);
 }
 
-void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, double4* vel, const double4* snap,
-                       const double* wall_center, StepScalars* scal, cudaGraphConditionalHandle rebuild,
-                       cudaGraphConditionalHandle sweep, cudaStream_t s) {
-    k_move<true><<<blocks(c.n, 256), 256, 0, s>>>(c, cellstart, pos, vel, snap, wall_center, scal, rebuild,
+void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
+                       const double4* snap, const double* wall_center, StepScalars* scal,
+                       cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle sweep, cudaStream_t s) {
+    k_move<true><<<blocks(c.n, 256), 256, 0, s>>>(c, cellstart, pos, vel, xv, snap, wall_center, scal, rebuild,
                                                   sweep);
 }
 
-void launch_sweep_a(const SimConst& c, const int* cellstart, const double4* pos, const double4* vel,
-                    const int* ncount, const int* nlist, const int* ncount_s, const int* nlist_s, double* dens_a,
-                    double* strain_p, double* div_p, double4* press, double4* gc, double* wall_center,
-                    cudaStream_t s) {
-    (void)cellstart;
+void launch_sweep_a(const SimConst& c, const double2* xv, const int* type, const int* ncount, const int* nlist,
+                    const int* ncount_s, const int* nlist_s, double* dens_a, double* strain_p, double* div_p,
+                    double4* press, double4* gc, double* wall_center, cudaStream_t s) {
     const bool warp = use_warp_sweeps(c);
-    const int nb = warp ? blocks(c.n, kWarpSweepWarps) : (blocks(c.n, 128) > 0 ? blocks(c.n, 128) : 1);
-    // with surface tension the list (DensityA, GravityCenter) and, when there
-    // is one, the short sublist (DensityP, DivergenceP); without, the short
-    // sublist alone
-    const bool split = c.has_st && nlist_s != nullptr;
-#define SWEEP_A(ST, RATIO, SPLIT, CNT, LIST)                                                                      \
-    if (warp)                                                                                                     \
-        k_sweep_a_w<ST, RATIO, ST><<<nb, 32 * kWarpSweepWarps, 0, s>>>(c, pos, vel, CNT, LIST, dens_a, strain_p,  \
-                                                                       div_p, press, gc, wall_center);            \
-    else                                                                                                          \
-        k_sweep_a<ST, RATIO, ST, SPLIT><<<nb, 128, 0, s>>>(c, pos, vel, CNT, LIST, ncount_s, nlist_s, dens_a,     \
-                                                           strain_p, div_p, press, gc, wall_center)
+    const int nb = blocks(c.n, warp ? kWarpSweepWarps : 128);
+    // the warp kernel walks one list: with surface tension the whole one,
+    // without the short sublist
+    const int* cw = c.has_st ? ncount : ncount_s;
+    const int* lw = c.has_st ? nlist : nlist_s;
+#define SWEEP_A(ST, RATIO)                                                                                          \
+    if (warp)                                                                                                       \
+        k_sweep_a_w<ST, RATIO><<<nb, 32 * kWarpSweepWarps, 0, s>>>(c, xv, type, cw, lw, dens_a, strain_p, div_p,    \
+                                                                   press, gc, wall_center);                         \
+    else                                                                                                            \
+        k_sweep_a<ST, RATIO><<<nb, 128, 0, s>>>(c, xv, type, ncount, nlist, ncount_s, nlist_s, dens_a, strain_p,    \
+                                                div_p, press, gc, wall_center)
     if (c.has_st) {
-        if (split) {
-            if (c.ratio_all_one) SWEEP_A(true, false, true, ncount, nlist); else SWEEP_A(true, true, true, ncount, nlist);
-        } else {
-            if (c.ratio_all_one) SWEEP_A(true, false, false, ncount, nlist); else SWEEP_A(true, true, false, ncount, nlist);
-        }
+        if (c.ratio_all_one) SWEEP_A(true, false); else SWEEP_A(true, true);
     } else {
-        if (c.ratio_all_one) SWEEP_A(false, false, false, ncount_s, nlist_s);
-        else SWEEP_A(false, true, false, ncount_s, nlist_s);
+        SWEEP_A(false, false);  // the ratios weigh surface-tension sums alone
     }
 #undef SWEEP_A
 }
@@ -1306,42 +1314,36 @@ void launch_density_a(const SimConst& c, const double4* pos, const int* ncount, 
         k_density_a<true><<<nb, 128, 0, s>>>(c, pos, ncount, nlist, dens_a, gc);
 }
 
-void launch_sweep_b(const SimConst& c, const int* cellstart, const double4* pos, const double4* vel_in,
-                    double4* vel_out, const double4* press, const double4* gc, const int* ncount,
-                    const int* nlist, const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal,
-                    cudaStream_t s, const int* eoff, const float4* eforce, float4* lsum, int part, int i0,
-                    int i1, double* vel_host) {
-    (void)vel_in;
+void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, const int* type, double4* vel_out,
+                    const double4* press, const double4* gc, const int* ncount, const int* nlist,
+                    const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
+                    const int* eoff, const float4* eforce, float4* lsum, int part, int i0, int i1,
+                    double* vel_host) {
     if (i1 < 0) i1 = c.n;
     if (i1 <= i0) return;
+    // the ratios weigh surface-tension terms alone
+    const bool ratio = c.has_st && !c.ratio_all_one;
     if (!eforce && i0 == 0 && i1 == c.n && use_warp_sweeps(c)) {
         const int nw = blocks(c.n, kWarpSweepWarps);
 #define SWEEP_BW(ST, RATIO)                                                                                       \
-    k_sweep_b_w<ST, RATIO><<<nw, 32 * kWarpSweepWarps, 0, s>>>(c, cellstart, pos, press, vel_out, gc, ncount,    \
+    k_sweep_b_w<ST, RATIO><<<nw, 32 * kWarpSweepWarps, 0, s>>>(c, cellstart, xv, type, press, vel_out, gc, ncount, \
                                                               nlist, force, scal, part, vel_host)
-        if (c.has_st) {
-            if (c.ratio_all_one) SWEEP_BW(true, false); else SWEEP_BW(true, true);
-        } else {
-            if (c.ratio_all_one) SWEEP_BW(false, false); else SWEEP_BW(false, true);
-        }
+        if (!c.has_st) SWEEP_BW(false, false);
+        else if (!ratio) SWEEP_BW(true, false);
+        else SWEEP_BW(true, true);
 #undef SWEEP_BW
         return;
     }
     const int nb = blocks(i1 - i0, 128);
-#define SWEEP_B(ST, RATIO, LRN, SPLIT) \
-    k_sweep_b<ST, RATIO, LRN, SPLIT><<<nb, 128, 0, s>>>(c, cellstart, pos, press, vel_out, gc, ncount, nlist,        \
-                                                        ncount_s, nlist_s, force, scal, eoff, eforce, lsum, part, \
-                                                        i0, i1, vel_host)
-#define SWEEP_B2(ST, RATIO)                                             \
-    if (eforce) SWEEP_B(ST, RATIO, true, false);                        \
-    else if (nlist_s) SWEEP_B(ST, RATIO, false, true);                  \
-    else SWEEP_B(ST, RATIO, false, false)
-    if (c.has_st) {
-        if (c.ratio_all_one) { SWEEP_B2(true, false); } else { SWEEP_B2(true, true); }
-    } else {
-        if (c.ratio_all_one) { SWEEP_B2(false, false); } else { SWEEP_B2(false, true); }
-    }
-#undef SWEEP_B2
+#define SWEEP_B(ST, RATIO, LRN, MU1)                                                                             \
+    k_sweep_b<ST, RATIO, LRN, MU1><<<nb, 128, 0, s>>>(c, cellstart, xv, type, press, vel_out, gc, ncount, nlist, \
+                                                      ncount_s, nlist_s, force, scal, eoff, eforce, lsum, part,  \
+                                                      i0, i1, vel_host)
+    if (eforce) SWEEP_B(false, false, true, true);
+    else if (!c.has_st) { if (c.mu_uniform) SWEEP_B(false, false, false, true); else SWEEP_B(false, false, false, false); }
+    else if (ratio) SWEEP_B(true, true, false, false);
+    else if (c.mu_uniform) SWEEP_B(true, false, false, true);
+    else SWEEP_B(true, false, false, false);
 #undef SWEEP_B
 }
 

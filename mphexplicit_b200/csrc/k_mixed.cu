@@ -1098,7 +1098,7 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     k_mix_place<<<blocks(n, 256), 256, 0, s>>>(n, m->keys_unsorted, m->slot, d.cellstart, m->tmp);
     k_mix_rank<<<blocks(n, 256), 256, 0, s>>>(n, m->keys_unsorted, d.cellstart, m->tmp, d.vals, d.keys);
     launch_reorder(c, d.vals, d.pidx[a], d.type[a], d.pos[a], d.vel[va], d.pidx[b], d.type[b], d.pos[b], d.vel[vb],
-                   d.snap, s);
+                   nullptr, d.snap, s);
     d.cur = b;
     d.vcur = vb;
     k_mix_home<<<blocks(n, 256), 256, 0, s>>>(c, m->mc, d.pos[d.cur], d.keys, d.vel[d.vcur], m->home, m->phl,

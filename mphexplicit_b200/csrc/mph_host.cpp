@@ -345,6 +345,10 @@ int mph::make_simconst(const mph_params& p, const mph_grid_header& h, const mph_
             s.visc_mu[t][u] = s.visc_c * muij;
         }
     const double margin = 0.1 * l0;
+    s.mu_uniform = 1;  // a NaN (two inviscid types) equals nothing
+    for (int t = 0; t < MPH_TYPE_COUNT; ++t)
+        for (int u = 0; u < MPH_TYPE_COUNT; ++u)
+            if (!(s.visc_mu[t][u] == s.visc_mu[0][0])) s.mu_uniform = 0;
     s.shift_thr = 0.5 * margin * 0.5 * margin;  // main.cpp:1102
     s.has_st = 0;
     s.ratio_all_one = 1;
@@ -390,7 +394,7 @@ static int dalloc(mph_ctx* ctx, T** ptr, size_t count) {
 
 static void free_fp64(mph::DevFP64& d) {
     void* ptrs[] = {d.pidx[0], d.pidx[1], d.type[0], d.type[1], d.pos[0], d.pos[1], d.vel[0], d.vel[1],
-                    d.snap, d.pos32, d.force, d.dens_a, d.strain_p, d.div_p, d.press, d.gc, d.virial_p, d.keys,
+                    d.xv, d.snap, d.pos32, d.force, d.dens_a, d.strain_p, d.div_p, d.press, d.gc, d.virial_p, d.keys,
                     d.vals, d.cellstart, d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.wall_center, d.staging,
                     d.scal};
     for (void* q : ptrs)
@@ -413,6 +417,7 @@ static int alloc_fp64(mph_ctx* ctx) {
         TRY(dalloc(ctx, &d.pos[k], n));
         TRY(dalloc(ctx, &d.vel[k], n));
     }
+    if (ctx->mode == MPH_MODE_FP64 || ctx->mode == MPH_MODE_LEARNED) TRY(dalloc(ctx, &d.xv, 3 * n));
     TRY(dalloc(ctx, &d.snap, n));
     TRY(dalloc(ctx, &d.pos32, n));
     TRY(dalloc(ctx, &d.force, n));
@@ -465,13 +470,6 @@ static int grow_table(mph_ctx* ctx, int need, int** table, int* capacity) {
 
 static int grow_list(mph_ctx* ctx, int need) { return grow_table(ctx, need, &ctx->d.nlist, &ctx->d.cap); }
 
-// The short sublist (the list's entries within RadiusP+MARGIN, in list order)
-// serves the pressure loops of both sweeps, with and without surface tension.
-static bool uses_short_list(const mph_ctx* ctx) {
-    (void)ctx;
-    return true;
-}
-
 // calculateCellParticle + calculateNeighbor (main.cpp:1111-1596).
 static int build_lists(mph_ctx* ctx);
 
@@ -486,7 +484,7 @@ static int rebuild_fp64(mph_ctx* ctx) {
     {
         Launch L(ctx, "reorder");
         mph::launch_reorder(s, d.vals, d.pidx[a], d.type[a], d.pos[a], d.vel[va], d.pidx[b], d.type[b], d.pos[b],
-                            d.vel[vb], d.snap, st);
+                            d.vel[vb], d.xv, d.snap, st);
     }
     d.cur = b;
     d.vcur = vb;
@@ -500,7 +498,6 @@ static int build_lists(mph_ctx* ctx) {
     mph::DevFP64& d = ctx->d;
     const SimConst& s = ctx->sc;
     cudaStream_t st = ctx->stream;
-    const bool sl = uses_short_list(ctx);
     int max_short = 0;
     for (int attempt = 0; attempt < 3; ++attempt) {
         CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_neighbors, 0, sizeof(int), st));
@@ -509,14 +506,14 @@ static int build_lists(mph_ctx* ctx) {
             Launch L(ctx, "neighbor_list");
             mph::launch_pos32(s, d.pos[d.cur], d.pos32, st);
             mph::launch_neighbor_list(s, d.pos[d.cur], d.pos32, d.cellstart, d.ncount, d.nlist, d.cap,
-                                      sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.cap_s, d.scal, st);
+                                      d.ncount_s, d.nlist_s, d.cap_s, d.scal, st);
             L.count = 2;
         }
         CUDA_TRY(ctx, cudaGetLastError());
         CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_scal, d.scal, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(ctx, cudaStreamSynchronize(st));
         ctx->max_neighbors = ctx->h_scal->max_neighbors;
-        max_short = sl ? ctx->h_scal->max_short : 0;
+        max_short = ctx->h_scal->max_short;
         if (ctx->max_neighbors <= d.cap && max_short <= d.cap_s) break;
         if (ctx->max_neighbors > d.cap) TRY(grow_list(ctx, ctx->max_neighbors));
         if (max_short > d.cap_s) TRY(grow_table(ctx, max_short, &d.nlist_s, &d.cap_s));
@@ -532,7 +529,7 @@ static int build_lists(mph_ctx* ctx) {
 static void sweep_a(mph_ctx* ctx, bool advance_wall) {
     mph::DevFP64& d = ctx->d;
     Launch L(ctx, "sweep_a");
-    mph::launch_sweep_a(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
+    mph::launch_sweep_a(ctx->sc, d.xv, d.type[d.cur], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
                         d.dens_a, d.strain_p, d.div_p, d.press, d.gc, advance_wall ? d.wall_center : nullptr,
                         ctx->stream);
     ctx->dens_a_valid = ctx->sc.has_st;  // without surface tension, computed when read
@@ -561,9 +558,8 @@ static void ensure_wall_force(mph_ctx* ctx) {
     if (ctx->mixed || ctx->wall_force_valid) return;
     mph::DevFP64& d = ctx->d;
     Launch L(ctx, "wall_force");
-    const bool sl = uses_short_list(ctx);
-    mph::launch_sweep_b(ctx->sc, d.cellstart, step_positions(ctx), nullptr, nullptr, d.press, d.gc, d.ncount,
-                        d.nlist, sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.force, d.scal, ctx->stream,
+    mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], nullptr, d.press, d.gc, d.ncount,
+                        d.nlist, d.ncount_s, d.nlist_s, d.force, d.scal, ctx->stream,
                         nullptr, nullptr, nullptr, 2);
     ctx->wall_force_valid = true;
 }
@@ -643,10 +639,8 @@ static int create_impl(mph_ctx* ctx, const int* type, const double* xyz, const d
         mph::mixed_set_cell_walk(ctx->mixed, ctx->cell_walk);
     } else {
         TRY(grow_list(ctx, initial_capacity(ctx, ctx->sc.rm2)));
-        if (uses_short_list(ctx)) {
-            TRY(dalloc(ctx, &d.ncount_s, n));
-            TRY(grow_table(ctx, initial_capacity(ctx, ctx->sc.rs2), &d.nlist_s, &d.cap_s));
-        }
+        TRY(dalloc(ctx, &d.ncount_s, n));
+        TRY(grow_table(ctx, initial_capacity(ctx, ctx->sc.rs2), &d.nlist_s, &d.cap_s));
         TRY(rebuild_fp64(ctx));
         sweep_a(ctx, false);
     }
@@ -717,7 +711,7 @@ static int step_fp64_head(mph_ctx* ctx) {
     CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
     {
         Launch L(ctx, "move");
-        mph::launch_move(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.snap, d.wall_center, d.scal, st);
+        mph::launch_move(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center, d.scal, st);
     }
     TRY(read_scalars(ctx));
     TRY(check_flags(ctx));
@@ -765,7 +759,6 @@ static int capture_step(mph_ctx* ctx, int v, cudaGraphExec_t* out, int* launches
     cudaStream_t st = ctx->stream;
     const int a = d.cur, b = 1 - d.cur, va = v, vb = 1 - v;
     const size_t n = (size_t)ctx->n;
-    const bool sl = uses_short_list(ctx);
     const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
     cudaGraph_t g = nullptr, g_reb = nullptr, g_sw = nullptr;
     cudaGraphConditionalHandle h_reb = 0, h_sw = 0;
@@ -784,7 +777,8 @@ static int capture_step(mph_ctx* ctx, int v, cudaGraphExec_t* out, int* launches
     if (ck(cudaGraphCreate(&g, 0)) && ck(cudaGraphConditionalHandleCreate(&h_reb, g, 0, 0)) &&
         ck(cudaGraphConditionalHandleCreate(&h_sw, g, 0, 0)) &&
         ck(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, mode))) {
-        mph::launch_move_graph(s, d.cellstart, d.pos[a], d.vel[va], d.snap, d.wall_center, d.scal, h_reb, h_sw, st);
+        mph::launch_move_graph(s, d.cellstart, d.pos[a], d.vel[va], d.xv, d.snap, d.wall_center, d.scal, h_reb, h_sw,
+                               st);
         ls += 1;
         if (rc == MPH_OK) rc = add_if_node(ctx, st, h_reb, &g_reb);
         if (rc == MPH_OK) rc = add_if_node(ctx, st, h_sw, &g_sw);
@@ -795,7 +789,7 @@ static int capture_step(mph_ctx* ctx, int v, cudaGraphExec_t* out, int* launches
         lr += 1 + mph::launch_bitonic_sort(s, d.keys, d.vals, st);
         mph::launch_cell_ranges(s, d.keys, d.cellstart, st);
         mph::launch_reorder(s, d.vals, d.pidx[a], d.type[a], d.pos[a], d.vel[va], d.pidx[b], d.type[b], d.pos[b],
-                            d.vel[vb], d.snap, st);
+                            d.vel[vb], d.xv, d.snap, st);
         ck(cudaMemcpyAsync(d.pos[a], d.pos[b], n * sizeof(double4), cudaMemcpyDeviceToDevice, st));
         ck(cudaMemcpyAsync(d.vel[va], d.vel[vb], n * sizeof(double4), cudaMemcpyDeviceToDevice, st));
         ck(cudaMemcpyAsync(d.pidx[a], d.pidx[b], n * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -804,16 +798,16 @@ static int capture_step(mph_ctx* ctx, int v, cudaGraphExec_t* out, int* launches
         ck(cudaMemsetAsync(&d.scal->max_short, 0, sizeof(int), st));
         mph::launch_pos32(s, d.pos[a], d.pos32, st);
         mph::launch_neighbor_list(s, d.pos[a], d.pos32, d.cellstart, d.ncount, d.nlist, d.cap,
-                                  sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.cap_s, d.scal, st);
-        mph::launch_graph_list_check(d.scal, d.cap, d.cap_s, sl ? 1 : 0, h_sw, st);
+                                  d.ncount_s, d.nlist_s, d.cap_s, d.scal, st);
+        mph::launch_graph_list_check(d.scal, d.cap, d.cap_s, 1, h_sw, st);
         lr += 6;
         end_capture();
     }
     if (rc == MPH_OK && ck(cudaStreamBeginCaptureToGraph(st, g_sw, nullptr, nullptr, 0, mode))) {
-        mph::launch_sweep_a(s, d.cellstart, d.pos[a], d.vel[va], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
+        mph::launch_sweep_a(s, d.xv, d.type[a], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
                             d.dens_a, d.strain_p, d.div_p, d.press, d.gc, d.wall_center, st);
-        mph::launch_sweep_b(s, d.cellstart, d.pos[a], d.vel[va], d.vel[vb], d.press, d.gc, d.ncount, d.nlist,
-                            sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.force, d.scal, st, nullptr,
+        mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[a], d.vel[vb], d.press, d.gc, d.ncount, d.nlist,
+                            d.ncount_s, d.nlist_s, d.force, d.scal, st, nullptr,
                             nullptr, nullptr, 1);
         ls += 2;
         end_capture();
@@ -905,9 +899,8 @@ static int step_fp64_graphs(mph_ctx* ctx, int nsteps) {
     sweep_a(ctx, true);
     {
         Launch L(ctx, "sweep_b");
-        const bool sl = uses_short_list(ctx);
-        mph::launch_sweep_b(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.vel[1 - d.vcur], d.press, d.gc,
-                            d.ncount, d.nlist, sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.force, d.scal,
+        mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc,
+                            d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.force, d.scal,
                             st, nullptr, nullptr, nullptr, 1);
         ctx->wall_force_valid = false;
     }
@@ -930,9 +923,8 @@ static int step_fp64(mph_ctx* ctx, int nsteps) {
         sweep_a(ctx, true);
         {
             Launch L(ctx, "sweep_b");
-            const bool sl = uses_short_list(ctx);
-            mph::launch_sweep_b(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.vel[1 - d.vcur], d.press, d.gc,
-                                d.ncount, d.nlist, sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.force,
+            mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc,
+                                d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.force,
                                 d.scal, st, nullptr, nullptr, nullptr, 1);
             ctx->wall_force_valid = false;  // computed when read
         }
@@ -1041,9 +1033,8 @@ static int learned_buffers(mph_ctx* ctx) {
 static void plain_sweep_b(mph_ctx* ctx, double4* vel_out, double4* force) {
     mph::DevFP64& d = ctx->d;
     Launch L(ctx, "sweep_b");
-    const bool sl = uses_short_list(ctx);
-    mph::launch_sweep_b(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], vel_out, d.press, d.gc, d.ncount, d.nlist,
-                        sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, force, d.scal, ctx->stream);
+    mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], vel_out, d.press, d.gc, d.ncount, d.nlist,
+                        d.ncount_s, d.nlist_s, force, d.scal, ctx->stream);
 }
 
 // The FP64 step with the learned pair terms, the judge and the fallback.
@@ -1059,7 +1050,7 @@ static int step_learned(mph_ctx* ctx, int nsteps) {
         CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
         {
             Launch Lm(ctx, "move");
-            mph::launch_move(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.snap, d.wall_center, d.scal, st);
+            mph::launch_move(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center, d.scal, st);
         }
         TRY(read_scalars(ctx));
         TRY(check_flags(ctx));
@@ -1097,10 +1088,8 @@ static int step_learned(mph_ctx* ctx, int nsteps) {
             {
                 Launch Lb(ctx, "sweep_b_learned");
                 // the learned sweep evaluates only the pairs within RadiusP
-                const bool sl = uses_short_list(ctx);
-                mph::launch_sweep_b(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], vout, d.press, d.gc,
-                                    sl ? d.ncount_s : d.ncount, sl ? d.nlist_s : d.nlist, nullptr, nullptr,
-                                    d.force, d.scal, st, L.eoff, L.eforce, L.lsum);
+                mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[d.cur], vout, d.press, d.gc, d.ncount, d.nlist,
+                                    d.ncount_s, d.nlist_s, d.force, d.scal, st, L.eoff, L.eforce, L.lsum);
             }
             bool use = true;
             if (L.info.steps % L.judge_interval == 0) {
@@ -1350,9 +1339,8 @@ static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
     double4* vout = d.vel[1 - d.vcur];
     {
         Launch L(ctx, "sweep_b");
-        const bool sl = uses_short_list(ctx);
-        mph::launch_sweep_b(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], vout, d.press, d.gc, d.ncount, d.nlist,
-                            sl ? d.ncount_s : nullptr, sl ? d.nlist_s : nullptr, d.force, d.scal, st, nullptr,
+        mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[d.cur], vout, d.press, d.gc, d.ncount, d.nlist,
+                            d.ncount_s, d.nlist_s, d.force, d.scal, st, nullptr,
                             nullptr, nullptr, 1, 0, -1, vh);
         ctx->wall_force_valid = false;  // computed when read
     }

@@ -24,6 +24,7 @@ struct SimConst {
     int pow2;              // PowerParticleCount
     int has_st;            // any surface tension -> diffuse-interface terms
     int ratio_all_one;     // InteractionRatio == 1 everywhere
+    int mu_uniform;        // visc_mu is one number for every pair of types
     double dmin[3], width[3], half_width[3], cell_width[3];
     // bits of 0.75*width: Mod(x, w) needs no division when 0 <= x < 0.75 w,
     // tested as one unsigned compare of x's bit pattern (negative x, -0.0
@@ -82,6 +83,7 @@ struct DevFP64 {
     double4* vel[2] = {nullptr, nullptr};   // vx,vy,vz,0
     int cur = 0;                            // index of the current pos/type/pidx
     int vcur = 0;                           // index of the current velocity
+    double2* xv = nullptr;                  // {x, y}, {z, vx}, {vy, vz}: the FP64 sweeps' gathers
     double4* snap = nullptr;                // NeighborCalculatedPosition
     float4* pos32 = nullptr;                // FP32 x - dmin for the list build's prefilter
     double4* force = nullptr;
@@ -110,9 +112,10 @@ void launch_cell_index(const SimConst& c, const double4* pos, const int* type, i
                        int* vals, cudaStream_t s);
 int launch_bitonic_sort(const SimConst& c, int* keys, int* vals, cudaStream_t s);  // returns #launches
 void launch_cell_ranges(const SimConst& c, const int* keys, int* cellstart, cudaStream_t s);
+// xv: the sweeps' records of the reordered particles (nullptr: not wanted)
 void launch_reorder(const SimConst& c, const int* vals, const int* pidx_in, const int* type_in,
                     const double4* pos_in, const double4* vel_in, int* pidx_out, int* type_out,
-                    double4* pos_out, double4* vel_out, double4* snap, cudaStream_t s);
+                    double4* pos_out, double4* vel_out, double2* xv, double4* snap, cudaStream_t s);
 // FP32 prefilter of the neighbour-list build: per axis whether it takes part,
 // the domain width, and the FP32 distance squared above which no candidate
 // can pass the exact FP64 test.
@@ -144,41 +147,39 @@ void launch_graph_list_check(StepScalars* scal, int cap, int cap_s, int short_li
 // makes the rebuild test of main.cpp:1102 (rebuild = 1 when it fires; sweep =
 // 1 unless the batch stopped, when the move does nothing), counts the step
 // and clears the maximum shift for the next step
-void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, double4* vel, const double4* snap,
-                       const double* wall_center, StepScalars* scal, cudaGraphConditionalHandle rebuild,
-                       cudaGraphConditionalHandle sweep, cudaStream_t s);
+void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
+                       const double4* snap, const double* wall_center, StepScalars* scal,
+                       cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle sweep, cudaStream_t s);
 void launch_unpack3(int n, const double* src, double4* dst, const int* type, cudaStream_t s);
 
 // ---- kernel launchers (k_fp64.cu) -----------------------------------------
-void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4* vel,
-                 const double4* snap, const double* wall_center, StepScalars* scal,
-                 cudaStream_t s);
+// xv receives the moved particles' {x, y}, {z, vx}, {vy, vz}
+void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
+                 const double4* snap, const double* wall_center, StepScalars* scal, cudaStream_t s);
 // Sweep A's DensityP and DivergenceP visit the short sublist (ncount_s,
 // nlist_s); with surface tension DensityA and GravityCenter the whole list.
-void launch_sweep_a(const SimConst& c, const int* cellstart, const double4* pos,
-                    const double4* vel, const int* ncount, const int* nlist, const int* ncount_s,
-                    const int* nlist_s, double* dens_a, double* strain_p, double* div_p, double4* press,
-                    double4* gc, double* wall_center, cudaStream_t s);
+void launch_sweep_a(const SimConst& c, const double2* xv, const int* type, const int* ncount, const int* nlist,
+                    const int* ncount_s, const int* nlist_s, double* dens_a, double* strain_p, double* div_p,
+                    double4* press, double4* gc, double* wall_center, cudaStream_t s);
 // DensityA and PressureA alone (into dens_a and gc[].w), in k_sweep_a's
 // order: what sweep A leaves out when there is no surface tension.
 void launch_density_a(const SimConst& c, const double4* pos, const int* ncount, const int* nlist, double* dens_a,
                       double4* gc, cudaStream_t s);
 // eforce != nullptr: the learned form (edge-MLP pair forces replace the
-// PressureA, DiffuseInterface and ViscosityV terms; see k_sweep_b; it then
-// needs only the pairs within RadiusP, so the short sublist may be passed).
+// PressureA, DiffuseInterface and ViscosityV terms; see k_sweep_b; it visits
+// the short sublist alone).
 // part: 0 every particle; 1 the fluid (walls copy their velocity, their
 // force is not written); 2 the walls' forces alone (vel_out unused).
-// ncount_s / nlist_s (not learned): the short sublist, over which the
-// PressureP force runs as its own loop (same result).
+// ncount_s / nlist_s: the short sublist, over which the PressureP force runs
+// as its own loop (same result).  xv: positions and velocities of the step.
 // [i0, i1): the particles (sorted order) this launch computes; i1 < 0 means
 // all n.  Every particle's result depends on the inputs alone, so a sweep
 // split into ranges gives the same bits as one launch.  vel_host (part 1): a
 // device-accessible [n][3] view of pinned host memory that also receives
 // each particle's new velocity.
-void launch_sweep_b(const SimConst& c, const int* cellstart, const double4* pos,
-                    const double4* vel_in, double4* vel_out, const double4* press,
-                    const double4* gc, const int* ncount, const int* nlist, const int* ncount_s,
-                    const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
+void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, const int* type, double4* vel_out,
+                    const double4* press, const double4* gc, const int* ncount, const int* nlist,
+                    const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
                     const int* eoff = nullptr, const float4* eforce = nullptr, float4* lsum = nullptr,
                     int part = 0, int i0 = 0, int i1 = -1, double* vel_host = nullptr);
 
