@@ -17,25 +17,23 @@
 #include "mph_exact.cuh"
 
 // Resident 128-thread blocks per SM the sweeps are compiled for (register cap
-// 65536 / (128 * blocks)); latency hiding vs. spills, set by measurement on
-// the full dam break.  Both sweeps keep the next neighbour's records in
-// flight: sweep A at 7 (72 registers; at 8 it spills), the force sweep at 6
-// (80 registers, a few spills outside the neighbour loops: 3.08 ms against
-// 3.13 ms at 5 blocks and 3.16 ms at 4, with the pressure loop split off).
+// 65536 / (128 * blocks)); latency hiding vs. spills, set by measurement.  The
+// FP64 pipe bounds the sweeps (71 % active in the force sweep, with the L1 data
+// pipe at 69 %): about 84 FP64 operations per list entry.  On the 2,779,256-particle
+// dam break the force sweep takes 2.34 ms at 6 blocks (80 registers, two spilled
+// values), 2.42 at 5; sweep A 0.314 ms at 7, 0.332 at 6, 0.366 at 8.  Blocks of 64 or
+// 256 threads give the same times, of 32 up to 13 % more.
 #ifndef MPH_SWEEP_MINB
 #define MPH_SWEEP_MINB 7
 #endif
 #ifndef MPH_SWEEPB_MINB
 #define MPH_SWEEPB_MINB 6
 #endif
-// The surface-tension variants hold more live values per pair; at the
-// bounds above they spilled (140 B in the force sweep) and ran the 8.5 M
-// particle two-fluid column's step at 40.6 + 13.9 ms.  Measured on that
-// column: the force sweep 26.7 ms at 4 blocks (no spills) and 29.6 ms at 3,
-// sweep A 12.5 ms at 5 (13.3 at 6); results bit-identical.  With the pressure
-// loops over the short sublist (SPLIT): 26.0 and 10.2 ms.
+// The surface-tension variants hold more live values per pair.  On the
+// 314,432-particle two-fluid column: the force sweep 0.75 ms at 4 blocks (no
+// spills), 0.85 at 5, 0.94 at 3; sweep A 0.323 ms at 7, 0.339 at 6, 0.376 at 5.
 #ifndef MPH_SWEEP_MINB_ST
-#define MPH_SWEEP_MINB_ST 5
+#define MPH_SWEEP_MINB_ST 7
 #endif
 #ifndef MPH_SWEEPB_MINB_ST
 #define MPH_SWEEPB_MINB_ST 4
@@ -53,14 +51,6 @@ __device__ __forceinline__ double omod_fast(double x, double w) {
     return (x >= 0.0 && x < 0.75 * w) ? x : omod(x, w);
 }
 
-// The same Mod with the range test as one unsigned compare of x's bits
-// against those of 0.75 w (SimConst::q75_bits): equal to omod_fast for every x
-// except -0.0, which takes omod and gives +0.0 instead of -0.0; the callers
-// then subtract half_width (non-zero), so their results are the same.
-__device__ __forceinline__ double omod_q(double x, double w, unsigned long long q75) {
-    return ((unsigned long long)__double_as_longlong(x) < q75) ? x : omod(x, w);
-}
-
 // The record the pair sweeps gather per neighbour: position and velocity, 48
 // bytes as three 16-byte words {x, y}, {z, vx}, {vy, vz}, written by the move
 // (k_move) and by the reorder.  The sweeps are bound by the L1 data pipe: a
@@ -72,6 +62,14 @@ __device__ __forceinline__ double omod_q(double x, double w, unsigned long long 
 // 13 -> 16 us and 0.058 -> 0.082 ms.
 struct XV {
     double2 a, b, c;
+};
+struct XVT {  // with the type
+    XV p;
+    int t;
+};
+struct XVP {  // with PressureP
+    XV p;
+    double pressure;
 };
 __device__ __forceinline__ XV ld_xv(const double2* __restrict__ xv, int j) {
     const double2* p = xv + 3 * (size_t)j;
@@ -97,16 +95,60 @@ __device__ __forceinline__ void st_xv(double2* __restrict__ xv, int i, const dou
     q[2] = make_double2(v.y, v.z);
 }
 
-// Minimum-image displacement x_j - x_i (main.cpp:1680 and every sweep).
+// Minimum-image displacement x_j - x_i (main.cpp:1680 and every sweep):
+// Mod(x_j - x_i + W/2, W) - W/2.  The division-free range 0 <= t < 0.75 W of Mod
+// is tested for the three axes at once on the high words of t against that of
+// 0.75 W (SimConst::q75_hi; a negative t, -0.0 and NaN have the sign bit set and
+// compare above it): one branch instead of three.  A t with the bound's own high
+// word takes Mod's general expression, which gives t itself where t < 0.75 W, and
+// so does -0.0, which becomes +0.0 and the same displacement.
+__device__ __forceinline__ void disp(const SimConst& c, double xi, double yi, double zi, double xj, double yj,
+                                     double zj, double* x) {
+    double t0 = xj - xi + c.half_width[0], t1 = yj - yi + c.half_width[1], t2 = zj - zi + c.half_width[2];
+    if (!((unsigned)__double2hiint(t0) < c.q75_hi[0] && (unsigned)__double2hiint(t1) < c.q75_hi[1] &&
+          (unsigned)__double2hiint(t2) < c.q75_hi[2])) {
+        t0 = omod(t0, c.width[0]);
+        t1 = omod(t1, c.width[1]);
+        t2 = omod(t2, c.width[2]);
+    }
+    x[0] = t0 - c.half_width[0];
+    x[1] = t1 - c.half_width[1];
+    x[2] = t2 - c.half_width[2];
+}
 __device__ __forceinline__ void disp(const SimConst& c, const XV& pi, const XV& pj, double* x) {
-    x[0] = omod_q(pj.a.x - pi.a.x + c.half_width[0], c.width[0], c.q75_bits[0]) - c.half_width[0];
-    x[1] = omod_q(pj.a.y - pi.a.y + c.half_width[1], c.width[1], c.q75_bits[1]) - c.half_width[1];
-    x[2] = omod_q(pj.b.x - pi.b.x + c.half_width[2], c.width[2], c.q75_bits[2]) - c.half_width[2];
+    disp(c, pi.a.x, pi.a.y, pi.b.x, pj.a.x, pj.a.y, pj.b.x, x);
 }
 __device__ __forceinline__ void disp(const SimConst& c, const double4& pi, const double4& pj, double* x) {
-    x[0] = omod_q(pj.x - pi.x + c.half_width[0], c.width[0], c.q75_bits[0]) - c.half_width[0];
-    x[1] = omod_q(pj.y - pi.y + c.half_width[1], c.width[1], c.q75_bits[1]) - c.half_width[1];
-    x[2] = omod_q(pj.z - pi.z + c.half_width[2], c.width[2], c.q75_bits[2]) - c.half_width[2];
+    disp(c, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, x);
+}
+
+// Visits the cnt entries of one particle's list (column lp, rows n apart) in
+// order: visit(j, load(j)).  Indices are loaded two to three entries ahead and
+// records one ahead, so the gathers overlap the previous pair's FP64
+// arithmetic; two entries per trip, so the records alternate between two sets
+// of registers instead of being moved.  With disp's single branch and
+// pair_root's, 158 -> 123 instructions per entry of the force sweep (2.60 -> 2.34
+// ms on the 2,779,256-particle dam break, 0.81 -> 0.75 ms on the 314,432-particle
+// column).
+template <class Load, class Visit>
+__device__ __forceinline__ void walk_list(const int* __restrict__ lp, size_t n, int cnt, Load&& load, Visit&& visit) {
+    if (cnt <= 0) return;
+    int ja = __ldg(lp), jb = cnt > 1 ? __ldg(lp + n) : ja;
+    auto a = load(ja);
+    for (int k = 0;; k += 2) {
+        lp += 2 * n;
+        int jc = ja, jd = jb;
+        if (k + 2 < cnt) jc = __ldg(lp);
+        if (k + 3 < cnt) jd = __ldg(lp + n);
+        auto b = load(jb);
+        visit(ja, a);
+        if (k + 1 >= cnt) break;
+        a = load(jc);
+        visit(jb, b);
+        if (k + 2 >= cnt) break;
+        ja = jc;
+        jb = jd;
+    }
 }
 
 // Kernel shapes, main.cpp:214-284, with q = r/h computed by division.
@@ -132,6 +174,19 @@ __device__ __forceinline__ double f_dwvdr(const SimConst& c, double r) {
 }
 
 __device__ __forceinline__ int type_of(const double4& p) { return (int)p.w; }
+
+// The distance r = sqrt(r2) of a pair that is in range (near) and its
+// reciprocal; false for one that is not, and for a particle paired with itself
+// (r2 = 0, which the list holds).  One branch on the way of every other pair.
+__device__ __forceinline__ bool pair_root(double r2, bool near, bool self, double& r, Recip& ri) {
+    if (near && plain_root(r2)) {
+        sqrt_recip(r2, r, ri);
+        return true;
+    }
+    if (!near || self) return false;
+    sqrt_recip_any(r2, r, ri);
+    return true;
+}
 
 // Convection (main.cpp:1605-1615), Wall (2013-2043), PeriodicBoundary
 // (2306-2317) and the displacement maximum of neighborCalculation (1086-1100).
@@ -258,81 +313,52 @@ k_sweep_a(SimConst c, const double2* __restrict__ xv, const int* __restrict__ ty
     const size_t n = (size_t)c.n;
     double sum_a = 0.0, sum_p = 0.0, sum_d = 0.0;
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    {  // DensityP, DivergenceP: indices two entries ahead, the neighbour's record one ahead
-        const int cs = ncount_p[i];
-        const int* lq = nlist_p + i;
-        int q1 = cs > 0 ? __ldg(lq) : i;
-        int q2 = cs > 1 ? __ldg(lq + n) : i;
-        lq += 2 * n;
-        XV qn = ld_xv(xv, q1);
-        for (int k = 0; k < cs; ++k) {
-            const int j = q1;
-            const XV pj = qn;
-            q1 = q2;
-            if (k + 2 < cs) q2 = __ldg(lq);
-            lq += n;
-            if (k + 1 < cs) qn = ld_xv(xv, q1);
-            if (j == i) continue;
-            double x[3];
-            disp(c, pi, pj, x);
-            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-            // R*R - r2 >= 0 (main.cpp:1683 and the other density sums) is r2 <= R*R:
-            // with gradual underflow a - b is zero only when a == b, and its sign exact
-            if (!(r2 <= c.rp2)) continue;
-            const double r = sqrt(r2);
-            const double qp = div_rs(r, c.rp, c.inv_rp);
-            sum_p += s_wp(c, qp);
-            const double dw = s_dwp(c, qp);
-            const double ri = __drcp_rn(r);
-            const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-            const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
-            sum_d -= u0 * e0 * dw;
-            sum_d -= u1 * e1 * dw;
-            sum_d -= u2 * e2 * dw;
-        }
-    }
+    walk_list(nlist_p + i, n, ncount_p[i], [&](int j) { return ld_xv(xv, j); }, [&](int j, const XV& pj) {
+        // DensityP, DivergenceP
+        double x[3];
+        disp(c, pi, pj, x);
+        const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+        // R*R - r2 >= 0 (main.cpp:1683 and the other density sums) is r2 <= R*R:
+        // with gradual underflow a - b is zero only when a == b, and its sign exact
+        double r;
+        Recip ri;
+        if (!pair_root(r2, r2 <= c.rp2, j == i, r, ri)) return;
+        const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
+        sum_p += s_wp(c, qp);
+        const double dw = s_dwp(c, qp);
+        const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
+        const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
+        sum_d -= u0 * e0 * dw;
+        sum_d -= u1 * e1 * dw;
+        sum_d -= u2 * e2 * dw;
+    });
     if (ST) {  // DensityA, GravityCenter
-        const int cnt = ncount[i];
-        const int* lp = nlist + i;
-        int j1 = cnt > 0 ? __ldg(lp) : i;
-        int j2 = cnt > 1 ? __ldg(lp + n) : i;
-        lp += 2 * n;
-        XV pn = ld_xv(xv, j1);  // the words that are not used are not loaded
-        int tn = RATIO ? __ldg(type + j1) : 0;
-        for (int k = 0; k < cnt; ++k) {
-            const int j = j1;
-            const XV pj = pn;
-            const int tj = tn;
-            j1 = j2;
-            if (k + 2 < cnt) j2 = __ldg(lp);
-            lp += n;
-            if (k + 1 < cnt) {
-                pn = ld_xv(xv, j1);
-                if (RATIO) tn = __ldg(type + j1);
-            }
-            if (j == i) continue;
+        walk_list(nlist + i, n, ncount[i],
+                  [&](int j) { return XVT{ld_xv(xv, j), RATIO ? __ldg(type + j) : 0}; },  // unused words: no loads
+                  [&](int j, const XVT& rj) {
             double x[3];
-            disp(c, pi, pj, x);
+            disp(c, pi, rj.p, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
             const bool in_a = r2 <= c.ra2;
             const bool in_g = r2 <= c.rg2;
-            if (!(in_a || in_g)) continue;
-            const double r = sqrt(r2);
+            double r;
+            Recip ri;  // not used: its operations are not compiled
+            if (!pair_root(r2, in_a || in_g, j == i, r, ri)) return;
             double ratio = 1.0;
-            if (RATIO) ratio = c.ratio[ti][tj];
-            const double qa = div_rs(r, c.ra, c.inv_ra);
+            if (RATIO) ratio = c.ratio[ti][rj.t];
+            const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
             if (in_a) {
                 const double w = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
                 sum_a += w;
             }
             if (in_g) {
-                const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
                 const double w = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
-                g0 += div_rs(x[0] * w, c.r2g, c.inv_r2g) * c.rg;
-                g1 += div_rs(x[1] * w, c.r2g, c.inv_r2g) * c.rg;
-                g2 += div_rs(x[2] * w, c.r2g, c.inv_r2g) * c.rg;
+                g0 += div_q(x[0] * w, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                g1 += div_q(x[1] * w, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                g2 += div_q(x[2] * w, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
             }
-        }
+        });
         dens_a[i] = sum_a;
     }
     const double strain = sum_p - c.n0p;
@@ -370,14 +396,14 @@ __global__ void __launch_bounds__(128) k_density_a(SimConst c, const double4* __
     double sum_a = 0.0;
     for (int k = 0; k < cnt; ++k) {
         const int j = __ldg(nlist + (size_t)k * n + i);
-        if (j == i) continue;
-        const double4 pj = pos[j];
+        const double4 pj = ld_d4(pos, j);
         double x[3];
         disp(c, pi, pj, x);
         const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        if (!(r2 <= c.ra2)) continue;
-        const double r = sqrt(r2);
-        const double qa = div_rs(r, c.ra, c.inv_ra);
+        double r;
+        Recip ri;
+        if (!pair_root(r2, r2 <= c.ra2, j == i, r, ri)) continue;
+        const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
         sum_a += RATIO ? c.ratio[ti][type_of(pj)] * s_wa(c, qa) : s_wa(c, qa);
     }
     dens_a[i] = sum_a;
@@ -433,71 +459,37 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
     double fd0 = 0.0, fd1 = 0.0, fd2 = 0.0;
     double fv0 = 0.0, fv1 = 0.0, fv2 = 0.0;
     {  // PressureP force (main.cpp:1908-1938) over the short sublist
-        // indices two entries ahead, the neighbour's position and PressureP one ahead
         const double ppi = velp[i].w;
-        const int cs = ncount_s[i];
-        const int* lq = nlist_s + i;
-        int q1 = cs > 0 ? __ldg(lq) : i;
-        int q2 = cs > 1 ? __ldg(lq + n) : i;
-        lq += 2 * n;
-        XV qn = ld_xv(xv, q1);
-        double qp1 = velp[q1].w;
-        for (int k = 0; k < cs; ++k) {
-            const int j = q1;
-            const XV pj = qn;
-            const double pjp = qp1;  // PressureP of j
-            q1 = q2;
-            if (k + 2 < cs) q2 = __ldg(lq);
-            lq += n;
-            if (k + 1 < cs) {
-                qn = ld_xv(xv, q1);
-                qp1 = velp[q1].w;
-            }
-            if (j == i) continue;
+        walk_list(nlist_s + i, n, ncount_s[i],
+                  [&](int j) { return XVP{ld_xv(xv, j), __ldg(&velp[j].w)}; },
+                  [&](int j, const XVP& rj) {
             double x[3];
-            disp(c, pi, pj, x);
+            disp(c, pi, rj.p, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
             // R*R - r2 > 0 (main.cpp:1926 and the other force sums) is r2 < R*R
-            if (!(r2 < c.rp2)) continue;
-            const double r = sqrt(r2);
-            const double ri = __drcp_rn(r);
-            const double qp = div_rs(r, c.rp, c.inv_rp);
+            double r;
+            Recip ri;
+            if (!pair_root(r2, r2 < c.rp2, j == i, r, ri)) return;
+            const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
             const double dw = s_dwp(c, qp);
-            const double gw0 = div_rs(dw * x[0], r, ri), gw1 = div_rs(dw * x[1], r, ri),
-                         gw2 = div_rs(dw * x[2], r, ri);
-            const double ps = ppi + pjp;
+            const double gw0 = div_q(dw * x[0], r, ri), gw1 = div_q(dw * x[1], r, ri),
+                         gw2 = div_q(dw * x[2], r, ri);
+            const double ps = ppi + rj.pressure;
             fp0 += ps * gw0 * c.vol;
             fp1 += ps * gw1 * c.vol;
             fp2 += ps * gw2 * c.vol;
-        }
+        });
     }
     if (!LRN) {
-        // software pipeline: list indices two entries ahead, the neighbour's
-        // record one ahead, so the gathers overlap the previous pair's FP64
-        // arithmetic
         const double ai = ST ? c.a_k[ti] : 0.0;
         double4 gci = make_double4(0, 0, 0, 0);
         if (ST) gci = gcpa[i];        // .w = PressureA
-        const int cnt = ncount[i];
-        const int* lp = nlist + i;
-        int j1 = cnt > 0 ? __ldg(lp) : i;
-        int j2 = cnt > 1 ? __ldg(lp + n) : i;
-        lp += 2 * n;
         constexpr bool TYPES = RATIO || !MU1;
-        XV pn = ld_xv(xv, j1);
-        int tn = TYPES ? __ldg(type + j1) : 0;
-        for (int k = 0; k < cnt; ++k) {
-            const int j = j1;
-            const XV pj = pn;
-            const int tj = tn;
-            j1 = j2;
-            if (k + 2 < cnt) j2 = __ldg(lp);
-            lp += n;
-            if (k + 1 < cnt) {
-                pn = ld_xv(xv, j1);
-                if (TYPES) tn = __ldg(type + j1);
-            }
-            if (j == i) continue;
+        walk_list(nlist + i, n, ncount[i],
+                  [&](int j) { return XVT{ld_xv(xv, j), TYPES ? __ldg(type + j) : 0}; },
+                  [&](int j, const XVT& rj) {
+            const XV& pj = rj.p;
+            const int tj = rj.t;
             double x[3];
             disp(c, pi, pj, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
@@ -507,11 +499,11 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
             const bool in_a = ST && (r2 < c.ra2);
             const bool in_g = ST && (r2 < c.rg2);
             const bool in_v = r2 < c.rv2;
-            if (!(in_a || in_g || in_v)) continue;
-            const double r = sqrt(r2);
-            const double ri = __drcp_rn(r);
-            const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-            const double qa = div_rs(r, c.ra, c.inv_ra);
+            double r;
+            Recip ri;
+            if (!pair_root(r2, in_a || in_g || in_v, j == i, r, ri)) return;
+            const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
+            const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
             double rij = 1.0, rji = 1.0;
             if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
             if (ST) {
@@ -527,13 +519,13 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
                 }
                 if (in_g) {
                     const double aj = ai;
-                    const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
                     const double wg = s_wg(c, qg);
                     const double wij = RATIO ? rij * wg : wg;
                     const double wji = RATIO ? rji * wg : wg;
-                    fd0 -= div_rs(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    fd1 -= div_rs(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    fd2 -= div_rs(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd0 -= div_q(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    fd1 -= div_q(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    fd2 -= div_q(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
                     const double dg = s_dwg(c, qg);
                     const double dwij = RATIO ? rij * dg : dg;
                     const double dwji = RATIO ? rji * dg : dg;
@@ -541,22 +533,22 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
                     gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
                     gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
                     gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
-                    fd0 -= div_rs((gr) * e0, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    fd1 -= div_rs((gr) * e1, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    fd2 -= div_rs((gr) * e2, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    fd0 -= div_q((gr) * e0, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    fd1 -= div_q((gr) * e1, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    fd2 -= div_q((gr) * e2, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
                 }
             }
             if (in_v) {
-                const double qv = c.rv_eq_ra ? qa : div_rs(r, c.rv, c.inv_rv);
+                const double qv = c.rv_eq_ra ? qa : div_q(r, c.rv, recip_const(c.inv_rv, c.inv_rv_lo));
                 const double dw = -s_dwv(c, qv);
                 const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
                 const double cm = MU1 ? c.visc_mu[0][0] : c.visc_mu[ti][tj];
                 const double dot = u0 * e0 + u1 * e1 + u2 * e2;
-                fv0 += div_rs(cm * dot * e0 * dw, r, ri) * c.vol;
-                fv1 += div_rs(cm * dot * e1 * dw, r, ri) * c.vol;
-                fv2 += div_rs(cm * dot * e2 * dw, r, ri) * c.vol;
+                fv0 += div_q(cm * dot * e0 * dw, r, ri) * c.vol;
+                fv1 += div_q(cm * dot * e1 * dw, r, ri) * c.vol;
+                fv2 += div_q(cm * dot * e2 * dw, r, ri) * c.vol;
             }
-        }
+        });
     }
     if (LRN) {
         float l0 = 0.f, l1 = 0.f, l2 = 0.f;
@@ -680,17 +672,18 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __rest
             const bool in_v = r2 < c.rv2;
             if (in_p || in_a || in_g || in_v) {
                 const int tj = __ldg(type + j);
-                const double r = sqrt(r2);
-                const double ri = __drcp_rn(r);
-                const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
-                const double qa = div_rs(r, c.ra, c.inv_ra);
+                double r;
+                Recip ri;
+                (void)pair_root(r2, true, false, r, ri);
+                const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
+                const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
                 double rij = 1.0, rji = 1.0;
                 if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
                 if (in_p) {
-                    const double qp = div_rs(r, c.rp, c.inv_rp);
+                    const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
                     const double dw = s_dwp(c, qp);
-                    const double gw0 = div_rs(dw * x[0], r, ri), gw1 = div_rs(dw * x[1], r, ri),
-                                 gw2 = div_rs(dw * x[2], r, ri);
+                    const double gw0 = div_q(dw * x[0], r, ri), gw1 = div_q(dw * x[1], r, ri),
+                                 gw2 = div_q(dw * x[2], r, ri);
                     const double ps = ppi + velp[j].w;
                     v[0] = ps * gw0 * c.vol;
                     v[1] = ps * gw1 * c.vol;
@@ -698,14 +691,14 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __rest
                     fl |= 1u;
                 }
                 if (in_v) {
-                    const double qv = c.rv_eq_ra ? qa : div_rs(r, c.rv, c.inv_rv);
+                    const double qv = c.rv_eq_ra ? qa : div_q(r, c.rv, recip_const(c.inv_rv, c.inv_rv_lo));
                     const double dw = -s_dwv(c, qv);
                     const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
                     const double cm = c.visc_mu[ti][tj];
                     const double dot = u0 * e0 + u1 * e1 + u2 * e2;
-                    v[3] = div_rs(cm * dot * e0 * dw, r, ri) * c.vol;
-                    v[4] = div_rs(cm * dot * e1 * dw, r, ri) * c.vol;
-                    v[5] = div_rs(cm * dot * e2 * dw, r, ri) * c.vol;
+                    v[3] = div_q(cm * dot * e0 * dw, r, ri) * c.vol;
+                    v[4] = div_q(cm * dot * e1 * dw, r, ri) * c.vol;
+                    v[5] = div_q(cm * dot * e2 * dw, r, ri) * c.vol;
                     fl |= 8u;
                 }
                 if (ST && in_a) {
@@ -721,13 +714,13 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __rest
                 if (ST && in_g) {
                     const double4 gcj = gcpa[j];
                     const double aj = ai;
-                    const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
                     const double wg = s_wg(c, qg);
                     const double wij = RATIO ? rij * wg : wg;
                     const double wji = RATIO ? rji * wg : wg;
-                    v[9 % NV] = div_rs(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    v[10 % NV] = div_rs(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    v[11 % NV] = div_rs(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    v[9 % NV] = div_q(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    v[10 % NV] = div_q(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    v[11 % NV] = div_q(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
                     const double dg = s_dwg(c, qg);
                     const double dwij = RATIO ? rij * dg : dg;
                     const double dwji = RATIO ? rji * dg : dg;
@@ -735,9 +728,9 @@ k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __rest
                     gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
                     gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
                     gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
-                    v[12 % NV] = div_rs((gr) * e0, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    v[13 % NV] = div_rs((gr) * e1, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
-                    v[14 % NV] = div_rs((gr) * e2, c.r2g, c.inv_r2g) * c.rg * c.vol_over_l0;
+                    v[12 % NV] = div_q((gr) * e0, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    v[13 % NV] = div_q((gr) * e1, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
+                    v[14 % NV] = div_q((gr) * e2, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
                     fl |= 4u;
                 }
             }
@@ -841,28 +834,29 @@ k_sweep_a_w(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
             const bool in_p = r2 <= c.rp2;
             const bool in_g = ST && (r2 <= c.rg2);
             if (in_a || in_p || in_g) {
-                const double r = sqrt(r2);
+                double r;
+                Recip ri;
+                (void)pair_root(r2, true, false, r, ri);
                 double ratio = 1.0;
                 if (RATIO) ratio = c.ratio[ti][__ldg(type + j)];
-                const double qa = div_rs(r, c.ra, c.inv_ra);
+                const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
                 if (in_a) {
                     v[0] = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
                     fl |= 1u;
                 }
                 if (ST && in_g) {
-                    const double qg = c.rg_eq_ra ? qa : div_rs(r, c.rg, c.inv_rg);
+                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
                     const double wgt = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
-                    v[5] = div_rs(x[0] * wgt, c.r2g, c.inv_r2g) * c.rg;
-                    v[6] = div_rs(x[1] * wgt, c.r2g, c.inv_r2g) * c.rg;
-                    v[7] = div_rs(x[2] * wgt, c.r2g, c.inv_r2g) * c.rg;
+                    v[5] = div_q(x[0] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                    v[6] = div_q(x[1] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                    v[7] = div_q(x[2] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
                     fl |= 4u;
                 }
                 if (in_p) {
-                    const double qp = div_rs(r, c.rp, c.inv_rp);
+                    const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
                     v[1] = s_wp(c, qp);
                     const double dw = s_dwp(c, qp);
-                    const double ri = __drcp_rn(r);
-                    const double e0 = div_rs(x[0], r, ri), e1 = div_rs(x[1], r, ri), e2 = div_rs(x[2], r, ri);
+                    const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
                     const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
                     v[2] = u0 * e0 * dw;
                     v[3] = u1 * e1 * dw;
@@ -916,12 +910,78 @@ k_sweep_a_w(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
     }
 }
 
-// Self-check of div_rn against the hardware IEEE division: operands with
-// random significands and exponents in [-40, 40], plus all-ones significands.
+// Self-check of div_rn, div_q and sqrt_recip against the hardware IEEE
+// operations: operands with random significands and exponents in [-40, 40],
+// all-ones significands, and the operands nearest to a wrong rounding.
+
+// Odd M in [2^53, 2^54) with M^2 = a 2^54 + k for a double a, k = 1 (mod 8): the
+// square roots nearest to the middle of two doubles.  2-adic Newton iteration for
+// 1/sqrt(k); each k has two such M.
+__device__ double hard_root(int k, int which) {
+    unsigned long long y = 1ull;
+    for (int it = 0; it < 8; ++it) y *= (3ull - (unsigned long long)(long long)k * y * y) >> 1;
+    unsigned long long m = (unsigned long long)(long long)k * y;  // sqrt(k)
+    if (which) m = 0ull - m;
+    m = (m & ((1ull << 53) - 1)) | (1ull << 53);
+    // a root modulo 2^54, or (that + 2^53) is one
+    if (((m * m - (unsigned long long)(long long)k) & ((1ull << 54) - 1)) != 0ull) m ^= 1ull << 53;
+    const unsigned long long lo = m * m, hi = __umul64hi(m, m);
+    const unsigned long long l2 = lo - (unsigned long long)(long long)k;
+    const unsigned long long h2 = hi - (k > 0 && lo < (unsigned long long)k) + (k < 0 && l2 < lo);
+    return (double)((h2 << 10) | (l2 >> 54));  // exact when the low bit allows, else a neighbour
+}
+
+// The x with |2^(j+1) x - T d| = 1 for an odd T in [2^53, 2^54): x/d nearest to the
+// middle of two doubles (0: there is none).
+__device__ double hard_numerator(unsigned long long d, int s, int j) {
+    unsigned long long inv = d;
+    for (int it = 0; it < 6; ++it) inv *= 2ull - d * inv;
+    unsigned long long t = s > 0 ? 0ull - inv : inv;
+    t &= (2ull << j) - 1;
+    if (j == 52) t |= 1ull << 53;
+    if (t < (1ull << 53)) return 0.0;
+    const unsigned long long lo = t * d, hi = __umul64hi(t, d);
+    const unsigned long long l2 = lo + (unsigned long long)(long long)s;
+    const unsigned long long h2 = hi + (s > 0 && l2 < lo) - (s < 0 && lo == 0ull);
+    const unsigned long long x = (h2 << (63 - j)) | (l2 >> (j + 1));
+    return x >= (1ull << 52) && x < (1ull << 53) ? (double)x : 0.0;
+}
+
 __global__ void k_check_division(unsigned long long seed, long long n, unsigned long long* mismatches,
                                  double* first) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += stride) {
+    auto same = [](double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); };
+    auto bad = [&](double x, double y) {
+        if (atomicAdd(mismatches, 1ull) == 0) { first[0] = x; first[1] = y; }
+    };
+    auto check = [&](double x, double y) {
+        const double h = __drcp_rn(y), ref = x / y;
+        if (!same(div_rn(x, y, h), ref)) bad(x, y);
+        if (!same(div_q(x, y, recip_const(h, __fma_rn(-y, h, 1.0) * h)), ref)) bad(x, y);
+    };
+    auto check_root = [&](double a, double x) {
+        double r;
+        Recip c;
+        if (plain_root(a)) sqrt_recip(a, r, c);
+        else sqrt_recip_any(a, r, c);
+        if (!same(r, sqrt(a))) bad(a, a);
+        if (!same(div_q(x, r, c), x / r)) bad(x, r);
+    };
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t0 < 40) {  // k = -79, -71, ..., 73, two roots each, and the doubles beside them
+        const double a = hard_root(-79 + 8 * (int)(t0 >> 1), (int)(t0 & 1));
+        for (int q = -4; q <= 4; ++q) check_root(a + q, 1.0 + q);
+    } else if (t0 >= 64 && t0 < 192) {  // divisors 2^53 - 1, - 3, ..., - 63
+        const int q = (int)t0 - 64;
+        const unsigned long long d = (1ull << 53) - 1 - 2 * (q >> 2);
+        const double x = hard_numerator(d, (q & 1) ? 1 : -1, (q & 2) ? 52 : 53);
+        if (x != 0.0) {
+            for (int e = -4; e <= 4; ++e) check(x + e, (double)d);
+            const double y = (double)d;  // the same through a square root's reciprocal
+            check_root(y * y, x);
+        }
+    }
+    for (long long t = t0; t < n; t += stride) {
         unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(t + 1);
         auto mix = [](unsigned long long v) {
             v ^= v >> 30; v *= 0xBF58476D1CE4E5B9ull;
@@ -936,11 +996,8 @@ __global__ void k_check_division(unsigned long long seed, long long n, unsigned 
         const unsigned long long sa = (e >> 40) & 1ull;
         const double x = __longlong_as_double((long long)((sa << 63) | ((unsigned long long)(1023 + ea) << 52) | ma));
         const double y = __longlong_as_double((long long)(((unsigned long long)(1023 + eb) << 52) | mb));
-        const double q = div_rn(x, y, __drcp_rn(y));
-        const double ref = x / y;
-        if (__double_as_longlong(q) != __double_as_longlong(ref)) {
-            if (atomicAdd(mismatches, 1ull) == 0) { first[0] = x; first[1] = y; }
-        }
+        check(x, y);
+        check_root(y, x);
     }
 }
 

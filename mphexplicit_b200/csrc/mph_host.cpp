@@ -295,7 +295,9 @@ int mph::make_simconst(const mph_params& p, const mph_grid_header& h, const mph_
         s.half_width[d] = 0.5 * c.domain_width[d];
         {
             const double q = 0.75 * c.domain_width[d];
-            std::memcpy(&s.q75_bits[d], &q, sizeof(q));
+            unsigned long long bits;
+            std::memcpy(&bits, &q, sizeof(q));
+            s.q75_hi[d] = (unsigned)(bits >> 32);
         }
         s.cell_width[d] = c.cell_width[d];
     }
@@ -336,6 +338,12 @@ int mph::make_simconst(const mph_params& p, const mph_grid_header& h, const mph_
     s.m2_rg = -2.0 / s.rg; s.m2_rp = -2.0 / s.rp; s.m2_rv = -2.0 / s.rv;
     s.visc_c = dim == 2 ? 8.0 : 10.0;
     s.inv_r2g = 1.0 / s.r2g;
+    auto rest = [](double h, double inv) { return std::fma(-h, inv, 1.0) * inv; };
+    s.inv_ra_lo = rest(s.ra, s.inv_ra);
+    s.inv_rg_lo = rest(s.rg, s.inv_rg);
+    s.inv_rp_lo = rest(s.rp, s.inv_rp);
+    s.inv_rv_lo = rest(s.rv, s.inv_rv);
+    s.inv_r2g_lo = rest(s.r2g, s.inv_r2g);
     s.rg_eq_ra = s.rg == s.ra;
     s.rv_eq_ra = s.rv == s.ra;
     for (int t = 0; t < MPH_TYPE_COUNT; ++t)

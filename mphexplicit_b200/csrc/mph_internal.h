@@ -26,10 +26,7 @@ struct SimConst {
     int ratio_all_one;     // InteractionRatio == 1 everywhere
     int mu_uniform;        // visc_mu is one number for every pair of types
     double dmin[3], width[3], half_width[3], cell_width[3];
-    // bits of 0.75*width: Mod(x, w) needs no division when 0 <= x < 0.75 w,
-    // tested as one unsigned compare of x's bit pattern (negative x, -0.0
-    // and NaN have the sign bit set and compare above every positive bound)
-    unsigned long long q75_bits[3];
+    unsigned q75_hi[3];  // high word of 0.75*width: Mod(x, w) needs no division when 0 <= x < 0.75 w
     double dt, l0, vol, vol_over_l0;
     double n0a, n0p, r2g, cof_k;
     double ra, rg, rp, rv;             // radii
@@ -41,6 +38,8 @@ struct SimConst {
     double m2_rg, m2_rp, m2_rv;        // -2.0/h
     double visc_c;                     // 8 (2-D) or 10 (3-D)
     double inv_r2g;                    // RN(1/R2g)
+    // what RN(1/h) lacks to 1/h, for the exact divisions by a constant (div_q)
+    double inv_ra_lo, inv_rg_lo, inv_rp_lo, inv_rv_lo, inv_r2g_lo;
     int rg_eq_ra, rv_eq_ra;            // radii equal: r/h shared
     int sweep_layout;                  // FP64 sweeps: 0 by size, 1 thread per particle, 2 warp per particle
     // visc_c * muij per type pair, muij = 2*(mu_i*mu_j)/(mu_i+mu_j) (main.cpp:1968)
