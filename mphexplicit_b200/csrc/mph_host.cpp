@@ -15,6 +15,7 @@
 #include <cstring>
 #include <exception>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include <algorithm>
 
@@ -344,6 +345,8 @@ int mph::make_simconst(const mph_params& p, const mph_grid_header& h, const mph_
     s.inv_rp_lo = rest(s.rp, s.inv_rp);
     s.inv_rv_lo = rest(s.rv, s.inv_rv);
     s.inv_r2g_lo = rest(s.r2g, s.inv_r2g);
+    s.inv_vol = 1.0 / s.vol;
+    s.inv_vol_lo = rest(s.vol, s.inv_vol);
     s.rg_eq_ra = s.rg == s.ra;
     s.rv_eq_ra = s.rv == s.ra;
     for (int t = 0; t < MPH_TYPE_COUNT; ++t)
@@ -401,10 +404,7 @@ static int dalloc(mph_ctx* ctx, T** ptr, size_t count) {
 }
 
 static void free_fp64(mph::DevFP64& d) {
-    void* ptrs[] = {d.pidx[0], d.pidx[1], d.type[0], d.type[1], d.pos[0], d.pos[1], d.vel[0], d.vel[1],
-                    d.xv, d.snap, d.pos32, d.force, d.dens_a, d.strain_p, d.div_p, d.press, d.gc, d.virial_p, d.keys,
-                    d.vals, d.cellstart, d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.wall_center, d.staging,
-                    d.scal};
+    void* ptrs[] = {d.slab, d.nlist, d.nlist_s};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     d = mph::DevFP64();
@@ -416,32 +416,48 @@ static void free_fp64(mph::DevFP64& d) {
         if (st_ != MPH_OK) return st_;  \
     } while (0)
 
+// The context's fixed arrays, cut from one allocation at 256-byte boundaries:
+// thirty small ones made and freed cost a short-lived context more than a
+// millisecond.
 static int alloc_fp64(mph_ctx* ctx) {
     mph::DevFP64& d = ctx->d;
     const size_t n = (size_t)ctx->n, P = (size_t)ctx->sc.pow2, tot = (size_t)ctx->sc.tot;
-    for (int k = 0; k < 2; ++k) {
-        TRY(dalloc(ctx, &d.pidx[k], n));
-        TRY(dalloc(ctx, &d.type[k], n));
-        TRY(dalloc(ctx, &d.pos[k], n));
-        TRY(dalloc(ctx, &d.vel[k], n));
+    const bool mixed = ctx->mode == MPH_MODE_MIXED || ctx->mode == MPH_MODE_MIXED_P64;
+    size_t used = 0;
+    auto take = [&](auto** ptr, size_t count) {
+        if (d.slab) *ptr = reinterpret_cast<std::remove_reference_t<decltype(*ptr)>>(d.slab + used);
+        used += (count * sizeof(**ptr) + 255) / 256 * 256;
+    };
+    for (int pass = 0; pass < 2; ++pass) {  // measure, allocate, cut
+        if (pass == 1) TRY(dalloc(ctx, &d.slab, used));
+        used = 0;
+        for (int k = 0; k < 2; ++k) {
+            take(&d.pidx[k], n);
+            take(&d.type[k], n);
+            take(&d.pos[k], n);
+            take(&d.vel[k], n);
+        }
+        if (!mixed) {
+            take(&d.xv, 3 * n);
+            take(&d.ncount_s, n);
+        }
+        take(&d.snap, n);
+        take(&d.pos32, n);
+        take(&d.force, n);
+        take(&d.dens_a, n);
+        take(&d.strain_p, n);
+        take(&d.div_p, n);
+        take(&d.press, n);
+        take(&d.gc, n);
+        take(&d.virial_p, n);
+        take(&d.keys, P);
+        take(&d.vals, P);
+        take(&d.cellstart, 2 * tot + 1);
+        take(&d.ncount, n);
+        take(&d.wall_center, 12);
+        take(&d.staging, 3 * n);
+        take(&d.scal, 1);
     }
-    if (ctx->mode == MPH_MODE_FP64 || ctx->mode == MPH_MODE_LEARNED) TRY(dalloc(ctx, &d.xv, 3 * n));
-    TRY(dalloc(ctx, &d.snap, n));
-    TRY(dalloc(ctx, &d.pos32, n));
-    TRY(dalloc(ctx, &d.force, n));
-    TRY(dalloc(ctx, &d.dens_a, n));
-    TRY(dalloc(ctx, &d.strain_p, n));
-    TRY(dalloc(ctx, &d.div_p, n));
-    TRY(dalloc(ctx, &d.press, n));
-    TRY(dalloc(ctx, &d.gc, n));
-    TRY(dalloc(ctx, &d.virial_p, n));
-    TRY(dalloc(ctx, &d.keys, P));
-    TRY(dalloc(ctx, &d.vals, P));
-    TRY(dalloc(ctx, &d.cellstart, 2 * tot + 1));
-    TRY(dalloc(ctx, &d.ncount, n));
-    TRY(dalloc(ctx, &d.wall_center, 12));
-    TRY(dalloc(ctx, &d.staging, 3 * n));
-    TRY(dalloc(ctx, &d.scal, 1));
     CUDA_TRY(ctx, cudaMemsetAsync(d.gc, 0, n * sizeof(double4), ctx->stream));
     CUDA_TRY(ctx, cudaMemsetAsync(d.force, 0, n * sizeof(double4), ctx->stream));
     CUDA_TRY(ctx, cudaMemsetAsync(d.virial_p, 0, n * sizeof(double), ctx->stream));
@@ -647,7 +663,6 @@ static int create_impl(mph_ctx* ctx, const int* type, const double* xyz, const d
         mph::mixed_set_cell_walk(ctx->mixed, ctx->cell_walk);
     } else {
         TRY(grow_list(ctx, initial_capacity(ctx, ctx->sc.rm2)));
-        TRY(dalloc(ctx, &d.ncount_s, n));
         TRY(grow_table(ctx, initial_capacity(ctx, ctx->sc.rs2), &d.nlist_s, &d.cap_s));
         TRY(rebuild_fp64(ctx));
         sweep_a(ctx, false);

@@ -40,6 +40,7 @@ struct SimConst {
     double inv_r2g;                    // RN(1/R2g)
     // what RN(1/h) lacks to 1/h, for the exact divisions by a constant (div_q)
     double inv_ra_lo, inv_rg_lo, inv_rp_lo, inv_rv_lo, inv_r2g_lo;
+    double inv_vol, inv_vol_lo;        // the same for the particle volume
     int rg_eq_ra, rv_eq_ra;            // radii equal: r/h shared
     int sweep_layout;                  // FP64 sweeps: 0 by size, 1 thread per particle, 2 warp per particle
     // visc_c * muij per type pair, muij = 2*(mu_i*mu_j)/(mu_i+mu_j) (main.cpp:1968)
@@ -76,6 +77,7 @@ enum : int {
 
 // Device buffers of the FP64 form.  Arrays are in cell-sorted order.
 struct DevFP64 {
+    char* slab = nullptr;                   // the one allocation of every array but the two lists
     int* pidx[2] = {nullptr, nullptr};
     int* type[2] = {nullptr, nullptr};
     double4* pos[2] = {nullptr, nullptr};   // x,y,z,(double)type
