@@ -521,8 +521,10 @@ int mph_learned_stats(mph_ctx* ctx, mph_learned_info* info);
  * integration.  All scenes of a batch have the same dimension; walls
  * must be static (zero Wall2/3 Velocity and Omega).  Scene s keeps its own
  * *.data parameters, domain and cell grid; a step advances every scene by its
- * own dt.  The sweeps are persistent kernels over (scene, cell tile) work
- * items; mph_batch_step replays steps as captured CUDA graphs of
+ * own dt.  The sweeps walk a neighbour table per particle where it fits in
+ * half of the free memory (0.3 KB a particle in 2-D, 1.3 KB in 3-D), else, or
+ * where a tile shape is asked for, they are persistent kernels over (scene, cell
+ * tile) work items; mph_batch_step replays steps as captured CUDA graphs of
  * MPH_BATCH_GRAPH_STEPS steps (the remainder as direct launches). */
 #define MPH_BATCH_GRAPH_STEPS 16
 typedef struct mph_batch mph_batch;
@@ -539,16 +541,18 @@ int mph_batch_synchronize(mph_batch* b);
  * mph_batch_create's xyz / vel). */
 int mph_batch_get_state(mph_batch* b, double* xyz, double* vel);
 /* Cell tile (tz ignored in 2-D), CTA size of the sweeps, and the resident CTAs
- * per SM their staging capacity is sized for (0: keep the current value). */
+ * per SM their staging capacity is sized for (0: keep the current value).  A tile
+ * of one cell selects the neighbour table, where there is one. */
 int mph_batch_set_tiles(mph_batch* b, int tx, int ty, int tz, int threads, int ctas_per_sm);
 typedef struct mph_batch_trial {
     int tile[3];
     int threads;
     int ctas_per_sm;   /* resident CTAs per SM the staging capacity is sized for */
-    int capacity;      /* particles a CTA stages (tile + halo) before splitting  */
+    int capacity;      /* particles a CTA stages (tile + halo) before splitting; */
+                       /* table: entries of a particle's list                    */
     double ms_per_step;
 } mph_batch_trial;
-/* Time every candidate tile shape, CTA size and staging capacity (sized for 2
+/* Time the table and every candidate tile shape, CTA size and staging capacity (sized for 2
  * to 4 resident CTAs per SM in 2-D, 1 or 2 in 3-D) on the batch itself for about
  * `steps` steps each, keep the fastest, and put the batch state back as it
  * was: the simulation does not advance.  trials[capacity] receives the

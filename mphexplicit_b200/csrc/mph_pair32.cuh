@@ -54,7 +54,7 @@ __device__ __forceinline__ void st_density(const K& m, int ti, int tj, float r2,
 // Surface-tension terms of one pair (PressureA, DiffuseInterface with aj the
 // a of i as the reference has it, main.cpp:1742-1828); returns the radial
 // part and adds the tangential part to t.
-template <bool RATIO, class K>
+template <bool RATIO, int DIM = 3, class K>
 __device__ __forceinline__ float st_terms(const K& m, int ti, int tj, float r2, float r, float rinv, float dx,
                                           float dy, float dz, const float4& gi, const float4& gj, float ai,
                                           float3& t) {
@@ -71,10 +71,12 @@ __device__ __forceinline__ float st_terms(const K& m, int ti, int tj, float r2, 
         const float k1 = m.inv_r2g_rg * m.vol_over_l0;
         t.x -= (ai * gj.x * rji * wg - ai * gi.x * rij * wg) * k1;
         t.y -= (ai * gj.y * rji * wg - ai * gi.y * rij * wg) * k1;
-        t.z -= (ai * gj.z * rji * wg - ai * gi.z * rij * wg) * k1;
-        const float gr = (ai * gj.x * rji * dwg - ai * gi.x * rij * dwg) * dx +
-                         (ai * gj.y * rji * dwg - ai * gi.y * rij * dwg) * dy +
-                         (ai * gj.z * rji * dwg - ai * gi.z * rij * dwg) * dz;
+        float gr = (ai * gj.x * rji * dwg - ai * gi.x * rij * dwg) * dx +
+                   (ai * gj.y * rji * dwg - ai * gi.y * rij * dwg) * dy;
+        if (DIM == 3) {  // in 2-D every z part is zero
+            t.z -= (ai * gj.z * rji * wg - ai * gi.z * rij * wg) * k1;
+            gr += (ai * gj.z * rji * dwg - ai * gi.z * rij * dwg) * dz;
+        }
         s -= gr * rinv * k1;
     }
     return s;
