@@ -277,7 +277,8 @@ k_sweep_a(SimConst c, const double2* __restrict__ xv, const int* __restrict__ ty
           const int* __restrict__ ncount, const int* __restrict__ nlist, const int* __restrict__ ncount_p,
           const int* __restrict__ nlist_p, double* __restrict__ dens_a,
           double* __restrict__ strain_p, double* __restrict__ div_p, double4* __restrict__ velp,
-          double4* __restrict__ gcpa, double* __restrict__ wall_center) {
+          double4* __restrict__ gcpa, double* __restrict__ wall_center, const StepScalars* __restrict__ skip) {
+    if (skip && skip->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
         // WallCenter += WallVelocity*Dt (main.cpp:2048-2052); the move kernel of
@@ -413,7 +414,9 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
           const double4* __restrict__ gcpa, const int* __restrict__ ncount, const int* __restrict__ nlist,
           const int* __restrict__ ncount_s, const int* __restrict__ nlist_s, double4* __restrict__ force,
           StepScalars* __restrict__ scal, const int* __restrict__ eoff, const float4* __restrict__ eforce,
-          float4* __restrict__ lsum, int part, int i0, int i1, double* __restrict__ vel_host) {
+          float4* __restrict__ lsum, int part, int i0, int i1, double* __restrict__ vel_host,
+          const StepScalars* __restrict__ skip) {
+    if (skip && skip->stop) return;
     const int i = i0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);  // particles [i0, i1)
     if (i >= i1) return;
     const int nf = cellstart[c.tot];
@@ -570,308 +573,148 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
     }
 }
 
-// ---- warp per particle (small scenes) ----------------------------------------
+// ---- G lanes per particle (small scenes) ---------------------------------------
 // With few particles the thread-per-particle sweeps leave most of the GPU idle
 // and each thread's chain of dependent FP64 work over its ~200 list entries
-// sets the time.  Here a warp takes one particle: its 32 lanes compute the
-// pair terms of 32 consecutive list entries at once (the expressions of
-// k_sweep_a / k_sweep_b), then one lane per sum adds the chunk's terms to it
-// in list order, each with the operation the thread kernels apply (+= or -=,
-// two in a row where they apply two): the same additions in the same order,
-// so the same bits.
-constexpr int kWarpSweepWarps = 4;
+// sets the time.  Here G lanes (4 to 32) take one particle: they compute the pair
+// terms of G consecutive list entries at once (the expressions of k_sweep_a /
+// k_sweep_b), stage them in shared memory, and one lane per sum adds them in list
+// order: the same additions in the same order, so the same bits.  An entry without
+// a term stages -0.0, which leaves any sum as it is (sums start at +0.0 and never
+// hold -0.0), and a subtracted term is staged negated (a - t is a + (-t)).
+constexpr int kGroupWarps = 4;
 
-// lane s's sum of k_sweep_b_w: flag bit, first term, second term (-1: none), subtract
-struct SumOp {
-    unsigned bit;
-    int q1, q2;
-    bool sub;
+// The warp's stage: NV terms of its 32 lanes' entries (rows one double apart from
+// a multiple of the banks, so the lanes that sum different terms do not collide).
+template <int NV>
+struct GroupStage {
+    double v[NV][33];
 };
-__device__ __forceinline__ SumOp sweep_b_sum(int s) {
-    // fp0..2 (+, bit 1), fv0..2 (+, bit 8), fa0..2 (+, bit 2), fd0..2 (-, -, bit 4)
-    if (s < 3) return {1u, s, -1, false};
-    if (s < 6) return {8u, s, -1, false};
-    if (s < 9) return {2u, s, -1, false};
-    return {4u, s, s + 3, true};
-}
 
-template <bool ST, bool RATIO>
-__global__ void __launch_bounds__(32 * kWarpSweepWarps)
-k_sweep_b_w(SimConst c, const int* __restrict__ cellstart, const double2* __restrict__ xv,
-            const int* __restrict__ type, const double4* __restrict__ velp, double4* __restrict__ vel_out,
-            const double4* __restrict__ gcpa,
-            const int* __restrict__ ncount, const int* __restrict__ nlist, double4* __restrict__ force,
-            StepScalars* __restrict__ scal, int part, double* __restrict__ vel_host) {
-    constexpr int NV = ST ? 15 : 6;  // terms per entry: fp 3, fv 3 [, fa 3, fd 3 + 3]
-    constexpr int NS = ST ? 12 : 6;  // sums
-    __shared__ double tv[kWarpSweepWarps][NV][33];
-    __shared__ unsigned tf[kWarpSweepWarps][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * kWarpSweepWarps + w;
-    if (i >= c.n) return;  // whole warp
-    const int nf = cellstart[c.tot];
-    const XV pi = ld_xv(xv, i);
-    if (part == 1 && i >= nf) {   // a wall keeps its velocity (see k_sweep_b)
-        if (lane == 0) {
-            vel_out[i] = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
-            if (vel_host) {
-                vel_host[3 * (size_t)i] = pi.b.y;
-                vel_host[3 * (size_t)i + 1] = pi.c.x;
-                vel_host[3 * (size_t)i + 2] = pi.c.y;
-            }
-        }
-        return;
-    }
-    if (part == 2 && i < nf) return;
-    const double ppi = velp[i].w;
-    const int ti = type[i];
-    const double ai = c.a_k[ti];
-    double4 gci = make_double4(0, 0, 0, 0);
-    if (ST) gci = gcpa[i];        // .w = PressureA
-    const int cnt = ncount[i];
-    const size_t n = (size_t)c.n;
-    const SumOp op = sweep_b_sum(lane < NS ? lane : 0);
-    double acc = 0.0;
-    for (int k0 = 0; k0 < cnt; k0 += 32) {
-        const int k = k0 + lane;
-        unsigned fl = 0u;
+// Walks the lists of the warp's particles, G entries of each per trip: lane sub of
+// a particle evaluates entry k0 + sub (eval(j, record, v), on -0.0 terms), then
+// add(stage, column of the particle's first entry) sums the G staged entries.
+// Indices are loaded two trips ahead and records one.
+template <int G, int NV, class Load, class Eval, class Add>
+__device__ __forceinline__ void group_walk(GroupStage<NV>& st, const int* __restrict__ lp, size_t n, int cnt, int self,
+                                           Load&& load, Eval&& eval, Add&& add) {
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    int ja = sub < cnt ? __ldg(lp + (size_t)sub * n) : self;
+    int jb = sub + G < cnt ? __ldg(lp + (size_t)(sub + G) * n) : self;
+    auto a = load(ja);
+    for (int k0 = 0; k0 < most; k0 += G) {
+        int jc = self;
+        if (k0 + 2 * G + sub < cnt) jc = __ldg(lp + (size_t)(k0 + 2 * G + sub) * n);
+        const auto b = load(jb);
         double v[NV];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) v[q] = 0.0;
-        const int j = k < cnt ? __ldg(nlist + (size_t)k * n + i) : i;
-        if (j != i) {
-            const XV pj = ld_xv(xv, j);
-            double x[3];
-            disp(c, pi, pj, x);
-            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-            const bool in_p = r2 < c.rp2;
-            const bool in_a = ST && (r2 < c.ra2);
-            const bool in_g = ST && (r2 < c.rg2);
-            const bool in_v = r2 < c.rv2;
-            if (in_p || in_a || in_g || in_v) {
-                const int tj = __ldg(type + j);
-                double r;
-                Recip ri;
-                (void)pair_root(r2, true, false, r, ri);
-                const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
-                const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
-                double rij = 1.0, rji = 1.0;
-                if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
-                if (in_p) {
-                    const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
-                    const double dw = s_dwp(c, qp);
-                    const double gw0 = div_q(dw * x[0], r, ri), gw1 = div_q(dw * x[1], r, ri),
-                                 gw2 = div_q(dw * x[2], r, ri);
-                    const double ps = ppi + velp[j].w;
-                    v[0] = ps * gw0 * c.vol;
-                    v[1] = ps * gw1 * c.vol;
-                    v[2] = ps * gw2 * c.vol;
-                    fl |= 1u;
-                }
-                if (in_v) {
-                    const double qv = c.rv_eq_ra ? qa : div_q(r, c.rv, recip_const(c.inv_rv, c.inv_rv_lo));
-                    const double dw = -s_dwv(c, qv);
-                    const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
-                    const double cm = c.visc_mu[ti][tj];
-                    const double dot = u0 * e0 + u1 * e1 + u2 * e2;
-                    v[3] = div_q(cm * dot * e0 * dw, r, ri) * c.vol;
-                    v[4] = div_q(cm * dot * e1 * dw, r, ri) * c.vol;
-                    v[5] = div_q(cm * dot * e2 * dw, r, ri) * c.vol;
-                    fl |= 8u;
-                }
-                if (ST && in_a) {
-                    const double dwa = s_dwa(c, qa);
-                    const double dwij = RATIO ? rij * dwa : dwa;
-                    const double dwji = RATIO ? rji * dwa : dwa;
-                    const double sa = gci.w * dwij + gcpa[j].w * dwji;
-                    v[6 % NV] = sa * e0 * c.vol;
-                    v[7 % NV] = sa * e1 * c.vol;
-                    v[8 % NV] = sa * e2 * c.vol;
-                    fl |= 2u;
-                }
-                if (ST && in_g) {
-                    const double4 gcj = gcpa[j];
-                    const double aj = ai;
-                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
-                    const double wg = s_wg(c, qg);
-                    const double wij = RATIO ? rij * wg : wg;
-                    const double wji = RATIO ? rji * wg : wg;
-                    v[9 % NV] = div_q(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    v[10 % NV] = div_q(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    v[11 % NV] = div_q(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    const double dg = s_dwg(c, qg);
-                    const double dwij = RATIO ? rij * dg : dg;
-                    const double dwji = RATIO ? rji * dg : dg;
-                    double gr = 0.0;
-                    gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
-                    gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
-                    gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
-                    v[12 % NV] = div_q((gr) * e0, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    v[13 % NV] = div_q((gr) * e1, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    v[14 % NV] = div_q((gr) * e2, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg * c.vol_over_l0;
-                    fl |= 4u;
-                }
-            }
-        }
+        for (int q = 0; q < NV; ++q) v[q] = -0.0;
+        if (k0 + sub < cnt) eval(ja, a, v);
 #pragma unroll
-        for (int q = 0; q < NV; ++q) tv[w][q][lane] = v[q];
-        tf[w][lane] = fl;
+        for (int q = 0; q < NV; ++q) st.v[q][lane] = v[q];
         __syncwarp();
-        const int m = min(32, cnt - k0);
-        if (lane < NS) {
-            // branch-free and the same for every lane: acc = (acc - a) - b, with
-            // a = -t, b = +0 for a += (acc + t, then - +0 changes nothing, -0
-            // included), a = t1, b = t2 for the two -=; an entry without the
-            // term keeps acc
-            const int q2 = op.q2 < 0 ? 0 : op.q2;
-#pragma unroll 4
-            for (int e = 0; e < m; ++e) {
-                const double t1 = tv[w][op.q1][e];
-                const double a = op.sub ? t1 : -t1;
-                const double b = op.sub ? tv[w][q2][e] : 0.0;
-                const double nx = (acc - a) - b;
-                acc = (tf[w][e] & op.bit) ? nx : acc;
-            }
-        }
+        add(lane - sub);
         __syncwarp();
-    }
-    double sums[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) sums[q] = q < NS ? __shfl_sync(0xffffffffu, acc, q) : 0.0;
-    if (lane != 0) return;
-    const double fp0 = sums[0], fp1 = sums[1], fp2 = sums[2];
-    const double fv0 = sums[3], fv1 = sums[4], fv2 = sums[5];
-    const double fa0 = sums[6], fa1 = sums[7], fa2 = sums[8];
-    const double fd0 = sums[9], fd1 = sums[10], fd2 = sums[11];
-    double F0 = 0.0, F1 = 0.0, F2 = 0.0;   // resetForce (main.cpp:1617-1628), as k_sweep_b
-    F0 += fp0; F1 += fp1; F2 += fp2;
-    F0 += fa0; F1 += fa1; F2 += fa2;
-    F0 += fd0; F1 += fd1; F2 += fd2;
-    F0 += fv0; F1 += fv1; F2 += fv2;
-    double4 vn = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
-    if (i < nf) {
-        const double m = c.density[ti] * c.vol;
-        F0 += m * c.gravity[0];
-        F1 += m * c.gravity[1];
-        F2 += m * c.gravity[2];
-        vn.x += F0 / m * c.dt;
-        vn.y += F1 / m * c.dt;
-        vn.z += F2 / m * c.dt;
-        if (!(isfinite(vn.x) && isfinite(vn.y) && isfinite(vn.z))) atomicOr(&scal->flags, DEVFLAG_NONFINITE);
-    }
-    force[i] = make_double4(F0, F1, F2, 0.0);
-    if (part != 2) {
-        vel_out[i] = vn;
-        if (vel_host) {
-            vel_host[3 * (size_t)i] = vn.x;
-            vel_host[3 * (size_t)i + 1] = vn.y;
-            vel_host[3 * (size_t)i + 2] = vn.z;
-        }
+        ja = jb;
+        jb = jc;
+        a = b;
     }
 }
 
-// Sweep A, warp per particle: sums DensityA (lane 0, bit 1), DensityP (lane 1,
-// bit 2), DivergenceP (lane 2, bit 2, three subtractions per entry) and
-// GravityCenter (lanes 3-5, bit 4), as k_sweep_a adds them.
-template <bool ST, bool RATIO>
-__global__ void __launch_bounds__(32 * kWarpSweepWarps)
-k_sweep_a_w(SimConst c, const double2* __restrict__ xv, const int* __restrict__ type,
-            const int* __restrict__ ncount, const int* __restrict__ nlist, double* __restrict__ dens_a,
+// Sweep A (see k_sweep_a), all particles.
+template <int G, bool ST, bool RATIO>
+__global__ void __launch_bounds__(32 * kGroupWarps)
+k_sweep_a_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ type,
+            const int* __restrict__ ncount, const int* __restrict__ nlist, const int* __restrict__ ncount_p,
+            const int* __restrict__ nlist_p, double* __restrict__ dens_a,
             double* __restrict__ strain_p, double* __restrict__ div_p, double4* __restrict__ velp,
-            double4* __restrict__ gcpa, double* __restrict__ wall_center) {
-    __shared__ double tv[kWarpSweepWarps][8][33];
-    __shared__ unsigned tf[kWarpSweepWarps][32];
+            double4* __restrict__ gcpa, double* __restrict__ wall_center, const StepScalars* __restrict__ skip) {
+    if (skip && skip->stop) return;
+    __shared__ GroupStage<4> stage[kGroupWarps];
     if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
         // WallCenter += WallVelocity*Dt (main.cpp:2048-2052), as k_sweep_a
         const int t = threadIdx.x / 3, d = threadIdx.x % 3;
         if (t >= 2) wall_center[3 * t + d] += c.wall_velocity[t][d] * c.dt;
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * kWarpSweepWarps + w;
-    if (i >= c.n) return;  // whole warp
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & (G - 1);
+    const int iw = (blockIdx.x * kGroupWarps + w) * (32 / G);
+    if (iw >= c.n) return;  // whole warp
+    const bool on = iw + lane / G < c.n;
+    const int i = on ? iw + lane / G : c.n - 1;
+    GroupStage<4>& st = stage[w];
     const XV pi = ld_xv(xv, i);
     const int ti = type[i];
-    const int cnt = ncount[i];
     const size_t n = (size_t)c.n;
-    // lane s's sum: 0 DensityA, 1 DensityP, 2 DivergenceP, 3-5 GravityCenter
-    const unsigned bit = lane == 0 ? 1u : (lane < 3 ? 2u : 4u);
-    double acc = 0.0;
-    for (int k0 = 0; k0 < cnt; k0 += 32) {
-        const int k = k0 + lane;
-        unsigned fl = 0u;
-        double v[8];
+    double acc = 0.0;  // lane 0: DensityP; lane 1: DivergenceP (three terms per entry)
+    group_walk<G, 4>(st, nlist_p + i, n, on ? ncount_p[i] : 0, i, [&](int j) { return ld_xv(xv, j); },
+                     [&](int j, const XV& pj, double* v) {
+        double x[3];
+        disp(c, pi, pj, x);
+        const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+        double r;
+        Recip ri;
+        if (!pair_root(r2, r2 <= c.rp2, j == i, r, ri)) return;
+        const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
+        v[0] = s_wp(c, qp);
+        const double dw = s_dwp(c, qp);
+        const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
+        const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
+        v[1] = -(u0 * e0 * dw);
+        v[2] = -(u1 * e1 * dw);
+        v[3] = -(u2 * e2 * dw);
+    }, [&](int col) {
+        if (sub < 2) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = 0.0;
-        const int j = k < cnt ? __ldg(nlist + (size_t)k * n + i) : i;
-        if (j != i) {
-            const XV pj = ld_xv(xv, j);
+            for (int e = 0; e < G; ++e) {
+                acc += st.v[sub][col + e];
+                if (sub == 1) {
+                    acc += st.v[2][col + e];
+                    acc += st.v[3][col + e];
+                }
+            }
+        }
+    });
+    const double sum_p = __shfl_sync(0xffffffffu, acc, lane - sub);
+    const double sum_d = __shfl_sync(0xffffffffu, acc, lane - sub + 1);
+    double sum_a = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
+    if (ST) {  // DensityA, GravityCenter: sum s on lane s
+        double as = 0.0;
+        group_walk<G, 4>(st, nlist + i, n, on ? ncount[i] : 0, i,
+                         [&](int j) { return XVT{ld_xv(xv, j), RATIO ? __ldg(type + j) : 0}; },
+                         [&](int j, const XVT& rj, double* v) {
             double x[3];
-            disp(c, pi, pj, x);
+            disp(c, pi, rj.p, x);
             const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-            const bool in_a = ST && (r2 <= c.ra2);
-            const bool in_p = r2 <= c.rp2;
-            const bool in_g = ST && (r2 <= c.rg2);
-            if (in_a || in_p || in_g) {
-                double r;
-                Recip ri;
-                (void)pair_root(r2, true, false, r, ri);
-                double ratio = 1.0;
-                if (RATIO) ratio = c.ratio[ti][__ldg(type + j)];
-                const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
-                if (in_a) {
-                    v[0] = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
-                    fl |= 1u;
-                }
-                if (ST && in_g) {
-                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
-                    const double wgt = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
-                    v[5] = div_q(x[0] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
-                    v[6] = div_q(x[1] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
-                    v[7] = div_q(x[2] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
-                    fl |= 4u;
-                }
-                if (in_p) {
-                    const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
-                    v[1] = s_wp(c, qp);
-                    const double dw = s_dwp(c, qp);
-                    const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
-                    const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
-                    v[2] = u0 * e0 * dw;
-                    v[3] = u1 * e1 * dw;
-                    v[4] = u2 * e2 * dw;
-                    fl |= 2u;
-                }
+            const bool in_a = r2 <= c.ra2;
+            const bool in_g = r2 <= c.rg2;
+            double r;
+            Recip ri;  // not used: its operations are not compiled
+            if (!pair_root(r2, in_a || in_g, j == i, r, ri)) return;
+            double ratio = 1.0;
+            if (RATIO) ratio = c.ratio[ti][rj.t];
+            const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
+            if (in_a) v[0] = RATIO ? ratio * s_wa(c, qa) : s_wa(c, qa);
+            if (in_g) {
+                const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
+                const double wgt = RATIO ? ratio * s_wg(c, qg) : s_wg(c, qg);
+                v[1] = div_q(x[0] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                v[2] = div_q(x[1] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
+                v[3] = div_q(x[2] * wgt, c.r2g, recip_const(c.inv_r2g, c.inv_r2g_lo)) * c.rg;
             }
-        }
+        }, [&](int col) {
+            if (sub < 4) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) tv[w][q][lane] = v[q];
-        tf[w][lane] = fl;
-        __syncwarp();
-        const int m = min(32, cnt - k0);
-        if (lane < 6) {
-            // as in k_sweep_b_w: acc = ((acc - a) - b) - c, a = -t, b = c = +0
-            // for a +=, the three DivergenceP terms for lane 2's three -=
-            const int q = lane < 2 ? lane : (lane == 2 ? 2 : lane + 2);
-            const bool sub = lane == 2;
-#pragma unroll 4
-            for (int e = 0; e < m; ++e) {
-                const double t = tv[w][q][e];
-                const double a = sub ? t : -t;
-                const double b = sub ? tv[w][3][e] : 0.0;
-                const double c3 = sub ? tv[w][4][e] : 0.0;
-                const double nx = ((acc - a) - b) - c3;
-                acc = (tf[w][e] & bit) ? nx : acc;
+                for (int e = 0; e < G; ++e) as += st.v[sub][col + e];
             }
-        }
-        __syncwarp();
+        });
+        const int l0 = lane - sub;
+        sum_a = __shfl_sync(0xffffffffu, as, l0);
+        g0 = __shfl_sync(0xffffffffu, as, l0 + 1);
+        g1 = __shfl_sync(0xffffffffu, as, l0 + 2);
+        g2 = __shfl_sync(0xffffffffu, as, l0 + 3);
     }
-    const double sum_a = __shfl_sync(0xffffffffu, acc, 0);
-    const double sum_p = __shfl_sync(0xffffffffu, acc, 1);
-    const double sum_d = __shfl_sync(0xffffffffu, acc, 2);
-    const double g0 = __shfl_sync(0xffffffffu, acc, 3);
-    const double g1 = __shfl_sync(0xffffffffu, acc, 4);
-    const double g2 = __shfl_sync(0xffffffffu, acc, 5);
-    if (lane != 0) return;
+    if (sub != 0 || !on) return;
     if (ST) dens_a[i] = sum_a;
     const double strain = sum_p - c.n0p;
     strain_p[i] = strain;
@@ -886,6 +729,181 @@ k_sweep_a_w(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
         if (c.n0a <= sum_a) pa = 0.0;
         gcpa[i] = make_double4(g0, g1, g2, pa);
     }
+}
+
+// Force sweep (see k_sweep_b) of the particles [i0, i1); with walls, the walls
+// [i1, n) keep their velocity in the blocks behind.
+template <int G, bool ST, bool RATIO>
+__global__ void __launch_bounds__(32 * kGroupWarps)
+k_sweep_b_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ type,
+            const double4* __restrict__ velp, double4* __restrict__ vel_out,
+            const double4* __restrict__ gcpa, const int* __restrict__ ncount, const int* __restrict__ nlist,
+            const int* __restrict__ ncount_s, const int* __restrict__ nlist_s, double4* __restrict__ force,
+            StepScalars* __restrict__ scal, int i0, int i1, int group_blocks, double* __restrict__ vel_host,
+            const StepScalars* __restrict__ skip) {
+    if (skip && skip->stop) return;
+    constexpr int NV = ST ? 12 : 3, NS = ST ? 9 : 3;  // terms; sums: fv, fa, fd (two terms each)
+    constexpr int PER = (NS + G - 1) / G;             // sums per lane
+    __shared__ GroupStage<NV> stage[kGroupWarps];
+    auto put_velocity = [&](int i, double x, double y, double z) {
+        vel_out[i] = make_double4(x, y, z, 0.0);
+        if (vel_host) {  // mapped pinned host memory: the read-back travels while the sweep runs
+            vel_host[3 * (size_t)i] = x;
+            vel_host[3 * (size_t)i + 1] = y;
+            vel_host[3 * (size_t)i + 2] = z;
+        }
+    };
+    if ((int)blockIdx.x >= group_blocks) {  // walls
+        const int i = i1 + ((int)blockIdx.x - group_blocks) * 32 * kGroupWarps + (int)threadIdx.x;
+        if (i >= c.n) return;
+        const XV p = ld_xv(xv, i);
+        put_velocity(i, p.b.y, p.c.x, p.c.y);
+        return;
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & (G - 1);
+    const int iw = i0 + (blockIdx.x * kGroupWarps + w) * (32 / G);
+    if (iw >= i1) return;  // whole warp
+    const bool on = iw + lane / G < i1;
+    const int i = on ? iw + lane / G : i1 - 1;
+    GroupStage<NV>& st = stage[w];
+    const XV pi = ld_xv(xv, i);
+    const int ti = type[i];
+    const size_t n = (size_t)c.n;
+    double fp = 0.0;  // lane s: component s
+    {  // PressureP over the short sublist
+        const double ppi = velp[i].w;
+        GroupStage<3>& sp = reinterpret_cast<GroupStage<3>&>(st);
+        group_walk<G, 3>(sp, nlist_s + i, n, on ? ncount_s[i] : 0, i,
+                         [&](int j) { return XVP{ld_xv(xv, j), __ldg(&velp[j].w)}; },
+                         [&](int j, const XVP& rj, double* v) {
+            double x[3];
+            disp(c, pi, rj.p, x);
+            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            double r;
+            Recip ri;
+            if (!pair_root(r2, r2 < c.rp2, j == i, r, ri)) return;
+            const double qp = div_q(r, c.rp, recip_const(c.inv_rp, c.inv_rp_lo));
+            const double dw = s_dwp(c, qp);
+            const double gw0 = div_q(dw * x[0], r, ri), gw1 = div_q(dw * x[1], r, ri),
+                         gw2 = div_q(dw * x[2], r, ri);
+            const double ps = ppi + rj.pressure;
+            v[0] = ps * gw0 * c.vol;
+            v[1] = ps * gw1 * c.vol;
+            v[2] = ps * gw2 * c.vol;
+        }, [&](int col) {
+            if (sub < 3) {
+#pragma unroll
+                for (int e = 0; e < G; ++e) fp += sp.v[sub][col + e];
+            }
+        });
+    }
+    double fs[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) fs[q] = 0.0;
+    {
+        const double ai = ST ? c.a_k[ti] : 0.0;
+        double4 gci = make_double4(0, 0, 0, 0);
+        if (ST) gci = gcpa[i];        // .w = PressureA
+        group_walk<G, NV>(st, nlist + i, n, on ? ncount[i] : 0, i,
+                          [&](int j) { return XVT{ld_xv(xv, j), __ldg(type + j)}; },
+                          [&](int j, const XVT& rj, double* v) {
+            const XV& pj = rj.p;
+            const int tj = rj.t;
+            double x[3];
+            disp(c, pi, pj, x);
+            const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+            const bool in_a = ST && (r2 < c.ra2);
+            const bool in_g = ST && (r2 < c.rg2);
+            const bool in_v = r2 < c.rv2;
+            double r;
+            Recip ri;
+            if (!pair_root(r2, in_a || in_g || in_v, j == i, r, ri)) return;
+            const double e0 = div_q(x[0], r, ri), e1 = div_q(x[1], r, ri), e2 = div_q(x[2], r, ri);
+            const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
+            double rij = 1.0, rji = 1.0;
+            if (RATIO) { rij = c.ratio[ti][tj]; rji = c.ratio[tj][ti]; }
+            if (in_v) {
+                const double qv = c.rv_eq_ra ? qa : div_q(r, c.rv, recip_const(c.inv_rv, c.inv_rv_lo));
+                const double dw = -s_dwv(c, qv);
+                const double u0 = pj.b.y - pi.b.y, u1 = pj.c.x - pi.c.x, u2 = pj.c.y - pi.c.y;
+                const double cm = c.visc_mu[ti][tj];
+                const double dot = u0 * e0 + u1 * e1 + u2 * e2;
+                v[0] = div_q(cm * dot * e0 * dw, r, ri) * c.vol;
+                v[1] = div_q(cm * dot * e1 * dw, r, ri) * c.vol;
+                v[2] = div_q(cm * dot * e2 * dw, r, ri) * c.vol;
+            }
+            if (ST) {
+                const double4 gcj = ld_d4(gcpa, j);  // .w = PressureA
+                if (in_a) {
+                    const double dwa = s_dwa(c, qa);
+                    const double dwij = RATIO ? rij * dwa : dwa;
+                    const double dwji = RATIO ? rji * dwa : dwa;
+                    const double sa = gci.w * dwij + gcj.w * dwji;
+                    v[3 % NV] = sa * e0 * c.vol;
+                    v[4 % NV] = sa * e1 * c.vol;
+                    v[5 % NV] = sa * e2 * c.vol;
+                }
+                if (in_g) {
+                    const Recip ir2g = recip_const(c.inv_r2g, c.inv_r2g_lo);
+                    const double aj = ai;
+                    const double qg = c.rg_eq_ra ? qa : div_q(r, c.rg, recip_const(c.inv_rg, c.inv_rg_lo));
+                    const double wg = s_wg(c, qg);
+                    const double wij = RATIO ? rij * wg : wg;
+                    const double wji = RATIO ? rji * wg : wg;
+                    v[6 % NV] = -(div_q(aj * gcj.x * wji - ai * gci.x * wij, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                    v[7 % NV] = -(div_q(aj * gcj.y * wji - ai * gci.y * wij, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                    v[8 % NV] = -(div_q(aj * gcj.z * wji - ai * gci.z * wij, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                    const double dg = s_dwg(c, qg);
+                    const double dwij = RATIO ? rij * dg : dg;
+                    const double dwji = RATIO ? rji * dg : dg;
+                    double gr = 0.0;
+                    gr += (aj * gcj.x * dwji - ai * gci.x * dwij) * x[0];
+                    gr += (aj * gcj.y * dwji - ai * gci.y * dwij) * x[1];
+                    gr += (aj * gcj.z * dwji - ai * gci.z * dwij) * x[2];
+                    v[9 % NV] = -(div_q((gr) * e0, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                    v[10 % NV] = -(div_q((gr) * e1, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                    v[11 % NV] = -(div_q((gr) * e2, c.r2g, ir2g) * c.rg * c.vol_over_l0);
+                }
+            }
+        }, [&](int col) {
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int s_ = sub + q * G;
+                if (s_ < NS) {
+#pragma unroll
+                    for (int e = 0; e < G; ++e) {
+                        fs[q] += st.v[s_][col + e];
+                        if (ST && s_ >= 6) fs[q] += st.v[(s_ + 3) % NV][col + e];
+                    }
+                }
+            }
+        });
+    }
+    const int l0 = lane - sub;
+    double S[9], P[3];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) S[q] = q < NS ? __shfl_sync(0xffffffffu, fs[(q / G) % PER], l0 + q % G) : 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) P[q] = __shfl_sync(0xffffffffu, fp, l0 + q);
+    if (sub != 0 || !on) return;
+    double F0 = 0.0, F1 = 0.0, F2 = 0.0;   // resetForce (main.cpp:1617-1628), as k_sweep_b
+    F0 += P[0]; F1 += P[1]; F2 += P[2];
+    F0 += S[3]; F1 += S[4]; F2 += S[5];
+    F0 += S[6]; F1 += S[7]; F2 += S[8];
+    F0 += S[0]; F1 += S[1]; F2 += S[2];
+    double4 vn = make_double4(pi.b.y, pi.c.x, pi.c.y, 0.0);
+    if (i < c.nf) {
+        const double m = c.density[ti] * c.vol;
+        F0 += m * c.gravity[0];
+        F1 += m * c.gravity[1];
+        F2 += m * c.gravity[2];
+        vn.x += F0 / m * c.dt;
+        vn.y += F1 / m * c.dt;
+        vn.z += F2 / m * c.dt;
+        if (!(isfinite(vn.x) && isfinite(vn.y) && isfinite(vn.z))) atomicOr(&scal->flags, DEVFLAG_NONFINITE);
+    }
+    force[i] = make_double4(F0, F1, F2, 0.0);
+    if (vel_out) put_velocity(i, vn.x, vn.y, vn.z);
 }
 
 // Self-check of div_rn, div_q and sqrt_recip against the hardware IEEE
@@ -1104,22 +1122,32 @@ k_conserved(SimConst c, const int* __restrict__ cellstart, const double4* __rest
 
 inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 
-// Small scenes take the warp-per-particle sweeps: below these sizes the
-// thread-per-particle sweeps leave most of the GPU idle.  Set by measurement
-// (sweep A + force sweep, one B200): 3-D dam breaks 0.065 ms (warp) against
-// 0.125 ms (thread) at 21,924 particles, 0.27 against 0.14 ms at 111,096;
-// 2-D droplets with surface tension 0.073 against 0.096 ms at 10,000, 0.52
-// against 0.36 ms at 40,000.  The ordered sums run on a few lanes of each
-// warp, so at scale the thread kernels win.
-#ifndef MPH_WARP_SWEEP_MAX_N
-#define MPH_WARP_SWEEP_MAX_N 40000
-#endif
-#ifndef MPH_WARP_SWEEP_MAX_N_2D
-#define MPH_WARP_SWEEP_MAX_N_2D 20000
-#endif
-inline bool use_warp_sweeps(const SimConst& c) {
-    if (c.sweep_layout != 0) return c.sweep_layout == 2;
-    return c.n <= (c.dim == 2 ? MPH_WARP_SWEEP_MAX_N_2D : MPH_WARP_SWEEP_MAX_N);
+// Lanes per particle of a sweep over m particles (1: the thread-per-particle
+// kernels): enough threads to fill the GPU, and no more, since every lane added
+// splits the list finer and adds the ordered sums' trips.  Set by measurement
+// (sweep A / force sweep in us at 1, 4, 8, 16, 32 lanes; long: lists of ~190
+// entries, 3-D whole lists; short: ~40 and fewer, 2-D, and sweep A without surface
+// tension):
+//   long, force sweep, 2,736 fluid     70 / 27 / 20 / 17 / 18
+//                      6,400           70 / 29 / 23 / 29 / 29
+//                     16,940           76 / 45 / 42 / 48 / 56
+//                     43,200           93 / 82 / 88 / 106 / 130
+//                    102,400          171 / 183 / 200 / 245 / 293
+//   long, surface tension, 4,096      136 / 52 / 35 / 29 / 31
+//                         39,304      178 / 171 / 172 / 177 / 215
+//                        110,592      365 / 416 / 463 / 500 / 638
+//   short, 2-D force sweep, 1,600      37 / 19 / 15 / 13 / 13
+//                          10,000      39 / 22 / 23 / 25 / 35
+//                          22,500      42 / 35 / 37 / 42 / 65
+//                          48,400      49 / 56 / 66 / 80 / 130
+//   short, sweep A, 14,724             18 / 14 / 13 / 15 / 16
+//                   26,128             18 / 14 / 15 / 18 / 22
+//                   52,724             18 / 19 / 21 / 27 / 35
+inline int group_lanes(const SimConst& c, int m, bool long_lists) {
+    if (c.sweep_layout == 1) return 1;
+    if (c.sweep_layout == 2) return 32;
+    if (long_lists) return m <= 2000 ? 32 : m <= 4500 ? 16 : m <= 20000 ? 8 : m <= 60000 ? 4 : 1;
+    return m <= 6000 ? 16 : m <= 16000 ? 8 : m <= 35000 ? 4 : 1;
 }
 
 // ---- learned form ----------------------------------------------------------
@@ -1330,25 +1358,34 @@ void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, do
 
 void launch_sweep_a(const SimConst& c, const double2* xv, const int* type, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double* dens_a, double* strain_p, double* div_p,
-                    double4* press, double4* gc, double* wall_center, cudaStream_t s) {
-    const bool warp = use_warp_sweeps(c);
-    const int nb = blocks(c.n, warp ? kWarpSweepWarps : 128);
-    // the warp kernel walks one list: with surface tension the whole one,
-    // without the short sublist
-    const int* cw = c.has_st ? ncount : ncount_s;
-    const int* lw = c.has_st ? nlist : nlist_s;
-#define SWEEP_A(ST, RATIO)                                                                                          \
-    if (warp)                                                                                                       \
-        k_sweep_a_w<ST, RATIO><<<nb, 32 * kWarpSweepWarps, 0, s>>>(c, xv, type, cw, lw, dens_a, strain_p, div_p,    \
-                                                                   press, gc, wall_center);                         \
-    else                                                                                                            \
-        k_sweep_a<ST, RATIO><<<nb, 128, 0, s>>>(c, xv, type, ncount, nlist, ncount_s, nlist_s, dens_a, strain_p,    \
-                                                div_p, press, gc, wall_center)
-    if (c.has_st) {
-        if (c.ratio_all_one) SWEEP_A(true, false); else SWEEP_A(true, true);
-    } else {
-        SWEEP_A(false, false);  // the ratios weigh surface-tension sums alone
+                    double4* press, double4* gc, double* wall_center, cudaStream_t s, const StepScalars* skip) {
+    const int g = group_lanes(c, c.n, c.dim == 3 && c.has_st);
+    if (g > 1) {
+        const int nb = blocks(c.n, kGroupWarps * (32 / g));
+#define SWEEP_AG(G, ST, RATIO)                                                                                    \
+    k_sweep_a_g<G, ST, RATIO><<<nb, 32 * kGroupWarps, 0, s>>>(c, xv, type, ncount, nlist, ncount_s, nlist_s, dens_a, \
+                                                              strain_p, div_p, press, gc, wall_center, skip)
+#define SWEEP_AG2(G)                                  \
+    if (!c.has_st) SWEEP_AG(G, false, false);         \
+    else if (c.ratio_all_one) SWEEP_AG(G, true, false); \
+    else SWEEP_AG(G, true, true)
+        switch (g) {
+            case 4: SWEEP_AG2(4); break;
+            case 8: SWEEP_AG2(8); break;
+            case 16: SWEEP_AG2(16); break;
+            default: SWEEP_AG2(32);
+        }
+#undef SWEEP_AG2
+#undef SWEEP_AG
+        return;
     }
+    const int nb = blocks(c.n, 128);
+#define SWEEP_A(ST, RATIO)                                                                                      \
+    k_sweep_a<ST, RATIO><<<nb, 128, 0, s>>>(c, xv, type, ncount, nlist, ncount_s, nlist_s, dens_a, strain_p,    \
+                                            div_p, press, gc, wall_center, skip)
+    if (!c.has_st) SWEEP_A(false, false);  // the ratios weigh surface-tension sums alone
+    else if (c.ratio_all_one) SWEEP_A(true, false);
+    else SWEEP_A(true, true);
 #undef SWEEP_A
 }
 
@@ -1365,27 +1402,41 @@ void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, 
                     const double4* press, const double4* gc, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
                     const int* eoff, const float4* eforce, float4* lsum, int part, int i0, int i1,
-                    double* vel_host) {
+                    double* vel_host, const StepScalars* skip) {
     if (i1 < 0) i1 = c.n;
     if (i1 <= i0) return;
     // the ratios weigh surface-tension terms alone
     const bool ratio = c.has_st && !c.ratio_all_one;
-    if (!eforce && i0 == 0 && i1 == c.n && use_warp_sweeps(c)) {
-        const int nw = blocks(c.n, kWarpSweepWarps);
-#define SWEEP_BW(ST, RATIO)                                                                                       \
-    k_sweep_b_w<ST, RATIO><<<nw, 32 * kWarpSweepWarps, 0, s>>>(c, cellstart, xv, type, press, vel_out, gc, ncount, \
-                                                              nlist, force, scal, part, vel_host)
-        if (!c.has_st) SWEEP_BW(false, false);
-        else if (!ratio) SWEEP_BW(true, false);
-        else SWEEP_BW(true, true);
-#undef SWEEP_BW
+    // the particles whose pairs this launch evaluates
+    const int b0 = part == 2 ? c.nf : 0, b1 = part == 1 ? c.nf : c.n;
+    const int g = !eforce && i0 == 0 && i1 == c.n ? group_lanes(c, b1 - b0, c.dim == 3) : 1;
+    if (g > 1) {
+        const int gb = blocks(b1 - b0, kGroupWarps * (32 / g));
+        const int nw = gb + (part == 1 ? blocks(c.n - c.nf, 32 * kGroupWarps) : 0);
+        if (nw == 0) return;
+#define SWEEP_BG(G, ST, RATIO)                                                                                    \
+    k_sweep_b_g<G, ST, RATIO><<<nw, 32 * kGroupWarps, 0, s>>>(c, xv, type, press, part == 2 ? nullptr : vel_out, gc, \
+                                                              ncount, nlist, ncount_s, nlist_s, force, scal, b0, b1, \
+                                                              gb, vel_host, skip)
+#define SWEEP_BG2(G)                                  \
+    if (!c.has_st) SWEEP_BG(G, false, false);         \
+    else if (!ratio) SWEEP_BG(G, true, false);        \
+    else SWEEP_BG(G, true, true)
+        switch (g) {
+            case 4: SWEEP_BG2(4); break;
+            case 8: SWEEP_BG2(8); break;
+            case 16: SWEEP_BG2(16); break;
+            default: SWEEP_BG2(32);
+        }
+#undef SWEEP_BG2
+#undef SWEEP_BG
         return;
     }
     const int nb = blocks(i1 - i0, 128);
 #define SWEEP_B(ST, RATIO, LRN, MU1)                                                                             \
     k_sweep_b<ST, RATIO, LRN, MU1><<<nb, 128, 0, s>>>(c, cellstart, xv, type, press, vel_out, gc, ncount, nlist, \
                                                       ncount_s, nlist_s, force, scal, eoff, eforce, lsum, part,  \
-                                                      i0, i1, vel_host)
+                                                      i0, i1, vel_host, skip)
     if (eforce) SWEEP_B(false, false, true, true);
     else if (!c.has_st) { if (c.mu_uniform) SWEEP_B(false, false, false, true); else SWEEP_B(false, false, false, false); }
     else if (ratio) SWEEP_B(true, true, false, false);

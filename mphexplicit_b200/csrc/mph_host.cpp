@@ -389,6 +389,7 @@ static int fill_simconst(mph_ctx* ctx) {
     std::string msg;
     const int st = mph::make_simconst(ctx->p, ctx->h, ctx->c, ctx->dim, ctx->n, ctx->sc, msg);
     if (st != MPH_OK) return fail(ctx, st, msg);
+    ctx->sc.nf = ctx->n_fluid;
     return MPH_OK;
 }
 

@@ -17,6 +17,7 @@ namespace mph {
 // ca = (1/Swa)/h^D and q = r/h.
 struct SimConst {
     int n;                 // particle count
+    int nf;                // fluid particles (sorted first)
     int dim;
     int tot;               // TotalCellCount
     int cc[3];             // CellCount
@@ -159,9 +160,11 @@ void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4*
                  const double4* snap, const double* wall_center, StepScalars* scal, cudaStream_t s);
 // Sweep A's DensityP and DivergenceP visit the short sublist (ncount_s,
 // nlist_s); with surface tension DensityA and GravityCenter the whole list.
+// skip: the sweep does nothing when skip->stop is set (step graphs)
 void launch_sweep_a(const SimConst& c, const double2* xv, const int* type, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double* dens_a, double* strain_p, double* div_p,
-                    double4* press, double4* gc, double* wall_center, cudaStream_t s);
+                    double4* press, double4* gc, double* wall_center, cudaStream_t s,
+                    const StepScalars* skip = nullptr);
 // DensityA and PressureA alone (into dens_a and gc[].w), in k_sweep_a's
 // order: what sweep A leaves out when there is no surface tension.
 void launch_density_a(const SimConst& c, const double4* pos, const int* ncount, const int* nlist, double* dens_a,
@@ -182,7 +185,8 @@ void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, 
                     const double4* press, const double4* gc, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
                     const int* eoff = nullptr, const float4* eforce = nullptr, float4* lsum = nullptr,
-                    int part = 0, int i0 = 0, int i1 = -1, double* vel_host = nullptr);
+                    int part = 0, int i0 = 0, int i1 = -1, double* vel_host = nullptr,
+                    const StepScalars* skip = nullptr);
 
 // ---- learned form (k_fp64.cu) ---------------------------------------------
 // CSR edges of the fluid particles' lists (i < nf): eoff[0..nf] = exclusive
