@@ -65,18 +65,16 @@ struct LearnedState {
     mph_learned_info info{};
 };
 
-// mph_step in the FP64 form for more than one step: one executable graph per
-// parity of the velocity ping-pong, replayed once per step, whose conditional
-// nodes take the host's per-step decisions (the rebuild test, made by the
-// move kernel's last block, and the table check); made for the buffers and
-// table capacities they were captured with.
-struct StepGraphs {
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};  // by the vcur of the step
-    int cur = -1, cap = -1, cap_s = -1;
-    const int* nlist = nullptr;
-    const int* nlist_s = nullptr;
-    int launches_step = 0, launches_rebuild = 0;  // kernels per step and per rebuild
-    bool enabled = true;  // mph_set_step_graphs
+// mph_step in the FP64 form for more than one step: batches of steps launched
+// ahead of the host, which reads how far they got; the kernels of a step whose
+// rebuild test fired, and of every later one, do nothing (StepScalars::stop).
+struct Ahead {
+    bool enabled = true;             // mph_set_step_graphs
+    StepScalars* seen = nullptr;     // pinned [2]: the counters after each batch in flight
+    cudaEvent_t ev[2] = {};          // ... and when they are there
+    int counted = 0;                 // StepScalars::steps_done accounted for so far
+    int since = 0;                   // steps since the last rebuild
+    double shift2 = 0.0;             // largest displacement squared since then
 };
 
 // mph_step_read_state: the copy stream (packs and device-to-host copies), its
@@ -111,7 +109,7 @@ struct mph_ctx {
     int max_neighbors = 0;
     long long launches = 0;
     ReadBack rb;
-    StepGraphs sg;
+    Ahead ahead;
     Profiler prof;
     std::string err;
     mph::TextWriter* text = nullptr;  // *.prof / *.vtk writer thread, made by the first write
@@ -513,6 +511,8 @@ static int rebuild_fp64(mph_ctx* ctx) {
     }
     d.cur = b;
     d.vcur = vb;
+    ctx->ahead.since = 0;
+    ctx->ahead.shift2 = 0.0;
     return build_lists(ctx);
 }
 
@@ -551,12 +551,12 @@ static int build_lists(mph_ctx* ctx) {
     return MPH_OK;
 }
 
-static void sweep_a(mph_ctx* ctx, bool advance_wall) {
+static void sweep_a(mph_ctx* ctx, bool advance_wall, bool skip = false) {
     mph::DevFP64& d = ctx->d;
     Launch L(ctx, "sweep_a");
     mph::launch_sweep_a(ctx->sc, d.xv, d.type[d.cur], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
                         d.dens_a, d.strain_p, d.div_p, d.press, d.gc, advance_wall ? d.wall_center : nullptr,
-                        ctx->stream);
+                        ctx->stream, skip ? d.scal : nullptr);
     ctx->dens_a_valid = ctx->sc.has_st;  // without surface tension, computed when read
     ctx->lazy_pos = -1;                  // this step's positions are the current ones
 }
@@ -629,8 +629,9 @@ extern "C" void mph_destroy(mph_ctx* ctx) {
         cudaFree(R.stage_v);
         if (R.copy) cudaStreamDestroy(R.copy);
     }
-    for (cudaGraphExec_t& e : ctx->sg.exec)
-        if (e) cudaGraphExecDestroy(e);
+    if (ctx->ahead.seen) cudaFreeHost(ctx->ahead.seen);
+    for (cudaEvent_t e : ctx->ahead.ev)
+        if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -732,15 +733,18 @@ static int step_fp64_head(mph_ctx* ctx) {
     mph::DevFP64& d = ctx->d;
     const SimConst& s = ctx->sc;
     cudaStream_t st = ctx->stream;
-    CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
     {
         Launch L(ctx, "move");
         mph::launch_move(s, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center, d.scal, st);
     }
     TRY(read_scalars(ctx));
+    // the maximum starts at zero for the next move, whichever kind it is
+    CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
     TRY(check_flags(ctx));
     double ms;
     std::memcpy(&ms, &ctx->h_scal->max_shift2_bits, sizeof(double));
+    ++ctx->ahead.since;
+    ctx->ahead.shift2 = ms;
     if (ms > s.shift_thr) {  // neighborCalculation() == 1 (main.cpp:1102)
         TRY(rebuild_fp64(ctx));
         ++ctx->rebuilds;
@@ -748,210 +752,146 @@ static int step_fp64_head(mph_ctx* ctx) {
     return MPH_OK;
 }
 
-// ---- the FP64 step as CUDA graphs --------------------------------------------
+// ---- FP64 steps launched ahead of the host -------------------------------------
 
-// Adds an IF node after the work captured so far on st and makes it the
-// capture's only dependency; *body is the graph the node runs.
-static int add_if_node(mph_ctx* ctx, cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t* body) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    CUDA_TRY(ctx, cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
-    if (cs != cudaStreamCaptureStatusActive) return fail(ctx, MPH_ERR_CUDA, "step graph: no active capture");
-    cudaGraphNodeParams p{};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = h;
-    p.conditional.type = cudaGraphCondTypeIf;
-    p.conditional.size = 1;
-    cudaGraphNode_t node = nullptr;
-    CUDA_TRY(ctx, cudaGraphAddNode(&node, g, deps, nd, &p));
-    *body = p.conditional.phGraph_out[0];
-    CUDA_TRY(ctx, cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+static void sweep_b_part1(mph_ctx* ctx, double* vel_host, bool skip) {
+    mph::DevFP64& d = ctx->d;
+    Launch L(ctx, "sweep_b");
+    mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc, d.ncount, d.nlist,
+                        d.ncount_s, d.nlist_s, d.force, d.scal, ctx->stream, nullptr, nullptr, nullptr, 1, 0, -1,
+                        vel_host, skip ? d.scal : nullptr);
+    ctx->wall_force_valid = false;  // computed when read
+}
+
+static int ahead_init(mph_ctx* ctx) {
+    Ahead& A = ctx->ahead;
+    if (A.seen) return MPH_OK;
+    CUDA_TRY(ctx, cudaMallocHost((void**)&A.seen, 2 * sizeof(StepScalars)));
+    for (cudaEvent_t& e : A.ev) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return MPH_OK;
 }
 
-// Captures one FP64 step for vcur == v:
-//   move (its last block makes the rebuild test and sets both conditionals)
-//   -> IF rebuild { cell index, bitonic sort, cell ranges, reorder (then copied
-//   back into the buffers this graph holds), pos32, neighbour list, table
-//   check } -> IF sweep { sweep A, force sweep }
-// The kernels and arguments of step_fp64, so the same bits.
-static int capture_step(mph_ctx* ctx, int v, cudaGraphExec_t* out, int* launches_step, int* launches_rebuild) {
+// The three kernels of one step, to run only if no earlier step stopped.
+static void launch_step_ahead(mph_ctx* ctx, double* vel_host = nullptr) {
     mph::DevFP64& d = ctx->d;
-    const SimConst& s = ctx->sc;
-    cudaStream_t st = ctx->stream;
-    const int a = d.cur, b = 1 - d.cur, va = v, vb = 1 - v;
-    const size_t n = (size_t)ctx->n;
-    const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-    cudaGraph_t g = nullptr, g_reb = nullptr, g_sw = nullptr;
-    cudaGraphConditionalHandle h_reb = 0, h_sw = 0;
-    int rc = MPH_OK;
-    auto ck = [&](cudaError_t e) {
-        if (e != cudaSuccess && rc == MPH_OK)
-            rc = fail(ctx, MPH_ERR_CUDA, std::string("step graph: ") + cudaGetErrorString(e));
-        return rc == MPH_OK;
-    };
-    auto end_capture = [&]() {
-        cudaGraph_t tmp = nullptr;
-        ck(cudaStreamEndCapture(st, &tmp));
-        ck(cudaGetLastError());
-    };
-    int ls = 0, lr = 0;
-    if (ck(cudaGraphCreate(&g, 0)) && ck(cudaGraphConditionalHandleCreate(&h_reb, g, 0, 0)) &&
-        ck(cudaGraphConditionalHandleCreate(&h_sw, g, 0, 0)) &&
-        ck(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, mode))) {
-        mph::launch_move_graph(s, d.cellstart, d.pos[a], d.vel[va], d.xv, d.snap, d.wall_center, d.scal, h_reb, h_sw,
-                               st);
-        ls += 1;
-        if (rc == MPH_OK) rc = add_if_node(ctx, st, h_reb, &g_reb);
-        if (rc == MPH_OK) rc = add_if_node(ctx, st, h_sw, &g_sw);
-        end_capture();
-    }
-    if (rc == MPH_OK && ck(cudaStreamBeginCaptureToGraph(st, g_reb, nullptr, nullptr, 0, mode))) {
-        mph::launch_cell_index(s, d.pos[a], d.type[a], d.keys, d.vals, st);
-        lr += 1 + mph::launch_bitonic_sort(s, d.keys, d.vals, st);
-        mph::launch_cell_ranges(s, d.keys, d.cellstart, st);
-        mph::launch_reorder(s, d.vals, d.pidx[a], d.type[a], d.pos[a], d.vel[va], d.pidx[b], d.type[b], d.pos[b],
-                            d.vel[vb], d.xv, d.snap, st);
-        ck(cudaMemcpyAsync(d.pos[a], d.pos[b], n * sizeof(double4), cudaMemcpyDeviceToDevice, st));
-        ck(cudaMemcpyAsync(d.vel[va], d.vel[vb], n * sizeof(double4), cudaMemcpyDeviceToDevice, st));
-        ck(cudaMemcpyAsync(d.pidx[a], d.pidx[b], n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-        ck(cudaMemcpyAsync(d.type[a], d.type[b], n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-        ck(cudaMemsetAsync(&d.scal->max_neighbors, 0, sizeof(int), st));
-        ck(cudaMemsetAsync(&d.scal->max_short, 0, sizeof(int), st));
-        mph::launch_pos32(s, d.pos[a], d.pos32, st);
-        mph::launch_neighbor_list(s, d.pos[a], d.pos32, d.cellstart, d.ncount, d.nlist, d.cap,
-                                  d.ncount_s, d.nlist_s, d.cap_s, d.scal, st);
-        mph::launch_graph_list_check(d.scal, d.cap, d.cap_s, 1, h_sw, st);
-        lr += 6;
-        end_capture();
-    }
-    if (rc == MPH_OK && ck(cudaStreamBeginCaptureToGraph(st, g_sw, nullptr, nullptr, 0, mode))) {
-        mph::launch_sweep_a(s, d.xv, d.type[a], d.ncount, d.nlist, d.ncount_s, d.nlist_s,
-                            d.dens_a, d.strain_p, d.div_p, d.press, d.gc, d.wall_center, st);
-        mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[a], d.vel[vb], d.press, d.gc, d.ncount, d.nlist,
-                            d.ncount_s, d.nlist_s, d.force, d.scal, st, nullptr,
-                            nullptr, nullptr, 1);
-        ls += 2;
-        end_capture();
-    }
-    if (rc == MPH_OK) ck(cudaGraphInstantiate(out, g, 0));
-    if (g) cudaGraphDestroy(g);
-    *launches_step = ls;
-    *launches_rebuild = lr;
-    return rc;
-}
-
-static void drop_step_graphs(mph_ctx* ctx) {
-    StepGraphs& G = ctx->sg;
-    for (cudaGraphExec_t& e : G.exec)
-        if (e) {
-            cudaGraphExecDestroy(e);
-            e = nullptr;
-        }
-    G.cur = -1;
-}
-
-static int ensure_step_graphs(mph_ctx* ctx) {
-    StepGraphs& G = ctx->sg;
-    const mph::DevFP64& d = ctx->d;
-    if (G.exec[0] && G.exec[1] && G.cur == d.cur && G.cap == d.cap && G.cap_s == d.cap_s && G.nlist == d.nlist &&
-        G.nlist_s == d.nlist_s)
-        return MPH_OK;
-    drop_step_graphs(ctx);
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int v = 0; v < 2; ++v) {
-        const int rc = capture_step(ctx, v, &G.exec[v], &G.launches_step, &G.launches_rebuild);
-        if (rc != MPH_OK) {
-            drop_step_graphs(ctx);
-            return rc;
-        }
-    }
-    G.cur = d.cur;
-    G.cap = d.cap;
-    G.cap_s = d.cap_s;
-    G.nlist = d.nlist;
-    G.nlist_s = d.nlist_s;
-    return MPH_OK;
-}
-
-// nsteps FP64 steps as graph launches with no host round trip in between;
-// the host reads the batch's counters at the end.  A list that outgrew its
-// table stops the batch after that step's reorder: the host then grows the
-// table, builds the list again from the same positions, finishes that step
-// and runs the rest.  A non-finite velocity is reported at the end of the
-// batch (the host path reports it at the next step's move).
-static int step_fp64(mph_ctx* ctx, int nsteps);
-
-static int step_fp64_graphs(mph_ctx* ctx, int nsteps) {
-    StepGraphs& G = ctx->sg;
-    mph::DevFP64& d = ctx->d;
-    cudaStream_t st = ctx->stream;
-    TRY(ensure_step_graphs(ctx));
-    // the graphs' move accumulates into a cleared maximum and clears it again
-    CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
-    CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->stop, 0, 4 * sizeof(int), st));  // stop, steps, rebuilds, blocks
-    for (int k = 0; k < nsteps; ++k) CUDA_TRY(ctx, cudaGraphLaunch(G.exec[(d.vcur + k) & 1], st));
-    TRY(read_scalars(ctx));
-    const StepScalars& h = *ctx->h_scal;
-    const int stopped = h.stop, reb = h.rebuilds_done;
-    const int done = h.steps_done - stopped;  // steps moved, less the one whose list overflowed
-    for (int k = 0; k < done; ++k) ctx->time += ctx->p.dt;  // main.cpp:449, one step at a time
-    ctx->step += done;
-    if (done & 1) d.vcur = 1 - d.vcur;
-    ctx->rebuilds += reb;
-    ctx->launches += (long long)G.launches_step * (done + stopped) + (long long)G.launches_rebuild * reb;
-    static_assert(offsetof(StepScalars, blocks_done) == offsetof(StepScalars, stop) + 3 * sizeof(int),
-                  "stop, steps_done, rebuilds_done and blocks_done are cleared together");
-    if (reb > 0) {
-        ctx->max_neighbors = h.max_neighbors;
-        ctx->lrn.edges_valid = false;
-    }
-    ctx->dens_a_valid = ctx->sc.has_st;
-    ctx->lazy_pos = -1;
-    ctx->wall_force_valid = false;
-    ctx->virial_valid = false;
-    if (h.flags & ~mph::DEVFLAG_NEIGHBOR_OVERFLOW) return check_flags(ctx);
-    if (!stopped) {
-        if (done != nsteps) return fail(ctx, MPH_ERR_DEVICE, "step graph: a step did not complete");
-        return MPH_OK;
-    }
-    // the stopped step: moved, sorted and reordered; build its lists with room
-    CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->flags, 0, sizeof(int), st));
-    TRY(build_lists(ctx));
-    sweep_a(ctx, true);
     {
-        Launch L(ctx, "sweep_b");
-        mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc,
-                            d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.force, d.scal,
-                            st, nullptr, nullptr, nullptr, 1);
-        ctx->wall_force_valid = false;
+        Launch L(ctx, "move");
+        mph::launch_move_ahead(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center, d.scal,
+                               ctx->stream);
     }
+    sweep_a(ctx, true, true);
+    sweep_b_part1(ctx, vel_host, true);
     d.vcur = 1 - d.vcur;
+}
+
+static int queue_counters(mph_ctx* ctx, int slot) {
+    Ahead& A = ctx->ahead;
+    CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, cudaMemcpyAsync(&A.seen[slot], ctx->d.scal, sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_TRY(ctx, cudaEventRecord(A.ev[slot], ctx->stream));
+    return MPH_OK;
+}
+
+// Takes in the counters of a batch of `launched` steps: those that completed (with
+// *stopped, one more has moved and waits for its rebuild).
+static int take_counters(mph_ctx* ctx, int slot, int launched, int* completed, bool* stopped) {
+    Ahead& A = ctx->ahead;
+    CUDA_TRY(ctx, cudaEventSynchronize(A.ev[slot]));
+    const StepScalars& h = A.seen[slot];
+    *ctx->h_scal = h;
+    const int moved = h.steps_done - A.counted;
+    A.counted = h.steps_done;
+    *stopped = h.stop != 0 && moved > 0;
+    *completed = moved - (*stopped ? 1 : 0);
+    if (moved > 0) {
+        A.since += moved;
+        std::memcpy(&A.shift2, &h.last_shift2_bits, sizeof(double));
+    }
+    if (moved > launched) return fail(ctx, MPH_ERR_DEVICE, "steps launched ahead: the counters disagree");
+    for (int k = 0; k < *completed; ++k) ctx->time += ctx->p.dt;  // main.cpp:449, one step at a time
+    ctx->step += *completed;
+    return check_flags(ctx);
+}
+
+// The step that stopped: rebuild, then its sweeps (main.cpp:399-431).
+static int finish_stopped(mph_ctx* ctx, double* vel_host = nullptr) {
+    CUDA_TRY(ctx, cudaMemsetAsync(&ctx->d.scal->stop, 0, sizeof(int), ctx->stream));
+    TRY(rebuild_fp64(ctx));
+    ++ctx->rebuilds;
+    sweep_a(ctx, true, false);
+    sweep_b_part1(ctx, vel_host, false);
+    ctx->d.vcur = 1 - ctx->d.vcur;
     CUDA_TRY(ctx, cudaGetLastError());
     ctx->time += ctx->p.dt;
     ++ctx->step;
-    const int rest = nsteps - done - 1;
-    return rest > 0 ? step_fp64(ctx, rest) : MPH_OK;
+    return MPH_OK;
+}
+
+// Steps of the next batch: half of those that the displacement so far leaves until
+// the next rebuild, so that few launches turn out empty, and at most 16.
+static int batch_steps(const mph_ctx* ctx) {
+    const Ahead& A = ctx->ahead;
+    if (A.since < 2 || !(A.shift2 > 0.0)) return 4;
+    const double rate = std::sqrt(A.shift2) / A.since, left = std::sqrt(ctx->sc.shift_thr) - std::sqrt(A.shift2);
+    return (int)std::min(16.0, std::max(1.0, 0.5 * left / rate));
+}
+
+// nsteps FP64 steps with the host one batch behind the GPU: while a batch runs the
+// next one is launched, then the first one's counters are read.  Measured against
+// the CUDA graphs with conditional nodes this replaced: 35 -> AHEAD_1600 us per step on
+// the 1,600-particle droplet (21 us of kernels), no graph to instantiate on the
+// first call, and rebuilds on the host's path (tables grow as they always do).
+static int step_fp64_ahead(mph_ctx* ctx, int nsteps) {
+    mph::DevFP64& d = ctx->d;
+    TRY(ahead_init(ctx));
+    int left = nsteps;  // steps not yet completed
+    while (left > 0) {
+        int size[2] = {0, 0}, queued = 0, slot = 0, done = 0, flight = 0;
+        bool stopped = false;
+        const int v0 = d.vcur;
+        auto launch_batch = [&](int s) {
+            size[s] = std::min(left - queued, batch_steps(ctx));
+            for (int k = 0; k < size[s]; ++k) launch_step_ahead(ctx);
+            queued += size[s];
+            ++flight;
+            return queue_counters(ctx, s);
+        };
+        TRY(launch_batch(0));
+        while (flight > 0) {
+            if (!stopped && queued < left) TRY(launch_batch(1 - slot));
+            int completed = 0;
+            bool s = false;
+            const int rc = take_counters(ctx, slot, size[slot], &completed, &s);
+            --flight;
+            done += completed;
+            stopped |= s;
+            slot = 1 - slot;
+            if (rc != MPH_OK) {
+                d.vcur = (v0 + done) & 1;
+                if (flight > 0 && cudaEventSynchronize(ctx->ahead.ev[slot]) == cudaSuccess)
+                    ctx->ahead.counted = ctx->ahead.seen[slot].steps_done;
+                return rc;
+            }
+        }
+        d.vcur = (v0 + done) & 1;
+        left -= done;
+        if (stopped) {
+            TRY(finish_stopped(ctx));
+            --left;
+        }
+    }
+    ctx->virial_valid = false;
+    return MPH_OK;
 }
 
 static int step_fp64(mph_ctx* ctx, int nsteps) {
-    // several steps: graph replay (per-kernel profiling needs the host path)
-    if (nsteps > 1 && ctx->sg.enabled && !ctx->prof.on) return step_fp64_graphs(ctx, nsteps);
+    // several steps: launched ahead (per-kernel profiling needs the host path)
+    if (nsteps > 1 && ctx->ahead.enabled && !ctx->prof.on) return step_fp64_ahead(ctx, nsteps);
     mph::DevFP64& d = ctx->d;
-    const SimConst& s = ctx->sc;
-    cudaStream_t st = ctx->stream;
     for (int k = 0; k < nsteps; ++k) {
         TRY(step_fp64_head(ctx));
         sweep_a(ctx, true);
-        {
-            Launch L(ctx, "sweep_b");
-            mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc,
-                                d.ncount, d.nlist, d.ncount_s, d.nlist_s, d.force,
-                                d.scal, st, nullptr, nullptr, nullptr, 1);
-            ctx->wall_force_valid = false;  // computed when read
-        }
+        sweep_b_part1(ctx, nullptr, false);
         d.vcur = 1 - d.vcur;
         CUDA_TRY(ctx, cudaGetLastError());
         ctx->time += ctx->p.dt;  // main.cpp:449
@@ -1217,14 +1157,12 @@ extern "C" int mph_set_sweep_layout(mph_ctx* ctx, int layout) {
     if (!ctx) return fail(nullptr, MPH_ERR_ARG, "ctx is NULL");
     if (layout < 0 || layout > 2) return fail(ctx, MPH_ERR_ARG, "layout must be 0, 1 or 2");
     ctx->sc.sweep_layout = layout;
-    drop_step_graphs(ctx);  // they hold the constants by value
     return MPH_OK;
 }
 
 extern "C" int mph_set_step_graphs(mph_ctx* ctx, int enable) {
     if (!ctx) return fail(nullptr, MPH_ERR_ARG, "ctx is NULL");
-    ctx->sg.enabled = enable != 0;
-    if (!enable) drop_step_graphs(ctx);
+    ctx->ahead.enabled = enable != 0;
     return MPH_OK;
 }
 
@@ -1342,50 +1280,89 @@ static double* mapped_host(double* p, size_t count) {
     return (double*)a.devicePointer;
 }
 
-// The FP64 form's last step with its read-back overlapped.  The positions are
-// final once the move and any rebuild are done: they are packed and copied on
-// a copy stream while the sweeps run.  The velocities: with a pinned, mapped
-// host buffer the force sweep stores each particle's new velocity into it as
-// well as into device memory (24 B per particle over PCIe while the sweep
-// runs); otherwise they are packed and copied after the sweep.  Same kernels
-// and inputs: the bits of mph_step + mph_get_state.
+// The FP64 form's last step with its read-back overlapped.  The step is launched
+// ahead of its rebuild test, whose answer the host reads with the state: the rare
+// step that has to rebuild does so then and copies again.  The positions are
+// final once the move and any rebuild are done: they are packed and copied on a
+// copy stream while the sweeps run.  The velocities: with a pinned, mapped host
+// buffer the force sweep stores each particle's new velocity into it as well as
+// into device memory (24 B per particle over PCIe while the sweep runs, 20 GB/s),
+// or, where the sweep is too short to hide that, a kernel behind it writes whole
+// lines (50 GB/s); otherwise they are packed and copied after the sweep.  Same
+// kernels and inputs: the bits of mph_step + mph_get_state.
+constexpr int kPackHostMax = 100000;  // particles up to which the line writer is faster
+
 static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
     TRY(readback_init(ctx));
+    TRY(ahead_init(ctx));
     ReadBack& R = ctx->rb;
     mph::DevFP64& d = ctx->d;
-    const SimConst& s = ctx->sc;
     cudaStream_t st = ctx->stream;
     const size_t n = (size_t)ctx->n;
+    const bool lines = ctx->n <= kPackHostMax;
     double* vh = mapped_host(vel, 3 * n);
-    TRY(step_fp64_head(ctx));
-    CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));  // positions final
-    sweep_a(ctx, true);
-    double4* vout = d.vel[1 - d.vcur];
-    {
-        Launch L(ctx, "sweep_b");
-        mph::launch_sweep_b(s, d.cellstart, d.xv, d.type[d.cur], vout, d.press, d.gc, d.ncount, d.nlist,
-                            d.ncount_s, d.nlist_s, d.force, d.scal, st, nullptr,
-                            nullptr, nullptr, 1, 0, -1, vh);
-        ctx->wall_force_valid = false;  // computed when read
+    double* xh = lines ? mapped_host(xyz, 3 * n) : nullptr;
+    double* in_sweep = lines ? nullptr : vh;
+    // after the launches of a step (vcur has flipped): the copies
+    auto copies = [&]() {
+        if (vel && vh && lines) {
+            mph::launch_pack3_lines(ctx->n, d.vel[d.vcur], vh, st);
+            ++ctx->launches;
+        }
+        CUDA_TRY(ctx, cudaEventRecord(R.ev[1], st));  // velocities final
+        // enqueued after the compute so pageable buffers do not hold it back
+        if (xyz) {
+            CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[0], 0));
+            ++ctx->launches;
+            if (xh) {
+                mph::launch_pack3_lines(ctx->n, d.pos[d.cur], xh, R.copy);
+            } else {
+                mph::launch_pack3(ctx->n, d.pos[d.cur], d.staging, R.copy);
+                CUDA_TRY(ctx, cudaMemcpyAsync(xyz, d.staging, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
+            }
+        }
+        if (vel && !vh) {
+            CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[1], 0));
+            mph::launch_pack3(ctx->n, d.vel[d.vcur], R.stage_v, R.copy);
+            ++ctx->launches;
+            CUDA_TRY(ctx, cudaMemcpyAsync(vel, R.stage_v, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
+        }
+        return MPH_OK;
+    };
+    if (ctx->prof.on) {  // per-kernel timing: the host path
+        TRY(step_fp64_head(ctx));
+        CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));  // positions final
+        sweep_a(ctx, true);
+        sweep_b_part1(ctx, in_sweep, false);
+        d.vcur = 1 - d.vcur;
+        TRY(copies());
+        ctx->time += ctx->p.dt;  // main.cpp:449
+        ++ctx->step;
+    } else {
+        {
+            Launch L(ctx, "move");
+            mph::launch_move_ahead(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center,
+                                   d.scal, st);
+        }
+        CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));  // positions final unless a rebuild follows
+        sweep_a(ctx, true, true);
+        sweep_b_part1(ctx, in_sweep, true);
+        d.vcur = 1 - d.vcur;
+        TRY(queue_counters(ctx, 0));
+        TRY(copies());
+        int completed = 0;
+        bool stopped = false;
+        const int rc = take_counters(ctx, 0, 1, &completed, &stopped);
+        if (stopped || rc != MPH_OK) {
+            CUDA_TRY(ctx, cudaStreamSynchronize(R.copy));
+            d.vcur = 1 - d.vcur;
+            if (rc != MPH_OK) return rc;
+            TRY(finish_stopped(ctx, in_sweep));
+            CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));
+            TRY(copies());
+        }
     }
-    CUDA_TRY(ctx, cudaEventRecord(R.ev[1], st));  // velocities final
-    // copies, enqueued after the compute so pageable buffers do not hold it back
-    if (xyz) {
-        CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[0], 0));
-        mph::launch_pack3(ctx->n, d.pos[d.cur], d.staging, R.copy);
-        ++ctx->launches;
-        CUDA_TRY(ctx, cudaMemcpyAsync(xyz, d.staging, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
-    }
-    if (vel && !vh) {
-        CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[1], 0));
-        mph::launch_pack3(ctx->n, vout, R.stage_v, R.copy);
-        ++ctx->launches;
-        CUDA_TRY(ctx, cudaMemcpyAsync(vel, R.stage_v, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
-    }
-    d.vcur = 1 - d.vcur;
     CUDA_TRY(ctx, cudaGetLastError());
-    ctx->time += ctx->p.dt;  // main.cpp:449
-    ++ctx->step;
     ctx->virial_valid = false;
     CUDA_TRY(ctx, cudaStreamSynchronize(R.copy));
     CUDA_TRY(ctx, cudaStreamSynchronize(st));

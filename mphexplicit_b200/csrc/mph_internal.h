@@ -59,14 +59,13 @@ struct SimConst {
 // Small per-step device scalars (one cache line, read back with one copy).
 struct StepScalars {
     unsigned long long max_shift2_bits;  // max |shift|^2 as ordered bits (>= 0)
+    unsigned long long last_shift2_bits; // steps launched ahead: the last moved step's maximum
     int flags;                           // MPH_DEVFLAG_*
     int max_neighbors;                   // longest list of the last build
-    int rebuild;                         // decision of the last move kernel
     int max_short, max_long;             // longest short / long part (mixed table)
-    int stop;                            // step graphs: a list overflowed, the later steps skip
-    int steps_done;                      // step graphs: steps started (moved) in this batch
-    int rebuilds_done;                   // step graphs: rebuilds started in this batch
-    unsigned blocks_done;                // step graphs: move blocks finished in this launch
+    int stop;                            // steps launched ahead: a step asked for a rebuild, the later ones do nothing
+    int steps_done;                      // steps launched ahead: steps moved so far
+    unsigned blocks_done;                // steps launched ahead: move blocks finished in this launch
     int pad[5];
 };
 
@@ -141,17 +140,15 @@ void launch_neighbor_list(const SimConst& c, const double4* pos, const float4* p
                           StepScalars* scal, cudaStream_t s);
 void launch_pack3(int n, const double4* src, double* dst, cudaStream_t s);
 
-// ---- step graphs (FP64 form) ------------------------------------------------
-// after a list build: a list longer than its table stops the batch (sweep = 0)
-void launch_graph_list_check(StepScalars* scal, int cap, int cap_s, int short_list,
-                             cudaGraphConditionalHandle sweep, cudaStream_t s);
-// the move of a step graph (k_fp64.cu): as launch_move, and its last block
-// makes the rebuild test of main.cpp:1102 (rebuild = 1 when it fires; sweep =
-// 1 unless the batch stopped, when the move does nothing), counts the step
-// and clears the maximum shift for the next step
-void launch_move_graph(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
-                       const double4* snap, const double* wall_center, StepScalars* scal,
-                       cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle sweep, cudaStream_t s);
+// the first three components, packed in `dst` by consecutive threads writing
+// consecutive doubles (whole lines over PCIe when dst is mapped host memory)
+void launch_pack3_lines(int n, const double4* src, double* dst, cudaStream_t s);
+// the move of a step launched ahead of the host (k_fp64.cu): as launch_move, and
+// its last block makes the rebuild test of main.cpp:1102 (when it fires, scal->stop
+// makes this step's sweeps and every later step's kernels do nothing), counts the
+// step and clears the maximum shift for the next step
+void launch_move_ahead(const SimConst& c, const int* cellstart, double4* pos, double4* vel, double2* xv,
+                       const double4* snap, const double* wall_center, StepScalars* scal, cudaStream_t s);
 void launch_unpack3(int n, const double* src, double4* dst, const int* type, cudaStream_t s);
 
 // ---- kernel launchers (k_fp64.cu) -----------------------------------------
@@ -160,7 +157,7 @@ void launch_move(const SimConst& c, const int* cellstart, double4* pos, double4*
                  const double4* snap, const double* wall_center, StepScalars* scal, cudaStream_t s);
 // Sweep A's DensityP and DivergenceP visit the short sublist (ncount_s,
 // nlist_s); with surface tension DensityA and GravityCenter the whole list.
-// skip: the sweep does nothing when skip->stop is set (step graphs)
+// skip: the sweep does nothing when skip->stop is set (steps launched ahead)
 void launch_sweep_a(const SimConst& c, const double2* xv, const int* type, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double* dens_a, double* strain_p, double* div_p,
                     double4* press, double4* gc, double* wall_center, cudaStream_t s,
