@@ -408,10 +408,10 @@ def measure_droplet(args, rank):
     """Benchmark config 1: the 2-D square droplet (40x40 type-0 particles,
     l0 = 0.004 m, mu 0.1, sigma 0.07, sound speed 10 m/s, dt 1e-5 s, no walls or
     gravity), FP64, `droplet_steps` steps in one mph_step call: the default
-    graph launches (the rebuild test on the device) and the host path (one
-    flag read per step, mph_set_step_graphs(0)), both bit-identical, and the
+    (steps launched ahead of the host, the rebuild test on the device) and the
+    host path (one flag read per step, mph_set_step_graphs(0)), both bit-identical, and the
     reference's own 2-D build on the same scene on all host threads and on
-    one.  At this size the sweeps run one warp per particle."""
+    one.  At this size the sweeps run several lanes per particle."""
     import torch
     import mphexplicit_b200 as M
     from mphexplicit_b200 import scenes
@@ -423,7 +423,7 @@ def measure_droplet(args, rank):
     for graphs in (True, False):
         s = M.Solver(sc.params, sc.header, sc.type, sc.xyz, sc.vel, dim=2, mode="fp64")
         s.set_step_graphs(graphs)
-        s.step(3)  # warm-up (the first several-step call captures the graphs)
+        s.step(3)  # warm-up
         s.synchronize()
         stream = torch.cuda.ExternalStream(s.stream_handle)
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -230,27 +230,26 @@ int mph_create(const mph_params* p, const mph_grid_header* h, int dim, int mode,
 
 /* Advance nsteps explicit steps: the loop body main.cpp:386-431 plus
  * Time += Dt (main.cpp:449).  No file output.  Returns when the steps are
- * done.  Several FP64 steps run as one CUDA graph launch each, whose
- * conditional nodes make the neighbour-rebuild test (in the move kernel's
- * last block) and check a rebuilt list against its table on the device, with
- * no host round trip until the end: the same kernels, so the same bits.  A
- * list that outgrows its table ends the graph launches after that step's
- * reorder; the host grows the table and finishes the steps.  One step, the
- * mixed and learned forms, profiling on (mph_profile_enable), or graphs off:
- * the host reads the rebuild flag after each step's move. */
+ * done.  Several FP64 steps are launched in batches ahead of the host: the
+ * move kernel's last block makes the neighbour-rebuild test on the device, and
+ * once it fires the sweeps of that step and everything launched after it do
+ * nothing until the host, a batch behind, has read the counters, rebuilt the
+ * list and finished that step: the same kernels, so the same bits.  One step,
+ * the mixed and learned forms, profiling on (mph_profile_enable), or launching
+ * ahead off: the host reads the rebuild flag after each step's move. */
 int mph_step(mph_ctx* ctx, int nsteps);
 
-/* enable == 0: mph_step takes the host path for every step; 1 (the
- * default): graph launches for several FP64 steps.  Measured on one B200:
- * 0.036 against 0.040 ms per step on a 1,600-particle droplet, 2-3 % on
- * 10-20 k particles, within 1 % at 0.1-2.8 M particles. */
+/* enable == 0: mph_step waits for every step's rebuild flag; 1 (the default):
+ * several FP64 steps are launched ahead of the host (see mph_step).  The name
+ * dates from when that was done with CUDA graphs.  Measured on one B200:
+ * 0.025 against 0.040 ms per step on a 1,600-particle droplet. */
 int mph_set_step_graphs(mph_ctx* ctx, int enable);
 
-/* The FP64 (and learned) form's pair sweeps: 0 (the default) by size, one
- * warp per particle up to 40,000 particles in 3-D and 20,000 in 2-D, one
- * thread per particle above; 1 always a thread per particle; 2 always a warp
- * per particle.  The same bits either way (the warp's lanes compute the terms
- * of 32 list entries, one lane per sum adds them in list order). */
+/* The FP64 (and learned) form's pair sweeps: 0 (the default) by size, 4 to 32
+ * lanes per particle in small scenes and one thread per particle above; 1
+ * always a thread per particle; 2 always a warp (32 lanes) per particle.  The
+ * same bits either way (the lanes compute the terms of as many list entries,
+ * one lane per sum adds them in list order). */
 int mph_set_sweep_layout(mph_ctx* ctx, int layout);
 
 /* Wait for the context's stream and report any device-side error flag. */

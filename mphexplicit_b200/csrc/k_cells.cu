@@ -150,22 +150,34 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
     }
 }
 
-// Neighbour list (main.cpp:1329-1585), one warp per home key: the particles
-// of one cell (fluid keys, then the wall keys of the same cells) share their
-// 3^D stencil and its visiting order, so the warp walks it in step, 32 home
-// particles at a time (one per lane).  Each candidate range is read 32
-// candidates at a time (one coalesced FP32 record per lane into shared
-// memory); every lane then tests all of them against its own particle with
-// the FP32 prefilter, giving a bit mask, and runs the exact FP64 test of the
-// reference only over the set bits, in ascending order.  A lane's entries
-// are therefore the reference's, in the reference's order: fluid candidates
-// of the 27 cells, then wall candidates (a wall with no fluid neighbour
-// skips the walls, main.cpp:1416), self included, each range ascending.
+// Neighbour list (main.cpp:1329-1585).  The particles of one home key (a cell's
+// fluid, or its walls) share their 3^D stencil and its visiting order; a warp walks
+// it with eight of them at a time, taken octant by octant of the cell so that the
+// box around them is small.  Each candidate range is read 32 candidates at a time
+// (one coalesced FP32 record per lane); those near the box are queued in order in
+// shared memory, and every full queue is tested with a candidate per lane against
+// one of the eight particles after the other: the FP32 prefilter, the exact FP64
+// test of the reference where that leaves a doubt, and a ballot that numbers the
+// hits in candidate order.  A particle's entries are therefore the reference's, in
+// the reference's order: fluid candidates of the 27 cells, then wall candidates (a
+// wall with no fluid neighbour skips the walls, main.cpp:1416), self included, each
+// range ascending.  The order in which the particles are taken changes no list.
+//
+// What bounds it: the instruction count.  A particle's list costs about 1150
+// warp instructions (its share of queueing 600 candidates for eight particles, then
+// 20 to test 32 candidates against one), issued at 65 % of the peak.  With a lane per particle, 32 candidates tested one after
+// the other into a bit mask and the hits pushed one by one, half of the lanes idled
+// in the pushes and in part-filled warps, and a small scene's few warps ran one long
+// serial chain: 8.03 -> 4.37 ms a build at 2,779,256 particles (3-D dam), 436 -> 311 us
+// at 213,868, 290 -> 106 at 20,116, 894 -> 710 at 314,432 (3-D column), 47 -> 36 at
+// 22,500 in 2-D.
 //
 // The count and the fill of the reference are one pass: entries go to a
-// column-major [cap][n] table; a list longer than cap is still counted,
+// table in rows of four, [cap / 4][n][4] (list_at): with single entries in rows
+// every store filled an eighth of a sector that was evicted before its neighbours
+// came (eight times the lists' bytes in DRAM traffic).  A list longer than cap is still counted,
 // raises DEVFLAG_NEIGHBOR_OVERFLOW and the host rebuilds with a larger table.
-// With nlist_s, the entries within rs2 also go, in the same order, to the
+// The entries within rs2 also go, in the same order, to the
 // short sublist: a particle moves at most MARGIN/2 between builds (the
 // rebuild test of main.cpp:1086-1108), so every pair within RadiusP until the
 // next build is in it, and a sum over the pairs within RadiusP visits them in
@@ -177,23 +189,25 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
 // cannot pass that test and is skipped.  An axis with fewer than 4 cells
 // contributes nothing to the FP32 distance (its minimum image need not be the
 // neighbouring cell's), which only keeps more candidates.
-constexpr int kListWarps = 4;  // warps (home keys) per 128-thread block
+constexpr int kListWarps = 4;     // warps per block
+constexpr int kListParts = 8;     // particles per group
+constexpr int kListSorted = 128;  // home particles that are taken octant by octant (more: in slot order)
 
-#ifndef MPH_LIST_MINB
-#define MPH_LIST_MINB 6
-#endif
 template <bool ALL3>  // every axis in the FP32 prefilter (pf.use all set)
-__global__ void __launch_bounds__(32 * kListWarps, MPH_LIST_MINB)
+__global__ void __launch_bounds__(32 * kListWarps, 8)
 k_neighbor_list(SimConst c, const double4* __restrict__ pos, const float4* __restrict__ pos32, Prefilter pf,
                 const int* __restrict__ cellstart, int* __restrict__ ncount, int* __restrict__ nlist, int cap,
-                int* __restrict__ ncount_s, int* __restrict__ nlist_s, int cap_s, StepScalars* __restrict__ scal) {
-    __shared__ float4 cand[kListWarps][32];
-    __shared__ int4 sten[kListWarps][27];  // the stencil in visiting order: cell, FP32 image offsets
+                int* __restrict__ ncount_s, int* __restrict__ nlist_s, int cap_s, StepScalars* __restrict__ scal,
+                int key_warps) {
+    __shared__ float4 queue_[kListWarps][64];           // candidates near the box, in order (a ring)
+    __shared__ float4 home_[kListWarps][kListParts];    // the group's FP32 positions and slots
+    __shared__ unsigned char order_[kListWarps][kListSorted];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int key = blockIdx.x * kListWarps + wib;  // home key in [0, 2*tot)
-    if (key >= 2 * c.tot) return;                   // whole warp
-    const int hb = cellstart[key], he = cellstart[key + 1];
-    if (hb == he) return;
+    const int gw = blockIdx.x * kListWarps + wib;
+    const int key = gw / key_warps;   // home key in [0, 2*tot), key_warps warps share it
+    if (key >= 2 * c.tot) return;     // whole warp
+    const int hb = cellstart[key], he = cellstart[key + 1], first = (gw % key_warps) * kListParts;
+    if (hb + first >= he) return;
     // the stencil of the home cell as main.cpp:1356-1392 computes it from the
     // key (a wall's key carries +TotalCellCount: its icx is cx + cc[0])
     const int icx = (key / (c.cc[1] * c.cc[2])) % c.tot;
@@ -213,35 +227,81 @@ k_neighbor_list(SimConst c, const double4* __restrict__ pos, const float4* __res
         off = raw < 0 ? -pf.width[d] : (raw >= c.cc[d] ? pf.width[d] : 0.0f);
         return ((ic[d] - c.range[d] + s_) % c.cc[d] + c.cc[d]) % c.cc[d];
     };
-    // lane s < w0*w1*w2 computes stencil slot s of the loop order of
-    // main.cpp:1356-1392 (x outer, z inner), once for all the key's chunks
+    // lane s < w0*w1*w2 holds stencil slot s of the loop order of
+    // main.cpp:1356-1392 (x outer, z inner): its ranges and image offsets
     const int nsl = w[0] * w[1] * w[2];  // at most 27: range <= 1 on every axis
+    int st_b[2] = {0, 0}, st_e[2] = {0, 0};
+    float st_x = 0.f, st_y = 0.f, st_z = 0.f;
     if (lane < nsl) {
         const int a0 = lane / (w[1] * w[2]), a1 = (lane / w[2]) % w[1], a2 = lane % w[2];
-        float gx, gy, gz;
-        const int cx = slot(0, (jmin[0] + a0) % w[0], gx), cy = slot(1, (jmin[1] + a1) % w[1], gy),
-                  cz = slot(2, (jmin[2] + a2) % w[2], gz);
-        sten[wib][lane] = make_int4(cell_id(c, cx, cy, cz), __float_as_int(gx), __float_as_int(gy),
-                                    __float_as_int(gz));
+        const int cx = slot(0, (jmin[0] + a0) % w[0], st_x), cy = slot(1, (jmin[1] + a1) % w[1], st_y),
+                  cz = slot(2, (jmin[2] + a2) % w[2], st_z);
+        const int cell = cell_id(c, cx, cy, cz);
+        st_b[0] = cellstart[cell];
+        st_e[0] = cellstart[cell + 1];
+        st_b[1] = cellstart[cell + c.tot];
+        st_e[1] = cellstart[cell + c.tot + 1];
     }
-    __syncwarp();
     const int wall_begin = cellstart[c.tot], wall_end = cellstart[2 * c.tot];
+    const bool is_wall = wall_begin <= hb && hb < wall_end;  // one key holds walls or fluid
     const size_t n = (size_t)c.n;
-    const bool short_list = nlist_s != nullptr;
-    float4* cw = cand[wib];
+    float4* const queue = queue_[wib];
+    float4* const homes = home_[wib];
+    unsigned char* const order = order_[wib];
+    const int nh = he - hb;
+    const bool sorted = nh > kListParts && nh <= kListSorted;
+    if (sorted) {  // a counting sort by octant of the home cell, along a Gray code (neighbouring octants in a row)
+        const float mx = ((float)home[0] + 0.5f) * pf.cell_width[0], my = ((float)home[1] + 0.5f) * pf.cell_width[1],
+                    mz = ((float)home[2] + 0.5f) * pf.cell_width[2];
+        int base[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (int pass = 0; pass < 2; ++pass) {
+            for (int h = 0; h < nh; h += 32) {
+                int o = 8;
+                if (h + lane < nh) {
+                    const float4 f = pos32[hb + h + lane];
+                    o = (f.x >= mx ? 4 : 0) | (f.y >= my ? 2 : 0) | (f.z >= mz ? 1 : 0);
+                    o = (0x54672310u >> (4 * o)) & 7;
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const unsigned mask = __ballot_sync(0xffffffffu, o == q);
+                    if (pass == 1 && o == q)
+                        order[base[q] + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)(h + lane);
+                    base[q] += __popc(mask);
+                }
+            }
+            if (pass == 0) {
+                int run = 0;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int v = base[q];
+                    base[q] = run;
+                    run += v;
+                }
+            }
+        }
+        __syncwarp();
+    }
     const float kInf = __int_as_float(0x7f800000);
-    for (int h0 = hb; h0 < he; h0 += 32) {
-        const int i = h0 + lane;
-        const bool active = i < he;
-        const double4 pi = pos[active ? i : hb];
-        const float4 fi = pos32[active ? i : hb];
-        const bool is_wall = wall_begin <= i && i < wall_end;
-        int cnt = 0, cnt_s = 0;
-        // box of the chunk's FP32 positions: a candidate farther than the
-        // cut-off from it is no lane's neighbour (Prefilter::r2_box)
-        float b0x = active ? fi.x : kInf, b0y = active ? fi.y : kInf, b0z = active ? fi.z : kInf;
-        float b1x = active ? fi.x : -kInf, b1y = active ? fi.y : -kInf, b1z = active ? fi.z : -kInf;
-        for (int o = 16; o > 0; o >>= 1) {
+    int most = 0, most_s = 0;
+    for (int h0 = first; h0 < nh; h0 += key_warps * kListParts) {
+        const int np = min(kListParts, nh - h0);
+        // the group, a particle per lane (0..7), and the box of its FP32 positions: a
+        // candidate farther than the cut-off from it is no particle's neighbour
+        // (Prefilter::r2_box)
+        float b0x = kInf, b0y = kInf, b0z = kInf, b1x = -kInf, b1y = -kInf, b1z = -kInf;
+        __syncwarp();
+        if (lane < np) {
+            const int i = hb + (sorted ? (int)order[h0 + lane] : h0 + lane);
+            float4 f = pos32[i];
+            b0x = b1x = f.x;
+            b0y = b1y = f.y;
+            b0z = b1z = f.z;
+            f.w = __int_as_float(i);
+            homes[lane] = f;
+        }
+#pragma unroll
+        for (int o = kListParts / 2; o > 0; o >>= 1) {
             b0x = fminf(b0x, __shfl_xor_sync(0xffffffffu, b0x, o));
             b0y = fminf(b0y, __shfl_xor_sync(0xffffffffu, b0y, o));
             b0z = fminf(b0z, __shfl_xor_sync(0xffffffffu, b0z, o));
@@ -249,97 +309,133 @@ k_neighbor_list(SimConst c, const double4* __restrict__ pos, const float4* __res
             b1y = fmaxf(b1y, __shfl_xor_sync(0xffffffffu, b1y, o));
             b1z = fmaxf(b1z, __shfl_xor_sync(0xffffffffu, b1z, o));
         }
+        b0x = __shfl_sync(0xffffffffu, b0x, 0);
+        b0y = __shfl_sync(0xffffffffu, b0y, 0);
+        b0z = __shfl_sync(0xffffffffu, b0z, 0);
+        b1x = __shfl_sync(0xffffffffu, b1x, 0);
+        b1y = __shfl_sync(0xffffffffu, b1y, 0);
+        b1z = __shfl_sync(0xffffffffu, b1z, 0);
+        __syncwarp();
+        int cnt = 0, cnt_s = 0;  // lane p: particle p's
+        unsigned takes = (1u << np) - 1u;
+        int head = 0, queued = 0;
+        auto test = [&](int m) {  // the first m (<= 32) of the queue
+            const float4 q = queue[(head + lane) & 63];
+            const int j = __float_as_int(q.w);
+            const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+            for (unsigned left = takes; left != 0u; left &= left - 1u) {
+                const int p = __ffs(left) - 1;
+                const float4 f = homes[p];
+                const float fx = (ALL3 || pf.use[0]) ? q.x - f.x : 0.f;
+                const float fy = (ALL3 || pf.use[1]) ? q.y - f.y : 0.f;
+                const float fz = (ALL3 || pf.use[2]) ? q.z - f.z : 0.f;
+                // FMA: fewer roundings than the bound allows for
+                const float r2f = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, __fmul_rn(fz, fz)));
+                bool in = lane < m && r2f <= pf.r2_hi;  // within rm unless in its shell
+                bool in_short = in && r2f <= pf.rs2_lo;  // within rs for certain
+                const int i = __float_as_int(f.w);
+                if (in && (r2f > pf.r2_lo || (r2f > pf.rs2_lo && r2f <= pf.rs2_hi))) {
+                    const double4 pi = pos[i], pj = pos[j];
+                    const double q0 = omod_fast(pj.x - pi.x + c.half_width[0], c.width[0]) - c.half_width[0];
+                    const double q1 = omod_fast(pj.y - pi.y + c.half_width[1], c.width[1]) - c.half_width[1];
+                    const double q2 = omod_fast(pj.z - pi.z + c.half_width[2], c.width[2]) - c.half_width[2];
+                    const double r2 = q0 * q0 + q1 * q1 + q2 * q2;
+                    in = r2 <= c.rm2;
+                    in_short = in && r2 <= c.rs2;
+                }
+                const unsigned hits = __ballot_sync(0xffffffffu, in);
+                const unsigned hits_s = __ballot_sync(0xffffffffu, in_short);
+                const int base_l = __shfl_sync(0xffffffffu, cnt, p);
+                if (in) {
+                    const int at = base_l + __popc(hits & below);
+                    if (at < cap) nlist[list_at(at, n, i)] = j;
+                }
+                if (hits_s != 0u) {
+                    const int base = __shfl_sync(0xffffffffu, cnt_s, p);
+                    if (in_short) {
+                        const int at = base + __popc(hits_s & below);
+                        if (at < cap_s) nlist_s[list_at(at, n, i)] = j;
+                    }
+                }
+                if (lane == p) {
+                    cnt += __popc(hits);
+                    cnt_s += __popc(hits_s);
+                }
+            }
+        };
         for (int kind = 0; kind < 2; ++kind) {
-            // main.cpp:1416: a wall with no fluid neighbour gets no wall entries
-            const bool take = active && !(kind == 1 && is_wall && cnt == 0);
-            const int off = kind ? c.tot : 0;
-            for (int sl = 0; sl < nsl; ++sl) {
-                const int4 st = sten[wib][sl];
-                const int cell = st.x;
-                const float gx = __int_as_float(st.y), gy = __int_as_float(st.z), gz = __int_as_float(st.w);
-                const float ox = (ALL3 || pf.use[0]) ? gx - fi.x : 0.f;
-                const float oy = (ALL3 || pf.use[1]) ? gy - fi.y : 0.f;
-                const float oz = (ALL3 || pf.use[2]) ? gz - fi.z : 0.f;
-                const int b = cellstart[cell + off], e = cellstart[cell + off + 1];
-                for (int cb = b; cb < e; cb += 32) {
-                    // the candidates near the box, compacted in order into the stage
-                    bool near = false;
-                    float4 q;
-                    if (cb + lane < e) {
-                        q = pos32[cb + lane];
-                        const float ax = q.x + gx, ay = q.y + gy, az = q.z + gz;
-                        const float ex = (ALL3 || pf.use[0]) ? fmaxf(0.f, fmaxf(b0x - ax, ax - b1x)) : 0.f;
-                        const float ey = (ALL3 || pf.use[1]) ? fmaxf(0.f, fmaxf(b0y - ay, ay - b1y)) : 0.f;
-                        const float ez = (ALL3 || pf.use[2]) ? fmaxf(0.f, fmaxf(b0z - az, az - b1z)) : 0.f;
-                        near = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez))) <= pf.r2_box;
+            if (kind == 1 && is_wall) {  // main.cpp:1416: a wall with no fluid neighbour gets no wall entries
+                takes &= __ballot_sync(0xffffffffu, cnt != 0);
+                if (takes == 0u) break;
+            }
+            // the candidate chunks one after the other, the next one's records loaded
+            // while this one is worked on
+            int sl = -1, cb = 0, e = 0;
+            float gx = 0.f, gy = 0.f, gz = 0.f;
+            auto next = [&]() {  // the next chunk: [cb, min(cb + 32, e)) of stencil slot sl
+                cb += 32;
+                while (cb >= e) {
+                    if (++sl >= nsl) return false;
+                    cb = __shfl_sync(0xffffffffu, st_b[kind], sl);
+                    e = __shfl_sync(0xffffffffu, st_e[kind], sl);
+                    if (cb < e) {
+                        gx = __shfl_sync(0xffffffffu, st_x, sl);
+                        gy = __shfl_sync(0xffffffffu, st_y, sl);
+                        gz = __shfl_sync(0xffffffffu, st_z, sl);
                     }
+                }
+                return true;
+            };
+            bool more = next();
+            float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (more && cb + lane < e) qn = pos32[cb + lane];
+            while (more || queued > 0) {
+                if (more) {
+                    float4 q = qn;
+                    const int j = cb + lane;
+                    const bool in_range = j < e;
+                    q.x += gx;
+                    q.y += gy;
+                    q.z += gz;
+                    more = next();
+                    if (more && cb + lane < e) qn = pos32[cb + lane];
+                    const float ex = (ALL3 || pf.use[0]) ? fmaxf(0.f, fmaxf(b0x - q.x, q.x - b1x)) : 0.f;
+                    const float ey = (ALL3 || pf.use[1]) ? fmaxf(0.f, fmaxf(b0y - q.y, q.y - b1y)) : 0.f;
+                    const float ez = (ALL3 || pf.use[2]) ? fmaxf(0.f, fmaxf(b0z - q.z, q.z - b1z)) : 0.f;
+                    const bool near =
+                        in_range && __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez))) <= pf.r2_box;
                     const unsigned kept = __ballot_sync(0xffffffffu, near);
-                    __syncwarp();
                     if (near) {
-                        q.w = __int_as_float(lane);
-                        cw[__popc(kept & ((1u << lane) - 1u))] = q;
+                        q.w = __int_as_float(j);
+                        queue[(head + queued + __popc(kept & ((1u << lane) - 1u))) & 63] = q;
                     }
+                    queued += __popc(kept);
                     __syncwarp();
-                    const int m = __popc(kept);
-                    // per candidate of the stage: may be within rm (mask), needs the
-                    // FP64 test (exact: in a shell of the rm or the rs bound), within
-                    // rs for certain (in_s)
-                    unsigned mask = 0u, exact = 0u, in_s = 0u;
-                    if (take) {
-                        for (int t = 0; t < m; ++t) {
-                            const float4 q = cw[t];
-                            const float fx = (ALL3 || pf.use[0]) ? q.x + ox : 0.f;
-                            const float fy = (ALL3 || pf.use[1]) ? q.y + oy : 0.f;
-                            const float fz = (ALL3 || pf.use[2]) ? q.z + oz : 0.f;
-                            // FMA: fewer roundings than the bound allows for
-                            const float r2f = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, __fmul_rn(fz, fz)));
-                            if (r2f <= pf.r2_hi) {
-                                const unsigned bit = 1u << t;
-                                mask |= bit;
-                                if (r2f > pf.r2_lo || (short_list && r2f > pf.rs2_lo && r2f <= pf.rs2_hi))
-                                    exact |= bit;
-                                else if (r2f <= pf.rs2_lo)
-                                    in_s |= bit;
-                            }
-                        }
-                    }
-                    while (mask) {
-                        const int t = __ffs(mask) - 1;
-                        const unsigned bit = mask & (0u - mask);
-                        mask &= mask - 1u;
-                        const int j = cb + __float_as_int(cw[t].w);
-                        bool in = true, in_short = (in_s & bit) != 0u;
-                        if (exact & bit) {
-                            const double4 pj = pos[j];
-                            const double q0 = omod_fast(pj.x - pi.x + c.half_width[0], c.width[0]) - c.half_width[0];
-                            const double q1 = omod_fast(pj.y - pi.y + c.half_width[1], c.width[1]) - c.half_width[1];
-                            const double q2 = omod_fast(pj.z - pi.z + c.half_width[2], c.width[2]) - c.half_width[2];
-                            const double r2 = q0 * q0 + q1 * q1 + q2 * q2;
-                            in = r2 <= c.rm2;
-                            in_short = r2 <= c.rs2;
-                        }
-                        if (in) {
-                            if (cnt < cap) nlist[(size_t)cnt * n + i] = j;
-                            cnt++;
-                            if (short_list && in_short) {
-                                if (cnt_s < cap_s) nlist_s[(size_t)cnt_s * n + i] = j;
-                                cnt_s++;
-                            }
-                        }
-                    }
+                }
+                if (queued >= 32 || (!more && queued > 0)) {
+                    const int m = min(queued, 32);
+                    test(m);
+                    head += m;
+                    queued -= m;
+                    __syncwarp();
                 }
             }
         }
-        if (active) {
+        if (lane < np) {
+            const int i = __float_as_int(homes[lane].w);
             ncount[i] = cnt;
-            atomicMax(&scal->max_neighbors, cnt);
-            if (cnt > cap) atomicOr(&scal->flags, DEVFLAG_NEIGHBOR_OVERFLOW);
-            if (short_list) {
-                ncount_s[i] = cnt_s;
-                atomicMax(&scal->max_short, cnt_s);
-                if (cnt_s > cap_s) atomicOr(&scal->flags, DEVFLAG_NEIGHBOR_OVERFLOW);
-            }
+            ncount_s[i] = cnt_s;
+            most = max(most, cnt);
+            most_s = max(most_s, cnt_s);
         }
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    most_s = __reduce_max_sync(0xffffffffu, most_s);
+    if (lane == 0) {
+        atomicMax(&scal->max_neighbors, most);
+        atomicMax(&scal->max_short, most_s);
+        if (most > cap || most_s > cap_s) atomicOr(&scal->flags, DEVFLAG_NEIGHBOR_OVERFLOW);
     }
 }
 
@@ -431,7 +527,7 @@ void launch_reorder(const SimConst& c, const int* vals, const int* pidx_in, cons
 
 // Bound of the prefilter (see k_neighbor_list).  An FP32 coordinate in
 // [0, W) is within 2^-24 W of its FP64 value (two coordinates: 2 * 2^-24 W);
-// a component is formed as q + (offset - p_i) with |offset - p_i| < 2W
+// a component is formed as (q + offset) - p_i with |q + offset| < 2W
 // (2 * 2^-24 W more) and a small result (less than 2^-24 W more), so each
 // component is within e = 5 * 2^-24 * W of the FP64 minimum-image
 // displacement (W rounded to FP32 for the offset adds 2^-24 W), which is
@@ -453,6 +549,7 @@ Prefilter make_prefilter(const SimConst& c) {
     for (int d = 0; d < 3; ++d) {
         pf.use[d] = c.cc[d] >= 4 && c.range[d] == 1;
         pf.width[d] = (float)c.width[d];
+        pf.cell_width[d] = (float)c.cell_width[d];
         if (pf.use[d]) wmax = std::fmax(wmax, c.width[d]);
     }
     const double e = 8.0 * std::ldexp(wmax, -24);
@@ -492,15 +589,20 @@ void launch_pos32(const SimConst& c, const double4* pos, float4* pos32, cudaStre
 void launch_neighbor_list(const SimConst& c, const double4* pos, const float4* pos32, const int* cellstart,
                           int* ncount, int* nlist, int cap, int* ncount_s, int* nlist_s, int cap_s,
                           StepScalars* scal, cudaStream_t s) {
-    const long long keys = 2LL * c.tot;
+    // Warps per key: enough to fill the GPU in small scenes.  Measured in us per
+    // build at 1, 2, 4, 6 warps: 3-D, 20,116 particles 360 / 186 / 106 / 101; 213,868 474 /
+    // 333 / 311 / 327; 2,779,256 4403 / 4368 / 4607 / 4879 (each warp sorts its key's
+    // particles anew); 2-D (13 particles a key), 22,500 50 / 36 / 37 / 42; 90,000 84 / 85 / 103 / 122.
+    const int key_warps = c.dim == 2 ? (c.n <= 50000 ? 2 : 1) : (c.n <= 250000 ? 4 : 2);
+    const long long warps = 2LL * c.tot * key_warps;
     const Prefilter pf = make_prefilter(c);
-    const int nb = (int)((keys + kListWarps - 1) / kListWarps);
+    const int nb = (int)((warps + kListWarps - 1) / kListWarps);
     if (pf.use[0] && pf.use[1] && pf.use[2])
         k_neighbor_list<true><<<nb, 32 * kListWarps, 0, s>>>(c, pos, pos32, pf, cellstart, ncount, nlist, cap,
-                                                              ncount_s, nlist_s, cap_s, scal);
+                                                              ncount_s, nlist_s, cap_s, scal, key_warps);
     else
         k_neighbor_list<false><<<nb, 32 * kListWarps, 0, s>>>(c, pos, pos32, pf, cellstart, ncount, nlist, cap,
-                                                               ncount_s, nlist_s, cap_s, scal);
+                                                               ncount_s, nlist_s, cap_s, scal, key_warps);
 }
 
 void launch_pack3(int n, const double4* src, double* dst, cudaStream_t s) {

@@ -122,32 +122,34 @@ __device__ __forceinline__ void disp(const SimConst& c, const double4& pi, const
     disp(c, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, x);
 }
 
-// Visits the cnt entries of one particle's list (column lp, rows n apart) in
-// order: visit(j, load(j)).  Indices are loaded two to three entries ahead and
-// records one ahead, so the gathers overlap the previous pair's FP64
-// arithmetic; two entries per trip, so the records alternate between two sets
-// of registers instead of being moved.  With disp's single branch and
-// pair_root's, 158 -> 123 instructions per entry of the force sweep (2.60 -> 2.34
-// ms on the 2,779,256-particle dam break, 0.81 -> 0.75 ms on the 314,432-particle
-// column).
+// Visits the cnt entries of particle i's list in order: visit(j, load(j)).  Two
+// indices are loaded at a time, two to three entries ahead, and records one entry
+// ahead, so the gathers overlap the previous pair's FP64 arithmetic; two entries
+// per trip, so the records alternate between two sets of registers instead of
+// being moved.  With disp's single branch and pair_root's, 158 -> 123 instructions
+// per entry of the force sweep (2.60 -> 2.34 ms on the 2,779,256-particle dam break, 0.81
+// -> 0.75 ms on the 314,432-particle column).  Whole rows of four indices and four entries
+// per trip take more registers: 2.38 ms.
 template <class Load, class Visit>
-__device__ __forceinline__ void walk_list(const int* __restrict__ lp, size_t n, int cnt, Load&& load, Visit&& visit) {
+__device__ __forceinline__ void walk_list(const int* __restrict__ list, size_t n, int i, int cnt, Load&& load,
+                                          Visit&& visit) {
     if (cnt <= 0) return;
-    int ja = __ldg(lp), jb = cnt > 1 ? __ldg(lp + n) : ja;
+    const int* lp = list + list_at(0, n, i);
+    const size_t row = 4 * n - 2;  // from the second half of a row to the next row
+    int2 q = __ldg(reinterpret_cast<const int2*>(lp));
+    int ja = q.x, jb = cnt > 1 ? q.y : q.x;
     auto a = load(ja);
     for (int k = 0;; k += 2) {
-        lp += 2 * n;
-        int jc = ja, jd = jb;
-        if (k + 2 < cnt) jc = __ldg(lp);
-        if (k + 3 < cnt) jd = __ldg(lp + n);
+        lp += (k & 2) ? row : (size_t)2;
+        if (k + 2 < cnt) q = __ldg(reinterpret_cast<const int2*>(lp));
         auto b = load(jb);
         visit(ja, a);
         if (k + 1 >= cnt) break;
-        a = load(jc);
+        a = load(q.x);  // past the end: a record again, not visited
         visit(jb, b);
         if (k + 2 >= cnt) break;
-        ja = jc;
-        jb = jd;
+        ja = q.x;
+        jb = k + 3 < cnt ? q.y : q.x;
     }
 }
 
@@ -288,7 +290,7 @@ k_sweep_a(SimConst c, const double2* __restrict__ xv, const int* __restrict__ ty
     const size_t n = (size_t)c.n;
     double sum_a = 0.0, sum_p = 0.0, sum_d = 0.0;
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    walk_list(nlist_p + i, n, ncount_p[i], [&](int j) { return ld_xv(xv, j); }, [&](int j, const XV& pj) {
+    walk_list(nlist_p, n, i, ncount_p[i], [&](int j) { return ld_xv(xv, j); }, [&](int j, const XV& pj) {
         // DensityP, DivergenceP
         double x[3];
         disp(c, pi, pj, x);
@@ -308,7 +310,7 @@ k_sweep_a(SimConst c, const double2* __restrict__ xv, const int* __restrict__ ty
         sum_d -= u2 * e2 * dw;
     });
     if (ST) {  // DensityA, GravityCenter
-        walk_list(nlist + i, n, ncount[i],
+        walk_list(nlist, n, i, ncount[i],
                   [&](int j) { return XVT{ld_xv(xv, j), RATIO ? __ldg(type + j) : 0}; },  // unused words: no loads
                   [&](int j, const XVT& rj) {
             double x[3];
@@ -369,18 +371,16 @@ __global__ void __launch_bounds__(128) k_density_a(SimConst c, const double4* __
     const int cnt = ncount[i];
     const size_t n = (size_t)c.n;
     double sum_a = 0.0;
-    for (int k = 0; k < cnt; ++k) {
-        const int j = __ldg(nlist + (size_t)k * n + i);
-        const double4 pj = ld_d4(pos, j);
+    walk_list(nlist, n, i, cnt, [&](int j) { return ld_d4(pos, j); }, [&](int j, const double4& pj) {
         double x[3];
         disp(c, pi, pj, x);
         const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
         double r;
         Recip ri;
-        if (!pair_root(r2, r2 <= c.ra2, j == i, r, ri)) continue;
+        if (!pair_root(r2, r2 <= c.ra2, j == i, r, ri)) return;
         const double qa = div_q(r, c.ra, recip_const(c.inv_ra, c.inv_ra_lo));
         sum_a += RATIO ? c.ratio[ti][type_of(pj)] * s_wa(c, qa) : s_wa(c, qa);
-    }
+    });
     dens_a[i] = sum_a;
     double pa = c.cof_a[ti] * (sum_a - c.n0a) / c.l0;
     if (c.n0a <= sum_a) pa = 0.0;
@@ -437,7 +437,7 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
     double fv0 = 0.0, fv1 = 0.0, fv2 = 0.0;
     {  // PressureP force (main.cpp:1908-1938) over the short sublist
         const double ppi = velp[i].w;
-        walk_list(nlist_s + i, n, ncount_s[i],
+        walk_list(nlist_s, n, i, ncount_s[i],
                   [&](int j) { return XVP{ld_xv(xv, j), __ldg(&velp[j].w)}; },
                   [&](int j, const XVP& rj) {
             double x[3];
@@ -462,7 +462,7 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
         double4 gci = make_double4(0, 0, 0, 0);
         if (ST) gci = gcpa[i];        // .w = PressureA
         constexpr bool TYPES = RATIO || !MU1;
-        walk_list(nlist + i, n, ncount[i],
+        walk_list(nlist, n, i, ncount[i],
                   [&](int j) { return XVT{ld_xv(xv, j), TYPES ? __ldg(type + j) : 0}; },
                   [&](int j, const XVT& rj) {
             const XV& pj = rj.p;
@@ -592,16 +592,16 @@ struct GroupStage {
 // add(stage, column of the particle's first entry) sums the G staged entries.
 // Indices are loaded two trips ahead and records one.
 template <int G, int NV, class Load, class Eval, class Add>
-__device__ __forceinline__ void group_walk(GroupStage<NV>& st, const int* __restrict__ lp, size_t n, int cnt, int self,
+__device__ __forceinline__ void group_walk(GroupStage<NV>& st, const int* __restrict__ list, size_t n, int cnt, int self,
                                            Load&& load, Eval&& eval, Add&& add) {
     const int lane = threadIdx.x & 31, sub = lane & (G - 1);
     const int most = __reduce_max_sync(0xffffffffu, cnt);
-    int ja = sub < cnt ? __ldg(lp + (size_t)sub * n) : self;
-    int jb = sub + G < cnt ? __ldg(lp + (size_t)(sub + G) * n) : self;
+    int ja = sub < cnt ? __ldg(list + list_at(sub, n, self)) : self;
+    int jb = sub + G < cnt ? __ldg(list + list_at(sub + G, n, self)) : self;
     auto a = load(ja);
     for (int k0 = 0; k0 < most; k0 += G) {
         int jc = self;
-        if (k0 + 2 * G + sub < cnt) jc = __ldg(lp + (size_t)(k0 + 2 * G + sub) * n);
+        if (k0 + 2 * G + sub < cnt) jc = __ldg(list + list_at(k0 + 2 * G + sub, n, self));
         const auto b = load(jb);
         double v[NV];
 #pragma unroll
@@ -643,7 +643,7 @@ k_sweep_a_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
     const int ti = type[i];
     const size_t n = (size_t)c.n;
     double acc = 0.0;  // lane 0: DensityP; lane 1: DivergenceP (three terms per entry)
-    group_walk<G, 4>(st, nlist_p + i, n, on ? ncount_p[i] : 0, i, [&](int j) { return ld_xv(xv, j); },
+    group_walk<G, 4>(st, nlist_p, n, on ? ncount_p[i] : 0, i, [&](int j) { return ld_xv(xv, j); },
                      [&](int j, const XV& pj, double* v) {
         double x[3];
         disp(c, pi, pj, x);
@@ -676,7 +676,7 @@ k_sweep_a_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
     double sum_a = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
     if (ST) {  // DensityA, GravityCenter: sum s on lane s
         double as = 0.0;
-        group_walk<G, 4>(st, nlist + i, n, on ? ncount[i] : 0, i,
+        group_walk<G, 4>(st, nlist, n, on ? ncount[i] : 0, i,
                          [&](int j) { return XVT{ld_xv(xv, j), RATIO ? __ldg(type + j) : 0}; },
                          [&](int j, const XVT& rj, double* v) {
             double x[3];
@@ -769,7 +769,7 @@ k_sweep_b_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
     {  // PressureP over the short sublist
         const double ppi = velp[i].w;
         GroupStage<3>& sp = reinterpret_cast<GroupStage<3>&>(st);
-        group_walk<G, 3>(sp, nlist_s + i, n, on ? ncount_s[i] : 0, i,
+        group_walk<G, 3>(sp, nlist_s, n, on ? ncount_s[i] : 0, i,
                          [&](int j) { return XVP{ld_xv(xv, j), __ldg(&velp[j].w)}; },
                          [&](int j, const XVP& rj, double* v) {
             double x[3];
@@ -800,7 +800,7 @@ k_sweep_b_g(SimConst c, const double2* __restrict__ xv, const int* __restrict__ 
         const double ai = ST ? c.a_k[ti] : 0.0;
         double4 gci = make_double4(0, 0, 0, 0);
         if (ST) gci = gcpa[i];        // .w = PressureA
-        group_walk<G, NV>(st, nlist + i, n, on ? ncount[i] : 0, i,
+        group_walk<G, NV>(st, nlist, n, on ? ncount[i] : 0, i,
                           [&](int j) { return XVT{ld_xv(xv, j), __ldg(type + j)}; },
                           [&](int j, const XVT& rj, double* v) {
             const XV& pj = rj.p;
@@ -1019,7 +1019,7 @@ k_virial(SimConst c, const double4* __restrict__ pos, const double4* __restrict_
     struct Rec {
         double4 p, v;
     };
-    walk_list(nlist + i, (size_t)c.n, ncount[i],
+    walk_list(nlist, (size_t)c.n, i, ncount[i],
               [&](int j) { return Rec{ld_d4(pos, j), ld_d4(vel, j)}; },
               [&](int j, const Rec& rj) {
         double x[3];
@@ -1227,7 +1227,7 @@ __global__ void __launch_bounds__(128) k_edge_fill(const int* __restrict__ ncoun
     const int b = eoff[i], cnt = ncount[i];
     for (int k = 0; k < cnt; ++k) {
         ei[b + k] = i;
-        ej[b + k] = nlist[(size_t)k * n + i];
+        ej[b + k] = nlist[list_at(k, (size_t)n, i)];
     }
 }
 

@@ -56,6 +56,12 @@ struct SimConst {
     double wall_rot[MPH_TYPE_COUNT][3][3];
 };
 
+// Entry k of particle i's neighbour list: the tables hold rows of four entries,
+// [cap / 4][n][4].
+__host__ __device__ inline size_t list_at(int k, size_t n, int i) {
+    return ((size_t)(k >> 2) * n + (size_t)i) * 4 + (size_t)(k & 3);
+}
+
 // Small per-step device scalars (one cache line, read back with one copy).
 struct StepScalars {
     unsigned long long max_shift2_bits;  // max |shift|^2 as ordered bits (>= 0)
@@ -98,10 +104,10 @@ struct DevFP64 {
     int* vals = nullptr;                    // CellParticle, pow2 entries
     int* cellstart = nullptr;               // 2*tot+1: #keys below each key value
     int* ncount = nullptr;                  // NeighborCount
-    int* nlist = nullptr;                   // [cap][n] column-major list
+    int* nlist = nullptr;                   // [cap / 4][n][4] (list_at)
     int cap = 0;
     int* ncount_s = nullptr;                // short sublist: the entries
-    int* nlist_s = nullptr;                 // within rs2, in list order, [cap_s][n]
+    int* nlist_s = nullptr;                 // within rs2, in list order, [cap_s / 4][n][4]
     int cap_s = 0;
     double* wall_center = nullptr;          // [4][3], advanced on the device
     double* staging = nullptr;              // [n][3] pack/unpack buffer
@@ -123,6 +129,7 @@ void launch_reorder(const SimConst& c, const int* vals, const int* pidx_in, cons
 struct Prefilter {
     int use[3];
     float width[3];
+    float cell_width[3];
     float r2_hi;   // per pair: FP32 distance squared at or below it for every pair within rm
     float r2_box;  // per candidate: FP32 distance squared to the box around a warp's particles
     float r2_lo;   // FP32 distance squared at or below it: within rm in FP64 for certain (-1: never)

@@ -148,7 +148,7 @@ int main(int argc, char** argv) {
         // mph_step call while no output falls between them (no VTK after, no
         // prof before, the loop not ending), found by running the loop's own
         // Time additions and tests ahead.  One call of several steps keeps
-        // the rebuild test on the device (step graphs).
+        // the rebuild test on the device.
         int k = 1;
         {
             double t = Time;
