@@ -102,7 +102,7 @@ extern "C" int mph_model_gradient(mph_model* m, const float* samples, long long 
     CU(cudaMalloc(&ds.p, bytes));
     CU(cudaMemcpyAsync(ds.p, samples, bytes, cudaMemcpyHostToDevice, m->m.stream));
     double l = 0.0;
-    const int rc = mph::mlp::model_grad(&m->m, (const float4*)ds.p, nullptr, n, &l, err);
+    const int rc = mph::mlp::model_grad(&m->m, (const float4*)ds.p, n, &l, err);
     if (rc) return map_rc(rc);
     CU(cudaMemcpyAsync(grad, m->m.grad, mph::mlp::NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->m.stream));
     CU(cudaStreamSynchronize(m->m.stream));
@@ -226,34 +226,42 @@ extern "C" int mph_model_train(mph_model* m, mph_dataset* d, int epochs, int bat
     std::string* err = &m->err;
     Model* md = &m->m;
     const long long n = d->n;
-    std::vector<long long> idx((size_t)n);
-    std::iota(idx.begin(), idx.end(), 0LL);
+    // 32-bit sample numbers: 2^32 samples of 48 bytes do not fit the device
+    std::vector<uint32_t> idx((size_t)n);
+    std::iota(idx.begin(), idx.end(), 0u);
     std::mt19937_64 rng(seed);
-    DevBuf order;
-    CU(cudaMalloc(&order.p, (size_t)n * sizeof(long long)));
+    if (md->order_cap < n) {
+        cudaFree(md->order);
+        md->order = nullptr;
+        md->order_cap = 0;
+        CU(cudaMalloc(&md->order, (size_t)n * sizeof(uint32_t)));
+        md->order_cap = n;
+    }
     const long long nb = (n + batch - 1) / batch;
     const long long total = nb * (long long)epochs;
     long long step = 0;
     double last = 0.0;
+    std::vector<float> rate((size_t)std::min<long long>(nb, mph::mlp::kLossSlots));
+    std::vector<double> l(rate.size());
     for (int ep = 0; ep < epochs; ++ep) {
         std::shuffle(idx.begin(), idx.end(), rng);
-        CU(cudaMemcpyAsync(order.p, idx.data(), (size_t)n * sizeof(long long), cudaMemcpyHostToDevice, md->stream));
+        CU(cudaMemcpyAsync(md->order, idx.data(), (size_t)n * sizeof(uint32_t), cudaMemcpyHostToDevice, md->stream));
         double sum = 0.0;
-        for (long long b = 0; b < nb; ++b, ++step) {
-            const long long first = b * batch, cnt = std::min<long long>(batch, n - first);
-            double l = 0.0;
-            int rc = mph::mlp::model_grad(md, d->s, (const long long*)order.p + first, cnt, &l, err);
+        for (long long b = 0; b < nb; b += mph::mlp::kLossSlots) {
+            const int k = (int)std::min<long long>(mph::mlp::kLossSlots, nb - b);
+            const long long first = b * batch, cnt = std::min<long long>((long long)k * batch, n - first);
+            for (int q = 0; q < k; ++q, ++step) {
+                // cosine decay to 5 % of the initial rate
+                const double frac = total > 1 ? (double)step / (double)(total - 1) : 1.0;
+                rate[q] = (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979323846 * frac))));
+            }
+            const int rc =
+                mph::mlp::model_train(md, d->s, md->order + first, cnt, batch, k, rate.data(), l.data(), err);
             if (rc) return map_rc(rc);
-            sum += l * (double)cnt;
-            // cosine decay to 5 % of the initial rate
-            const double frac = total > 1 ? (double)step / (double)(total - 1) : 1.0;
-            const double rate = lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979323846 * frac)));
-            rc = mph::mlp::model_adam(md, (float)rate, 0.9f, 0.999f, 1e-8f, err);
-            if (rc) return map_rc(rc);
+            for (int q = 0; q < k; ++q) sum += l[q] * (double)std::min<long long>(batch, n - (b + q) * batch);
         }
         last = sum / (double)n;
     }
-    CU(cudaStreamSynchronize(md->stream));
     if (loss) *loss = last;
     return MPH_OK;
 }

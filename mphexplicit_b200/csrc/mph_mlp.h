@@ -63,7 +63,9 @@ struct Model {
     float* gpart = nullptr;   // per-CTA partial gradients [ctas][NPARAM]
     double* lossp = nullptr;  // per-CTA loss partials
     uint8_t* image = nullptr; // packed BF16 image [PK_BYTES]
-    int* err = nullptr;       // device error flag (tensor-core wait timeout)
+    int* err = nullptr;       // device error flag (tensor-core wait timeout), update count, loss sums
+    uint32_t* order = nullptr;  // a training epoch's order of the samples [order_cap]
+    long long order_cap = 0;
     int ctas = 0;
     long long adam_t = 0;
     Scales sc{1.f, 1.f, 1.f, 0.f};
@@ -76,13 +78,17 @@ void model_destroy(Model* m);
 // upload FP32 parameters (and repack), read them back
 int model_set_params(Model* m, const float* host, std::string* err);
 int model_get_params(Model* m, float* host, std::string* err);
-// one pass of forward + backward over `n` device samples (indices `order`
-// into `samples`, or 0..n-1 when order is null); the gradient of the mean
-// squared error of the scaled outputs lands in m->grad, the loss in *loss
-int model_grad(Model* m, const float4* samples, const long long* order, long long n, double* loss,
-               std::string* err);
-// Adam update from m->grad, then repack the BF16 image
-int model_adam(Model* m, float lr, float beta1, float beta2, float eps, std::string* err);
+// one pass of forward + backward over `n` device samples; the gradient of the
+// mean squared error of the scaled outputs lands in m->grad, the loss in *loss
+int model_grad(Model* m, const float4* samples, long long n, double* loss, std::string* err);
+// `nb` <= kLossSlots batches of training: batch b is the samples order[b * batch ..]
+// (device, at most `batch` of them, `n` over all batches), one Adam update (0.9,
+// 0.999, 1e-8) at rate lr[b], its loss before the update in loss[b].  The batches are
+// launched one after the other with one wait at the end; after a wait that
+// timed out on the device no further update is made (-5).
+constexpr int kLossSlots = 1024;
+int model_train(Model* m, const float4* samples, const uint32_t* order, long long n, int batch, int nb,
+                const float* lr, double* loss, std::string* err);
 // predictions for `n` device samples: out[e] = (fx, fy, fz, 0) in N (scaled back)
 int model_predict(Model* m, const float4* samples, long long n, float4* out, std::string* err);
 
