@@ -34,11 +34,12 @@ constexpr int kCodeBits = 5;  // 27 neighbour-cell offsets
 #ifndef MPH_MIXB_MINB_FUSED
 #define MPH_MIXB_MINB_FUSED 8
 #endif
-// ... and of its surface-tension variants (more live values per pair): on the
-// 8.5 M-particle two-fluid column 10.06 ms at 8 blocks (some spilling), 10.28
-// at 6 and 11.06 at 5, results identical.
+// ... and of its surface-tension variants (more live values per pair).  They were
+// bound by the latency of the gravity centre's gather, sent after the distance test, and
+// spilled at 8 blocks: 730 us a launch on the 592,704-particle two-fluid column.  With the
+// four centres of a row gathered with its records: 619 at 6 blocks, 656 at 5, 709 at 7.
 #ifndef MPH_MIXB_MINB_ST
-#define MPH_MIXB_MINB_ST 8
+#define MPH_MIXB_MINB_ST 6
 #endif
 // Resident 128-thread blocks per SM of the table-free force sweep.
 #ifndef MPH_WALK_MINB
@@ -52,6 +53,7 @@ struct MixConst {
     double grid, inv_grid;             // hi-part grid (a power of two, metres)
     float dhi[27][4];                  // cell-origin offset per code: hi part (on the grid)
     float dlo[27][4];                  //                              lo part
+    float half_cell[3];                // half of dhi's step of one cell
     float list_r2, short_r2;           // (MaxRadius+m)^2, (RP+m)^2
     float walk_r2, walk_short2;        // cell walk: (largest force radius + s)^2, (RP + s)^2, s = 8 grid steps
     float ra2, rp2, rv2, rg2;
@@ -141,29 +143,65 @@ __global__ void k_mix_cellkey(SimConst c, const double4* __restrict__ pos, int* 
     slot[i] = atomicAdd(&counts[id], 1);
 }
 
-// Exclusive scan of counts[0..m) into out[0..m] (out[m] = total), one block:
-// each thread scans a contiguous chunk; chunk totals are scanned in shared memory.
-__global__ void __launch_bounds__(1024) k_mix_scan(const int* __restrict__ counts, int m, int* __restrict__ out) {
-    __shared__ int part[1024];
-    const int t = threadIdx.x;
-    const int chunk = (m + blockDim.x - 1) / blockDim.x;
-    const int b = min(m, t * chunk), e = min(m, b + chunk);
-    int s = 0;
-    for (int k = b; k < e; ++k) s += counts[k];
-    part[t] = s;
+// Exclusive scan of counts[0..m) into out[0..m] (out[m] = total).  Two launches,
+// 4096 keys a block: the blocks' sums, then every block adds up the sums before its
+// own and scans its keys.  (One block scanning all keys was a serial chain of 130
+// loads a thread: 179 us a build at 130,000 keys, 1,526,488 particles; now 10 us.)
+constexpr int kScanThreads = 1024, kScanKeys = 4096;
+
+__device__ __forceinline__ int block_scan(int v, int* part, int& total) {  // exclusive
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += a;
+    }
+    if (lane == 31) part[w] = x;
     __syncthreads();
-    for (int off = 1; off < (int)blockDim.x; off <<= 1) {  // Hillis-Steele inclusive scan
-        const int v = t >= off ? part[t - off] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int k = 0; k < kScanThreads / 32; ++k) {
+        const int q = part[k];
+        if (k < w) before += q;
+        total += q;
     }
-    int run = part[t] - s;
-    for (int k = b; k < e; ++k) {
-        out[k] = run;
-        run += counts[k];
+    __syncthreads();
+    return before + x - v;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_mix_scan_sums(const int* __restrict__ counts, int m,
+                                                                int* __restrict__ sums) {
+    __shared__ int part[kScanThreads / 32];
+    int v = 0, total;
+    for (int q = 0; q < kScanKeys / kScanThreads; ++q) {
+        const int k = blockIdx.x * kScanKeys + q * kScanThreads + threadIdx.x;
+        if (k < m) v += counts[k];
     }
-    if (t == blockDim.x - 1) out[m] = part[t];
+    block_scan(v, part, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+k_mix_scan(const int* __restrict__ counts, int m, const int* __restrict__ sums, int* __restrict__ out) {
+    __shared__ int part[kScanThreads / 32];
+    int before = 0, total;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += kScanThreads) before += sums[k];
+    block_scan(before, part, total);
+    constexpr int kEach = kScanKeys / kScanThreads;
+    const int k0 = blockIdx.x * kScanKeys + threadIdx.x * kEach;
+    int cnt[kEach], v = 0;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        cnt[q] = k0 + q < m ? counts[k0 + q] : 0;
+        v += cnt[q];
+    }
+    before = total;
+    int run = before + block_scan(v, part, total);
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        if (k0 + q <= m) out[k0 + q] = run;  // the last key's end is the total
+        run += cnt[q];
+    }
 }
 
 __global__ void k_mix_place(int n, const int* __restrict__ keys, const int* __restrict__ slot,
@@ -417,11 +455,28 @@ k_mix_move(SimConst c, MixConst m, const int* __restrict__ cellstart, double4* _
     }
 }
 
+// The hi offset of a code from one 32-bit word instead of four: per axis two bits
+// that read, as the top bits of a float, 0.0, +2.0 or -2.0 for an offset of 0, 1 or
+// -1 cells, so pj + offset is one FMA with half a cell's (rounded) width.  The
+// offsets are these multiples of the grid exactly, so the sum is the same.  A
+// shared-memory word at 27 addresses takes one wavefront of the L1 data pipe, the
+// four words of dhi took 4.7 of the 30 that a long pair cost.
+__device__ __forceinline__ unsigned cell_steps(int code) {
+    const unsigned x = (unsigned)(code / 9 + 3) & 3u, y = (unsigned)(code / 3 % 3 + 3) & 3u,
+                   z = (unsigned)(code % 3 + 3) & 3u;  // 0, 1, 2 -> 3, 0, 1
+    return x << 30 | y << 28 | z << 26;
+}
+
+__device__ __forceinline__ float add_step(float a, unsigned steps, float half_width) {
+    return fmaf(__uint_as_float(steps & 0xc0000000u), half_width, a);
+}
+
 // Offset tables in shared memory: per-lane codes differ, and shared memory
 // serves divergent addresses in one access where the constant bank serialises.
 struct SharedTables {
     float4 dhi[27];
     float4 dlo[27];
+    unsigned steps[27];  // cell_steps
     float mu[MPH_TYPE_COUNT * MPH_TYPE_COUNT];
 };
 
@@ -429,6 +484,7 @@ __device__ __forceinline__ void load_tables(const MixConst& m, SharedTables& t) 
     for (int k = threadIdx.x; k < 27; k += blockDim.x) {
         t.dhi[k] = make_float4(m.dhi[k][0], m.dhi[k][1], m.dhi[k][2], 0.f);
         t.dlo[k] = make_float4(m.dlo[k][0], m.dlo[k][1], m.dlo[k][2], 0.f);
+        t.steps[k] = cell_steps(k);
     }
     for (int k = threadIdx.x; k < 16; k += blockDim.x) t.mu[k] = m.visc_mu[k / 4][k % 4];
     __syncthreads();
@@ -488,7 +544,7 @@ __device__ __forceinline__ void wp_df(const MixConst& m, float hx, float hy, flo
 // coefficients, PressureP, PressureA (main.cpp:1631-1662, 1735-1740, 1831-1906).
 template <bool ST, bool RATIO, bool S64>
 __global__ void __launch_bounds__(128)
-k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ v32,
+k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p32, const float4* __restrict__ v32,
         const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
         float4* __restrict__ pv, float4* __restrict__ gca, double* __restrict__ strain_out,
         double* __restrict__ div_out, double* __restrict__ dens_a_out, double* __restrict__ wall_center,
@@ -557,15 +613,28 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ v
         }
         if (ST) st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r, dx, dy, dz, sa, cak, g0, g1, g2);
     });
-    if (ST) {  // surface tension only: the long part
-        for_entries(tab + (size_t)(m.cap_s >> 2) * n, n, na - ns, [&](unsigned e) {
-            const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
-            const float4 pj = phl[2 * (size_t)j];
-            const float4 dh = tb.dhi[code];
-            const float dx = (pj.x - pi.x) + dh.x, dy = (pj.y - pi.y) + dh.y, dz = (pj.z - pi.z) + dh.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rsqrtf(r2), dx, dy, dz, sa, cak, g0, g1, g2);
-        });
+    if (ST) {  // surface tension only: the long part, on the 16-byte hi records
+        const uint4* tl = tab + (size_t)(m.cap_s >> 2) * n;
+        const int nl = na - ns;
+        for (int k = 0; k < nl; k += 4, tl += n) {
+            const uint4 q = __ldg(tl);
+            const unsigned e[4] = {q.x, q.y, q.z, q.w};
+            float4 pj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < nl) pj[u] = __ldg(p32 + (e[u] >> kCodeBits));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < nl) {
+                    const unsigned st = tb.steps[e[u] & 31u];
+                    const float dx = add_step(pj[u].x - pi.x, st, m.half_cell[0]),
+                                dy = add_step(pj[u].y - pi.y, st << 2, m.half_cell[1]),
+                                dz = add_step(pj[u].z - pi.z, st << 4, m.half_cell[2]);
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    st_density<RATIO>(m, ti, __float_as_int(pj[u].w), r2, r2 * rsqrtf(r2), dx, dy, dz, sa, cak, g0, g1,
+                                      g2);
+                }
+        }
     }
     double strain, div;
     if (S64) {
@@ -605,6 +674,13 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ v
 // sums.  The long part: the hi displacement, ViscosityV (+ surface tension),
 // plain FP32 sum.  Then gravity and the FP64 velocity update
 // (main.cpp:1908-2010).
+//
+// What bounds it: the L1 data pipe (94 % of its cycles without surface tension), which
+// spends 17.6 of them on a warp's gather, one for each 128-byte line that holds
+// some of its 32 records.  With the offset's one word (cell_steps) a launch takes 656 us
+// instead of 696 at 1,024,000 fluid particles.  A thread per two neighbouring particles
+// with a common list gathered once took 884: the warp runs the longest of its lanes'
+// lists, and the order within cells that keeps its records in few lines is lost.
 template <bool ST, bool RATIO, bool WALLS>
 __global__ void __launch_bounds__(128, ST ? MPH_MIXB_MINB_ST : MPH_MIXB_MINB_FUSED)
 k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4* __restrict__ phl,
@@ -663,10 +739,19 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     });
     // long part: a row of four pairs per iteration, their gathers issued
     // together so a thread keeps four independent loads in flight
-    auto long_pair = [&](unsigned e, const float4& pj, const float4& vj) {
-        const int code = (int)(e & 31u);
-        const float4 dh = tb.dhi[code];
-        const float dx = (pj.x - pi.x) + dh.x, dy = (pj.y - pi.y) + dh.y, dz = (pj.z - pi.z) + dh.z;
+    auto long_pair = [&](unsigned e, const float4& pj, const float4& vj, const float4& gj) {
+        float dx, dy, dz;
+        if (ST) {  // short of registers: the table's three words cost less (619 us against 623 on the column, and the steps' words spill at 8 blocks)
+            const float4 dh = tb.dhi[e & 31u];
+            dx = (pj.x - pi.x) + dh.x;
+            dy = (pj.y - pi.y) + dh.y;
+            dz = (pj.z - pi.z) + dh.z;
+        } else {
+            const unsigned st = tb.steps[e & 31u];
+            dx = add_step(pj.x - pi.x, st, m.half_cell[0]);
+            dy = add_step(pj.y - pi.y, st << 2, m.half_cell[1]);
+            dz = add_step(pj.z - pi.z, st << 4, m.half_cell[2]);
+        }
         const float r2 = dx * dx + dy * dy + dz * dz;
         const float rinv = rsqrtf(r2);
         float s = 0.0f;
@@ -678,9 +763,8 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
         }
         if (ST) {
             if (r2 < m.ra2 || r2 < m.rg2) {
-                const int j = (int)(e >> kCodeBits);
                 float3 t = make_float3(0.f, 0.f, 0.f);
-                s += st_terms<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gca[j], ai, t);
+                s += st_terms<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gj, ai, t);
                 gx += t.x;
                 gy += t.y;
                 gz += t.z;
@@ -695,13 +779,16 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     for (int k = 0; k < nl; k += 4) {
         const uint4 q = __ldg(tl + (size_t)(k >> 2) * n);
         const unsigned e[4] = {q.x, q.y, q.z, q.w};
-        float4 pj[4], vj[4];
+        float4 pj[4], vj[4], gj[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (k + u < nl) ldg_pv(pv, (int)(e[u] >> kCodeBits), pj[u], vj[u]);
+            if (k + u < nl) {
+                ldg_pv(pv, (int)(e[u] >> kCodeBits), pj[u], vj[u]);
+                if (ST) gj[u] = __ldg(gca + (e[u] >> kCodeBits));
+            }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (k + u < nl) long_pair(e[u], pj[u], vj[u]);
+            if (k + u < nl) long_pair(e[u], pj[u], vj[u], gj[u]);
     }
     double F0 = ((double)fx - (double)cx) + (double)gx;
     double F1 = ((double)fy - (double)cy) + (double)gy;
@@ -1033,6 +1120,7 @@ struct MixedState {
     int* keys_unsorted = nullptr;
     int* slot = nullptr;
     int* counts = nullptr;
+    int* sums = nullptr;  // of the scan's blocks
     int* tmp = nullptr;
     int* home = nullptr;
     float4* phl = nullptr;  // [2n]: {hi position + type, lo position} per particle (home-cell relative)
@@ -1054,7 +1142,7 @@ struct MixedState {
 };
 
 static void mfree(MixedState* m) {
-    void* ptrs[] = {m->keys_unsorted, m->slot, m->counts, m->tmp, m->home, m->phl, m->p32, m->v32, m->pv,
+    void* ptrs[] = {m->keys_unsorted, m->slot, m->counts, m->sums, m->tmp, m->home, m->phl, m->p32, m->v32, m->pv,
                     m->gca, m->list, m->cnt_short, m->cnt_all};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1094,7 +1182,8 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     int nl = 0;
     MTRY(cudaMemsetAsync(m->counts, 0, sizeof(int) * (size_t)(nb + 1), s));
     k_mix_cellkey<<<blocks(n, 256), 256, 0, s>>>(c, d.pos[a], m->keys_unsorted, m->slot, m->counts);
-    k_mix_scan<<<1, 1024, 0, s>>>(m->counts, nb, d.cellstart);
+    k_mix_scan_sums<<<blocks(nb + 1, kScanKeys), kScanThreads, 0, s>>>(m->counts, nb, m->sums);
+    k_mix_scan<<<blocks(nb + 1, kScanKeys), kScanThreads, 0, s>>>(m->counts, nb, m->sums, d.cellstart);
     k_mix_place<<<blocks(n, 256), 256, 0, s>>>(n, m->keys_unsorted, m->slot, d.cellstart, m->tmp);
     k_mix_rank<<<blocks(n, 256), 256, 0, s>>>(n, m->keys_unsorted, d.cellstart, m->tmp, d.vals, d.keys);
     launch_reorder(c, d.vals, d.pidx[a], d.type[a], d.pos[a], d.vel[va], d.pidx[b], d.type[b], d.pos[b], d.vel[vb],
@@ -1103,7 +1192,7 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     d.vcur = vb;
     k_mix_home<<<blocks(n, 256), 256, 0, s>>>(c, m->mc, d.pos[d.cur], d.keys, d.vel[d.vcur], m->home, m->phl,
                                               m->p32, m->v32);
-    nl += 6;
+    nl += 7;
     for (int attempt = 0; attempt < 3; ++attempt) {
         MTRY(cudaMemsetAsync(&d.scal->max_neighbors, 0, sizeof(int), s));
         MTRY(cudaMemsetAsync(&d.scal->max_short, 0, 2 * sizeof(int), s));
@@ -1135,7 +1224,7 @@ void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wa
     const int nb = blocks(c.n, 128);
     double* wc = advance_wall ? d.wall_center : nullptr;
 #define MIX_A(ST, RATIO, S64)                                                                                   \
-    k_mix_a<ST, RATIO, S64><<<nb, 128, 0, s>>>(m->mc, m->phl, m->v32, m->list, m->cnt_short,          \
+    k_mix_a<ST, RATIO, S64><<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short,          \
                                                m->cnt_all, m->pv, m->gca, d.strain_p, d.div_p, d.dens_a, wc, c, \
                                                d.vel[d.vcur], d.press)
 #define MIX_A2(ST, RATIO) \
@@ -1232,6 +1321,8 @@ int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, De
         }
         mc.dhi[code][3] = mc.dlo[code][3] = 0.0f;
     }
+    const int one[3] = {22, 16, 14};  // the codes of one cell up along x, y, z
+    for (int dd = 0; dd < 3; ++dd) mc.half_cell[dd] = 0.5f * mc.dhi[one[dd]][dd];
     mc.uniform_mu = 1;
     for (int t = 0; t < MPH_TYPE_COUNT; ++t)
         for (int u = 0; u < MPH_TYPE_COUNT; ++u)
@@ -1300,6 +1391,7 @@ int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, De
     if (e == cudaSuccess) e = malloc_n(&m->keys_unsorted, n);
     if (e == cudaSuccess) e = malloc_n(&m->slot, n);
     if (e == cudaSuccess) e = malloc_n(&m->counts, 2 * (size_t)c.tot + 1);
+    if (e == cudaSuccess) e = malloc_n(&m->sums, (size_t)blocks(2LL * c.tot + 1, kScanKeys));
     if (e == cudaSuccess) e = malloc_n(&m->tmp, n);
     if (e == cudaSuccess) e = malloc_n(&m->home, n);
     if (e == cudaSuccess) e = malloc_n(&m->phl, 2 * n);
