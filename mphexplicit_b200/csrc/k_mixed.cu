@@ -667,6 +667,40 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
     div_out[i] = div;
 }
 
+// Surface-tension terms of one pair (PressureA, DiffuseInterface with aj the
+// a of i as the reference has it, main.cpp:1742-1828); returns the radial
+// part and adds the tangential part to t.  The difference of the two gravity
+// centres, scaled by a of i, is formed once per axis (exact product, one rounding) and
+// shared by the kernel's and its derivative's term; with every product formed anew, as
+// the batched sweeps' st_terms has it, the force sweep of the 592,704-particle column took 707
+// us instead of 619.
+template <bool RATIO>
+__device__ __forceinline__ float st_force(const MixConst& m, int ti, int tj, float r2, float r, float rinv, float dx,
+                                          float dy, float dz, const float4& gi, const float4& gj, float ai,
+                                          float3& t) {
+    const float rij = RATIO ? m.ratio[ti][tj] : 1.0f, rji = RATIO ? m.ratio[tj][ti] : 1.0f;
+    float s = 0.0f;
+    if (r2 < m.ra2) {
+        const float q = r * m.inv_ra;
+        const float dwa = (m.ca_inv * m.vol) * (1.0f - q) * fmaf(-3.0f, q, 1.0f);
+        s = (RATIO ? fmaf(gi.w, rij, gj.w * rji) : gi.w + gj.w) * dwa * rinv;
+    }
+    if (r2 < m.rg2) {
+        const float q = 1.0f - r * m.inv_rg;
+        const float k1 = m.inv_r2g_rg * m.vol_over_l0;
+        const float wg = (m.cg * k1) * q * q, dwg = (m.cg_m2 * k1) * q;
+        const float bi = RATIO ? ai * rij : ai, bj = RATIO ? ai * rji : ai;
+        const float d0 = fmaf(bj, gj.x, -(bi * gi.x)), d1 = fmaf(bj, gj.y, -(bi * gi.y)),
+                    d2 = fmaf(bj, gj.z, -(bi * gi.z));
+        t.x = fmaf(-d0, wg, t.x);
+        t.y = fmaf(-d1, wg, t.y);
+        t.z = fmaf(-d2, wg, t.z);
+        const float gr = fmaf(d2, dz, fmaf(d0, dx, d1 * dy));
+        s = fmaf(-gr, dwg * rinv, s);
+    }
+    return s;
+}
+
 // Sweep B for fluid particles (WALLS: for the wall particles, output only),
 // FP32 in both mixed forms (the FP64 density sweep of MPH_MODE_MIXED_P64 sets
 // the pressures this sweep reads).  The short part of the list: exact
@@ -732,7 +766,7 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
             s += mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
         }
         float3 t = make_float3(0.f, 0.f, 0.f);
-        if (ST) s += st_terms<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gca[j], ai, t);
+        if (ST) s += st_force<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gca[j], ai, t);
         kahan_add(fx, cx, fmaf(s, dx, t.x));
         kahan_add(fy, cy, fmaf(s, dy, t.y));
         kahan_add(fz, cz, fmaf(s, dz, t.z));
@@ -764,7 +798,7 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
         if (ST) {
             if (r2 < m.ra2 || r2 < m.rg2) {
                 float3 t = make_float3(0.f, 0.f, 0.f);
-                s += st_terms<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gj, ai, t);
+                s += st_force<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gj, ai, t);
                 gx += t.x;
                 gy += t.y;
                 gz += t.z;
@@ -948,7 +982,7 @@ k_mix_b_walk(MixConst m, SimConst c, const int* __restrict__ cellstart, const fl
                                             sc += mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
                                         }
                                         float3 tt = make_float3(0.f, 0.f, 0.f);
-                                        if (ST) sc += st_terms<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gstage[q], ai, tt);
+                                        if (ST) sc += st_force<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gstage[q], ai, tt);
                                         kahan_add(fx, cx, fmaf(sc, dx, tt.x));
                                         kahan_add(fy, cy, fmaf(sc, dy, tt.y));
                                         kahan_add(fz, cz, fmaf(sc, dz, tt.z));
@@ -964,7 +998,7 @@ k_mix_b_walk(MixConst m, SimConst c, const int* __restrict__ cellstart, const fl
                                         if (ST) {
                                             if (r2h < m.ra2 || r2h < m.rg2) {
                                                 float3 tt = make_float3(0.f, 0.f, 0.f);
-                                                sc += st_terms<RATIO>(m, ti, tj, r2h, r2h * rinv, rinv, hx, hy, hz, gi,
+                                                sc += st_force<RATIO>(m, ti, tj, r2h, r2h * rinv, rinv, hx, hy, hz, gi,
                                                                       gstage[q], ai, tt);
                                                 gx += tt.x;
                                                 gy += tt.y;

@@ -53,9 +53,7 @@ __device__ __forceinline__ void st_density(const K& m, int ti, int tj, float r2,
 
 // Surface-tension terms of one pair (PressureA, DiffuseInterface with aj the
 // a of i as the reference has it, main.cpp:1742-1828); returns the radial
-// part and adds the tangential part to t.  The difference of the two gravity
-// centres, scaled by a of i, is formed once per axis (exact product, one rounding) and
-// shared by the kernel's and its derivative's term.
+// part and adds the tangential part to t.
 template <bool RATIO, int DIM = 3, class K>
 __device__ __forceinline__ float st_terms(const K& m, int ti, int tj, float r2, float r, float rinv, float dx,
                                           float dy, float dz, const float4& gi, const float4& gj, float ai,
@@ -64,24 +62,22 @@ __device__ __forceinline__ float st_terms(const K& m, int ti, int tj, float r2, 
     float s = 0.0f;
     if (r2 < m.ra2) {
         const float q = r * m.inv_ra;
-        const float dwa = (m.ca_inv * m.vol) * (1.0f - q) * fmaf(-3.0f, q, 1.0f);
-        s = (RATIO ? fmaf(gi.w, rij, gj.w * rji) : gi.w + gj.w) * dwa * rinv;
+        const float dwa = m.ca_inv * (1.0f - q) * (1.0f - 3.0f * q);
+        s += (gi.w * rij * dwa + gj.w * rji * dwa) * rinv * m.vol;
     }
     if (r2 < m.rg2) {
         const float q = 1.0f - r * m.inv_rg;
+        const float wg = m.cg * q * q, dwg = m.cg_m2 * q;
         const float k1 = m.inv_r2g_rg * m.vol_over_l0;
-        const float wg = (m.cg * k1) * q * q, dwg = (m.cg_m2 * k1) * q;
-        const float bi = RATIO ? ai * rij : ai, bj = RATIO ? ai * rji : ai;
-        const float d0 = fmaf(bj, gj.x, -(bi * gi.x)), d1 = fmaf(bj, gj.y, -(bi * gi.y));
-        t.x = fmaf(-d0, wg, t.x);
-        t.y = fmaf(-d1, wg, t.y);
-        float gr = fmaf(d0, dx, d1 * dy);
+        t.x -= (ai * gj.x * rji * wg - ai * gi.x * rij * wg) * k1;
+        t.y -= (ai * gj.y * rji * wg - ai * gi.y * rij * wg) * k1;
+        float gr = (ai * gj.x * rji * dwg - ai * gi.x * rij * dwg) * dx +
+                   (ai * gj.y * rji * dwg - ai * gi.y * rij * dwg) * dy;
         if (DIM == 3) {  // in 2-D every z part is zero
-            const float d2 = fmaf(bj, gj.z, -(bi * gi.z));
-            t.z = fmaf(-d2, wg, t.z);
-            gr = fmaf(d2, dz, gr);
+            t.z -= (ai * gj.z * rji * wg - ai * gi.z * rij * wg) * k1;
+            gr += (ai * gj.z * rji * dwg - ai * gi.z * rij * dwg) * dz;
         }
-        s = fmaf(-gr, dwg * rinv, s);
+        s -= gr * rinv * k1;
     }
     return s;
 }
