@@ -1219,15 +1219,35 @@ __global__ void __launch_bounds__(1024) k_edge_scan3(int* __restrict__ eoff, con
     if (i == 0) eoff[nf] = bsum[nb];
 }
 
+// The fluid's lists as CSR edges.  32 particles a block: the rows of the table
+// (512 bytes a warp) go through shared memory, 64 entries of each particle at a time,
+// and leave as consecutive entries of one particle.  (A thread per particle wrote
+// 4 bytes to 32 lines at once: 451 us for 23.1 M edges, now 78; 51 us for 0.2 M, now 14.)
+constexpr int kFillEntries = 64;
+
 __global__ void __launch_bounds__(128) k_edge_fill(const int* __restrict__ ncount, const int* __restrict__ nlist,
                                                    int n, int nf, const int* __restrict__ eoff, int* __restrict__ ei,
                                                    int* __restrict__ ej) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nf) return;
-    const int b = eoff[i], cnt = ncount[i];
-    for (int k = 0; k < cnt; ++k) {
-        ei[b + k] = i;
-        ej[b + k] = nlist[list_at(k, (size_t)n, i)];
+    __shared__ __align__(16) int tile[32][kFillEntries + 4];  // rows 4 banks apart
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * 32, i = i0 + lane;
+    const int cnt = i < nf ? ncount[i] : 0, b = i < nf ? eoff[i] : 0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    for (int k0 = 0; k0 < most; k0 += kFillEntries) {
+        for (int r = 4 * warp; r < kFillEntries; r += 16)
+            if (k0 + r < cnt)
+                *reinterpret_cast<int4*>(&tile[lane][r]) =
+                    reinterpret_cast<const int4*>(nlist)[(size_t)((k0 + r) >> 2) * n + i];
+        __syncthreads();
+        for (int q = warp; q < 32; q += 4) {
+            const int c = min(kFillEntries, __shfl_sync(0xffffffffu, cnt, q) - k0);
+            const int to = __shfl_sync(0xffffffffu, b, q) + k0;
+            for (int u = lane; u < c; u += 32) {
+                ei[to + u] = i0 + q;
+                ej[to + u] = tile[q][u];
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1472,7 +1492,7 @@ void launch_edge_offsets(const int* ncount, int nf, int* eoff, int* bsum, cudaSt
 
 void launch_edge_fill(const int* ncount, const int* nlist, int n, int nf, const int* eoff, int* ei, int* ej,
                       cudaStream_t s) {
-    if (nf > 0) k_edge_fill<<<blocks(nf, 128), 128, 0, s>>>(ncount, nlist, n, nf, eoff, ei, ej);
+    if (nf > 0) k_edge_fill<<<blocks(nf, 32), 128, 0, s>>>(ncount, nlist, n, nf, eoff, ei, ej);
 }
 
 void launch_collect(const SimConst& c, const double4* pos, const double4* press, const double4* gc, const int* ei,
