@@ -1352,6 +1352,7 @@ struct mph_batch {
     int4* d_items = nullptr;
     int* d_sid = nullptr;
     int2* d_items_t = nullptr;         // table form: sweep A's blocks, then sweep B's
+    char* slab = nullptr;              // the arrays of d, d_scenes and d_sid
     bool table_ok = false;             // the table fits: allocated at creation
     bool sorted = false;               // the initial sort is done
     bool table_valid = false;          // the table holds the lists of the current sort
@@ -1378,6 +1379,28 @@ static int bfail(mph_batch* b, int code, const std::string& msg) {
             return bfail(b, MPH_ERR_CUDA, std::string(#expr ": ") + cudaGetErrorString(e_)); \
     } while (0)
 
+// Device arrays that live as long as their batch, in one allocation (thirty of
+// their own cost a batch 0.5 to 4 ms: 64 droplets 20-31 ms to create, now 19-21; 24 dam
+// breaks 31, now 21-27).
+class Slab {
+public:
+    template <class T>
+    void want(T** p, size_t n) {
+        list_.push_back({(void**)p, bytes_});
+        bytes_ += ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+    }
+    cudaError_t alloc(char** base) {
+        const cudaError_t e = cudaMalloc((void**)base, bytes_);
+        if (e == cudaSuccess)
+            for (const auto& w : list_) *w.first = *base + w.second;
+        return e;
+    }
+
+private:
+    std::vector<std::pair<void**, size_t>> list_;
+    size_t bytes_ = 0;
+};
+
 template <class T>
 static cudaError_t balloc(T** p, size_t n) {
     *p = nullptr;
@@ -1395,10 +1418,7 @@ extern "C" void mph_batch_destroy(mph_batch* b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     free_graph(b);
-    BatchDev& d = b->d;
-    void* ptrs[] = {b->d_items_t, (void*)d.cell_scene, d.home, d.rel, d.v32, d.tile2, d.cfluid, d.fcount, d.flist, d.tab,
-                    d.tab_s, d.tcnt, d.tcnt_s, b->d_scenes, b->d_items, b->d_sid, d.pos, d.vel, d.snap, d.pidx, d.pos_t, d.vel_t, d.pidx_t,
-                    d.key, d.slot, d.tmp, d.counts, d.start, d.vp, d.gc, d.flags, d.ctl};
+    void* ptrs[] = {b->d_items_t, b->d_items, b->slab};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (auto& pe : b->prof.pending) {
@@ -1810,7 +1830,7 @@ static int lattice_count(int dim, double r) {
 // over the lattice's (longer ones are walked from the cells).  They cost 0.3 KB a
 // particle in 2-D and 1.3 KB in 3-D; where that is more than half of the free
 // memory the batch runs the tile sweeps.
-static cudaError_t alloc_table(mph_batch* b, int lat_l, int lat_s) {
+static cudaError_t want_table(mph_batch* b, int lat_l, int lat_s, Slab& slab) {
     BatchDev& d = b->d;
     const size_t n = (size_t)b->n, cells = (size_t)b->cells;
     d.tcap = ((int)(lat_l * 1.25) + 8 + 3) / 4 * 4;
@@ -1823,26 +1843,19 @@ static cudaError_t alloc_table(mph_batch* b, int lat_l, int lat_s) {
         b->table_ok = false;
         return cudaSuccess;
     }
-    std::vector<int> cs(cells);
-    for (int s = 0; s < b->S; ++s)
-        std::fill(cs.begin() + b->hs[s].cbase, cs.begin() + b->hs[s].cbase + b->hs[s].tot, s);
-    int* dcs = nullptr;
-    if ((e = balloc(&dcs, cells)) != cudaSuccess) return e;
-    d.cell_scene = dcs;
-    if ((e = balloc(&d.home, n)) != cudaSuccess) return e;
-    if ((e = balloc(&d.rel, n)) != cudaSuccess) return e;
-    if ((e = balloc(&d.v32, n)) != cudaSuccess) return e;
-    if (b->dim == 2 && (e = balloc(&d.tile2, n)) != cudaSuccess) return e;
-    if ((e = balloc(&d.cfluid, cells)) != cudaSuccess) return e;
-    if ((e = balloc(&d.fcount, (size_t)b->S)) != cudaSuccess) return e;
-    if ((e = balloc(&d.flist, (size_t)b->n_fluid)) != cudaSuccess) return e;
-    if ((e = balloc(&d.tab, n * (size_t)(d.tcap / 4))) != cudaSuccess) return e;
-    if ((e = balloc(&d.tab_s, n * (size_t)(d.tcap_s / 4))) != cudaSuccess) return e;
-    if ((e = balloc(&d.tcnt, n)) != cudaSuccess) return e;
-    if ((e = balloc(&d.tcnt_s, n)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(dcs, cs.data(), cells * sizeof(int), cudaMemcpyHostToDevice, b->stream)) != cudaSuccess)
-        return e;
-    return cudaStreamSynchronize(b->stream);
+    slab.want(&d.cell_scene, cells);
+    slab.want(&d.home, n);
+    slab.want(&d.rel, n);
+    slab.want(&d.v32, n);
+    if (b->dim == 2) slab.want(&d.tile2, n);
+    slab.want(&d.cfluid, cells);
+    slab.want(&d.fcount, (size_t)b->S);
+    slab.want(&d.flist, (size_t)b->n_fluid);
+    slab.want(&d.tab, n * (size_t)(d.tcap / 4));
+    slab.want(&d.tab_s, n * (size_t)(d.tcap_s / 4));
+    slab.want(&d.tcnt, n);
+    slab.want(&d.tcnt_s, n);
+    return cudaSuccess;
 }
 
 extern "C" int mph_batch_create(int n_scenes, const mph_params* params, const mph_grid_header* headers, int dim,
@@ -1953,37 +1966,32 @@ extern "C" int mph_batch_create(int n_scenes, const mph_params* params, const mp
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     BatchDev& d = b->d;
     const size_t n = (size_t)ntot;
-    if (e == cudaSuccess) e = balloc(&b->d_scenes, (size_t)n_scenes);
-    if (e == cudaSuccess) e = balloc(&b->d_sid, n);
-    if (e == cudaSuccess) e = balloc(&d.pos, n);
-    if (e == cudaSuccess) e = balloc(&d.vel, n);
-    if (e == cudaSuccess) e = balloc(&d.snap, n);
-    if (e == cudaSuccess) e = balloc(&d.pidx, n);
-    if (e == cudaSuccess) e = balloc(&d.pos_t, n);
-    if (e == cudaSuccess) e = balloc(&d.vel_t, n);
-    if (e == cudaSuccess) e = balloc(&d.pidx_t, n);
-    if (e == cudaSuccess) e = balloc(&d.key, n);
-    if (e == cudaSuccess) e = balloc(&d.slot, n);
-    if (e == cudaSuccess) e = balloc(&d.tmp, n);
-    if (e == cudaSuccess) e = balloc(&d.counts, (size_t)ctot);
-    if (e == cudaSuccess) e = balloc(&d.start, (size_t)ctot + 1);
-    if (e == cudaSuccess) e = balloc(&d.vp, n);
-    if (e == cudaSuccess) e = balloc(&d.gc, n);
-    if (e == cudaSuccess) e = balloc(&d.flags, (size_t)n_scenes);
-    if (e == cudaSuccess) e = balloc(&d.ctl, 8);
+    Slab slab;
+    slab.want(&b->d_scenes, (size_t)n_scenes);
+    slab.want(&b->d_sid, n);
+    slab.want(&d.pos, n);
+    slab.want(&d.vel, n);
+    slab.want(&d.snap, n);
+    slab.want(&d.pidx, n);
+    slab.want(&d.pos_t, n);
+    slab.want(&d.vel_t, n);
+    slab.want(&d.pidx_t, n);
+    slab.want(&d.key, n);
+    slab.want(&d.slot, n);
+    slab.want(&d.tmp, n);
+    slab.want(&d.counts, (size_t)ctot);
+    slab.want(&d.start, (size_t)ctot + 1);
+    slab.want(&d.vp, n);
+    slab.want(&d.gc, n);
+    slab.want(&d.flags, (size_t)n_scenes);
+    slab.want(&d.ctl, 8);
+    if (e == cudaSuccess && b->table_ok) e = want_table(b, tab_l, tab_s, slab);
+    if (e == cudaSuccess) e = slab.alloc(&b->slab);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_ctl, 8 * sizeof(int));
     if (e != cudaSuccess) {
         const std::string m = std::string("batch allocation: ") + cudaGetErrorString(e);
         mph_batch_destroy(b);
         return bfail(nullptr, MPH_ERR_NOMEM, m);
-    }
-    if (b->table_ok) {
-        e = alloc_table(b, tab_l, tab_s);
-        if (e != cudaSuccess) {
-            const std::string m = std::string("batch table: ") + cudaGetErrorString(e);
-            mph_batch_destroy(b);
-            return bfail(nullptr, MPH_ERR_NOMEM, m);
-        }
     }
     d.n = b->n;
     d.S = n_scenes;
@@ -2004,6 +2012,14 @@ extern "C" int mph_batch_create(int n_scenes, const mph_params* params, const mp
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d.flags, hflags.data(), hflags.size() * sizeof(int), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d.ctl, ctl0, sizeof(ctl0), cudaMemcpyHostToDevice, st);
+    std::vector<int> hcs;
+    if (b->table_ok) {
+        hcs.resize((size_t)ctot);
+        for (int s = 0; s < n_scenes; ++s)
+            std::fill(hcs.begin() + b->hs[s].cbase, hcs.begin() + b->hs[s].cbase + b->hs[s].tot, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync((void*)d.cell_scene, hcs.data(), hcs.size() * sizeof(int), cudaMemcpyHostToDevice, st);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // host vectors go out of scope below
     if (e != cudaSuccess) {
         const std::string m = std::string("batch upload: ") + cudaGetErrorString(e);

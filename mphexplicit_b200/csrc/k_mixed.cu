@@ -1264,7 +1264,7 @@ struct MixedState {
     int* keys_unsorted = nullptr;
     int* slot = nullptr;
     int* counts = nullptr;
-    int* sums = nullptr;  // of the scan's blocks
+    int* sums = nullptr;  // of the scan's blocks, behind counts
     int* tmp = nullptr;
     int* home = nullptr;
     float4* phl = nullptr;  // [2n]: {hi position + type, lo position} per particle (home-cell relative)
@@ -1286,7 +1286,7 @@ struct MixedState {
 };
 
 static void mfree(MixedState* m) {
-    void* ptrs[] = {m->keys_unsorted, m->slot, m->counts, m->sums, m->tmp, m->home, m->phl, m->p32, m->v32, m->pv,
+    void* ptrs[] = {m->keys_unsorted, m->slot, m->counts, m->tmp, m->home, m->phl, m->p32, m->v32, m->pv,
                     m->gca, m->list, m->cnt_short, m->cnt_all};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1534,8 +1534,8 @@ int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, De
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = malloc_n(&m->keys_unsorted, n);
     if (e == cudaSuccess) e = malloc_n(&m->slot, n);
-    if (e == cudaSuccess) e = malloc_n(&m->counts, 2 * (size_t)c.tot + 1);
-    if (e == cudaSuccess) e = malloc_n(&m->sums, (size_t)blocks(2LL * c.tot + 1, kScanKeys));
+    if (e == cudaSuccess) e = malloc_n(&m->counts, 2 * (size_t)c.tot + 1 + blocks(2LL * c.tot + 1, kScanKeys));
+    if (e == cudaSuccess) m->sums = m->counts + 2 * (size_t)c.tot + 1;
     if (e == cudaSuccess) e = malloc_n(&m->tmp, n);
     if (e == cudaSuccess) e = malloc_n(&m->home, n);
     if (e == cudaSuccess) e = malloc_n(&m->phl, 2 * n);

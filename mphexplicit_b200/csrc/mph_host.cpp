@@ -629,7 +629,6 @@ extern "C" void mph_destroy(mph_ctx* ctx) {
         cudaFree(R.stage_v);
         if (R.copy) cudaStreamDestroy(R.copy);
     }
-    if (ctx->ahead.seen) cudaFreeHost(ctx->ahead.seen);
     for (cudaEvent_t e : ctx->ahead.ev)
         if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -638,7 +637,8 @@ extern "C" void mph_destroy(mph_ctx* ctx) {
 
 static int create_impl(mph_ctx* ctx, const int* type, const double* xyz, const double* vel) {
     CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    CUDA_TRY(ctx, cudaMallocHost((void**)&ctx->h_scal, sizeof(StepScalars)));
+    CUDA_TRY(ctx, cudaMallocHost((void**)&ctx->h_scal, 3 * sizeof(StepScalars)));  // [1], [2]: Ahead::seen
+    ctx->ahead.seen = ctx->h_scal + 1;
     TRY(alloc_fp64(ctx));
     mph::DevFP64& d = ctx->d;
     const size_t n = (size_t)ctx->n;
@@ -765,8 +765,7 @@ static void sweep_b_part1(mph_ctx* ctx, double* vel_host, bool skip) {
 
 static int ahead_init(mph_ctx* ctx) {
     Ahead& A = ctx->ahead;
-    if (A.seen) return MPH_OK;
-    CUDA_TRY(ctx, cudaMallocHost((void**)&A.seen, 2 * sizeof(StepScalars)));
+    if (A.ev[1]) return MPH_OK;
     for (cudaEvent_t& e : A.ev) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return MPH_OK;
 }
