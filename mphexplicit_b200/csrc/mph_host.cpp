@@ -54,13 +54,15 @@ struct LearnedState {
     int* ei = nullptr;          // edge -> i
     int* ej = nullptr;          // edge -> j
     float4* eforce = nullptr;   // edge-MLP pair forces
+    char* edges = nullptr;      // the allocation of eforce, ei, ej
     long long ecap = 0, ne = 0;
     bool edges_valid = false;
     float4* lsum = nullptr;     // per-particle learned force
     double4* force_j = nullptr; // the judge's forces and velocities
     double4* vel_j = nullptr;
     double* sums = nullptr;     // device [3]
-    double* h_sums = nullptr;   // pinned [3]
+    double* h_sums = nullptr;   // pinned [3], behind mph_ctx::h_scal
+    char* slab = nullptr;       // the allocation of lsum, force_j, vel_j, sums
     int fallback_left = 0;
     mph_learned_info info{};
 };
@@ -610,15 +612,8 @@ extern "C" void mph_destroy(mph_ctx* ctx) {
     {
         LearnedState& L = ctx->lrn;
         cudaFree(L.eoff);
-        cudaFree(L.bsum);
-        cudaFree(L.ei);
-        cudaFree(L.ej);
-        cudaFree(L.eforce);
-        cudaFree(L.lsum);
-        cudaFree(L.force_j);
-        cudaFree(L.vel_j);
-        cudaFree(L.sums);
-        if (L.h_sums) cudaFreeHost(L.h_sums);
+        cudaFree(L.edges);
+        cudaFree(L.slab);
     }
     if (ctx->h_scal) cudaFreeHost(ctx->h_scal);
     {
@@ -637,8 +632,9 @@ extern "C" void mph_destroy(mph_ctx* ctx) {
 
 static int create_impl(mph_ctx* ctx, const int* type, const double* xyz, const double* vel) {
     CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    CUDA_TRY(ctx, cudaMallocHost((void**)&ctx->h_scal, 3 * sizeof(StepScalars)));  // [1], [2]: Ahead::seen
+    CUDA_TRY(ctx, cudaMallocHost((void**)&ctx->h_scal, 4 * sizeof(StepScalars)));  // [1], [2]: Ahead::seen
     ctx->ahead.seen = ctx->h_scal + 1;
+    ctx->lrn.h_sums = reinterpret_cast<double*>(ctx->h_scal + 3);
     TRY(alloc_fp64(ctx));
     mph::DevFP64& d = ctx->d;
     const size_t n = (size_t)ctx->n;
@@ -947,8 +943,8 @@ static int build_edges(mph_ctx* ctx) {
     cudaStream_t st = ctx->stream;
     const int nf = ctx->n_fluid;
     if (!L.eoff) {
-        TRY(dalloc(ctx, &L.eoff, (size_t)nf + 1));
-        TRY(dalloc(ctx, &L.bsum, (size_t)mph::edge_scan_blocks(nf) + 1));
+        TRY(dalloc(ctx, &L.eoff, (size_t)nf + 1 + mph::edge_scan_blocks(nf) + 1));
+        L.bsum = L.eoff + nf + 1;
     }
     {
         Launch Lc(ctx, "edge_offsets");
@@ -959,16 +955,17 @@ static int build_edges(mph_ctx* ctx) {
     CUDA_TRY(ctx, cudaMemcpyAsync(&ne, L.eoff + nf, sizeof(int), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(ctx, cudaStreamSynchronize(st));
     if (ne > L.ecap) {
-        cudaFree(L.ei);
-        cudaFree(L.ej);
-        cudaFree(L.eforce);
+        cudaFree(L.edges);
+        L.edges = nullptr;
         L.ei = L.ej = nullptr;
         L.eforce = nullptr;
         L.ecap = 0;
-        const long long cap = (long long)(ne * 1.2) + 1024;
-        TRY(dalloc(ctx, &L.ei, (size_t)cap));
-        TRY(dalloc(ctx, &L.ej, (size_t)cap));
-        if (ctx->mode == MPH_MODE_LEARNED) TRY(dalloc(ctx, &L.eforce, (size_t)cap));
+        const long long cap = ((long long)(ne * 1.2) + 1024 + 3) / 4 * 4;
+        const bool forces = ctx->mode == MPH_MODE_LEARNED;
+        TRY(dalloc(ctx, &L.edges, (size_t)cap * ((forces ? sizeof(float4) : 0) + 2 * sizeof(int))));
+        if (forces) L.eforce = reinterpret_cast<float4*>(L.edges);
+        L.ei = reinterpret_cast<int*>(L.edges + (forces ? (size_t)cap * sizeof(float4) : 0));
+        L.ej = L.ei + cap;
         L.ecap = cap;
     }
     L.ne = ne;
@@ -985,11 +982,11 @@ static int learned_buffers(mph_ctx* ctx) {
     LearnedState& L = ctx->lrn;
     if (L.lsum) return MPH_OK;
     const size_t n = (size_t)ctx->n;
-    TRY(dalloc(ctx, &L.lsum, n));
-    TRY(dalloc(ctx, &L.force_j, n));
-    TRY(dalloc(ctx, &L.vel_j, n));
-    TRY(dalloc(ctx, &L.sums, 3));
-    CUDA_TRY(ctx, cudaMallocHost((void**)&L.h_sums, 3 * sizeof(double)));
+    TRY(dalloc(ctx, &L.slab, n * (sizeof(*L.lsum) + sizeof(*L.force_j) + sizeof(*L.vel_j)) + 3 * sizeof(double)));
+    L.force_j = reinterpret_cast<double4*>(L.slab);
+    L.vel_j = L.force_j + n;
+    L.lsum = reinterpret_cast<float4*>(L.vel_j + n);
+    L.sums = reinterpret_cast<double*>(L.lsum + n);
     return MPH_OK;
 }
 
