@@ -230,17 +230,17 @@ int mph_create(const mph_params* p, const mph_grid_header* h, int dim, int mode,
 
 /* Advance nsteps explicit steps: the loop body main.cpp:386-431 plus
  * Time += Dt (main.cpp:449).  No file output.  Returns when the steps are
- * done.  Several FP64 steps are launched in batches ahead of the host: the
+ * done.  Several FP64 or mixed steps are launched in batches ahead of the host: the
  * move kernel's last block makes the neighbour-rebuild test on the device, and
  * once it fires the sweeps of that step and everything launched after it do
  * nothing until the host, a batch behind, has read the counters, rebuilt the
  * list and finished that step: the same kernels, so the same bits.  One step,
- * the mixed and learned forms, profiling on (mph_profile_enable), or launching
+ * the learned form, profiling on (mph_profile_enable), or launching
  * ahead off: the host reads the rebuild flag after each step's move. */
 int mph_step(mph_ctx* ctx, int nsteps);
 
 /* enable == 0: mph_step waits for every step's rebuild flag; 1 (the default):
- * several FP64 steps are launched ahead of the host (see mph_step).  The name
+ * several FP64 or mixed steps are launched ahead of the host (see mph_step).  The name
  * dates from when that was done with CUDA graphs.  Measured on one B200:
  * 0.025 against 0.040 ms per step on a 1,600-particle droplet. */
 int mph_set_step_graphs(mph_ctx* ctx, int enable);

@@ -495,13 +495,16 @@ k_mix_list(SimConst c, MixConst m, const float4* __restrict__ p32, const int* __
 
 // Convection, wall motion, periodic wrap and the displacement maximum (the
 // same FP64 expressions as the FP64 form's move), plus the FP32 copies of
-// position (home-relative, hi/lo) and velocity for the pair sweeps.
+// position (home-relative, hi/lo) and velocity for the pair sweeps.  AHEAD: a step
+// launched ahead of the host, with the counters and the rebuild test of k_move.
+template <bool AHEAD>
 __global__ void __launch_bounds__(256)
 k_mix_move(SimConst c, MixConst m, const int* __restrict__ cellstart, double4* __restrict__ pos,
            double4* __restrict__ vel, const double4* __restrict__ snap, const double* __restrict__ wall_center,
            const int* __restrict__ home, float4* __restrict__ phl, float4* __restrict__ p32,
            float4* __restrict__ v32, StepScalars* __restrict__ scal) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (AHEAD && scal->stop) return;  // set by an earlier launch only, or by this one's last block
     double s2 = 0.0;
     if (i < c.n) {
         const int nf = cellstart[c.tot], we = cellstart[2 * c.tot];
@@ -557,6 +560,18 @@ k_mix_move(SimConst c, MixConst m, const int* __restrict__ cellstart, double4* _
         double mx = red[0];
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = red[w] > mx ? red[w] : mx;
         if (mx > 0.0) atomicMax(&scal->max_shift2_bits, (unsigned long long)__double_as_longlong(mx));
+        if (AHEAD) {
+            __threadfence();
+            if (atomicAdd(&scal->blocks_done, 1u) == gridDim.x - 1) {  // the last block
+                __threadfence();
+                const unsigned long long bits = atomicAdd(&scal->max_shift2_bits, 0ull);
+                scal->last_shift2_bits = bits;
+                scal->max_shift2_bits = 0ull;
+                scal->blocks_done = 0u;
+                scal->steps_done += 1;
+                if (__longlong_as_double((long long)bits) > c.shift_thr) scal->stop = 1;
+            }
+        }
     }
 }
 
@@ -654,8 +669,9 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
         float4* __restrict__ pv, float4* __restrict__ gca, double* __restrict__ strain_out,
         double* __restrict__ div_out, double* __restrict__ dens_a_out, double* __restrict__ wall_center,
         const SimConst c, const double4* __restrict__ vel64,
-        double4* __restrict__ press64) {
+        double4* __restrict__ press64, const StepScalars* __restrict__ skip) {
     __shared__ SharedTables tb;
+    if (skip != nullptr && skip->stop) return;  // launched ahead of a step that has to rebuild
     load_tables(m, tb);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
@@ -826,8 +842,9 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
         const float4* __restrict__ pv, const float4* __restrict__ gca,
         const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
         const double4* __restrict__ vel, double4* __restrict__ vel_out, double4* __restrict__ force,
-        StepScalars* __restrict__ scal) {
+        StepScalars* __restrict__ scal, bool ahead) {
     __shared__ SharedTables tb;
+    if (ahead && scal->stop) return;
     load_tables(m, tb);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
@@ -973,7 +990,9 @@ template <bool ST, bool RATIO>
 __global__ void __launch_bounds__(32 * kWalkWarps, MPH_WALK_MINB)
 k_mix_b_walk(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4* __restrict__ phl,
              const float4* __restrict__ pv, const float4* __restrict__ gca, const double4* __restrict__ vel,
-             double4* __restrict__ vel_out, double4* __restrict__ force, StepScalars* __restrict__ scal) {
+             double4* __restrict__ vel_out, double4* __restrict__ force, StepScalars* __restrict__ scal,
+             bool ahead) {
+    if (ahead && scal->stop) return;
     __shared__ WalkRec stage_all[kWalkWarps][32];
     __shared__ float4 gstage_all[kWalkWarps][ST ? 32 : 1];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1364,13 +1383,13 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     return MPH_OK;
 }
 
-void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s) {
+void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s, bool ahead) {
     const int nb = blocks(c.n, 128);
     double* wc = advance_wall ? d.wall_center : nullptr;
 #define MIX_A(ST, RATIO, S64)                                                                                   \
     k_mix_a<ST, RATIO, S64><<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short,          \
                                                m->cnt_all, m->pv, m->gca, d.strain_p, d.div_p, d.dens_a, wc, c, \
-                                               d.vel[d.vcur], d.press)
+                                               d.vel[d.vcur], d.press, ahead ? d.scal : nullptr)
 #define MIX_A2(ST, RATIO) \
     if (m->s64) MIX_A(ST, RATIO, true); else MIX_A(ST, RATIO, false)
     if (m->mc.has_st) {
@@ -1384,13 +1403,13 @@ void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wa
 }
 
 template <bool WALLS>
-static void launch_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s) {
+static void launch_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
     const int nb = blocks(c.n, 128);
     double4* vout = WALLS ? nullptr : d.vel[1 - d.vcur];
 #define MIX_B1(ST, RATIO)                                                                                   \
     k_mix_b<ST, RATIO, WALLS><<<nb, 128, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca,   \
                                                  m->list, m->cnt_short, m->cnt_all, d.vel[d.vcur], vout,   \
-                                                 d.force, d.scal)
+                                                 d.force, d.scal, ahead)
     if (m->mc.has_st) {
         if (m->mc.ratio_all_one) { MIX_B1(true, false); } else { MIX_B1(true, true); }
     } else {
@@ -1399,11 +1418,11 @@ static void launch_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t 
 #undef MIX_B1
 }
 
-static void launch_b_walk(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s) {
+static void launch_b_walk(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
     const int nb = (2 * c.tot + kWalkWarps - 1) / kWalkWarps;
 #define MIX_W(ST, RATIO)                                                                                      \
     k_mix_b_walk<ST, RATIO><<<nb, 32 * kWalkWarps, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca,    \
-                                                          d.vel[d.vcur], d.vel[1 - d.vcur], d.force, d.scal)
+                                                          d.vel[d.vcur], d.vel[1 - d.vcur], d.force, d.scal, ahead)
     if (m->mc.has_st) {
         if (m->mc.ratio_all_one) { MIX_W(true, false); } else { MIX_W(true, true); }
     } else {
@@ -1412,18 +1431,23 @@ static void launch_b_walk(MixedState* m, const SimConst& c, DevFP64& d, cudaStre
 #undef MIX_W
 }
 
-int mixed_sweep_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s) {
-    if (m->walk) launch_b_walk(m, c, d, s);
-    else launch_b<false>(m, c, d, s);
+int mixed_sweep_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
+    if (m->walk) launch_b_walk(m, c, d, s, ahead);
+    else launch_b<false>(m, c, d, s, ahead);
     m->exported = false;
     return 1;
 }
 
 void mixed_set_cell_walk(MixedState* m, bool on) { m->walk = on; }
 
-void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s) {
-    k_mix_move<<<blocks(c.n, 256), 256, 0, s>>>(c, m->mc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.snap,
-                                                d.wall_center, m->home, m->phl, m->p32, m->v32, d.scal);
+void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
+    const int nb = blocks(c.n, 256);
+    if (ahead)
+        k_mix_move<true><<<nb, 256, 0, s>>>(c, m->mc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.snap, d.wall_center,
+                                            m->home, m->phl, m->p32, m->v32, d.scal);
+    else
+        k_mix_move<false><<<nb, 256, 0, s>>>(c, m->mc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.snap, d.wall_center,
+                                             m->home, m->phl, m->p32, m->v32, d.scal);
     m->exported = false;
 }
 
@@ -1567,7 +1591,7 @@ int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, De
     int st = grow_list(m, (int)(lat_s * 1.1) + 4, (int)(lat_l * 1.1) + 8, c.n, err);
     if (st == MPH_OK) st = mixed_rebuild(m, c, d, s, err, nullptr);
     if (st == MPH_OK) {
-        mixed_sweep_a(m, c, d, false, s);
+        mixed_sweep_a(m, c, d, false, s, false);
         e = cudaGetLastError();
         if (e != cudaSuccess) {
             if (err) *err = cudaGetErrorString(e);
@@ -1591,7 +1615,7 @@ int mixed_export(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, s
                                                                d.dens_a);
             ++nl;
         }
-        launch_b<true>(m, c, d, s);  // wall forces
+        launch_b<true>(m, c, d, s, false);  // wall forces
         k_mix_counts<<<blocks(c.n, 256), 256, 0, s>>>(c.n, m->cnt_all, d.cellstart, c.tot, d.ncount);
         nl += 2;
         MTRY(cudaGetLastError());

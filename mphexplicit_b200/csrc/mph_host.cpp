@@ -766,9 +766,39 @@ static int ahead_init(mph_ctx* ctx) {
     return MPH_OK;
 }
 
+// The parts of a mixed step.
+static void mixed_move(mph_ctx* ctx, bool ahead) {
+    Launch L(ctx, "mix_move");
+    mph::mixed_move(ctx->mixed, ctx->sc, ctx->d, ctx->stream, ahead);
+}
+
+static int mixed_rebuild(mph_ctx* ctx) {
+    Launch L(ctx, "mix_rebuild");
+    const int rc = mph::mixed_rebuild(ctx->mixed, ctx->sc, ctx->d, ctx->stream, &ctx->err, &L.count);
+    if (rc != MPH_OK) return fail(ctx, rc, ctx->err);
+    ctx->ahead.since = 0;
+    ctx->ahead.shift2 = 0.0;
+    return MPH_OK;
+}
+
+static void mixed_sweeps(mph_ctx* ctx, bool ahead) {
+    {
+        Launch L(ctx, "mix_sweep_a");
+        mph::mixed_sweep_a(ctx->mixed, ctx->sc, ctx->d, true, ctx->stream, ahead);
+    }
+    Launch L(ctx, "mix_sweep_b");
+    L.count = mph::mixed_sweep_b(ctx->mixed, ctx->sc, ctx->d, ctx->stream, ahead);
+}
+
 // The three kernels of one step, to run only if no earlier step stopped.
 static void launch_step_ahead(mph_ctx* ctx, double* vel_host = nullptr) {
     mph::DevFP64& d = ctx->d;
+    if (ctx->mixed) {
+        mixed_move(ctx, true);
+        mixed_sweeps(ctx, true);
+        d.vcur = 1 - d.vcur;
+        return;
+    }
     {
         Launch L(ctx, "move");
         mph::launch_move_ahead(ctx->sc, d.cellstart, d.pos[d.cur], d.vel[d.vcur], d.xv, d.snap, d.wall_center, d.scal,
@@ -811,10 +841,15 @@ static int take_counters(mph_ctx* ctx, int slot, int launched, int* completed, b
 // The step that stopped: rebuild, then its sweeps (main.cpp:399-431).
 static int finish_stopped(mph_ctx* ctx, double* vel_host = nullptr) {
     CUDA_TRY(ctx, cudaMemsetAsync(&ctx->d.scal->stop, 0, sizeof(int), ctx->stream));
-    TRY(rebuild_fp64(ctx));
+    if (ctx->mixed) TRY(mixed_rebuild(ctx));
+    else TRY(rebuild_fp64(ctx));
     ++ctx->rebuilds;
-    sweep_a(ctx, true, false);
-    sweep_b_part1(ctx, vel_host, false);
+    if (ctx->mixed) {
+        mixed_sweeps(ctx, false);
+    } else {
+        sweep_a(ctx, true, false);
+        sweep_b_part1(ctx, vel_host, false);
+    }
     ctx->d.vcur = 1 - ctx->d.vcur;
     CUDA_TRY(ctx, cudaGetLastError());
     ctx->time += ctx->p.dt;
@@ -831,12 +866,12 @@ static int batch_steps(const mph_ctx* ctx) {
     return (int)std::min(16.0, std::max(1.0, 0.5 * left / rate));
 }
 
-// nsteps FP64 steps with the host one batch behind the GPU: while a batch runs the
+// nsteps FP64 or mixed steps with the host one batch behind the GPU: while a batch runs the
 // next one is launched, then the first one's counters are read.  Measured against
 // the CUDA graphs with conditional nodes this replaced: 36 -> 25 us per step on
 // the 1,600-particle droplet (21 us of kernels), no graph to instantiate on the
 // first call, and rebuilds on the host's path (tables grow as they always do).
-static int step_fp64_ahead(mph_ctx* ctx, int nsteps) {
+static int step_ahead(mph_ctx* ctx, int nsteps) {
     mph::DevFP64& d = ctx->d;
     TRY(ahead_init(ctx));
     int left = nsteps;  // steps not yet completed
@@ -881,7 +916,7 @@ static int step_fp64_ahead(mph_ctx* ctx, int nsteps) {
 
 static int step_fp64(mph_ctx* ctx, int nsteps) {
     // several steps: launched ahead (per-kernel profiling needs the host path)
-    if (nsteps > 1 && ctx->ahead.enabled && !ctx->prof.on) return step_fp64_ahead(ctx, nsteps);
+    if (nsteps > 1 && ctx->ahead.enabled && !ctx->prof.on) return step_ahead(ctx, nsteps);
     mph::DevFP64& d = ctx->d;
     for (int k = 0; k < nsteps; ++k) {
         TRY(step_fp64_head(ctx));
@@ -898,33 +933,24 @@ static int step_fp64(mph_ctx* ctx, int nsteps) {
 
 // The mixed form: same step order, its own kernels (k_mixed.cu).
 static int step_mixed(mph_ctx* ctx, int nsteps) {
+    if (nsteps > 1 && ctx->ahead.enabled && !ctx->prof.on) return step_ahead(ctx, nsteps);
     mph::DevFP64& d = ctx->d;
-    const SimConst& s = ctx->sc;
     cudaStream_t st = ctx->stream;
     for (int k = 0; k < nsteps; ++k) {
-        CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
-        {
-            Launch L(ctx, "mix_move");
-            mph::mixed_move(ctx->mixed, s, d, st);
-        }
+        mixed_move(ctx, false);
         TRY(read_scalars(ctx));
+        // the maximum starts at zero for the next move, whichever kind it is
+        CUDA_TRY(ctx, cudaMemsetAsync(&d.scal->max_shift2_bits, 0, sizeof(unsigned long long), st));
         TRY(check_flags(ctx));
         double ms;
         std::memcpy(&ms, &ctx->h_scal->max_shift2_bits, sizeof(double));
-        if (ms > s.shift_thr) {
-            Launch L(ctx, "mix_rebuild");
-            const int rc = mph::mixed_rebuild(ctx->mixed, s, d, st, &ctx->err, &L.count);
-            if (rc != MPH_OK) return fail(ctx, rc, ctx->err);
+        ++ctx->ahead.since;
+        ctx->ahead.shift2 = ms;
+        if (ms > ctx->sc.shift_thr) {
+            TRY(mixed_rebuild(ctx));
             ++ctx->rebuilds;
         }
-        {
-            Launch L(ctx, "mix_sweep_a");
-            mph::mixed_sweep_a(ctx->mixed, s, d, true, st);
-        }
-        {
-            Launch L(ctx, "mix_sweep_b");
-            L.count = mph::mixed_sweep_b(ctx->mixed, s, d, st);
-        }
+        mixed_sweeps(ctx, false);
         d.vcur = 1 - d.vcur;
         CUDA_TRY(ctx, cudaGetLastError());
         ctx->time += ctx->p.dt;  // main.cpp:449

@@ -16,15 +16,16 @@ struct MixedState;
 // (MPH_MODE_MIXED_P64).
 int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, DevFP64& d, bool fp64_pressure,
                  cudaStream_t s, std::string* err);
-// Convection/wall/periodic + displacement maximum + FP32 copies (1 launch).
-void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s);
+// Convection/wall/periodic + displacement maximum + FP32 copies (1 launch).  ahead, here
+// and below: of a step launched ahead of the host, to run only if no earlier one stopped.
+void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead);
 // Counting sort by cell, reorder, neighbour table; *launches gets the count.
 int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, std::string* err, int* launches);
 // Density sweep (1 launch); advance_wall moves the wall centres one step.
-void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s);
+void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s, bool ahead);
 // Force sweep (FP32 pairs) + FP64 velocity update into d.vel[1 - d.vcur];
 // returns the number of launches (1).
-int mixed_sweep_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s);
+int mixed_sweep_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead);
 // Force sweep by cell walk (no long table read) instead of the table sweep.
 void mixed_set_cell_walk(MixedState* m, bool on);
 // Fill the output-only fields (DensityA, wall forces, neighbour counts).

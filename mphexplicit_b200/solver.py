@@ -318,7 +318,7 @@ class Solver:
         _check(self._lib.mph_set_sweep_layout(self._ctx, code), self._ctx)
 
     def set_step_graphs(self, enable: bool) -> None:
-        """Several FP64 steps launched ahead of the host (default), or a wait per step."""
+        """Several FP64 or mixed steps launched ahead of the host (default), or a wait per step."""
         _check(self._lib.mph_set_step_graphs(self._ctx, 1 if enable else 0), self._ctx)
 
     def step_read_state(self, nsteps: int, xyz: np.ndarray | None, vel: np.ndarray | None) -> None:
