@@ -111,16 +111,29 @@ __device__ __forceinline__ void rel32(const SimConst& c, const MixConst& m, cons
 // The neighbour table holds entries in rows of four: entries 4r..4r+3 of
 // particle i are one uint4 at row r, column i (tab[r * n + i]), so a lane
 // writes 16 bytes at a time when the table is built and the lanes of a warp
-// read consecutive uint4 when it is swept.  Visits entries [0, cnt) in order.
-template <class F>
-__device__ __forceinline__ void for_entries(const uint4* __restrict__ tab, size_t n, int cnt, F&& f) {
-    for (int k = 0; k < cnt; k += 4) {
+// read consecutive uint4 when it is swept.  Visits entries [0, cnt) in order; with G
+// lanes per particle, lane sub's: every G-th row.
+template <int G = 1, class F>
+__device__ __forceinline__ void for_entries(const uint4* __restrict__ tab, size_t n, int cnt, F&& f, int sub = 0) {
+    for (int k = 4 * sub; k < cnt; k += 4 * G) {
         const uint4 q = __ldg(tab + (size_t)(k >> 2) * n);
         f(q.x);
         if (k + 1 < cnt) f(q.y);
         if (k + 2 < cnt) f(q.z);
         if (k + 3 < cnt) f(q.w);
     }
+}
+
+// The sum over a particle's G lanes, in each of them (mask: those lanes).
+template <int G, class T>
+__device__ __forceinline__ T lane_sum(unsigned mask, T v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+    return v;
+}
+template <int G>
+__device__ __forceinline__ unsigned lane_mask() {
+    return G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
 }
 
 // ---- counting sort by cell ------------------------------------------------
@@ -660,9 +673,10 @@ __device__ __forceinline__ void wp_df(const MixConst& m, float hx, float hy, flo
 // Sweep A: DensityP and DivergenceP over the short part of the list with the
 // exact FP32 displacement (S64: pair arithmetic in FP64, the displacement
 // assembled in FP64 from the hi/lo parts, FP32 velocities), plus, with
-// surface tension, DensityA and GravityCenter over all of it; epilogue:
+// surface tension, DensityA and GravityCenter over all of it, by G lanes per
+// particle (lanes_a), whose sums are added in FP64; epilogue:
 // coefficients, PressureP, PressureA (main.cpp:1631-1662, 1735-1740, 1831-1906).
-template <bool ST, bool RATIO, bool S64>
+template <bool ST, bool RATIO, bool S64, int G>
 __global__ void __launch_bounds__(128)
 k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p32, const float4* __restrict__ v32,
         const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
@@ -673,7 +687,7 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
     __shared__ SharedTables tb;
     if (skip != nullptr && skip->stop) return;  // launched ahead of a step that has to rebuild
     load_tables(m, tb);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = G == 1 ? 0 : (int)(threadIdx.x % G);
     if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
         const int t = threadIdx.x / 3, d = threadIdx.x % 3;
         if (t >= 2) wall_center[3 * t + d] += c.wall_velocity[t][d] * c.dt;
@@ -690,7 +704,7 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
     double spd = 0.0, sdd = 0.0;
     float sa = 0.f, cak = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
     const uint4* tab = reinterpret_cast<const uint4*>(list) + i;
-    for_entries(tab, n, ns, [&](unsigned e) {
+    for_entries<G>(tab, n, ns, [&](unsigned e) {
         const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
         float4 pj, lj;
         ldg_pv(phl, j, pj, lj);  // {hi, lo} in one 256-bit load
@@ -733,11 +747,11 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
             kahan_add(sd, cdk, -ue * dw);
         }
         if (ST) st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r, dx, dy, dz, sa, cak, g0, g1, g2);
-    });
+    }, sub);
     if (ST) {  // surface tension only: the long part, on the 16-byte hi records
-        const uint4* tl = tab + (size_t)(m.cap_s >> 2) * n;
+        const uint4* tl = tab + (size_t)((m.cap_s >> 2) + sub) * n;
         const int nl = na - ns;
-        for (int k = 0; k < nl; k += 4, tl += n) {
+        for (int k = 4 * sub; k < nl; k += 4 * G, tl += G * n) {
             const uint4 q = __ldg(tl);
             const unsigned e[4] = {q.x, q.y, q.z, q.w};
             float4 pj[4];
@@ -759,20 +773,31 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
     }
     double strain, div;
     if (S64) {
-        strain = spd - m.n0p_d;
+        strain = spd;
         div = sdd;
     } else {
-        // the pair sum is exact to ~2^-44: N0p is subtracted in FP64 (the
-        // strain is a small difference of two numbers near N0p)
-        strain = ((double)sph + (double)spl) - m.n0p_d;
+        strain = (double)sph + (double)spl;  // the pair sum is exact to ~2^-44
         div = (double)sd - (double)cdk;
     }
+    float dens = sa - cak;
+    if (G > 1) {
+        const unsigned mask = lane_mask<G>();
+        strain = lane_sum<G>(mask, strain);
+        div = lane_sum<G>(mask, div);
+        if (ST) {
+            dens = (float)lane_sum<G>(mask, (double)sa - (double)cak);
+            g0 = lane_sum<G>(mask, g0);
+            g1 = lane_sum<G>(mask, g1);
+            g2 = lane_sum<G>(mask, g2);
+        }
+        if (sub != 0) return;
+    }
+    strain -= m.n0p_d;  // the strain is a small difference of two numbers near N0p
     double kappa = c.bulk_modulus[ti];
     if (strain < 0.0) kappa = 0.0;
     const double pp = -c.bulk_viscosity[ti] * div + kappa * strain;
     float pa = 0.0f;
     if (ST) {
-        const float dens = sa - cak;
         pa = m.cof_a[ti] * (dens - m.n0a) / m.l0;
         if (m.n0a <= dens) pa = 0.0f;
         dens_a_out[i] = dens;
@@ -822,7 +847,8 @@ __device__ __forceinline__ float st_force(const MixConst& m, int ti, int tj, flo
     return s;
 }
 
-// Sweep B for fluid particles (WALLS: for the wall particles, output only),
+// Sweep B for fluid particles (WALLS: for the wall particles, output only), G lanes
+// per particle (lanes_b), whose forces are added in FP64,
 // FP32 in both mixed forms (the FP64 density sweep of MPH_MODE_MIXED_P64 sets
 // the pressures this sweep reads).  The short part of the list: exact
 // displacement, PressureP + ViscosityV (+ the surface-tension terms), Kahan
@@ -836,7 +862,7 @@ __device__ __forceinline__ float st_force(const MixConst& m, int ti, int tj, flo
 // instead of 696 at 1,024,000 fluid particles.  A thread per two neighbouring particles
 // with a common list gathered once took 884: the warp runs the longest of its lanes'
 // lists, and the order within cells that keeps its records in few lines is lost.
-template <bool ST, bool RATIO, bool WALLS>
+template <bool ST, bool RATIO, bool WALLS, int G>
 __global__ void __launch_bounds__(128, ST ? MPH_MIXB_MINB_ST : MPH_MIXB_MINB_FUSED)
 k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4* __restrict__ phl,
         const float4* __restrict__ pv, const float4* __restrict__ gca,
@@ -846,11 +872,11 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     __shared__ SharedTables tb;
     if (ahead && scal->stop) return;
     load_tables(m, tb);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = G == 1 ? 0 : (int)(threadIdx.x % G);
     if (i >= m.n) return;
     const int nf = cellstart[c.tot];
     if (WALLS ? i < nf : i >= nf) {
-        if (!WALLS) vel_out[i] = vel[i];
+        if (!WALLS && sub == 0) vel_out[i] = vel[i];
         return;
     }
     const float4 pi = phl[2 * (size_t)i];
@@ -866,7 +892,7 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;  // short part, Kahan
     float gx = 0.f, gy = 0.f, gz = 0.f;                                 // long part
     const uint4* tab = reinterpret_cast<const uint4*>(list) + i;
-    for_entries(tab, n, ns, [&](unsigned e) {
+    for_entries<G>(tab, n, ns, [&](unsigned e) {
         const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
         float4 pj, vj;
         ldg_pv(pv, j, pj, vj);
@@ -892,7 +918,7 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
         kahan_add(fx, cx, fmaf(s, dx, t.x));
         kahan_add(fy, cy, fmaf(s, dy, t.y));
         kahan_add(fz, cz, fmaf(s, dz, t.z));
-    });
+    }, sub);
     // long part: a row of four pairs per iteration, their gathers issued
     // together so a thread keeps four independent loads in flight
     auto long_pair = [&](unsigned e, const float4& pj, const float4& vj, const float4& gj) {
@@ -932,7 +958,7 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     };
     const uint4* tl = tab + (size_t)(m.cap_s >> 2) * n;
     const int nl = na - ns;
-    for (int k = 0; k < nl; k += 4) {
+    for (int k = 4 * sub; k < nl; k += 4 * G) {
         const uint4 q = __ldg(tl + (size_t)(k >> 2) * n);
         const unsigned e[4] = {q.x, q.y, q.z, q.w};
         float4 pj[4], vj[4], gj[4];
@@ -949,6 +975,13 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     double F0 = ((double)fx - (double)cx) + (double)gx;
     double F1 = ((double)fy - (double)cy) + (double)gy;
     double F2 = ((double)fz - (double)cz) + (double)gz;
+    if (G > 1) {
+        const unsigned mask = lane_mask<G>();
+        F0 = lane_sum<G>(mask, F0);
+        F1 = lane_sum<G>(mask, F1);
+        F2 = lane_sum<G>(mask, F2);
+        if (sub != 0) return;
+    }
     if (WALLS) {
         force[i] = make_double4(F0, F1, F2, 0.0);
         return;
@@ -1299,6 +1332,7 @@ struct MixedState {
     int* cnt_all = nullptr;
     StepScalars* h_scal = nullptr;
     int max_neighbors = 0;
+    int n_fluid = 0;
     bool exported = false;
     bool s64 = false;  // FP64 pressure core (MPH_MODE_MIXED_P64)
     bool walk = false; // force sweep by cell walk (MPH_MIXED_CELL_WALK)
@@ -1383,38 +1417,72 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     return MPH_OK;
 }
 
+// Lanes per particle of a sweep: enough threads to fill the GPU, and no more (the
+// lanes' sums and the rows they share cost more than one thread's walk then).  us at
+// 1, 4, 8 lanes (a particle's list: 40 entries in 2-D and in sweep A without surface
+// tension, else 200):
+//   2-D, sweep A / B         1,600   20 / 11 / 9    26 / 14 / 11
+//                           10,000   23 / 12 / 11   29 / 15 / 14
+//                           25,600   23 / 13 / 18   30 / 18 / 24
+//                           57,600   23 / 22 / 31   32 / 37 / 47
+//   3-D, sweep A, no surface tension, 19,548 particles  22 / 11 / 9; 40,872  23 / 12 / 12;
+//                           87,396   23 / 20 / 22; 157,212  26 / 29 / 38
+//   3-D, sweep A, surface tension, 13,824   76 / 27 / 19; 32,768  80 / 31 / 34;
+//                          157,464  140 / 124 / 139; 314,432  216 / 225 / -
+//   3-D, sweep B, 4,116 fluid  73 / 26 / 17; 12,000  76 / 28 / 23; 32,928  77 / 36 / 43;
+//                          165,888  171 / 147 / 181; 281,216  202 / 237 / -
+//   same with surface tension, 8,000  108 / 37 / 27; 21,952  115 / 46 / 51;
+//                          125,000  240 / 191 / 220; 262,144  369 / 377 / -
+static int lanes_for(int n, int eight, int four) { return n <= eight ? 8 : n <= four ? 4 : 1; }
+static int lanes_a(const MixedState* m) {
+    if (m->mc.dim == 2) return lanes_for(m->mc.n, 15000, 45000);
+    return m->mc.has_st ? lanes_for(m->mc.n, 25000, 200000) : lanes_for(m->mc.n, 30000, 100000);
+}
+static int lanes_b(const MixedState* m) {
+    return m->mc.dim == 2 ? lanes_for(m->n_fluid, 15000, 45000) : lanes_for(m->n_fluid, 18000, 200000);
+}
+
 void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s, bool ahead) {
-    const int nb = blocks(c.n, 128);
+    const int g = lanes_a(m), nb = blocks((long long)c.n * g, 128);
     double* wc = advance_wall ? d.wall_center : nullptr;
-#define MIX_A(ST, RATIO, S64)                                                                                   \
-    k_mix_a<ST, RATIO, S64><<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short,          \
-                                               m->cnt_all, m->pv, m->gca, d.strain_p, d.div_p, d.dens_a, wc, c, \
-                                               d.vel[d.vcur], d.press, ahead ? d.scal : nullptr)
+#define MIX_A(ST, RATIO, S64, G)                                                                                   \
+    k_mix_a<ST, RATIO, S64, G><<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short,          \
+                                                  m->cnt_all, m->pv, m->gca, d.strain_p, d.div_p, d.dens_a, wc, c, \
+                                                  d.vel[d.vcur], d.press, ahead ? d.scal : nullptr)
+#define MIX_A3(ST, RATIO, S64)                    \
+    if (g == 1) MIX_A(ST, RATIO, S64, 1);         \
+    else if (g == 4) MIX_A(ST, RATIO, S64, 4);    \
+    else MIX_A(ST, RATIO, S64, 8)
 #define MIX_A2(ST, RATIO) \
-    if (m->s64) MIX_A(ST, RATIO, true); else MIX_A(ST, RATIO, false)
+    if (m->s64) { MIX_A3(ST, RATIO, true); } else { MIX_A3(ST, RATIO, false); }
     if (m->mc.has_st) {
         if (m->mc.ratio_all_one) { MIX_A2(true, false); } else { MIX_A2(true, true); }
     } else {
         if (m->mc.ratio_all_one) { MIX_A2(false, false); } else { MIX_A2(false, true); }
     }
 #undef MIX_A2
+#undef MIX_A3
 #undef MIX_A
     m->exported = false;
 }
 
 template <bool WALLS>
 static void launch_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
-    const int nb = blocks(c.n, 128);
+    const int g = WALLS ? 1 : lanes_b(m), nb = blocks((long long)c.n * g, 128);
     double4* vout = WALLS ? nullptr : d.vel[1 - d.vcur];
-#define MIX_B1(ST, RATIO)                                                                                   \
-    k_mix_b<ST, RATIO, WALLS><<<nb, 128, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca,   \
-                                                 m->list, m->cnt_short, m->cnt_all, d.vel[d.vcur], vout,   \
-                                                 d.force, d.scal, ahead)
+#define MIX_B1(ST, RATIO, W, G)                                                                                  \
+    k_mix_b<ST, RATIO, W, G><<<nb, 128, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca, m->list,         \
+                                                m->cnt_short, m->cnt_all, d.vel[d.vcur], vout, d.force, d.scal, ahead)
+#define MIX_B(ST, RATIO)                               \
+    if (g == 1) MIX_B1(ST, RATIO, WALLS, 1);           \
+    else if (g == 4) MIX_B1(ST, RATIO, false, 4);      \
+    else MIX_B1(ST, RATIO, false, 8)
     if (m->mc.has_st) {
-        if (m->mc.ratio_all_one) { MIX_B1(true, false); } else { MIX_B1(true, true); }
+        if (m->mc.ratio_all_one) { MIX_B(true, false); } else { MIX_B(true, true); }
     } else {
-        if (m->mc.ratio_all_one) { MIX_B1(false, false); } else { MIX_B1(false, true); }
+        if (m->mc.ratio_all_one) { MIX_B(false, false); } else { MIX_B(false, true); }
     }
+#undef MIX_B
 #undef MIX_B1
 }
 
@@ -1451,8 +1519,8 @@ void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bo
     m->exported = false;
 }
 
-int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, DevFP64& d, bool fp64_pressure,
-                 cudaStream_t s, std::string* err) {
+int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, DevFP64& d, int n_fluid,
+                 bool fp64_pressure, cudaStream_t s, std::string* err) {
     *out = nullptr;
     if (c.cc[0] > 1024 || c.cc[1] > 1024 || c.cc[2] > 1024) {
         if (err) *err = "mixed form: at most 1024 cells per axis";
@@ -1464,6 +1532,7 @@ int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, De
     }
     MixedState* m = new MixedState();
     m->s64 = fp64_pressure;
+    m->n_fluid = n_fluid;
     MixConst& mc = m->mc;
     std::memset(&mc, 0, sizeof(mc));
     mc.n = c.n;

@@ -657,7 +657,7 @@ static int create_impl(mph_ctx* ctx, const int* type, const double* xyz, const d
     // start-up: calculateCellParticle, calculateNeighbor, DensityA, GravityCenter,
     // DensityP (main.cpp:358-364)
     if (ctx->mode == MPH_MODE_MIXED || ctx->mode == MPH_MODE_MIXED_P64) {
-        TRY(mph::mixed_create(&ctx->mixed, ctx->sc, ctx->c, d, ctx->mode == MPH_MODE_MIXED_P64, st, &ctx->err));
+        TRY(mph::mixed_create(&ctx->mixed, ctx->sc, ctx->c, d, ctx->n_fluid, ctx->mode == MPH_MODE_MIXED_P64, st, &ctx->err));
         mph::mixed_set_cell_walk(ctx->mixed, ctx->cell_walk);
     } else {
         TRY(grow_list(ctx, initial_capacity(ctx, ctx->sc.rm2)));

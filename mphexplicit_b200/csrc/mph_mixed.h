@@ -14,8 +14,8 @@ struct MixedState;
 // fp64_pressure: the density sweep's short-range pairs (DensityP,
 // DivergenceP, hence the PressureP values) in FP64, the rest in FP32
 // (MPH_MODE_MIXED_P64).
-int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, DevFP64& d, bool fp64_pressure,
-                 cudaStream_t s, std::string* err);
+int mixed_create(MixedState** out, const SimConst& c, const mph_constants& k, DevFP64& d, int n_fluid,
+                 bool fp64_pressure, cudaStream_t s, std::string* err);
 // Convection/wall/periodic + displacement maximum + FP32 copies (1 launch).  ahead, here
 // and below: of a step launched ahead of the host, to run only if no earlier one stopped.
 void mixed_move(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead);
