@@ -1430,16 +1430,21 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
 //   3-D, sweep A, surface tension, 13,824   76 / 27 / 19; 32,768  80 / 31 / 34;
 //                          157,464  140 / 124 / 139; 314,432  216 / 225 / -
 //   3-D, sweep B, 4,116 fluid  73 / 26 / 17; 12,000  76 / 28 / 23; 32,928  77 / 36 / 43;
-//                          165,888  171 / 147 / 181; 281,216  202 / 237 / -
+//                          69,984   83 / 67 / 82; 165,888  171 / 147 / 181; 281,216  202 / 237 / -
 //   same with surface tension, 8,000  108 / 37 / 27; 21,952  115 / 46 / 51;
 //                          125,000  240 / 191 / 220; 262,144  369 / 377 / -
+// Sweep B without surface tension runs 151,552 threads at once, so a thread per particle
+// is one wave up to there and the better one from 100,000 on (a step of the dam with 128,000
+// fluid particles 192 us, with four lanes 210; 107,520: 198 and 201); with surface
+// tension it runs 113,664 (column of 125,000: 405 and 355; 175,616: 473 and 476).
 static int lanes_for(int n, int eight, int four) { return n <= eight ? 8 : n <= four ? 4 : 1; }
 static int lanes_a(const MixedState* m) {
     if (m->mc.dim == 2) return lanes_for(m->mc.n, 15000, 45000);
     return m->mc.has_st ? lanes_for(m->mc.n, 25000, 200000) : lanes_for(m->mc.n, 30000, 100000);
 }
 static int lanes_b(const MixedState* m) {
-    return m->mc.dim == 2 ? lanes_for(m->n_fluid, 15000, 45000) : lanes_for(m->n_fluid, 18000, 200000);
+    if (m->mc.dim == 2) return lanes_for(m->n_fluid, 15000, 45000);
+    return lanes_for(m->n_fluid, 18000, m->mc.has_st ? 150000 : 100000);
 }
 
 void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s, bool ahead) {

@@ -34,7 +34,8 @@ def dam(fluid, st):
 
 CASES = [(f"droplet {n}", lambda n=n: droplet(n)) for n in (1, 33, 15000, 15001, 45000, 45001)]
 CASES += [(f"dam {f} {st}", lambda f=f, st=st: dam(f, st)) for st in (False, True)
-          for f in ((9, 10, 11), (26, 26, 26), (27, 26, 26), (40, 41, 40), (58, 58, 59), (58, 58, 60))]
+          for f in ((9, 10, 11), (26, 26, 26), (27, 26, 26), (40, 41, 40), (46, 47, 46), (46, 46, 48), (53, 53, 53),
+                    (53, 53, 54), (58, 58, 59), (58, 58, 60))]
 
 
 @pytest.mark.parametrize("mode", ["mixed", "mixed_p64"])
