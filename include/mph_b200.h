@@ -245,11 +245,11 @@ int mph_step(mph_ctx* ctx, int nsteps);
  * 0.025 against 0.040 ms per step on a 1,600-particle droplet. */
 int mph_set_step_graphs(mph_ctx* ctx, int enable);
 
-/* The FP64 (and learned) form's pair sweeps: 0 (the default) by size, 4 to 32
- * lanes per particle in small scenes and one thread per particle above; 1
- * always a thread per particle; 2 always a warp (32 lanes) per particle.  The
- * same bits either way (the lanes compute the terms of as many list entries,
- * one lane per sum adds them in list order). */
+/* The pair sweeps of the FP64, learned and mixed forms: 0 (the default) by size,
+ * several lanes per particle in small scenes (4 to 32; mixed 4 or 8) and one thread per
+ * particle above; 1 always a thread per particle; 2 always a warp (32 lanes) per
+ * particle, in the mixed form 8 lanes.  The same bits either way (the lanes compute the
+ * terms of as many list entries, one lane per sum adds them in list order). */
 int mph_set_sweep_layout(mph_ctx* ctx, int layout);
 
 /* Wait for the context's stream and report any device-side error flag. */

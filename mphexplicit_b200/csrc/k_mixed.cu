@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include "mph_mixed.h"
 #include "mph_pair32.cuh"
@@ -34,12 +35,11 @@ constexpr int kCodeBits = 5;  // 27 neighbour-cell offsets
 #ifndef MPH_MIXB_MINB_FUSED
 #define MPH_MIXB_MINB_FUSED 8
 #endif
-// ... and of its surface-tension variants (more live values per pair).  They were
-// bound by the latency of the gravity centre's gather, sent after the distance test, and
-// spilled at 8 blocks: 730 us a launch on the 592,704-particle two-fluid column.  With the
-// four centres of a row gathered with its records: 619 at 6 blocks, 656 at 5, 709 at 7.
+// ... and of its surface-tension variants (more live values per pair), bound by latency:
+// us a launch at 4 / 5 / 6 / 7 / 8 blocks on the 592,704-particle two-fluid column
+// 728 / 703 / 730 / 794 / 947, on the 830,584-particle one 1031 / 969 / 1025 / 1126 / 1308.
 #ifndef MPH_MIXB_MINB_ST
-#define MPH_MIXB_MINB_ST 6
+#define MPH_MIXB_MINB_ST 5
 #endif
 // Resident 128-thread blocks per SM of the table-free force sweep.
 #ifndef MPH_WALK_MINB
@@ -111,11 +111,10 @@ __device__ __forceinline__ void rel32(const SimConst& c, const MixConst& m, cons
 // The neighbour table holds entries in rows of four: entries 4r..4r+3 of
 // particle i are one uint4 at row r, column i (tab[r * n + i]), so a lane
 // writes 16 bytes at a time when the table is built and the lanes of a warp
-// read consecutive uint4 when it is swept.  Visits entries [0, cnt) in order; with G
-// lanes per particle, lane sub's: every G-th row.
-template <int G = 1, class F>
-__device__ __forceinline__ void for_entries(const uint4* __restrict__ tab, size_t n, int cnt, F&& f, int sub = 0) {
-    for (int k = 4 * sub; k < cnt; k += 4 * G) {
+// read consecutive uint4 when it is swept.  Visits entries [0, cnt) in order.
+template <class F>
+__device__ __forceinline__ void for_entries(const uint4* __restrict__ tab, size_t n, int cnt, F&& f) {
+    for (int k = 0; k < cnt; k += 4) {
         const uint4 q = __ldg(tab + (size_t)(k >> 2) * n);
         f(q.x);
         if (k + 1 < cnt) f(q.y);
@@ -124,16 +123,38 @@ __device__ __forceinline__ void for_entries(const uint4* __restrict__ tab, size_
     }
 }
 
-// The sum over a particle's G lanes, in each of them (mask: those lanes).
-template <int G, class T>
-__device__ __forceinline__ T lane_sum(unsigned mask, T v) {
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-    return v;
-}
+// The warp's stage of the sweeps with G lanes per particle: one float4 a lane, a
+// particle's G behind one another and the particles one more apart, so that the lanes
+// which sum different particles' terms meet different banks.
 template <int G>
-__device__ __forceinline__ unsigned lane_mask() {
-    return G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+struct LaneStage {
+    float4 v[32 + 32 / G];
+    __device__ __forceinline__ static int slot(int lane) { return lane + lane / G; }
+};
+
+// Walks a list by G lanes per particle, G entries a trip: lane sub evaluates
+// entry k0 + sub (eval(record): it stages the terms), then add(m) adds the first m
+// of the G staged entries in list order.  tab: the list's first row; self: an entry that names the
+// particle, loaded where the list has ended.  Entries are loaded two trips ahead and
+// records one.  All lanes of the warp take part; cnt is the particle's.
+template <int G, class Load, class Eval, class Add>
+__device__ __forceinline__ void lane_walk(const unsigned* __restrict__ tab, size_t n, int i, int cnt, unsigned self,
+                                          Load&& load, Eval&& eval, Add&& add) {
+    const int sub = threadIdx.x & (G - 1);
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    auto entry = [&](int k) { return k < cnt ? __ldg(tab + ((size_t)(k >> 2) * n + i) * 4 + (k & 3)) : self; };
+    unsigned eb = entry(sub + G);
+    auto a = load(entry(sub));
+    for (int k0 = 0; k0 < most; k0 += G) {
+        const unsigned ec = entry(k0 + 2 * G + sub);
+        const auto b = load(eb);
+        const int m = min(G, max(0, cnt - k0));
+        eval(a, sub < m);
+        add(m);
+        __syncwarp();
+        eb = ec;
+        a = b;
+    }
 }
 
 // ---- counting sort by cell ------------------------------------------------
@@ -631,8 +652,9 @@ __device__ __forceinline__ void load_tables(const MixConst& m, SharedTables& t) 
 // Arithmetic, chs. 4-5) carry r^2, r, 1 - r/RP and the square to about 2^-44
 // relative.  The strain is a small difference of a sum near N0p, so the
 // per-term rounding of plain FP32 (~1e-7 relative) would dominate the error.
-__device__ __forceinline__ void wp_df(const MixConst& m, float hx, float hy, float hz, float lx, float ly,
-                                      float lz, float& sh, float& sl) {
+// wp_square: the square, p2 + p2e; wp_add: times Cp, to the sum.
+__device__ __forceinline__ void wp_square(const MixConst& m, float hx, float hy, float hz, float lx, float ly,
+                                          float lz, float& p2, float& p2e) {
     // renormalise each axis so that hi is the FP32 rounding of hi + lo
     { const float t = hx + lx; lx -= t - hx; hx = t; }
     { const float t = hy + ly; ly -= t - hy; hy = t; }
@@ -657,142 +679,113 @@ __device__ __forceinline__ void wp_df(const MixConst& m, float hx, float hy, flo
     const float te = fmaf(r0, m.inv_rp, -t) + r0 * m.inv_rp_lo + rl * m.inv_rp;
     const float qh = 1.0f - t;
     const float ql = ((1.0f - qh) - t) - te;
+    p2 = qh * qh;
+    p2e = fmaf(qh, qh, -p2) + 2.0f * qh * ql;
+}
+__device__ __forceinline__ void wp_add(const MixConst& m, float p2, float p2e, float& sh, float& sl) {
     // w = Cp q^2: wh + wl
-    const float p2 = qh * qh;
-    const float p2e = fmaf(qh, qh, -p2) + 2.0f * qh * ql;
     const float wh = m.cp * p2;
     const float wl = fmaf(m.cp, p2, -wh) + m.cp * p2e + m.cp_lo * p2;
     // (sh, sl) += (wh, wl)
     const float sn = sh + wh;
-    bb = sn - sh;
+    const float bb = sn - sh;
     const float se = (sh - (sn - bb)) + (wh - bb);
     sh = sn;
     sl += se + wl;
 }
 
-// Sweep A: DensityP and DivergenceP over the short part of the list with the
-// exact FP32 displacement (S64: pair arithmetic in FP64, the displacement
-// assembled in FP64 from the hi/lo parts, FP32 velocities), plus, with
-// surface tension, DensityA and GravityCenter over all of it, by G lanes per
-// particle (lanes_a), whose sums are added in FP64; epilogue:
-// coefficients, PressureP, PressureA (main.cpp:1631-1662, 1735-1740, 1831-1906).
-template <bool ST, bool RATIO, bool S64, int G>
-__global__ void __launch_bounds__(128)
-k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p32, const float4* __restrict__ v32,
-        const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
-        float4* __restrict__ pv, float4* __restrict__ gca, double* __restrict__ strain_out,
-        double* __restrict__ div_out, double* __restrict__ dens_a_out, double* __restrict__ wall_center,
-        const SimConst c, const double4* __restrict__ vel64,
-        double4* __restrict__ press64, const StepScalars* __restrict__ skip) {
-    __shared__ SharedTables tb;
-    if (skip != nullptr && skip->stop) return;  // launched ahead of a step that has to rebuild
-    load_tables(m, tb);
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = G == 1 ? 0 : (int)(threadIdx.x % G);
-    if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
-        const int t = threadIdx.x / 3, d = threadIdx.x % 3;
-        if (t >= 2) wall_center[3 * t + d] += c.wall_velocity[t][d] * c.dt;
-    }
-    if (i >= m.n) return;
-    const float4 pi = phl[2 * (size_t)i];
-    const float4 li = phl[2 * (size_t)i + 1];
-    const float4 vi = v32[i];
-    const int ti = __float_as_int(pi.w);
-    const int ns = cnt_short[i];
-    const int na = ST ? cnt_all[i] : ns;
-    const size_t n = (size_t)m.n;
+// A pair's terms of sweep A as the factors of their last product, which the sums take
+// in with that product's rounding (the compiler's or the sums' own fused
+// multiply-add), whoever adds them: this thread, or another lane.
+struct DensityTerms {   // DensityP, DivergenceP, within RadiusP
+    float p2, p2e;      // wp_square
+    float ue, dw;       // u.e, dwp/dr
+};
+struct DensityTerms64 {
+    double wa, wb;      // DensityP: wa wb
+    double da, db;      // DivergenceP: - da db
+};
+template <bool S64>
+using DensityTermsOf = std::conditional_t<S64, DensityTerms64, DensityTerms>;
+
+struct DensitySums {
     float sph = 0.f, spl = 0.f, sd = 0.f, cdk = 0.f;
     double spd = 0.0, sdd = 0.0;
-    float sa = 0.f, cak = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
-    const uint4* tab = reinterpret_cast<const uint4*>(list) + i;
-    for_entries<G>(tab, n, ns, [&](unsigned e) {
-        const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
-        float4 pj, lj;
-        ldg_pv(phl, j, pj, lj);  // {hi, lo} in one 256-bit load
-        const float4 dh = tb.dhi[code], dl = tb.dlo[code];
-        float dx, dy, dz;
-        if (S64) {
-            // FP64 displacement: the hi difference plus the cell offset is exact in
-            // FP32 (grid multiples), the lo parts carry the rest to ~1e-14 l0
-            const double dxd = (double)((pj.x - pi.x) + dh.x) + (((double)lj.x - (double)li.x) + (double)dl.x);
-            const double dyd = (double)((pj.y - pi.y) + dh.y) + (((double)lj.y - (double)li.y) + (double)dl.y);
-            const double dzd = (double)((pj.z - pi.z) + dh.z) + (((double)lj.z - (double)li.z) + (double)dl.z);
-            const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
-            if (r2d <= c.rp2) {
-                const double y = rsqrt_dnr(r2d);
-                const double q = 1.0 - r2d * y * m.inv_rp_d;
-                spd += m.cp_d * q * q;
-                const double dw = m.cp_m2_d * q;
-                const float4 vj = v32[j];
-                sdd -= (((double)vj.x - (double)vi.x) * dxd + ((double)vj.y - (double)vi.y) * dyd +
-                        ((double)vj.z - (double)vi.z) * dzd) * y * dw;
-            }
-            dx = (float)dxd;
-            dy = (float)dyd;
-            dz = (float)dzd;
-        } else {
-            dx = ((pj.x - pi.x) + dh.x) + ((lj.x - li.x) + dl.x);
-            dy = ((pj.y - pi.y) + dh.y) + ((lj.y - li.y) + dl.y);
-            dz = ((pj.z - pi.z) + dh.z) + ((lj.z - li.z) + dl.z);
-        }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const float rinv = rsqrt_nr(r2);
-        const float r = r2 * rinv;
-        if (!S64 && r2 <= m.rp2) {
-            wp_df(m, (pj.x - pi.x) + dh.x, (pj.y - pi.y) + dh.y, (pj.z - pi.z) + dh.z, (lj.x - li.x) + dl.x,
-                  (lj.y - li.y) + dl.y, (lj.z - li.z) + dl.z, sph, spl);  // wp
-            const float q = 1.0f - r * m.inv_rp;
-            const float dw = m.cp_m2 * q;                        // dwpdr
-            const float4 vj = v32[j];
-            const float ue = ((vj.x - vi.x) * dx + (vj.y - vi.y) * dy + (vj.z - vi.z) * dz) * rinv;
-            kahan_add(sd, cdk, -ue * dw);
-        }
-        if (ST) st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r, dx, dy, dz, sa, cak, g0, g1, g2);
-    }, sub);
-    if (ST) {  // surface tension only: the long part, on the 16-byte hi records
-        const uint4* tl = tab + (size_t)((m.cap_s >> 2) + sub) * n;
-        const int nl = na - ns;
-        for (int k = 4 * sub; k < nl; k += 4 * G, tl += G * n) {
-            const uint4 q = __ldg(tl);
-            const unsigned e[4] = {q.x, q.y, q.z, q.w};
-            float4 pj[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (k + u < nl) pj[u] = __ldg(p32 + (e[u] >> kCodeBits));
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (k + u < nl) {
-                    const unsigned st = tb.steps[e[u] & 31u];
-                    const float dx = add_step(pj[u].x - pi.x, st, m.half_cell[0]),
-                                dy = add_step(pj[u].y - pi.y, st << 2, m.half_cell[1]),
-                                dz = add_step(pj[u].z - pi.z, st << 4, m.half_cell[2]);
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    st_density<RATIO>(m, ti, __float_as_int(pj[u].w), r2, r2 * rsqrtf(r2), dx, dy, dz, sa, cak, g0, g1,
-                                      g2);
-                }
-        }
+    __device__ __forceinline__ void add_p(const MixConst& m, float p2, float p2e) { wp_add(m, p2, p2e, sph, spl); }
+    __device__ __forceinline__ void add_p64(double wa, double wb) { spd += wa * wb; }
+    __device__ __forceinline__ void add_d(float ue, float dw) { kahan_add(sd, cdk, -ue * dw); }
+    __device__ __forceinline__ void add_d64(double da, double db) { sdd -= da * db; }
+    // the pair sum is exact to ~2^-44: N0p is subtracted in FP64 (the strain is a
+    // small difference of two numbers near N0p)
+    template <bool S64>
+    __device__ __forceinline__ double strain(const MixConst& m) const {
+        return S64 ? spd - m.n0p_d : ((double)sph + (double)spl) - m.n0p_d;
     }
-    double strain, div;
-    if (S64) {
-        strain = spd;
-        div = sdd;
+    template <bool S64>
+    __device__ __forceinline__ double div() const {
+        return S64 ? sdd : (double)sd - (double)cdk;
+    }
+};
+
+// A pair of the short part: its displacement d (FP32) and squared distance r2, and, where it is within
+// RadiusP (the return value), its terms.  FP32: the exact displacement from the hi and lo parts.
+// S64: pair arithmetic in FP64.
+template <bool S64>
+__device__ __forceinline__ bool density_pair(const MixConst& m, const SimConst& c, const float4& pi, const float4& li,
+                                             const float4& vi, const float4& pj, const float4& lj, const float4& vj,
+                                             const float4& dh, const float4& dl, float* d, float& r2,
+                                             DensityTermsOf<S64>& t) {
+    bool in;
+    if constexpr (S64) {
+        // FP64 displacement: the hi difference plus the cell offset is exact in
+        // FP32 (grid multiples), the lo parts carry the rest to ~1e-14 l0
+        const double dxd = (double)((pj.x - pi.x) + dh.x) + (((double)lj.x - (double)li.x) + (double)dl.x);
+        const double dyd = (double)((pj.y - pi.y) + dh.y) + (((double)lj.y - (double)li.y) + (double)dl.y);
+        const double dzd = (double)((pj.z - pi.z) + dh.z) + (((double)lj.z - (double)li.z) + (double)dl.z);
+        const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
+        in = r2d <= c.rp2;
+        if (in) {
+            const double y = rsqrt_dnr(r2d);
+            const double q = 1.0 - r2d * y * m.inv_rp_d;
+            t.wa = m.cp_d * q;
+            t.wb = q;
+            const double dw = m.cp_m2_d * q;
+            t.da = (((double)vj.x - (double)vi.x) * dxd + ((double)vj.y - (double)vi.y) * dyd +
+                    ((double)vj.z - (double)vi.z) * dzd) * y;
+            t.db = dw;
+        }
+        d[0] = (float)dxd;
+        d[1] = (float)dyd;
+        d[2] = (float)dzd;
+        r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
     } else {
-        strain = (double)sph + (double)spl;  // the pair sum is exact to ~2^-44
-        div = (double)sd - (double)cdk;
-    }
-    float dens = sa - cak;
-    if (G > 1) {
-        const unsigned mask = lane_mask<G>();
-        strain = lane_sum<G>(mask, strain);
-        div = lane_sum<G>(mask, div);
-        if (ST) {
-            dens = (float)lane_sum<G>(mask, (double)sa - (double)cak);
-            g0 = lane_sum<G>(mask, g0);
-            g1 = lane_sum<G>(mask, g1);
-            g2 = lane_sum<G>(mask, g2);
+        d[0] = ((pj.x - pi.x) + dh.x) + ((lj.x - li.x) + dl.x);
+        d[1] = ((pj.y - pi.y) + dh.y) + ((lj.y - li.y) + dl.y);
+        d[2] = ((pj.z - pi.z) + dh.z) + ((lj.z - li.z) + dl.z);
+        r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        in = r2 <= m.rp2;
+        if (in) {
+            wp_square(m, (pj.x - pi.x) + dh.x, (pj.y - pi.y) + dh.y, (pj.z - pi.z) + dh.z, (lj.x - li.x) + dl.x,
+                      (lj.y - li.y) + dl.y, (lj.z - li.z) + dl.z, t.p2, t.p2e);  // wp
+            const float rinv = rsqrt_nr(r2);
+            const float r = r2 * rinv;
+            const float q = 1.0f - r * m.inv_rp;
+            t.dw = m.cp_m2 * q;  // dwpdr
+            t.ue = ((vj.x - vi.x) * d[0] + (vj.y - vi.y) * d[1] + (vj.z - vi.z) * d[2]) * rinv;
         }
-        if (sub != 0) return;
     }
-    strain -= m.n0p_d;  // the strain is a small difference of two numbers near N0p
+    return in;
+}
+
+// Epilogue of sweep A: coefficients, PressureP, PressureA (main.cpp:1631-1662, 1735-1740, 1904-1906).
+template <bool ST, bool S64>
+__device__ __forceinline__ void density_finish(const MixConst& m, const SimConst& c, int i, const float4& pi,
+                                               const float4& vi, double strain, double div, float dens, float g0,
+                                               float g1, float g2, float4* __restrict__ pv, float4* __restrict__ gca,
+                                               double* __restrict__ strain_out, double* __restrict__ div_out,
+                                               double* __restrict__ dens_a_out, const double4* __restrict__ vel64,
+                                               double4* __restrict__ press64) {
+    const int ti = __float_as_int(pi.w);
     double kappa = c.bulk_modulus[ti];
     if (strain < 0.0) kappa = 0.0;
     const double pp = -c.bulk_viscosity[ti] * div + kappa * strain;
@@ -813,46 +806,347 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
     div_out[i] = div;
 }
 
-// Surface-tension terms of one pair (PressureA, DiffuseInterface with aj the
-// a of i as the reference has it, main.cpp:1742-1828); returns the radial
-// part and adds the tangential part to t.  The difference of the two gravity
-// centres, scaled by a of i, is formed once per axis (exact product, one rounding) and
-// shared by the kernel's and its derivative's term; with every product formed anew, as
-// the batched sweeps' st_terms has it, the force sweep of the 592,704-particle column took 707
-// us instead of 619.
-template <bool RATIO>
-__device__ __forceinline__ float st_force(const MixConst& m, int ti, int tj, float r2, float r, float rinv, float dx,
-                                          float dy, float dz, const float4& gi, const float4& gj, float ai,
-                                          float3& t) {
-    const float rij = RATIO ? m.ratio[ti][tj] : 1.0f, rji = RATIO ? m.ratio[tj][ti] : 1.0f;
-    float s = 0.0f;
-    if (r2 < m.ra2) {
-        const float q = r * m.inv_ra;
-        const float dwa = (m.ca_inv * m.vol) * (1.0f - q) * fmaf(-3.0f, q, 1.0f);
-        s = (RATIO ? fmaf(gi.w, rij, gj.w * rji) : gi.w + gj.w) * dwa * rinv;
+__device__ __forceinline__ void advance_wall_centers(const SimConst& c, double* __restrict__ wall_center) {
+    if (wall_center != nullptr && blockIdx.x == 0 && threadIdx.x < 12) {
+        const int t = threadIdx.x / 3, d = threadIdx.x % 3;
+        if (t >= 2) wall_center[3 * t + d] += c.wall_velocity[t][d] * c.dt;
     }
-    if (r2 < m.rg2) {
-        const float q = 1.0f - r * m.inv_rg;
-        const float k1 = m.inv_r2g_rg * m.vol_over_l0;
-        const float wg = (m.cg * k1) * q * q, dwg = (m.cg_m2 * k1) * q;
-        const float bi = RATIO ? ai * rij : ai, bj = RATIO ? ai * rji : ai;
-        const float d0 = fmaf(bj, gj.x, -(bi * gi.x)), d1 = fmaf(bj, gj.y, -(bi * gi.y)),
-                    d2 = fmaf(bj, gj.z, -(bi * gi.z));
-        t.x = fmaf(-d0, wg, t.x);
-        t.y = fmaf(-d1, wg, t.y);
-        t.z = fmaf(-d2, wg, t.z);
-        const float gr = fmaf(d2, dz, fmaf(d0, dx, d1 * dy));
-        s = fmaf(-gr, dwg * rinv, s);
-    }
-    return s;
 }
 
-// Sweep B for fluid particles (WALLS: for the wall particles, output only), G lanes
-// per particle (lanes_b), whose forces are added in FP64,
+// Sweep A: DensityP and DivergenceP over the short part of the list
+// (density_pair), plus, with surface tension, DensityA and GravityCenter over all
+// of it (main.cpp:1665-1727, 1831-1896), a thread per particle.
+template <bool ST, bool RATIO, bool S64>
+__global__ void __launch_bounds__(128)
+k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p32, const float4* __restrict__ v32,
+        const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
+        float4* __restrict__ pv, float4* __restrict__ gca, double* __restrict__ strain_out,
+        double* __restrict__ div_out, double* __restrict__ dens_a_out, double* __restrict__ wall_center,
+        const SimConst c, const double4* __restrict__ vel64,
+        double4* __restrict__ press64, const StepScalars* __restrict__ skip) {
+    __shared__ SharedTables tb;
+    if (skip != nullptr && skip->stop) return;  // launched ahead of a step that has to rebuild
+    load_tables(m, tb);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    advance_wall_centers(c, wall_center);
+    if (i >= m.n) return;
+    const float4 pi = phl[2 * (size_t)i];
+    const float4 li = phl[2 * (size_t)i + 1];
+    const float4 vi = v32[i];
+    const int ti = __float_as_int(pi.w);
+    const int ns = cnt_short[i];
+    const int na = ST ? cnt_all[i] : ns;
+    const size_t n = (size_t)m.n;
+    DensitySums q;
+    float sa = 0.f, cak = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
+    const uint4* tab = reinterpret_cast<const uint4*>(list) + i;
+    for_entries(tab, n, ns, [&](unsigned e) {
+        const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
+        float4 pj, lj;
+        ldg_pv(phl, j, pj, lj);  // {hi, lo} in one 256-bit load
+        float d[3], r2;
+        DensityTermsOf<S64> t;
+        if (density_pair<S64>(m, c, pi, li, vi, pj, lj, v32[j], tb.dhi[code], tb.dlo[code], d, r2, t)) {
+            if constexpr (S64) {
+                q.add_p64(t.wa, t.wb);
+                q.add_d64(t.da, t.db);
+            } else {
+                q.add_p(m, t.p2, t.p2e);
+                q.add_d(t.ue, t.dw);
+            }
+        }
+        if (ST) {
+            const float rinv = rsqrt_nr(r2);
+            st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, d[0], d[1], d[2], sa, cak, g0, g1, g2);
+        }
+    });
+    if (ST) {  // surface tension only: the long part, on the 16-byte hi records
+        const uint4* tl = tab + (size_t)(m.cap_s >> 2) * n;
+        const int nl = na - ns;
+        for (int k = 0; k < nl; k += 4, tl += n) {
+            const uint4 q4 = __ldg(tl);
+            const unsigned e[4] = {q4.x, q4.y, q4.z, q4.w};
+            float4 pj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < nl) pj[u] = __ldg(p32 + (e[u] >> kCodeBits));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < nl) {
+                    const unsigned st = tb.steps[e[u] & 31u];
+                    const float dx = add_step(pj[u].x - pi.x, st, m.half_cell[0]),
+                                dy = add_step(pj[u].y - pi.y, st << 2, m.half_cell[1]),
+                                dz = add_step(pj[u].z - pi.z, st << 4, m.half_cell[2]);
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    st_density<RATIO>(m, ti, __float_as_int(pj[u].w), r2, r2 * rsqrtf(r2), dx, dy, dz, sa, cak, g0, g1,
+                                      g2);
+                }
+        }
+    }
+    density_finish<ST, S64>(m, c, i, pi, vi, q.strain<S64>(m), q.div<S64>(), sa - cak, g0, g1, g2, pv, gca, strain_out,
+                            div_out, dens_a_out, vel64, press64);
+}
+
+// A pair's terms of DensityA (sa x y) and GravityCenter (g += d w), as st_density has
+// them; bit 0 of the return value: the first is in range, bit 1: the second.
+template <bool RATIO>
+__device__ __forceinline__ int st_density_terms(const MixConst& m, int ti, int tj, float r2, float r, float& x,
+                                                float& y, float& w) {
+    const float ratio = RATIO ? m.ratio[ti][tj] : 1.0f;
+    int in = 0;
+    if (r2 <= m.ra2) {
+        const float q = r * m.inv_ra;
+        x = ratio * m.ca * q * (1.0f - q);
+        y = 1.0f - q;
+        in = 1;
+    }
+    if (r2 <= m.rg2) {
+        const float q = 1.0f - r * m.inv_rg;
+        w = ratio * m.cg * q * q * m.inv_r2g_rg;
+        in |= 2;
+    }
+    return in;
+}
+
+// Sweep A with G lanes per particle (small scenes, lanes_a): the lanes compute the
+// terms of G consecutive entries, stage them in shared memory, and one lane per sum adds
+// them in list order: the additions of k_mix_a in its order, so the same bits.
+template <bool ST, bool RATIO, bool S64, int G>
+__global__ void __launch_bounds__(128)
+k_mix_a_g(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p32, const float4* __restrict__ v32,
+          const unsigned* __restrict__ list, const int* __restrict__ cnt_short, const int* __restrict__ cnt_all,
+          float4* __restrict__ pv, float4* __restrict__ gca, double* __restrict__ strain_out,
+          double* __restrict__ div_out, double* __restrict__ dens_a_out, double* __restrict__ wall_center,
+          const SimConst c, const double4* __restrict__ vel64,
+          double4* __restrict__ press64, const StepScalars* __restrict__ skip) {
+    __shared__ SharedTables tb;
+    __shared__ LaneStage<G> stage_[4][S64 ? 2 : 1];            // DensityP's and DivergenceP's factors
+    __shared__ LaneStage<G> stage_st_[ST ? 4 : 1][ST ? 2 : 1];  // {d, w}; {x, y} of DensityA
+    if (skip != nullptr && skip->stop) return;  // launched ahead of a step that has to rebuild
+    load_tables(m, tb);
+    advance_wall_centers(c, wall_center);
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), wib = threadIdx.x >> 5;
+    const int iw = (blockIdx.x * 4 + wib) * (32 / G);
+    if (iw >= m.n) return;  // whole warp
+    const bool on = iw + lane / G < m.n;
+    const int i = on ? iw + lane / G : m.n - 1;
+    LaneStage<G>* const st = stage_[wib];
+    LaneStage<G>* const ss = stage_st_[ST ? wib : 0];
+    const int mine = LaneStage<G>::slot(lane), col = LaneStage<G>::slot(lane - sub);
+    const float4 pi = phl[2 * (size_t)i];
+    const float4 li = phl[2 * (size_t)i + 1];
+    const float4 vi = v32[i];
+    const int ti = __float_as_int(pi.w);
+    const int ns = on ? cnt_short[i] : 0;
+    const int nl = ST && on ? cnt_all[i] - ns : 0;
+    const size_t n = (size_t)m.n;
+    const unsigned self = (unsigned)i << kCodeBits | 13u;  // code 13: the home cell
+    DensitySums q;              // lane 0: DensityP; lane 1: DivergenceP
+    float sa = 0.f, cak = 0.f;  // lane 2: DensityA
+    float gs = 0.f;             // GravityCenter: component gcomp
+    const int gcomp = G >= 8 ? sub - 3 : (sub + 1) & 3;
+    unsigned in_p = 0u, in_a = 0u, in_g = 0u;
+    // DensityA and GravityCenter of one entry into the stage
+    auto stage_st = [&](bool have, int tj, float r2, float r, float dx, float dy, float dz) {
+        float x = 0.f, y = 0.f, w = 0.f;
+        const int in = have ? st_density_terms<RATIO>(m, ti, tj, r2, r, x, y, w) : 0;
+        ss[0].v[mine] = make_float4(dx, dy, dz, w);
+        ss[ST ? 1 : 0].v[mine].x = x;
+        ss[ST ? 1 : 0].v[mine].y = y;
+        in_a = __ballot_sync(0xffffffffu, in & 1) >> (lane - sub);
+        in_g = __ballot_sync(0xffffffffu, in & 2) >> (lane - sub);
+    };
+    auto add_st = [&]() {
+        if (sub == 2) {
+#pragma unroll
+            for (int e = 0; e < G; ++e)
+                if (in_a >> e & 1u) {
+                    const float4 t = ss[ST ? 1 : 0].v[col + e];
+                    kahan_add(sa, cak, t.x * t.y);
+                }
+        }
+        if (gcomp >= 0 && gcomp < 3) {
+#pragma unroll
+            for (int e = 0; e < G; ++e)
+                if (in_g >> e & 1u) {
+                    const float* t = reinterpret_cast<const float*>(&ss[0].v[col + e]);
+                    gs += t[gcomp] * t[3];
+                }
+        }
+    };
+    struct Rec {
+        float4 p, l, v;
+        unsigned code;
+    };
+    lane_walk<G>(
+        list, n, i, ns, self,
+        [&](unsigned e) {
+            Rec r;
+            ldg_pv(phl, (int)(e >> kCodeBits), r.p, r.l);
+            r.v = __ldg(v32 + (e >> kCodeBits));
+            r.code = e & 31u;
+            return r;
+        },
+        [&](const Rec& rj, bool have) {
+            float d[3] = {0.f, 0.f, 0.f}, r2 = 0.f;
+            DensityTermsOf<S64> t{};
+            const bool in = have && density_pair<S64>(m, c, pi, li, vi, rj.p, rj.l, rj.v, tb.dhi[rj.code],
+                                                      tb.dlo[rj.code], d, r2, t);
+            if constexpr (S64) {
+                *reinterpret_cast<double2*>(&st[0].v[mine]) = make_double2(t.wa, t.wb);
+                *reinterpret_cast<double2*>(&st[1].v[mine]) = make_double2(t.da, t.db);
+            } else {
+                st[0].v[mine] = make_float4(t.p2, t.p2e, t.ue, t.dw);
+            }
+            in_p = __ballot_sync(0xffffffffu, in) >> (lane - sub);
+            if (ST) {
+                const float rinv = rsqrt_nr(r2);
+                stage_st(have, __float_as_int(rj.p.w), r2, r2 * rinv, d[0], d[1], d[2]);
+            }
+            __syncwarp();
+        },
+        [&](int) {
+            if (sub < 2) {
+#pragma unroll
+                for (int e = 0; e < G; ++e)
+                    if (in_p >> e & 1u) {
+                        if constexpr (S64) {
+                            const double2 t = *reinterpret_cast<const double2*>(&st[sub].v[col + e]);
+                            if (sub == 0) q.add_p64(t.x, t.y);
+                            else q.add_d64(t.x, t.y);
+                        } else {
+                            const float4 t = st[0].v[col + e];
+                            if (sub == 0) q.add_p(m, t.x, t.y);
+                            else q.add_d(t.z, t.w);
+                        }
+                    }
+            }
+            if (ST) add_st();
+        });
+    if (ST) {  // the long part, on the 16-byte hi records
+        struct RecL {
+            float4 p;
+            unsigned steps;
+        };
+        lane_walk<G>(
+            list + (size_t)m.cap_s * n, n, i, nl, self,
+            [&](unsigned e) { return RecL{__ldg(p32 + (e >> kCodeBits)), tb.steps[e & 31u]}; },
+            [&](const RecL& rj, bool have) {
+                const float dx = add_step(rj.p.x - pi.x, rj.steps, m.half_cell[0]),
+                            dy = add_step(rj.p.y - pi.y, rj.steps << 2, m.half_cell[1]),
+                            dz = add_step(rj.p.z - pi.z, rj.steps << 4, m.half_cell[2]);
+                const float r2 = dx * dx + dy * dy + dz * dz;
+                stage_st(have, __float_as_int(rj.p.w), r2, r2 * rsqrtf(r2), dx, dy, dz);
+                __syncwarp();
+            },
+            [&](int) { add_st(); });
+    }
+    const int l0 = lane - sub;
+    const double strain = q.strain<S64>(m);
+    const double div = __shfl_sync(0xffffffffu, q.div<S64>(), l0 + 1);
+    float dens = 0.f, g[3] = {0.f, 0.f, 0.f};
+    if (ST) {
+        dens = __shfl_sync(0xffffffffu, sa - cak, l0 + 2);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g[k] = __shfl_sync(0xffffffffu, gs, l0 + (G >= 8 ? k + 3 : (k + 3) & 3));
+    }
+    if (sub != 0 || !on) return;
+    density_finish<ST, S64>(m, c, i, pi, vi, strain, div, dens, g[0], g[1], g[2], pv, gca, strain_out, div_out,
+                            dens_a_out, vel64, press64);
+}
+
+// A pair of the short part: exact displacement d, PressureP and ViscosityV (and the
+// surface-tension terms); false when it is out of every range.  The force is s d + t.
+template <bool ST, bool RATIO>
+__device__ __forceinline__ bool force_pair_short(const MixConst& m, const SharedTables& tb, unsigned code,
+                                                 const float4& pi, const float4& li, const float4& vi, int ti,
+                                                 float mu_u, const float4& gi, float ai, const float4& pj,
+                                                 const float4& lj, const float4& vj, const float4& gj, float* d,
+                                                 float& s, float3& t) {
+    const float4 dh = tb.dhi[code], dl = tb.dlo[code];
+    const float dx = ((pj.x - pi.x) + dh.x) + ((lj.x - li.x) + dl.x);
+    const float dy = ((pj.y - pi.y) + dh.y) + ((lj.y - li.y) + dl.y);
+    const float dz = ((pj.z - pi.z) + dh.z) + ((lj.z - li.z) + dl.z);
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    if (!(r2 < m.rv2 || r2 < m.rp2 || (ST && (r2 < m.ra2 || r2 < m.rg2)))) return false;
+    const float rinv = rsqrt_nr(r2);
+    const float r = r2 * rinv;
+    const int tj = __float_as_int(pj.w);
+    s = 0.0f;
+    if (r2 < m.rp2) s += (vi.w + vj.w) * fmaf(m.p_b, r, m.p_a) * rinv;
+    if (r2 < m.rv2) {
+        const float mu = m.uniform_mu ? mu_u : tb.mu[ti * 4 + tj];
+        const float ud = (vj.x - vi.x) * dx + (vj.y - vi.y) * dy + (vj.z - vi.z) * dz;
+        s += mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
+    }
+    t = make_float3(0.f, 0.f, 0.f);
+    if (ST) s += st_terms<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gj, ai, t);
+    d[0] = dx;
+    d[1] = dy;
+    d[2] = dz;
+    return true;
+}
+
+// A pair of the long part: the hi displacement, ViscosityV (and surface tension); the
+// force is t, where the return value says that there is one, then s d.
+template <bool ST, bool RATIO>
+__device__ __forceinline__ bool force_pair_long(const MixConst& m, const SharedTables& tb, unsigned code,
+                                                const float4& pi, const float4& vi, int ti, float mu_u,
+                                                const float4& gi, float ai, const float4& pj, const float4& vj,
+                                                const float4& gj, float* d, float& s, float3& t) {
+    float dx, dy, dz;
+    if (ST) {  // short of registers: the table's three words cost less than the steps' one
+        const float4 dh = tb.dhi[code];
+        dx = (pj.x - pi.x) + dh.x;
+        dy = (pj.y - pi.y) + dh.y;
+        dz = (pj.z - pi.z) + dh.z;
+    } else {
+        const unsigned st = tb.steps[code];
+        dx = add_step(pj.x - pi.x, st, m.half_cell[0]);
+        dy = add_step(pj.y - pi.y, st << 2, m.half_cell[1]);
+        dz = add_step(pj.z - pi.z, st << 4, m.half_cell[2]);
+    }
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float rinv = rsqrtf(r2);
+    s = 0.0f;
+    if (r2 < m.rv2) {
+        const float r = r2 * rinv;
+        const float mu = m.uniform_mu ? mu_u : tb.mu[ti * 4 + __float_as_int(pj.w)];
+        const float ud = (vj.x - vi.x) * dx + (vj.y - vi.y) * dy + (vj.z - vi.z) * dz;
+        s = mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
+    }
+    d[0] = dx;
+    d[1] = dy;
+    d[2] = dz;
+    if (ST && (r2 < m.ra2 || r2 < m.rg2)) {
+        t = make_float3(0.f, 0.f, 0.f);
+        s += st_terms<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gj, ai, t);
+        return true;
+    }
+    return false;
+}
+
+// Gravity and the FP64 velocity update of a fluid particle with pair force F.
+__device__ __forceinline__ void force_finish(const SimConst& c, int i, int ti, double F0, double F1, double F2,
+                                             const double4* __restrict__ vel, double4* __restrict__ vel_out,
+                                             double4* __restrict__ force, StepScalars* __restrict__ scal) {
+    double4 v = vel[i];
+    const double mass = c.density[ti] * c.vol;
+    F0 += mass * c.gravity[0];
+    F1 += mass * c.gravity[1];
+    F2 += mass * c.gravity[2];
+    v.x += F0 / mass * c.dt;
+    v.y += F1 / mass * c.dt;
+    v.z += F2 / mass * c.dt;
+    if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z))) atomicOr(&scal->flags, DEVFLAG_NONFINITE);
+    force[i] = make_double4(F0, F1, F2, 0.0);
+    vel_out[i] = v;
+}
+
+// Sweep B for fluid particles (WALLS: for the wall particles, output only), a thread per particle,
 // FP32 in both mixed forms (the FP64 density sweep of MPH_MODE_MIXED_P64 sets
-// the pressures this sweep reads).  The short part of the list: exact
-// displacement, PressureP + ViscosityV (+ the surface-tension terms), Kahan
-// sums.  The long part: the hi displacement, ViscosityV (+ surface tension),
+// the pressures this sweep reads).  The short part of the list
+// (force_pair_short): Kahan sums.  The long part (force_pair_long):
 // plain FP32 sum.  Then gravity and the FP64 velocity update
 // (main.cpp:1908-2010).
 //
@@ -862,7 +1156,7 @@ __device__ __forceinline__ float st_force(const MixConst& m, int ti, int tj, flo
 // instead of 696 at 1,024,000 fluid particles.  A thread per two neighbouring particles
 // with a common list gathered once took 884: the warp runs the longest of its lanes'
 // lists, and the order within cells that keeps its records in few lines is lost.
-template <bool ST, bool RATIO, bool WALLS, int G>
+template <bool ST, bool RATIO, bool WALLS>
 __global__ void __launch_bounds__(128, ST ? MPH_MIXB_MINB_ST : MPH_MIXB_MINB_FUSED)
 k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4* __restrict__ phl,
         const float4* __restrict__ pv, const float4* __restrict__ gca,
@@ -872,11 +1166,11 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     __shared__ SharedTables tb;
     if (ahead && scal->stop) return;
     load_tables(m, tb);
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = G == 1 ? 0 : (int)(threadIdx.x % G);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
     const int nf = cellstart[c.tot];
     if (WALLS ? i < nf : i >= nf) {
-        if (!WALLS && sub == 0) vel_out[i] = vel[i];
+        if (!WALLS) vel_out[i] = vel[i];
         return;
     }
     const float4 pi = phl[2 * (size_t)i];
@@ -892,73 +1186,25 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
     float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;  // short part, Kahan
     float gx = 0.f, gy = 0.f, gz = 0.f;                                 // long part
     const uint4* tab = reinterpret_cast<const uint4*>(list) + i;
-    for_entries<G>(tab, n, ns, [&](unsigned e) {
-        const int j = (int)(e >> kCodeBits), code = (int)(e & 31u);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for_entries(tab, n, ns, [&](unsigned e) {
+        const int j = (int)(e >> kCodeBits);
         float4 pj, vj;
         ldg_pv(pv, j, pj, vj);
-        const float4 lj = phl[2 * (size_t)j + 1];
-        const float4 dh = tb.dhi[code], dl = tb.dlo[code];
-        const float dx = ((pj.x - pi.x) + dh.x) + ((lj.x - li.x) + dl.x);
-        const float dy = ((pj.y - pi.y) + dh.y) + ((lj.y - li.y) + dl.y);
-        const float dz = ((pj.z - pi.z) + dh.z) + ((lj.z - li.z) + dl.z);
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (!(r2 < m.rv2 || r2 < m.rp2 || (ST && (r2 < m.ra2 || r2 < m.rg2)))) return;
-        const float rinv = rsqrt_nr(r2);
-        const float r = r2 * rinv;
-        const int tj = __float_as_int(pj.w);
-        float s = 0.0f;
-        if (r2 < m.rp2) s += (vi.w + vj.w) * fmaf(m.p_b, r, m.p_a) * rinv;
-        if (r2 < m.rv2) {
-            const float mu = m.uniform_mu ? mu_u : tb.mu[ti * 4 + tj];
-            const float ud = (vj.x - vi.x) * dx + (vj.y - vi.y) * dy + (vj.z - vi.z) * dz;
-            s += mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
-        }
-        float3 t = make_float3(0.f, 0.f, 0.f);
-        if (ST) s += st_force<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gca[j], ai, t);
-        kahan_add(fx, cx, fmaf(s, dx, t.x));
-        kahan_add(fy, cy, fmaf(s, dy, t.y));
-        kahan_add(fz, cz, fmaf(s, dz, t.z));
-    }, sub);
+        float d[3], s;
+        float3 t;
+        if (!force_pair_short<ST, RATIO>(m, tb, e & 31u, pi, li, vi, ti, mu_u, gi, ai, pj, phl[2 * (size_t)j + 1], vj,
+                                         ST ? gca[j] : zero, d, s, t))
+            return;
+        kahan_add(fx, cx, fmaf(s, d[0], t.x));
+        kahan_add(fy, cy, fmaf(s, d[1], t.y));
+        kahan_add(fz, cz, fmaf(s, d[2], t.z));
+    });
     // long part: a row of four pairs per iteration, their gathers issued
     // together so a thread keeps four independent loads in flight
-    auto long_pair = [&](unsigned e, const float4& pj, const float4& vj, const float4& gj) {
-        float dx, dy, dz;
-        if (ST) {  // short of registers: the table's three words cost less (619 us against 623 on the column, and the steps' words spill at 8 blocks)
-            const float4 dh = tb.dhi[e & 31u];
-            dx = (pj.x - pi.x) + dh.x;
-            dy = (pj.y - pi.y) + dh.y;
-            dz = (pj.z - pi.z) + dh.z;
-        } else {
-            const unsigned st = tb.steps[e & 31u];
-            dx = add_step(pj.x - pi.x, st, m.half_cell[0]);
-            dy = add_step(pj.y - pi.y, st << 2, m.half_cell[1]);
-            dz = add_step(pj.z - pi.z, st << 4, m.half_cell[2]);
-        }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const float rinv = rsqrtf(r2);
-        float s = 0.0f;
-        if (r2 < m.rv2) {
-            const float r = r2 * rinv;
-            const float mu = m.uniform_mu ? mu_u : tb.mu[ti * 4 + __float_as_int(pj.w)];
-            const float ud = (vj.x - vi.x) * dx + (vj.y - vi.y) * dy + (vj.z - vi.z) * dz;
-            s = mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
-        }
-        if (ST) {
-            if (r2 < m.ra2 || r2 < m.rg2) {
-                float3 t = make_float3(0.f, 0.f, 0.f);
-                s += st_force<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, rinv, dx, dy, dz, gi, gj, ai, t);
-                gx += t.x;
-                gy += t.y;
-                gz += t.z;
-            }
-        }
-        gx = fmaf(s, dx, gx);
-        gy = fmaf(s, dy, gy);
-        gz = fmaf(s, dz, gz);
-    };
     const uint4* tl = tab + (size_t)(m.cap_s >> 2) * n;
     const int nl = na - ns;
-    for (int k = 4 * sub; k < nl; k += 4 * G) {
+    for (int k = 0; k < nl; k += 4) {
         const uint4 q = __ldg(tl + (size_t)(k >> 2) * n);
         const unsigned e[4] = {q.x, q.y, q.z, q.w};
         float4 pj[4], vj[4], gj[4];
@@ -970,33 +1216,139 @@ k_mix_b(MixConst m, SimConst c, const int* __restrict__ cellstart, const float4*
             }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (k + u < nl) long_pair(e[u], pj[u], vj[u], gj[u]);
+            if (k + u < nl) {
+                float d[3], s;
+                float3 t;
+                if (force_pair_long<ST, RATIO>(m, tb, e[u] & 31u, pi, vi, ti, mu_u, gi, ai, pj[u], vj[u], gj[u], d, s,
+                                               t)) {
+                    gx += t.x;
+                    gy += t.y;
+                    gz += t.z;
+                }
+                gx = fmaf(s, d[0], gx);
+                gy = fmaf(s, d[1], gy);
+                gz = fmaf(s, d[2], gz);
+            }
     }
-    double F0 = ((double)fx - (double)cx) + (double)gx;
-    double F1 = ((double)fy - (double)cy) + (double)gy;
-    double F2 = ((double)fz - (double)cz) + (double)gz;
-    if (G > 1) {
-        const unsigned mask = lane_mask<G>();
-        F0 = lane_sum<G>(mask, F0);
-        F1 = lane_sum<G>(mask, F1);
-        F2 = lane_sum<G>(mask, F2);
-        if (sub != 0) return;
-    }
-    if (WALLS) {
-        force[i] = make_double4(F0, F1, F2, 0.0);
+    const double F0 = ((double)fx - (double)cx) + (double)gx;
+    const double F1 = ((double)fy - (double)cy) + (double)gy;
+    const double F2 = ((double)fz - (double)cz) + (double)gz;
+    if (WALLS) force[i] = make_double4(F0, F1, F2, 0.0);
+    else force_finish(c, i, ti, F0, F1, F2, vel, vel_out, force, scal);
+}
+
+// Sweep B with G lanes per fluid particle (small scenes, lanes_b), as k_mix_a_g: lane k
+// < 3 adds component k of the staged terms in list order, with the additions of k_mix_b, so
+// the same bits.  The walls keep their velocity in the blocks behind.
+template <bool ST, bool RATIO, int G>
+__global__ void __launch_bounds__(128)
+k_mix_b_g(MixConst m, SimConst c, int nf, int group_blocks, const float4* __restrict__ phl,
+          const float4* __restrict__ pv, const float4* __restrict__ gca, const unsigned* __restrict__ list,
+          const int* __restrict__ cnt_short, const int* __restrict__ cnt_all, const double4* __restrict__ vel,
+          double4* __restrict__ vel_out, double4* __restrict__ force, StepScalars* __restrict__ scal, bool ahead) {
+    __shared__ SharedTables tb;
+    __shared__ LaneStage<G> stage_[4][ST ? 2 : 1];  // short: s d + t; long: {d, s}, t
+    if (ahead && scal->stop) return;
+    if ((int)blockIdx.x >= group_blocks) {  // walls
+        const int i = nf + ((int)blockIdx.x - group_blocks) * 128 + (int)threadIdx.x;
+        if (i < m.n) vel_out[i] = vel[i];
         return;
     }
-    double4 v = vel[i];
-    const double mass = c.density[ti] * c.vol;
-    F0 += mass * c.gravity[0];
-    F1 += mass * c.gravity[1];
-    F2 += mass * c.gravity[2];
-    v.x += F0 / mass * c.dt;
-    v.y += F1 / mass * c.dt;
-    v.z += F2 / mass * c.dt;
-    if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z))) atomicOr(&scal->flags, DEVFLAG_NONFINITE);
-    force[i] = make_double4(F0, F1, F2, 0.0);
-    vel_out[i] = v;
+    load_tables(m, tb);
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), wib = threadIdx.x >> 5;
+    const int iw = (blockIdx.x * 4 + wib) * (32 / G);
+    if (iw >= nf) return;  // whole warp
+    const bool on = iw + lane / G < nf;
+    const int i = on ? iw + lane / G : nf - 1;
+    LaneStage<G>* const st = stage_[wib];
+    const int mine = LaneStage<G>::slot(lane), col = LaneStage<G>::slot(lane - sub);
+    const float4 pi = phl[2 * (size_t)i];
+    const float4 li = phl[2 * (size_t)i + 1];
+    const float4 vi = pv[2 * (size_t)i + 1];
+    const int ti = __float_as_int(pi.w);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 gi = ST ? gca[i] : zero;
+    const float ai = m.a_k[ti];
+    const int ns = on ? cnt_short[i] : 0, nl = on ? cnt_all[i] - ns : 0;
+    const size_t n = (size_t)m.n;
+    const float mu_u = tb.mu[ti * 4 + ti];
+    const unsigned self = (unsigned)i << kCodeBits | 13u;  // code 13: the home cell
+    float f = 0.f, ck = 0.f;  // lane k < 3: component k of the short part, Kahan
+    float g = 0.f;            // ... of the long part
+    unsigned in = 0u;
+    struct Rec {
+        float4 p, v, l, g;
+        unsigned code;
+    };
+    lane_walk<G>(
+        list, n, i, ns, self,
+        [&](unsigned e) {
+            const int j = (int)(e >> kCodeBits);
+            Rec r;
+            ldg_pv(pv, j, r.p, r.v);
+            r.l = __ldg(phl + 2 * (size_t)j + 1);
+            r.g = ST ? __ldg(gca + j) : zero;
+            r.code = e & 31u;
+            return r;
+        },
+        [&](const Rec& rj, bool have) {
+            float d[3], s;
+            float3 t;
+            const bool hit = have && force_pair_short<ST, RATIO>(m, tb, rj.code, pi, li, vi, ti, mu_u, gi, ai, rj.p,
+                                                                 rj.l, rj.v, rj.g, d, s, t);
+            if (hit) st[0].v[mine] = make_float4(fmaf(s, d[0], t.x), fmaf(s, d[1], t.y), fmaf(s, d[2], t.z), 0.f);
+            in = __ballot_sync(0xffffffffu, hit) >> (lane - sub);
+            __syncwarp();
+        },
+        [&](int) {
+            if (sub < 3) {
+#pragma unroll
+                for (int e = 0; e < G; ++e)
+                    if (in >> e & 1u) kahan_add(f, ck, reinterpret_cast<const float*>(&st[0].v[col + e])[sub]);
+            }
+        });
+    struct RecL {
+        float4 p, v, g;
+        unsigned code;
+    };
+    lane_walk<G>(
+        list + (size_t)m.cap_s * n, n, i, nl, self,
+        [&](unsigned e) {
+            const int j = (int)(e >> kCodeBits);
+            RecL r;
+            ldg_pv(pv, j, r.p, r.v);
+            r.g = ST ? __ldg(gca + j) : zero;
+            r.code = e & 31u;
+            return r;
+        },
+        [&](const RecL& rj, bool have) {
+            if (have) {
+                float d[3], s;
+                float3 t;
+                const bool has_t =
+                    force_pair_long<ST, RATIO>(m, tb, rj.code, pi, vi, ti, mu_u, gi, ai, rj.p, rj.v, rj.g, d, s, t);
+                st[0].v[mine] = make_float4(d[0], d[1], d[2], s);
+                if (ST)  // none: -0.0, which leaves a sum as it is
+                    st[ST ? 1 : 0].v[mine] = has_t ? make_float4(t.x, t.y, t.z, 0.f) : make_float4(-0.f, -0.f, -0.f, 0.f);
+            }
+            __syncwarp();
+        },
+        [&](int mm) {
+            if (sub < 3) {
+#pragma unroll
+                for (int e = 0; e < G; ++e)
+                    if (e < mm) {
+                        const float* q = reinterpret_cast<const float*>(&st[0].v[col + e]);
+                        if (ST) g += reinterpret_cast<const float*>(&st[ST ? 1 : 0].v[col + e])[sub];
+                        g = fmaf(q[3], q[sub], g);
+                    }
+            }
+        });
+    const double F = ((double)f - (double)ck) + (double)g;
+    const int l0 = lane - sub;
+    const double F0 = __shfl_sync(0xffffffffu, F, l0), F1 = __shfl_sync(0xffffffffu, F, l0 + 1),
+                 F2 = __shfl_sync(0xffffffffu, F, l0 + 2);
+    if (sub == 0 && on) force_finish(c, i, ti, F0, F1, F2, vel, vel_out, force, scal);
 }
 
 // The force sweep without the long table (MPH_MIXED_CELL_WALK).  One warp per
@@ -1139,7 +1491,7 @@ k_mix_b_walk(MixConst m, SimConst c, const int* __restrict__ cellstart, const fl
                                             sc += mu * ud * fmaf(m.v_b, r, m.v_a) * (rinv * rinv * rinv);
                                         }
                                         float3 tt = make_float3(0.f, 0.f, 0.f);
-                                        if (ST) sc += st_force<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gstage[q], ai, tt);
+                                        if (ST) sc += st_terms<RATIO>(m, ti, tj, r2, r, rinv, dx, dy, dz, gi, gstage[q], ai, tt);
                                         kahan_add(fx, cx, fmaf(sc, dx, tt.x));
                                         kahan_add(fy, cy, fmaf(sc, dy, tt.y));
                                         kahan_add(fz, cz, fmaf(sc, dz, tt.z));
@@ -1155,7 +1507,7 @@ k_mix_b_walk(MixConst m, SimConst c, const int* __restrict__ cellstart, const fl
                                         if (ST) {
                                             if (r2h < m.ra2 || r2h < m.rg2) {
                                                 float3 tt = make_float3(0.f, 0.f, 0.f);
-                                                sc += st_force<RATIO>(m, ti, tj, r2h, r2h * rinv, rinv, hx, hy, hz, gi,
+                                                sc += st_terms<RATIO>(m, ti, tj, r2h, r2h * rinv, rinv, hx, hy, hz, gi,
                                                                       gstage[q], ai, tt);
                                                 gx += tt.x;
                                                 gy += tt.y;
@@ -1418,53 +1770,51 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
 }
 
 // Lanes per particle of a sweep: enough threads to fill the GPU, and no more (the
-// lanes' sums and the rows they share cost more than one thread's walk then).  us at
-// 1, 4, 8 lanes (a particle's list: 40 entries in 2-D and in sweep A without surface
-// tension, else 200):
-//   2-D, sweep A / B         1,600   20 / 11 / 9    26 / 14 / 11
-//                           10,000   23 / 12 / 11   29 / 15 / 14
-//                           25,600   23 / 13 / 18   30 / 18 / 24
-//                           57,600   23 / 22 / 31   32 / 37 / 47
-//   3-D, sweep A, no surface tension, 19,548 particles  22 / 11 / 9; 40,872  23 / 12 / 12;
-//                           87,396   23 / 20 / 22; 157,212  26 / 29 / 38
-//   3-D, sweep A, surface tension, 13,824   76 / 27 / 19; 32,768  80 / 31 / 34;
-//                          157,464  140 / 124 / 139; 314,432  216 / 225 / -
-//   3-D, sweep B, 4,116 fluid  73 / 26 / 17; 12,000  76 / 28 / 23; 32,928  77 / 36 / 43;
-//                          69,984   83 / 67 / 82; 165,888  171 / 147 / 181; 281,216  202 / 237 / -
-//   same with surface tension, 8,000  108 / 37 / 27; 21,952  115 / 46 / 51;
-//                          125,000  240 / 191 / 220; 262,144  369 / 377 / -
-// Sweep B without surface tension runs 151,552 threads at once, so a thread per particle
-// is one wave up to there and the better one from 100,000 on (a step of the dam with 128,000
-// fluid particles 192 us, with four lanes 210; 107,520: 198 and 201); with surface
-// tension it runs 113,664 (column of 125,000: 405 and 355; 175,616: 473 and 476).
-static int lanes_for(int n, int eight, int four) { return n <= eight ? 8 : n <= four ? 4 : 1; }
-static int lanes_a(const MixedState* m) {
-    if (m->mc.dim == 2) return lanes_for(m->mc.n, 15000, 45000);
-    return m->mc.has_st ? lanes_for(m->mc.n, 25000, 200000) : lanes_for(m->mc.n, 30000, 100000);
+// ordered sums cost more than one thread's walk then).  us at 1, 4, 8 lanes (a particle's
+// list: 40 entries in 2-D and in sweep A without surface tension, else 200):
+//   2-D, sweep A / B         1,600   23 / 17 / 15   28 / 13 / 11
+//                           12,100   23 / 17 / 15   27 / 15 / 15
+//                           16,900   23 / 19 / 21   29 / 16 / 19
+//                           32,400   25 / 22 / 27   31 / 24 / 25
+//                           46,225   23 / 26 / 30   31 / 27 / 33
+//                           57,600   25 / 30 / 37   33 / 33 / 37
+//   3-D, sweep A, no surface tension, 13,320 particles  23 / 17 / 17; 27,936  22 / 16 / 17;
+//                           45,561   24 / 19 / 23; 58,848  23 / 24 / 26
+//   3-D, sweep A, surface tension, 8,000   59 / 32 / 26; 13,824  62 / 34 / 30;
+//                           32,768   66 / 48 / 61; 64,000  66 / 82 / 104
+//   3-D, sweep B, 2,304 fluid  55 / 21 / 17; 9,600  56 / 26 / 23; 14,283  58 / 27 / 28;
+//                           36,864   60 / 54 / 51; 60,648  70 / 69 / 79; 75,645  80 / 91 / 95
+//   same with surface tension, 8,000  99 / 29 / 25; 21,952  103 / 50 / 48;
+//                           85,184   - / 134 / 152; 125,000  237 / 195 / 217; 262,144  372 / 385 / 438
+// Sixteen lanes win 1 or 2 us below 5,000 particles alone.
+static int lanes_for(const SimConst& c, int n, int eight, int four) {
+    if (c.sweep_layout) return c.sweep_layout == 1 ? 1 : 8;  // mph_set_sweep_layout
+    return n <= eight ? 8 : n <= four ? 4 : 1;
 }
-static int lanes_b(const MixedState* m) {
-    if (m->mc.dim == 2) return lanes_for(m->n_fluid, 15000, 45000);
-    return lanes_for(m->n_fluid, 18000, m->mc.has_st ? 150000 : 100000);
+static int lanes_a(const MixedState* m, const SimConst& c) {
+    if (m->mc.dim == 2) return lanes_for(c, m->mc.n, 14000, 35000);
+    return m->mc.has_st ? lanes_for(c, m->mc.n, 20000, 48000) : lanes_for(c, m->mc.n, 14000, 50000);
+}
+static int lanes_b(const MixedState* m, const SimConst& c) {
+    if (m->mc.dim == 2) return lanes_for(c, m->n_fluid, 12000, 50000);
+    return m->mc.has_st ? lanes_for(c, m->n_fluid, 25000, 150000) : lanes_for(c, m->n_fluid, 12000, 62000);
 }
 
 void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wall, cudaStream_t s, bool ahead) {
-    const int g = lanes_a(m), nb = blocks((long long)c.n * g, 128);
+    const int g = lanes_a(m, c), nb = blocks((long long)c.n * g, 128);
     double* wc = advance_wall ? d.wall_center : nullptr;
-#define MIX_A(ST, RATIO, S64, G)                                                                                   \
-    k_mix_a<ST, RATIO, S64, G><<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short,          \
-                                                  m->cnt_all, m->pv, m->gca, d.strain_p, d.div_p, d.dens_a, wc, c, \
-                                                  d.vel[d.vcur], d.press, ahead ? d.scal : nullptr)
-#define MIX_A3(ST, RATIO, S64)                    \
-    if (g == 1) MIX_A(ST, RATIO, S64, 1);         \
-    else if (g == 4) MIX_A(ST, RATIO, S64, 4);    \
-    else MIX_A(ST, RATIO, S64, 8)
+#define MIX_A(KERNEL)                                                                                               \
+    KERNEL<<<nb, 128, 0, s>>>(m->mc, m->phl, m->p32, m->v32, m->list, m->cnt_short, m->cnt_all, m->pv, m->gca,      \
+                              d.strain_p, d.div_p, d.dens_a, wc, c, d.vel[d.vcur], d.press, ahead ? d.scal : nullptr)
+#define MIX_A3(ST, RATIO, S64)                                  \
+    if (g == 1) MIX_A((k_mix_a<ST, RATIO, S64>));               \
+    else if (g == 4) MIX_A((k_mix_a_g<ST, RATIO, S64, 4>));     \
+    else MIX_A((k_mix_a_g<ST, RATIO, S64, 8>))
 #define MIX_A2(ST, RATIO) \
     if (m->s64) { MIX_A3(ST, RATIO, true); } else { MIX_A3(ST, RATIO, false); }
-    if (m->mc.has_st) {
-        if (m->mc.ratio_all_one) { MIX_A2(true, false); } else { MIX_A2(true, true); }
-    } else {
-        if (m->mc.ratio_all_one) { MIX_A2(false, false); } else { MIX_A2(false, true); }
-    }
+    if (!m->mc.has_st) { MIX_A2(false, false); }  // the ratios weigh surface-tension sums alone
+    else if (m->mc.ratio_all_one) { MIX_A2(true, false); }
+    else { MIX_A2(true, true); }
 #undef MIX_A2
 #undef MIX_A3
 #undef MIX_A
@@ -1473,22 +1823,32 @@ void mixed_sweep_a(MixedState* m, const SimConst& c, DevFP64& d, bool advance_wa
 
 template <bool WALLS>
 static void launch_b(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {
-    const int g = WALLS ? 1 : lanes_b(m), nb = blocks((long long)c.n * g, 128);
-    double4* vout = WALLS ? nullptr : d.vel[1 - d.vcur];
-#define MIX_B1(ST, RATIO, W, G)                                                                                  \
-    k_mix_b<ST, RATIO, W, G><<<nb, 128, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca, m->list,         \
-                                                m->cnt_short, m->cnt_all, d.vel[d.vcur], vout, d.force, d.scal, ahead)
-#define MIX_B(ST, RATIO)                               \
-    if (g == 1) MIX_B1(ST, RATIO, WALLS, 1);           \
-    else if (g == 4) MIX_B1(ST, RATIO, false, 4);      \
-    else MIX_B1(ST, RATIO, false, 8)
-    if (m->mc.has_st) {
-        if (m->mc.ratio_all_one) { MIX_B(true, false); } else { MIX_B(true, true); }
-    } else {
-        if (m->mc.ratio_all_one) { MIX_B(false, false); } else { MIX_B(false, true); }
+    const int g = WALLS ? 1 : lanes_b(m, c);
+    if (g > 1) {
+        const int gb = blocks((long long)m->n_fluid * g, 128), nw = gb + blocks(c.n - m->n_fluid, 128);
+#define MIX_BG(ST, RATIO, G)                                                                                        \
+    k_mix_b_g<ST, RATIO, G><<<nw, 128, 0, s>>>(m->mc, c, m->n_fluid, gb, m->phl, m->pv, m->gca, m->list,          \
+                                               m->cnt_short, m->cnt_all, d.vel[d.vcur], d.vel[1 - d.vcur], d.force, \
+                                               d.scal, ahead)
+#define MIX_BG2(ST, RATIO)               \
+    if (g == 4) MIX_BG(ST, RATIO, 4);    \
+    else MIX_BG(ST, RATIO, 8)
+        if (!m->mc.has_st) { MIX_BG2(false, false); }
+        else if (m->mc.ratio_all_one) { MIX_BG2(true, false); }
+        else { MIX_BG2(true, true); }
+#undef MIX_BG2
+#undef MIX_BG
+        return;
     }
+    const int nb = blocks(c.n, 128);
+    double4* vout = WALLS ? nullptr : d.vel[1 - d.vcur];
+#define MIX_B(ST, RATIO)                                                                                            \
+    k_mix_b<ST, RATIO, WALLS><<<nb, 128, 0, s>>>(m->mc, c, d.cellstart, m->phl, m->pv, m->gca, m->list,           \
+                                                 m->cnt_short, m->cnt_all, d.vel[d.vcur], vout, d.force, d.scal, ahead)
+    if (!m->mc.has_st) MIX_B(false, false);
+    else if (m->mc.ratio_all_one) MIX_B(true, false);
+    else MIX_B(true, true);
 #undef MIX_B
-#undef MIX_B1
 }
 
 static void launch_b_walk(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, bool ahead) {

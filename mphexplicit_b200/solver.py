@@ -313,7 +313,7 @@ class Solver:
                self._ctx)
 
     def set_sweep_layout(self, layout: str) -> None:
-        """FP64 pair sweeps: "auto" (by size), "thread" or "warp" per particle."""
+        """Pair sweeps: "auto" (by size), "thread" or "warp" (mixed: 8 lanes) per particle."""
         code = {"auto": 0, "thread": 1, "warp": 2}[layout]
         _check(self._lib.mph_set_sweep_layout(self._ctx, code), self._ctx)
 
