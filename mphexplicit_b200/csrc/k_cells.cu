@@ -189,7 +189,6 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
 // cannot pass that test and is skipped.  An axis with fewer than 4 cells
 // contributes nothing to the FP32 distance (its minimum image need not be the
 // neighbouring cell's), which only keeps more candidates.
-constexpr int kListWarps = 4;     // warps per block
 constexpr int kListParts = 8;     // particles per group
 constexpr int kListSorted = 128;  // home particles that are taken octant by octant (more: in slot order)
 
@@ -589,11 +588,7 @@ void launch_pos32(const SimConst& c, const double4* pos, float4* pos32, cudaStre
 void launch_neighbor_list(const SimConst& c, const double4* pos, const float4* pos32, const int* cellstart,
                           int* ncount, int* nlist, int cap, int* ncount_s, int* nlist_s, int cap_s,
                           StepScalars* scal, cudaStream_t s) {
-    // Warps per key: enough to fill the GPU in small scenes.  Measured in us per
-    // build at 1, 2, 4, 6 warps: 3-D, 20,116 particles 360 / 186 / 106 / 101; 213,868 474 /
-    // 333 / 311 / 327; 2,779,256 4403 / 4368 / 4607 / 4879 (each warp sorts its key's
-    // particles anew); 2-D (13 particles a key), 22,500 50 / 36 / 37 / 42; 90,000 84 / 85 / 103 / 122.
-    const int key_warps = c.dim == 2 ? (c.n <= 50000 ? 2 : 1) : (c.n <= 250000 ? 4 : 2);
+    const int key_warps = list_key_warps(c.dim, c.n, c.tot);
     const long long warps = 2LL * c.tot * key_warps;
     const Prefilter pf = make_prefilter(c);
     const int nb = (int)((warps + kListWarps - 1) / kListWarps);

@@ -299,19 +299,18 @@ __global__ void k_mix_home(SimConst c, MixConst m, const double4* __restrict__ p
 // long chain: us a build at 1,526,488 particles (3-D dam) 2447 -> 2049, 258,392 441 -> 347,
 // 21,924 324 -> 83, 592,704 (3-D column) 1111 -> 1076, 39,304 316 -> 115, in 2-D 90,000
 // 73 -> 62, 3,600 30 -> 14.
-constexpr int kMixListWarps = 4;
 constexpr int kMixListParts = 8;     // particles per group
 constexpr int kMixListSorted = 128;  // home particles that are taken octant by octant (more: in slot order)
 
-__global__ void __launch_bounds__(32 * kMixListWarps, 8)
+__global__ void __launch_bounds__(32 * kListWarps, 8)
 k_mix_list(SimConst c, MixConst m, const float4* __restrict__ p32, const int* __restrict__ cellstart,
            unsigned* __restrict__ list, int cap_l, int* __restrict__ cnt_short, int* __restrict__ cnt_all,
            StepScalars* __restrict__ scal, int key_warps) {
-    __shared__ float4 queue_[kMixListWarps][64];  // candidates near the box, in order (a ring)
-    __shared__ float4 home_[kMixListWarps][kMixListParts];
-    __shared__ unsigned char order_[kMixListWarps][kMixListSorted];
+    __shared__ float4 queue_[kListWarps][64];  // candidates near the box, in order (a ring)
+    __shared__ float4 home_[kListWarps][kMixListParts];
+    __shared__ unsigned char order_[kListWarps][kMixListSorted];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * kMixListWarps + wib;
+    const int gw = blockIdx.x * kListWarps + wib;
     const int key = gw / key_warps;  // key_warps warps share a key
     if (key >= 2 * c.tot) return;    // whole warp
     const int hb = cellstart[key], nh = cellstart[key + 1] - hb, first = (gw % key_warps) * kMixListParts;
@@ -1656,11 +1655,6 @@ __global__ void k_mix_counts(int n, const int* __restrict__ cnt_all, const int* 
 
 inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 
-// Warps per key of the table build: enough to fill the GPU in small scenes.  us a
-// build at 1, 2, 4 warps: 3-D, 21,924 particles 279 / - / 83; 258,392 429 / 347 / 335; 1,526,488
-// 2100 / 2049 / 2150; 592,704 1163 / 1076 / 1062; 2-D, 3,600 22 / 14 / 15; 90,000 62 / - / 86.
-int list_key_warps(const SimConst& c) { return c.dim == 2 ? (c.n <= 50000 ? 2 : 1) : (c.n <= 250000 ? 4 : 2); }
-
 }  // namespace
 
 struct MixedState {
@@ -1745,8 +1739,8 @@ int mixed_rebuild(MixedState* m, const SimConst& c, DevFP64& d, cudaStream_t s, 
     for (int attempt = 0; attempt < 3; ++attempt) {
         MTRY(cudaMemsetAsync(&d.scal->max_neighbors, 0, sizeof(int), s));
         MTRY(cudaMemsetAsync(&d.scal->max_short, 0, 2 * sizeof(int), s));
-        const int key_warps = list_key_warps(c);
-        k_mix_list<<<blocks(2LL * c.tot * key_warps, kMixListWarps), 32 * kMixListWarps, 0, s>>>(
+        const int key_warps = list_key_warps(c.dim, n, c.tot);
+        k_mix_list<<<blocks(2LL * c.tot * key_warps, kListWarps), 32 * kListWarps, 0, s>>>(
             c, m->mc, m->p32, d.cellstart, m->list, m->cap_l, m->cnt_short, m->cnt_all, d.scal, key_warps);
         ++nl;
         MTRY(cudaGetLastError());

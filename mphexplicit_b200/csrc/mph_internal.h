@@ -56,6 +56,24 @@ struct SimConst {
     double wall_rot[MPH_TYPE_COUNT][3][3];
 };
 
+// Warps that share a key (a cell's fluid, or its walls) in the list builds of the FP64
+// and the mixed form: enough to fill the GPU in small scenes.  us a build at 1, 2, 4 warps
+// (FP64): 3-D, 20,116 particles 360 / 186 / 106; 213,868 474 / 333 / 311; 2,779,256 4403 /
+// 4368 / 4607 (each warp sorts its key's particles anew); 2-D (13 particles a key), 22,500
+// 50 / 36 / 37; 90,000 84 / 85 / 103.  Mixed: 3-D, 21,924 279 / - / 83; 258,392 429 / 347 /
+// 335; 1,526,488 2100 / 2049 / 2150; 2-D, 3,600 22 / 14 / 15; 90,000 62 / - / 86.
+// A warp without particles costs 0.14 ns, so a mostly empty grid gets no more of them: 8,000
+// particles in 432,000 keys 354 / 198 / 248, in 2,000,000 382 / 562 / 1109; 2-D, 3,600 in 180,000
+// 43 / 60 / 109.  The kernels number the warps in 32 bits: at most 2^30 (make_simconst takes up
+// to 2^29 cells, two keys each).
+constexpr int kListWarps = 4;  // warps per block
+inline int list_key_warps(int dim, int n, int tot) {
+    const long long keys = 2LL * tot, most = dim == 2 ? 1 << 17 : 1 << 20;
+    int w = dim == 2 ? (n <= 50000 ? 2 : 1) : (n <= 250000 ? 4 : 2);
+    while (w > 1 && keys * w > most) w /= 2;
+    return w;
+}
+
 // Entry k of particle i's neighbour list: the tables hold rows of four entries,
 // [cap / 4][n][4].
 __host__ __device__ inline size_t list_at(int k, size_t n, int i) {
@@ -141,7 +159,7 @@ void launch_pos32(const SimConst& c, const double4* pos, float4* pos32, cudaStre
 // nlist_s != nullptr: also the short sublist (entries within rs2, in list
 // order; its longest length in scal->max_short).  pos32 (launch_pos32) feeds
 // the FP32 prefilter that skips candidates surely beyond the cut-off (the
-// list is the same).  One warp per cell key.
+// list is the same).
 void launch_neighbor_list(const SimConst& c, const double4* pos, const float4* pos32, const int* cellstart,
                           int* ncount, int* nlist, int cap, int* ncount_s, int* nlist_s, int cap_s,
                           StepScalars* scal, cudaStream_t s);
