@@ -1353,6 +1353,7 @@ struct mph_batch {
     int* d_sid = nullptr;
     int2* d_items_t = nullptr;         // table form: sweep A's blocks, then sweep B's
     char* slab = nullptr;              // the arrays of d, d_scenes and d_sid
+    int table_cta = 0;                 // block size its items are cut for
     bool table_ok = false;             // the table fits: allocated at creation
     bool sorted = false;               // the initial sort is done
     bool table_valid = false;          // the table holds the lists of the current sort
@@ -1532,7 +1533,8 @@ static void fill_bscene(BScene& s, const mph::SimConst& c, const mph_constants& 
 }
 
 // The table form (a tile of one cell): blocks of `threads` slots (sweep A) and
-// of `threads` fluid particles (sweep B), scene by scene.
+// of `threads` fluid particles (sweep B), scene by scene.  Here and in configure() the
+// batch changes only once nothing can fail any more: after an error it steps on as it was.
 static int configure_table(mph_batch* b, int threads, int ctas_per_sm) {
     const int cta = std::min(threads, 128);  // the kernels' bound; the asked-for size is reported back
     std::vector<int2> ia, ib;
@@ -1541,21 +1543,27 @@ static int configure_table(mph_batch* b, int threads, int ctas_per_sm) {
         for (int k = 0; k < sc.n; k += cta) ia.push_back(make_int2(s, sc.pbase + k));
         for (int k = 0; k < sc.nfl; k += cta) ib.push_back(make_int2(s, sc.fbase + k));
     }
+    int2* items = nullptr;
+    BTRY(b, balloc(&items, ia.size() + ib.size()));
+    cudaError_t e = cudaMemcpyAsync(items, ia.data(), ia.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(items + ia.size(), ib.data(), ib.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->d_scenes, b->hs.data(), b->hs.size() * sizeof(BScene), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);  // the vectors go out of scope
+    if (e != cudaSuccess) {
+        cudaFree(items);
+        return bfail(b, MPH_ERR_CUDA, std::string("table form: ") + cudaGetErrorString(e));
+    }
     if (b->d_items_t) cudaFree(b->d_items_t);
-    b->d_items_t = nullptr;
-    BTRY(b, balloc(&b->d_items_t, ia.size() + ib.size()));
-    BTRY(b, cudaMemcpyAsync(b->d_items_t, ia.data(), ia.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
-    BTRY(b, cudaMemcpyAsync(b->d_items_t + ia.size(), ib.data(), ib.size() * sizeof(int2), cudaMemcpyHostToDevice,
-                            b->stream));
-    BTRY(b, cudaMemcpyAsync(b->d_scenes, b->hs.data(), b->hs.size() * sizeof(BScene), cudaMemcpyHostToDevice,
-                            b->stream));
-    BTRY(b, cudaStreamSynchronize(b->stream));  // the vectors go out of scope
+    b->d_items_t = items;
     BatchDev& d = b->d;
     d.table = 1;
     d.items_a = b->d_items_t;
     d.items_b = b->d_items_t + ia.size();
     for (int k = 0; k < 3; ++k) b->tile[k] = 1;
     b->threads = threads;
+    b->table_cta = cta;
     b->occ = std::max(1, std::min(ctas_per_sm, 8));
     b->cap = d.tcap;
     b->n_items = b->grid_a = (int)ia.size();
@@ -1579,9 +1587,10 @@ static int configure(mph_batch* b, const int t[3], int threads, int ctas_per_sm 
         long long cost;
     };
     std::vector<Item> items;
+    std::vector<BScene> hs = b->hs;
     long long max_halo = 0;
     for (int s = 0; s < b->S; ++s) {
-        BScene& sc = b->hs[s];
+        BScene& sc = hs[s];
         for (int d = 0; d < 3; ++d) sc.tile[d] = 1;
         for (int d = 0; d < dim; ++d) sc.tile[d] = std::max(1, std::min(t[d], sc.cc[d] - 2));  // distinct halo cells
         for (int d = 0; d < 3; ++d) tmax[d] = std::max(tmax[d], sc.tile[d]);
@@ -1633,15 +1642,38 @@ static int configure(mph_batch* b, const int t[3], int threads, int ctas_per_sm 
     while (cap > 64 && std::max(mph::sweep_smem(dim, 0, b->has_st, cap, hmax, ncol),
                                 mph::sweep_smem(dim, 1, b->has_st, cap, hmax, ncol)) > budget)
         cap -= 32;
-    // free old items, upload new
-    if (b->d_items) cudaFree(b->d_items);
-    b->d_items = nullptr;
+    const size_t smem[2] = {mph::sweep_smem(dim, 0, b->has_st, cap, hmax, ncol),
+                            mph::sweep_smem(dim, 1, b->has_st, cap, hmax, ncol)};
+    int g[2];
+    for (int sw = 0; sw < 2; ++sw) {
+        mph::SweepFn f = dim == 2 ? mph::sweep_fn<2>(sw, b->has_st) : mph::sweep_fn<3>(sw, b->has_st);
+        cudaFuncAttributes fa{};
+        BTRY(b, cudaFuncGetAttributes(&fa, f));
+        if (smem[sw] + fa.sharedSizeBytes > (size_t)smem_optin)
+            return bfail(b, MPH_ERR_ARG, "sweep kernel does not fit on an SM with this tile");
+        // the limit belongs to the kernel: never below what another batch asked for
+        if ((int)smem[sw] > fa.maxDynamicSharedSizeBytes)
+            BTRY(b, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[sw]));
+        int per = 0;
+        BTRY(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, threads, smem[sw]));
+        if (per < 1) return bfail(b, MPH_ERR_ARG, "sweep kernel does not fit on an SM with this tile");
+        g[sw] = std::max(1, std::min(per * b->sms, (int)items.size()));
+    }
     std::vector<int4> hv(items.size());
     for (size_t k = 0; k < items.size(); ++k) hv[k] = items[k].v;
-    BTRY(b, balloc(&b->d_items, hv.size()));
-    BTRY(b, cudaMemcpyAsync(b->d_items, hv.data(), hv.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
-    BTRY(b, cudaMemcpyAsync(b->d_scenes, b->hs.data(), b->hs.size() * sizeof(BScene), cudaMemcpyHostToDevice,
-                            b->stream));
+    int4* d_items = nullptr;
+    BTRY(b, balloc(&d_items, hv.size()));
+    cudaError_t e = cudaMemcpyAsync(d_items, hv.data(), hv.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->d_scenes, hs.data(), hs.size() * sizeof(BScene), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);  // the vectors go out of scope
+    if (e != cudaSuccess) {
+        cudaFree(d_items);
+        return bfail(b, MPH_ERR_CUDA, std::string("tile items: ") + cudaGetErrorString(e));
+    }
+    if (b->d_items) cudaFree(b->d_items);
+    b->d_items = d_items;
+    b->hs = std::move(hs);
     for (int d = 0; d < 3; ++d) b->tile[d] = t[d];
     if (dim == 2) b->tile[2] = 1;
     b->threads = threads;
@@ -1649,19 +1681,9 @@ static int configure(mph_batch* b, const int t[3], int threads, int ctas_per_sm 
     b->cap = cap;
     b->hmax = hmax;
     b->ncol = ncol;
-    b->n_items = (int)items.size();
-    b->smem_a = mph::sweep_smem(dim, 0, b->has_st, cap, hmax, ncol);
-    b->smem_b = mph::sweep_smem(dim, 1, b->has_st, cap, hmax, ncol);
-    int g[2];
-    for (int sw = 0; sw < 2; ++sw) {
-        mph::SweepFn f = dim == 2 ? mph::sweep_fn<2>(sw, b->has_st) : mph::sweep_fn<3>(sw, b->has_st);
-        const size_t sm = sw == 0 ? b->smem_a : b->smem_b;
-        BTRY(b, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        int per = 0;
-        BTRY(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, threads, sm));
-        if (per < 1) return bfail(b, MPH_ERR_ARG, "sweep kernel does not fit on an SM with this tile");
-        g[sw] = std::max(1, std::min(per * b->sms, b->n_items));
-    }
+    b->n_items = (int)hv.size();
+    b->smem_a = smem[0];
+    b->smem_b = smem[1];
     b->grid_a = g[0];
     b->grid_b = g[1];
     BatchDev& d = b->d;
@@ -1755,7 +1777,7 @@ static void launch_sweep(mph_batch* b, int sw) {
     if (b->d.table) {
         const int nb = sw == 0 ? b->grid_a : b->grid_b;
         if (nb == 0) return;  // no fluid
-        const int cta = std::min(b->threads, 128);
+        const int cta = b->table_cta;
 #define TABLE_SWEEP(DIM, ST)                                                     \
     if (sw == 0) mph::k_bt_a<DIM, ST><<<nb, cta, 0, b->stream>>>(b->d);   \
     else mph::k_bt_b<DIM, ST><<<nb, cta, 0, b->stream>>>(b->d)
