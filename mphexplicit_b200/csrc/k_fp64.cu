@@ -240,6 +240,7 @@ k_move(SimConst c, const int* __restrict__ cellstart, double4* __restrict__ pos,
                 scal->max_shift2_bits = 0ull;
                 scal->blocks_done = 0u;
                 scal->steps_done += 1;
+                scal->move_flags = scal->flags;
                 if (__longlong_as_double((long long)bits) > c.shift_thr) scal->stop = 1;
             }
         }

@@ -714,13 +714,13 @@ static int read_scalars(mph_ctx* ctx) {
     return MPH_OK;
 }
 
-static int check_flags(mph_ctx* ctx) {
-    const int f = ctx->h_scal->flags;
+static int check_flags(mph_ctx* ctx, int f) {
     if (f & mph::DEVFLAG_NONFINITE) return fail(ctx, MPH_ERR_NONFINITE, "non-finite velocity produced by a step");
     if (f & mph::DEVFLAG_NEIGHBOR_OVERFLOW) return fail(ctx, MPH_ERR_CAPACITY, "neighbour table overflow");
     if (f) return fail(ctx, MPH_ERR_DEVICE, "device error flag " + std::to_string(f));
     return MPH_OK;
 }
+static int check_flags(mph_ctx* ctx) { return check_flags(ctx, ctx->h_scal->flags); }
 
 // One FP64 step up to the pair sweeps: convection, wall motion, periodic wrap
 // and the displacement test, then the list rebuild when it fires
@@ -818,8 +818,10 @@ static int queue_counters(mph_ctx* ctx, int slot) {
 }
 
 // Takes in the counters of a batch of `launched` steps: those that completed (with
-// *stopped, one more has moved and waits for its rebuild).
-static int take_counters(mph_ctx* ctx, int slot, int launched, int* completed, bool* stopped) {
+// *stopped, one more has moved and waits for its rebuild).  An error of the device is
+// returned with the steps accounted for all the same.  at_move (one step): the error flags as the
+// step's move found them, and after an error the step has only moved.
+static int take_counters(mph_ctx* ctx, int slot, int launched, int* completed, bool* stopped, bool at_move = false) {
     Ahead& A = ctx->ahead;
     CUDA_TRY(ctx, cudaEventSynchronize(A.ev[slot]));
     const StepScalars& h = A.seen[slot];
@@ -833,9 +835,13 @@ static int take_counters(mph_ctx* ctx, int slot, int launched, int* completed, b
         std::memcpy(&A.shift2, &h.last_shift2_bits, sizeof(double));
     }
     if (moved > launched) return fail(ctx, MPH_ERR_DEVICE, "steps launched ahead: the counters disagree");
+    if (at_move && h.move_flags) {
+        *completed = 0;
+        return check_flags(ctx, h.move_flags);
+    }
     for (int k = 0; k < *completed; ++k) ctx->time += ctx->p.dt;  // main.cpp:449, one step at a time
     ctx->step += *completed;
-    return check_flags(ctx);
+    return at_move ? MPH_OK : check_flags(ctx);
 }
 
 // The step that stopped: rebuild, then its sweeps (main.cpp:399-431).
@@ -887,23 +893,20 @@ static int step_ahead(mph_ctx* ctx, int nsteps) {
             return queue_counters(ctx, s);
         };
         TRY(launch_batch(0));
+        int rc = MPH_OK;
         while (flight > 0) {
-            if (!stopped && queued < left) TRY(launch_batch(1 - slot));
+            if (!stopped && rc == MPH_OK && queued < left) TRY(launch_batch(1 - slot));
             int completed = 0;
             bool s = false;
-            const int rc = take_counters(ctx, slot, size[slot], &completed, &s);
+            const int r = take_counters(ctx, slot, size[slot], &completed, &s);
+            if (rc == MPH_OK) rc = r;  // a batch in flight behind an error has run too: count it
             --flight;
             done += completed;
             stopped |= s;
             slot = 1 - slot;
-            if (rc != MPH_OK) {
-                d.vcur = (v0 + done) & 1;
-                if (flight > 0 && cudaEventSynchronize(ctx->ahead.ev[slot]) == cudaSuccess)
-                    ctx->ahead.counted = ctx->ahead.seen[slot].steps_done;
-                return rc;
-            }
         }
         d.vcur = (v0 + done) & 1;
+        if (rc != MPH_OK) return rc;
         left -= done;
         if (stopped) {
             TRY(finish_stopped(ctx));
@@ -1372,9 +1375,10 @@ static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
         d.vcur = 1 - d.vcur;
         TRY(queue_counters(ctx, 0));
         TRY(copies());
+        // as on the host path, an error of this step's own sweeps is the next call's
         int completed = 0;
         bool stopped = false;
-        const int rc = take_counters(ctx, 0, 1, &completed, &stopped);
+        const int rc = take_counters(ctx, 0, 1, &completed, &stopped, true);
         if (stopped || rc != MPH_OK) {
             CUDA_TRY(ctx, cudaStreamSynchronize(R.copy));
             d.vcur = 1 - d.vcur;

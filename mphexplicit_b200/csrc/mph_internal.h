@@ -90,7 +90,8 @@ struct StepScalars {
     int stop;                            // steps launched ahead: a step asked for a rebuild, the later ones do nothing
     int steps_done;                      // steps launched ahead: steps moved so far
     unsigned blocks_done;                // steps launched ahead: move blocks finished in this launch
-    int pad[5];
+    int move_flags;                      // steps launched ahead: `flags` at the last moved step's end of the move
+    int pad[4];
 };
 
 enum : int {
