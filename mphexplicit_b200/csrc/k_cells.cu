@@ -468,17 +468,7 @@ __global__ void k_unpack3(int n, const double* __restrict__ src, double4* __rest
 
 inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 
-__global__ void k_pack3_lines(int n, const double4* __restrict__ src, double* __restrict__ dst) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * n) return;
-    dst[t] = reinterpret_cast<const double*>(src + t / 3)[t % 3];
-}
-
 }  // namespace
-
-void launch_pack3_lines(int n, const double4* src, double* dst, cudaStream_t s) {
-    k_pack3_lines<<<blocks(3LL * n, 256), 256, 0, s>>>(n, src, dst);
-}
 
 void launch_cell_index(const SimConst& c, const double4* pos, const int* type, int* keys, int* vals,
                        cudaStream_t s) {

@@ -809,11 +809,11 @@ static void launch_step_ahead(mph_ctx* ctx, double* vel_host = nullptr) {
     d.vcur = 1 - d.vcur;
 }
 
-static int queue_counters(mph_ctx* ctx, int slot) {
+static int queue_counters(mph_ctx* ctx, int slot, cudaStream_t st) {
     Ahead& A = ctx->ahead;
     CUDA_TRY(ctx, cudaGetLastError());
-    CUDA_TRY(ctx, cudaMemcpyAsync(&A.seen[slot], ctx->d.scal, sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(ctx, cudaEventRecord(A.ev[slot], ctx->stream));
+    CUDA_TRY(ctx, cudaMemcpyAsync(&A.seen[slot], ctx->d.scal, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(ctx, cudaEventRecord(A.ev[slot], st));
     return MPH_OK;
 }
 
@@ -890,7 +890,7 @@ static int step_ahead(mph_ctx* ctx, int nsteps) {
             for (int k = 0; k < size[s]; ++k) launch_step_ahead(ctx);
             queued += size[s];
             ++flight;
-            return queue_counters(ctx, s);
+            return queue_counters(ctx, s, ctx->stream);
         };
         TRY(launch_batch(0));
         int rc = MPH_OK;
@@ -1306,17 +1306,17 @@ static double* mapped_host(double* p, size_t count) {
 }
 
 // The FP64 form's last step with its read-back overlapped.  The step is launched
-// ahead of its rebuild test, whose answer the host reads with the state: the rare
-// step that has to rebuild does so then and copies again.  The positions are
-// final once the move and any rebuild are done: they are packed and copied on a
-// copy stream while the sweeps run.  The velocities: with a pinned, mapped host
-// buffer the force sweep stores each particle's new velocity into it as well as
-// into device memory (24 B per particle over PCIe while the sweep runs, 20 GB/s),
-// or, where the sweep is too short to hide that, a kernel behind it writes whole
-// lines (50 GB/s); otherwise they are packed and copied after the sweep.  Same
+// ahead of its rebuild test, whose answer comes through a copy stream while the sweeps
+// run; the rare step that has to rebuild does so then.  The positions are final after
+// that: they are packed and copied, once, on the copy stream behind the sweeps' launches.  The
+// velocities: with a pinned, mapped host buffer the force sweep stores each particle's new
+// velocity into it as well as into device memory (24 B per particle over PCIe while
+// the sweep runs); otherwise they are packed and copied after the sweep.  Same
 // kernels and inputs: the bits of mph_step + mph_get_state.
-constexpr int kPackHostMax = 100000;  // particles up to which the line writer is faster
-
+// us per step with the state into pinned buffers, against kernels behind the move and the sweep
+// that write both to the mapped buffers in whole lines, launched before the test's answer
+// and again after a rebuild: 4,860 particles 52 and 56, 17,388 67 and 71, 51,064 95 and 132,
+// 258,392 345 and 504; two-fluid column of 64,000 294 and 353; 2-D droplet of 25,600 72 and 108.
 static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
     TRY(readback_init(ctx));
     TRY(ahead_init(ctx));
@@ -1324,27 +1324,16 @@ static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
     mph::DevFP64& d = ctx->d;
     cudaStream_t st = ctx->stream;
     const size_t n = (size_t)ctx->n;
-    const bool lines = ctx->n <= kPackHostMax;
     double* vh = mapped_host(vel, 3 * n);
-    double* xh = lines ? mapped_host(xyz, 3 * n) : nullptr;
-    double* in_sweep = lines ? nullptr : vh;
     // after the launches of a step (vcur has flipped): the copies
     auto copies = [&]() {
-        if (vel && vh && lines) {
-            mph::launch_pack3_lines(ctx->n, d.vel[d.vcur], vh, st);
-            ++ctx->launches;
-        }
         CUDA_TRY(ctx, cudaEventRecord(R.ev[1], st));  // velocities final
         // enqueued after the compute so pageable buffers do not hold it back
         if (xyz) {
             CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[0], 0));
+            mph::launch_pack3(ctx->n, d.pos[d.cur], d.staging, R.copy);
             ++ctx->launches;
-            if (xh) {
-                mph::launch_pack3_lines(ctx->n, d.pos[d.cur], xh, R.copy);
-            } else {
-                mph::launch_pack3(ctx->n, d.pos[d.cur], d.staging, R.copy);
-                CUDA_TRY(ctx, cudaMemcpyAsync(xyz, d.staging, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
-            }
+            CUDA_TRY(ctx, cudaMemcpyAsync(xyz, d.staging, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, R.copy));
         }
         if (vel && !vh) {
             CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[1], 0));
@@ -1358,9 +1347,8 @@ static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
         TRY(step_fp64_head(ctx));
         CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));  // positions final
         sweep_a(ctx, true);
-        sweep_b_part1(ctx, in_sweep, false);
+        sweep_b_part1(ctx, vh, false);
         d.vcur = 1 - d.vcur;
-        TRY(copies());
         ctx->time += ctx->p.dt;  // main.cpp:449
         ++ctx->step;
     } else {
@@ -1371,23 +1359,22 @@ static int step_fp64_read(mph_ctx* ctx, double* xyz, double* vel) {
         }
         CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));  // positions final unless a rebuild follows
         sweep_a(ctx, true, true);
-        sweep_b_part1(ctx, in_sweep, true);
+        sweep_b_part1(ctx, vh, true);
         d.vcur = 1 - d.vcur;
-        TRY(queue_counters(ctx, 0));
-        TRY(copies());
+        CUDA_TRY(ctx, cudaStreamWaitEvent(R.copy, R.ev[0], 0));
+        TRY(queue_counters(ctx, 0, R.copy));
         // as on the host path, an error of this step's own sweeps is the next call's
         int completed = 0;
         bool stopped = false;
         const int rc = take_counters(ctx, 0, 1, &completed, &stopped, true);
         if (stopped || rc != MPH_OK) {
-            CUDA_TRY(ctx, cudaStreamSynchronize(R.copy));
             d.vcur = 1 - d.vcur;
             if (rc != MPH_OK) return rc;
-            TRY(finish_stopped(ctx, in_sweep));
+            TRY(finish_stopped(ctx, vh));
             CUDA_TRY(ctx, cudaEventRecord(R.ev[0], st));
-            TRY(copies());
         }
     }
+    TRY(copies());
     CUDA_TRY(ctx, cudaGetLastError());
     ctx->virial_valid = false;
     CUDA_TRY(ctx, cudaStreamSynchronize(R.copy));

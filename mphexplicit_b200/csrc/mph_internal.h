@@ -166,9 +166,6 @@ void launch_neighbor_list(const SimConst& c, const double4* pos, const float4* p
                           StepScalars* scal, cudaStream_t s);
 void launch_pack3(int n, const double4* src, double* dst, cudaStream_t s);
 
-// the first three components, packed in `dst` by consecutive threads writing
-// consecutive doubles (whole lines over PCIe when dst is mapped host memory)
-void launch_pack3_lines(int n, const double4* src, double* dst, cudaStream_t s);
 // the move of a step launched ahead of the host (k_fp64.cu): as launch_move, and
 // its last block makes the rebuild test of main.cpp:1102 (when it fires, scal->stop
 // makes this step's sweeps and every later step's kernels do nothing), counts the
