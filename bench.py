@@ -625,6 +625,10 @@ def bench_config(workload: str, mode: str) -> dict:
             "l2": "inputs larger than L2 (particle state and neighbour lists, several GB)"}
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's own program is not built on this machine."""
+
+
 def cpu_reference_sample(args, threads: int, steps: int, warmup: int, budget: float, rebuild_at: int):
     """The reference's own step (oracle/_ref/ref_mph3d, OpenMP) on the bench
     scene, written by oracle/ref_inputs (nothing of the product is loaded):
@@ -633,11 +637,12 @@ def cpu_reference_sample(args, threads: int, steps: int, warmup: int, budget: fl
     the cell and neighbour lists (the developed flow rebuilds about every 20
     steps; a dam break at rest does not for its first few hundred)."""
     from oracle import ref_inputs as RI
+    if not RI.ref_available(3):
+        raise ReferenceMissing("oracle/_ref/ref_mph3d is missing: build it with "
+                               "`make -C oracle ref REF=<reference>`")
     fluid, box = SCENES[args.scene]
     with tempfile.TemporaryDirectory() as td:
         d, g, n, nf = RI.dam_break_files(td, seed=0, fluid=fluid, box=box)
-        if not RI.ref_available(3):
-            raise SystemExit("oracle/_ref/ref_mph3d is missing: build it with `make -C oracle ref REF=<reference>`")
         r = RI.time_reference(d, g, 3, warmup, steps, threads, max_seconds=budget, timeout=3600,
                               rebuild_at=rebuild_at)
     r["workload"] = workload_name(fluid, box, 3, 0.005, n, nf)
@@ -655,16 +660,33 @@ def cpu_baseline_entry(r, cores) -> dict:
                          r["threads"])}
 
 
+def cpu_baseline_sample(args):
+    """The product line's cpu_baseline: the steps that fit in --ref-seconds, the first
+    of them a neighbour rebuild; null where the reference is not built."""
+    from oracle import ref_inputs as RI
+    cores = RI.host_cores()
+    try:
+        return cpu_baseline_entry(cpu_reference_sample(args, cores["logical"], 1000, 1, args.ref_seconds, 0), cores)
+    except ReferenceMissing as e:
+        print("no cpu_baseline: %s" % e, file=sys.stderr, flush=True)
+        return None
+
+
 def run_reference_arm(args, rank, world):
     """`--impl reference`: the reference's own CPU step on this line's workload,
     all host threads, exactly --steps timed steps after --warmup untimed ones,
     with one neighbour rebuild inside the window; then one step on one thread.
-    Rank 0 alone runs it (the other ranks exit without work)."""
+    Rank 0 alone runs it (the other ranks exit without work).  Where the reference is not
+    built, the line says so."""
     if rank != 0:
         return
     from oracle import ref_inputs as RI
     cores = RI.host_cores()
-    r = cpu_reference_sample(args, cores["logical"], args.steps, args.warmup, 1.0e30, args.steps // 2)
+    try:
+        r = cpu_reference_sample(args, cores["logical"], args.steps, args.warmup, 1.0e30, args.steps // 2)
+    except ReferenceMissing as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     base = cpu_baseline_entry(r, cores)
     if args.ref_single_steps > 0:
         r1 = cpu_reference_sample(args, 1, args.ref_single_steps, 0, 1.0e30, -1)
@@ -883,10 +905,7 @@ def main():
 
     base = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        from oracle import ref_inputs as RI
-        cores = RI.host_cores()
-        # bounded sample: the steps that fit in --ref-seconds, the first of them a neighbour rebuild
-        base = cpu_baseline_entry(cpu_reference_sample(args, cores["logical"], 1000, 1, args.ref_seconds, 0), cores)
+        base = cpu_baseline_sample(args)
 
     if rank == 0:
         n_all = sc.n
