@@ -411,11 +411,11 @@ k_sweep_b(SimConst c, const int* __restrict__ cellstart, const double2* __restri
           const double4* __restrict__ gcpa, const int* __restrict__ ncount, const int* __restrict__ nlist,
           const int* __restrict__ ncount_s, const int* __restrict__ nlist_s, double4* __restrict__ force,
           StepScalars* __restrict__ scal, const int* __restrict__ eoff, const float4* __restrict__ eforce,
-          float4* __restrict__ lsum, int part, int i0, int i1, double* __restrict__ vel_host,
+          float4* __restrict__ lsum, int part, double* __restrict__ vel_host,
           const StepScalars* __restrict__ skip) {
     if (skip && skip->stop) return;
-    const int i = i0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);  // particles [i0, i1)
-    if (i >= i1) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
     const int nf = cellstart[c.tot];
     const XV pi = ld_xv(xv, i);
     // part 1: fluid only; a wall keeps its velocity (what the full sweep
@@ -1416,15 +1416,13 @@ void launch_density_a(const SimConst& c, const double4* pos, const int* ncount, 
 void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, const int* type, double4* vel_out,
                     const double4* press, const double4* gc, const int* ncount, const int* nlist,
                     const int* ncount_s, const int* nlist_s, double4* force, StepScalars* scal, cudaStream_t s,
-                    const int* eoff, const float4* eforce, float4* lsum, int part, int i0, int i1,
+                    const int* eoff, const float4* eforce, float4* lsum, int part,
                     double* vel_host, const StepScalars* skip) {
-    if (i1 < 0) i1 = c.n;
-    if (i1 <= i0) return;
     // the ratios weigh surface-tension terms alone
     const bool ratio = c.has_st && !c.ratio_all_one;
     // the particles whose pairs this launch evaluates
     const int b0 = part == 2 ? c.nf : 0, b1 = part == 1 ? c.nf : c.n;
-    const int g = !eforce && i0 == 0 && i1 == c.n ? group_lanes(c, b1 - b0, c.dim == 3) : 1;
+    const int g = !eforce ? group_lanes(c, b1 - b0, c.dim == 3) : 1;
     if (g > 1) {
         const int gb = blocks(b1 - b0, kGroupWarps * (32 / g));
         const int nw = gb + (part == 1 ? blocks(c.n - c.nf, 32 * kGroupWarps) : 0);
@@ -1447,11 +1445,11 @@ void launch_sweep_b(const SimConst& c, const int* cellstart, const double2* xv, 
 #undef SWEEP_BG
         return;
     }
-    const int nb = blocks(i1 - i0, 128);
+    const int nb = blocks(c.n, 128);
 #define SWEEP_B(ST, RATIO, LRN, MU1)                                                                             \
     k_sweep_b<ST, RATIO, LRN, MU1><<<nb, 128, 0, s>>>(c, cellstart, xv, type, press, vel_out, gc, ncount, nlist, \
                                                       ncount_s, nlist_s, force, scal, eoff, eforce, lsum, part,  \
-                                                      i0, i1, vel_host, skip)
+                                                      vel_host, skip)
     if (eforce) SWEEP_B(false, false, true, true);
     else if (!c.has_st) { if (c.mu_uniform) SWEEP_B(false, false, false, true); else SWEEP_B(false, false, false, false); }
     else if (ratio) SWEEP_B(true, true, false, false);

@@ -754,8 +754,8 @@ static void sweep_b_part1(mph_ctx* ctx, double* vel_host, bool skip) {
     mph::DevFP64& d = ctx->d;
     Launch L(ctx, "sweep_b");
     mph::launch_sweep_b(ctx->sc, d.cellstart, d.xv, d.type[d.cur], d.vel[1 - d.vcur], d.press, d.gc, d.ncount, d.nlist,
-                        d.ncount_s, d.nlist_s, d.force, d.scal, ctx->stream, nullptr, nullptr, nullptr, 1, 0, -1,
-                        vel_host, skip ? d.scal : nullptr);
+                        d.ncount_s, d.nlist_s, d.force, d.scal, ctx->stream, nullptr, nullptr, nullptr, 1, vel_host,
+                        skip ? d.scal : nullptr);
     ctx->wall_force_valid = false;  // computed when read
 }
 
@@ -791,7 +791,7 @@ static void mixed_sweeps(mph_ctx* ctx, bool ahead) {
 }
 
 // The three kernels of one step, to run only if no earlier step stopped.
-static void launch_step_ahead(mph_ctx* ctx, double* vel_host = nullptr) {
+static void launch_step_ahead(mph_ctx* ctx) {
     mph::DevFP64& d = ctx->d;
     if (ctx->mixed) {
         mixed_move(ctx, true);
@@ -805,7 +805,7 @@ static void launch_step_ahead(mph_ctx* ctx, double* vel_host = nullptr) {
                                ctx->stream);
     }
     sweep_a(ctx, true, true);
-    sweep_b_part1(ctx, vel_host, true);
+    sweep_b_part1(ctx, nullptr, true);
     d.vcur = 1 - d.vcur;
 }
 
