@@ -165,7 +165,8 @@ __global__ void k_reorder(int n, const int* __restrict__ vals, const int* __rest
 //
 // What bounds it: the instruction count.  A particle's list costs about 1150
 // warp instructions (its share of queueing 600 candidates for eight particles, then
-// 20 to test 32 candidates against one), issued at 65 % of the peak.  With a lane per particle, 32 candidates tested one after
+// 20 to test 32 candidates against one), issued at 80 % of the peak (2,779,256 particles;
+// 78 % at 258,392).  With a lane per particle, 32 candidates tested one after
 // the other into a bit mask and the hits pushed one by one, half of the lanes idled
 // in the pushes and in part-filled warps, and a small scene's few warps ran one long
 // serial chain: 8.03 -> 4.37 ms a build at 2,779,256 particles (3-D dam), 436 -> 311 us

@@ -2,7 +2,8 @@
 // reference's x86-64 build.
 //
 // The reference runs eight neighbour sweeps per step (main.cpp:1665-1985).
-// Here they are two, one thread per particle, list order kept:
+// Here they are two, a thread per particle or, in small scenes, several lanes,
+// list order kept:
 //   sweep A = DensityA + GravityCenter + DensityP + DivergenceP
 //             (four independent sums over the same list) and, in the epilogue,
 //             PhysicalCoefficients + PressureP value + PressureA value;
@@ -18,8 +19,9 @@
 
 // Resident 128-thread blocks per SM the sweeps are compiled for (register cap
 // 65536 / (128 * blocks)); latency hiding vs. spills, set by measurement.  The
-// FP64 pipe bounds the sweeps (71 % active in the force sweep, with the L1 data
-// pipe at 69 %): about 84 FP64 operations per list entry.  On the 2,779,256-particle
+// FP64 pipe and the L1 data pipe bound the sweeps (76 and 77 % active in the force sweep of
+// the 2,779,256-particle dam break, 64 and 56 at 258,392): about 84 FP64 operations and
+// one 48-byte gather per list entry.  On the 2,779,256-particle
 // dam break the force sweep takes 2.34 ms at 6 blocks (80 registers, two spilled
 // values), 2.42 at 5; sweep A 0.314 ms at 7, 0.332 at 6, 0.366 at 8.  Blocks of 64 or
 // 256 threads give the same times, of 32 up to 13 % more.
@@ -53,10 +55,10 @@ __device__ __forceinline__ double omod_fast(double x, double w) {
 
 // The record the pair sweeps gather per neighbour: position and velocity, 48
 // bytes as three 16-byte words {x, y}, {z, vx}, {vy, vz}, written by the move
-// (k_move) and by the reorder.  The sweeps are bound by the L1 data pipe: a
-// warp's gather of one neighbour per lane costs it 50-57 cycles as two 32-byte
-// double4 (four 16-byte loads), 37 as two 32-byte loads and 27-32 as this record
-// (measured with 40 to 1000 records in reach of a warp).  Force sweep 299 -> 255
+// (k_move) and by the reorder.  The gathers are the L1 data pipe's work, which bounded
+// the sweeps before: a warp's gather of one neighbour per lane costs it 50-57 cycles as
+// two 32-byte double4 (four 16-byte loads), 37 as two 32-byte loads and 27-32 as this
+// record (measured with 40 to 1000 records in reach of a warp).  Force sweep 299 -> 255
 // us on the 258,392-particle dam break and 3.08 -> 2.90 ms on the 2,779,256 one,
 // sweep A 49 -> 43 us and 0.39 -> 0.36 ms, the move, which writes the records,
 // 13 -> 16 us and 0.058 -> 0.082 ms.

@@ -1149,7 +1149,7 @@ __device__ __forceinline__ void force_finish(const SimConst& c, int i, int ti, d
 // plain FP32 sum.  Then gravity and the FP64 velocity update
 // (main.cpp:1908-2010).
 //
-// What bounds it: the L1 data pipe (94 % of its cycles without surface tension), which
+// What bounds it: the L1 data pipe (90 % of its cycles without surface tension), which
 // spends 17.6 of them on a warp's gather, one for each 128-byte line that holds
 // some of its 32 records.  With the offset's one word (cell_steps) a launch takes 656 us
 // instead of 696 at 1,024,000 fluid particles.  A thread per two neighbouring particles
