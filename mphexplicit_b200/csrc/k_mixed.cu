@@ -727,14 +727,14 @@ struct DensitySums {
 };
 
 // A pair of the short part: its displacement d (FP32) and squared distance r2, and, where it is within
-// RadiusP (the return value), its terms.  FP32: the exact displacement from the hi and lo parts.
-// S64: pair arithmetic in FP64.
-template <bool S64>
-__device__ __forceinline__ bool density_pair(const MixConst& m, const SimConst& c, const float4& pi, const float4& li,
-                                             const float4& vi, const float4& pj, const float4& lj, const float4& vj,
-                                             const float4& dh, const float4& dl, float* d, float& r2,
-                                             DensityTermsOf<S64>& t) {
-    bool in;
+// RadiusP, its terms to put(terms).  FP32: the exact displacement from the hi and lo parts.
+// S64: pair arithmetic in FP64.  velocity(): the neighbour's.
+template <bool S64, class Velocity, class Put>
+__device__ __forceinline__ void density_pair(const MixConst& m, const SimConst& c, const float4& pi, const float4& li,
+                                             const float4& vi, const float4& pj, const float4& lj,
+                                             Velocity&& velocity, const float4& dh, const float4& dl, float* d,
+                                             float& r2, Put&& put) {
+    DensityTermsOf<S64> t;
     if constexpr (S64) {
         // FP64 displacement: the hi difference plus the cell offset is exact in
         // FP32 (grid multiples), the lo parts carry the rest to ~1e-14 l0
@@ -742,16 +742,17 @@ __device__ __forceinline__ bool density_pair(const MixConst& m, const SimConst& 
         const double dyd = (double)((pj.y - pi.y) + dh.y) + (((double)lj.y - (double)li.y) + (double)dl.y);
         const double dzd = (double)((pj.z - pi.z) + dh.z) + (((double)lj.z - (double)li.z) + (double)dl.z);
         const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
-        in = r2d <= c.rp2;
-        if (in) {
+        if (r2d <= c.rp2) {
             const double y = rsqrt_dnr(r2d);
             const double q = 1.0 - r2d * y * m.inv_rp_d;
             t.wa = m.cp_d * q;
             t.wb = q;
             const double dw = m.cp_m2_d * q;
+            const float4 vj = velocity();
             t.da = (((double)vj.x - (double)vi.x) * dxd + ((double)vj.y - (double)vi.y) * dyd +
                     ((double)vj.z - (double)vi.z) * dzd) * y;
             t.db = dw;
+            put(t);
         }
         d[0] = (float)dxd;
         d[1] = (float)dyd;
@@ -762,18 +763,18 @@ __device__ __forceinline__ bool density_pair(const MixConst& m, const SimConst& 
         d[1] = ((pj.y - pi.y) + dh.y) + ((lj.y - li.y) + dl.y);
         d[2] = ((pj.z - pi.z) + dh.z) + ((lj.z - li.z) + dl.z);
         r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-        in = r2 <= m.rp2;
-        if (in) {
+        if (r2 <= m.rp2) {
             wp_square(m, (pj.x - pi.x) + dh.x, (pj.y - pi.y) + dh.y, (pj.z - pi.z) + dh.z, (lj.x - li.x) + dl.x,
                       (lj.y - li.y) + dl.y, (lj.z - li.z) + dl.z, t.p2, t.p2e);  // wp
             const float rinv = rsqrt_nr(r2);
             const float r = r2 * rinv;
             const float q = 1.0f - r * m.inv_rp;
             t.dw = m.cp_m2 * q;  // dwpdr
+            const float4 vj = velocity();
             t.ue = ((vj.x - vi.x) * d[0] + (vj.y - vi.y) * d[1] + (vj.z - vi.z) * d[2]) * rinv;
+            put(t);
         }
     }
-    return in;
 }
 
 // Epilogue of sweep A: coefficients, PressureP, PressureA (main.cpp:1631-1662, 1735-1740, 1904-1906).
@@ -844,8 +845,8 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
         float4 pj, lj;
         ldg_pv(phl, j, pj, lj);  // {hi, lo} in one 256-bit load
         float d[3], r2;
-        DensityTermsOf<S64> t;
-        if (density_pair<S64>(m, c, pi, li, vi, pj, lj, v32[j], tb.dhi[code], tb.dlo[code], d, r2, t)) {
+        density_pair<S64>(m, c, pi, li, vi, pj, lj, [&] { return v32[j]; }, tb.dhi[code], tb.dlo[code], d, r2,
+                          [&](const DensityTermsOf<S64>& t) {
             if constexpr (S64) {
                 q.add_p64(t.wa, t.wb);
                 q.add_d64(t.da, t.db);
@@ -853,7 +854,7 @@ k_mix_a(MixConst m, const float4* __restrict__ phl, const float4* __restrict__ p
                 q.add_p(m, t.p2, t.p2e);
                 q.add_d(t.ue, t.dw);
             }
-        }
+        });
         if (ST) {
             const float rinv = rsqrt_nr(r2);
             st_density<RATIO>(m, ti, __float_as_int(pj.w), r2, r2 * rinv, d[0], d[1], d[2], sa, cak, g0, g1, g2);
@@ -989,8 +990,13 @@ k_mix_a_g(MixConst m, const float4* __restrict__ phl, const float4* __restrict__
         [&](const Rec& rj, bool have) {
             float d[3] = {0.f, 0.f, 0.f}, r2 = 0.f;
             DensityTermsOf<S64> t{};
-            const bool in = have && density_pair<S64>(m, c, pi, li, vi, rj.p, rj.l, rj.v, tb.dhi[rj.code],
-                                                      tb.dlo[rj.code], d, r2, t);
+            bool in = false;
+            if (have)
+                density_pair<S64>(m, c, pi, li, vi, rj.p, rj.l, [&] { return rj.v; }, tb.dhi[rj.code],
+                                  tb.dlo[rj.code], d, r2, [&](const DensityTermsOf<S64>& terms) {
+                    t = terms;
+                    in = true;
+                });
             if constexpr (S64) {
                 *reinterpret_cast<double2*>(&st[0].v[mine]) = make_double2(t.wa, t.wb);
                 *reinterpret_cast<double2*>(&st[1].v[mine]) = make_double2(t.da, t.db);
